@@ -267,6 +267,29 @@ int strata_adaln_cond_bf16(const void* tokens, int B, int D, int h, int w, int C
  * 0 when the geometry has no such form. With table_ws NULL every pixel is evaluated tap by tap. */
 int64_t strata_adaln_cond_table_floats(int Cb, int factor, int ks);
 
+/* That table alone, for weights that serve many calls (strata_network_forward_f32 takes it ready). */
+int strata_adaln_cond_table_f32(const float* w_dw, int Cb, int factor, int ks, float* table,
+                                void* stream);
+
+/* Rotary modes of strata_tile_tables and strata_network_forward_f32. */
+#define STRATA_ROPE_NONE 0
+#define STRATA_ROPE_AXIAL 1         /* row / column of the token */
+#define STRATA_ROPE_STEREOGRAPHIC 2 /* stereographic coordinates about the tile's spherical centroid */
+
+/* Per-tile geometry from the pixels' latitudes and longitudes [B, H, W] (radians): the tile centre
+ * (lat0, lon0 [B]: mean latitude, circular mean longitude in [0, 2 pi); both NULL to skip) and the
+ * packed rotary table rope_cs [B, (H/patch)*(W/patch), head_dim/2] of strata_qkv_rope_bf16 (unused
+ * for STRATA_ROPE_NONE). Stereographic coordinates are the mean over a token's patch x patch
+ * pixels in units of length_scale. Evaluated in double precision, rounded once.
+ * workspace: strata_tile_tables_workspace_bytes(B, H, W) bytes (may be 0), 8-byte aligned.
+ * Replaces TileGeometry.tile_center (screamcast/tile_geometry.py:33-61) and the RoPE table helpers
+ * the reference imports (screamcast/strata_wrappers.py:50-52, 636-642). */
+int64_t strata_tile_tables_workspace_bytes(int B, int H, int W);
+int strata_tile_tables(const float* lat, const float* lon, int B, int H, int W, float* lat0,
+                       float* lon0, int rope_mode, int patch, double length_scale, double rope_base,
+                       int head_dim, void* rope_cs, void* workspace, int64_t workspace_bytes,
+                       void* stream);
+
 /* Operand rows of the de-aliased patch embedding (screamcast/dealias.py:28-143,
  * DealiasedPatchEmbed3D): x_rows = pixel rows [B, D, H, W, ldx] bf16, channels last (what
  * strata_preprocess_patches_bf16 writes at patch 1x1x1); a[token, (c, v, y, x)] = the low-pass
@@ -276,6 +299,67 @@ int64_t strata_adaln_cond_table_floats(int Cb, int factor, int ks);
 int strata_dealias_patches_bf16(const void* x_rows, int64_t ldx, int B, int C, int D, int H, int W,
                                 int pv, int ph, int pw, const float* taps, int n_taps, void* a,
                                 int64_t lda, void* stream);
+
+/* ---- whole networks ----------------------------------------------------------------------- */
+/* Single-stage backbone (screamcast/strata_wrappers.py:252-415). Pointers named h_* are HOST
+ * arrays read during the call; the weights are DEVICE pointers. w_embed: [dim, k_embed] bf16, the
+ * patch convolution in (channel, dv, dh, dw) order, columns zero-padded to k_embed (a multiple of
+ * 8); w_head: [n_head, dim] bf16, rows in (dv, dh, dw, channel) order, zero-padded to n_head (a
+ * multiple of 8; ignored in front of a pixel stage). in_channels counts the raw fields; two more
+ * channels follow when concat_lat is set. u_idx = v_idx = -1: no wind rotation. */
+typedef struct strata_backbone_desc {
+  int32_t in_channels, out_channels, patch_v, patch_h, patch_w;
+  int32_t dim, heads, hidden, n_blocks, qk_norm;
+  int32_t concat_lat, u_idx, v_idx, rope_mode;
+  double rope_length_scale, rope_base;
+  const void* w_embed;
+  const float* b_embed;
+  int64_t k_embed;
+  const strata_block_weights* h_blocks; /* [n_blocks] */
+  const int32_t* h_kernels;             /* [n_blocks][3]: kd, kh, kw */
+  const void* w_head;
+  const float* b_head;
+  int32_t n_head;
+} strata_backbone_desc;
+
+/* One AdaLN pixel block ("bilinear_dw" mode): w_mod NULL = unmodulated. cond_table: what
+ * strata_adaln_cond_table_f32 wrote for w_dw, or NULL where the geometry has no table. */
+typedef struct strata_pixel_block_weights {
+  strata_block_weights block;
+  const float* cond_table;
+  const float* w_dw;   /* [backbone dim, ks, ks] */
+  const float* b_dw;
+  const void* w_mod;   /* [6*dim, backbone dim] */
+  const float* b_mod;
+} strata_pixel_block_weights;
+
+/* Pixel stage of the two-stage model (screamcast/strata_wrappers.py:418-687), patch 1. */
+typedef struct strata_pixel_desc {
+  int32_t dim, heads, hidden, n_blocks, qk_norm, rope_mode, cond_ks;
+  double rope_length_scale, rope_base;
+  const void* w_embed;
+  const float* b_embed;
+  int64_t k_embed;
+  const strata_pixel_block_weights* h_blocks;
+  const int32_t* h_kernels;
+  const void* w_head;
+  const float* b_head;
+  int32_t n_head;
+} strata_pixel_desc;
+
+/* Device scratch of strata_network_forward_f32 (-1: sizes out of range). px NULL = single stage. */
+int64_t strata_network_workspace_bytes(const strata_backbone_desc* h_backbone,
+                                       const strata_pixel_desc* h_pixel, int B, int D, int H, int W);
+
+/* network(x[B, C_in, D, H, W], lat / lon [B, H, W]) -> out [B, C_out, D, H, W], fp32 fields: tile
+ * geometry, wind rotation and patch gathering, patch embedding, blocks, [pixel stage], final layer
+ * and un-patchify, all launched on `stream` by this one call (replaces
+ * StrataBackboneModel.forward / StrataModel.forward, screamcast/strata_wrappers.py:408-415,
+ * 673-680). workspace: 256-byte aligned, strata_network_workspace_bytes() bytes. */
+int strata_network_forward_f32(const strata_backbone_desc* h_backbone, const strata_pixel_desc* h_pixel,
+                               const float* x, const float* lat, const float* lon, int B, int D, int H,
+                               int W, float* out, void* workspace, int64_t workspace_bytes,
+                               void* stream);
 
 /* Cross-GPU barrier on the stream: publishes `epoch` (monotonically increasing per use) in slot
  * [me] of every rank's flag array h_flags[r] (int32[world], zero-initialised, peer-mapped) and

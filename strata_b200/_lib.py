@@ -6,7 +6,7 @@ error, the call raises.
 from __future__ import annotations
 
 import ctypes
-from ctypes import c_char_p, c_float, c_int, c_int64, c_void_p, POINTER, Structure
+from ctypes import c_char_p, c_double, c_float, c_int, c_int32, c_int64, c_void_p, POINTER, Structure
 from pathlib import Path
 
 _LIB_PATH = Path(__file__).resolve().parent / "libstrata_b200.so"
@@ -21,6 +21,33 @@ class BlockWeights(Structure):
     """struct strata_block_weights (device pointers)."""
     _fields_ = [(n, c_void_p) for n in ("w_qkv", "b_qkv", "w_proj", "b_proj", "w_gate", "b_gate",
                                         "w_fc1", "b_fc1", "w_fc2", "b_fc2")]
+
+
+class BackboneDesc(Structure):
+    """struct strata_backbone_desc."""
+    _fields_ = ([(n, c_int32) for n in ("in_channels", "out_channels", "patch_v", "patch_h", "patch_w",
+                                        "dim", "heads", "hidden", "n_blocks", "qk_norm", "concat_lat",
+                                        "u_idx", "v_idx", "rope_mode")]
+                + [("rope_length_scale", c_double), ("rope_base", c_double), ("w_embed", c_void_p),
+                   ("b_embed", c_void_p), ("k_embed", c_int64), ("h_blocks", POINTER(BlockWeights)),
+                   ("h_kernels", POINTER(c_int32)), ("w_head", c_void_p), ("b_head", c_void_p),
+                   ("n_head", c_int32)])
+
+
+class PixelBlockWeights(Structure):
+    """struct strata_pixel_block_weights."""
+    _fields_ = [("block", BlockWeights)] + [(n, c_void_p) for n in ("cond_table", "w_dw", "b_dw", "w_mod",
+                                                                   "b_mod")]
+
+
+class PixelDesc(Structure):
+    """struct strata_pixel_desc."""
+    _fields_ = ([(n, c_int32) for n in ("dim", "heads", "hidden", "n_blocks", "qk_norm", "rope_mode",
+                                        "cond_ks")]
+                + [("rope_length_scale", c_double), ("rope_base", c_double), ("w_embed", c_void_p),
+                   ("b_embed", c_void_p), ("k_embed", c_int64), ("h_blocks", POINTER(PixelBlockWeights)),
+                   ("h_kernels", POINTER(c_int32)), ("w_head", c_void_p), ("b_head", c_void_p),
+                   ("n_head", c_int32)])
 
 
 _SIGNATURES = {
@@ -77,6 +104,16 @@ _SIGNATURES = {
                                        c_void_p, c_void_p, c_int, c_int64, c_int64, c_void_p,
                                        c_void_p, c_void_p]),
     "strata_adaln_cond_table_floats": (c_int64, [c_int, c_int, c_int]),
+    "strata_adaln_cond_table_f32": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]),
+    "strata_tile_tables_workspace_bytes": (c_int64, [c_int, c_int, c_int]),
+    "strata_tile_tables": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
+                                   c_int, c_double, c_double, c_int, c_void_p, c_void_p, c_int64,
+                                   c_void_p]),
+    "strata_network_workspace_bytes": (c_int64, [POINTER(BackboneDesc), POINTER(PixelDesc), c_int, c_int,
+                                                 c_int, c_int]),
+    "strata_network_forward_f32": (c_int, [POINTER(BackboneDesc), POINTER(PixelDesc), c_void_p, c_void_p,
+                                           c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
+                                           c_int64, c_void_p]),
     "strata_dealias_patches_bf16": (c_int, [c_void_p, c_int64, c_int, c_int, c_int, c_int, c_int,
                                             c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_int64,
                                             c_void_p]),

@@ -551,8 +551,17 @@ inline long long adaln_cond_table_floats(int Cb, int factor, int ks) {
   return 9LL * factor * factor * 9 * Cb;
 }
 
-// table: device scratch of adaln_cond_table_floats() floats, or null for the direct kernel.
-inline int launch_adaln_cond(const AdalnCondParams& p, float* table, int sm_count,
+inline int launch_adaln_cond_table(const float* wdw, int Cb, int factor, int ks, float* table,
+                                   cudaStream_t stream) {
+  const int n = 9 * factor * factor * Cb;
+  adaln_cond_table_kernel<<<(n + 255) / 256, 256, 0, stream>>>(wdw, Cb, factor, ks, table);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
+}
+
+// table: what launch_adaln_cond_table wrote for these weights (adaln_cond_table_floats() floats),
+// or null for the direct kernel.
+inline int launch_adaln_cond(const AdalnCondParams& p, const float* table, int sm_count,
                              cudaStream_t stream) {
   if (p.Cb % 8 != 0 || p.Cb <= 0 || p.factor <= 0 || p.ks <= 0 || (p.ks & 1) == 0 || p.ks > 9 ||
       p.D <= 0 || p.h <= 0 || p.w <= 0 || p.row0 < 0)
@@ -560,8 +569,6 @@ inline int launch_adaln_cond(const AdalnCondParams& p, float* table, int sm_coun
   if (p.n_rows <= 0) return 0;
   if (table != nullptr && p.h >= 3 && p.w >= 3 &&
       adaln_cond_table_floats(p.Cb, p.factor, p.ks) > 0) {
-    const int n = 9 * p.factor * p.factor * p.Cb;
-    adaln_cond_table_kernel<<<(n + 255) / 256, 256, 0, stream>>>(p.wdw, p.Cb, p.factor, p.ks, table);
     const long long W = static_cast<long long>(p.w) * p.factor;
     const long long cell_rows = (p.row0 + p.n_rows - 1) / W / p.factor - p.row0 / W / p.factor + 1;
     const long long items =

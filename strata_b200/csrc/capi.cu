@@ -2,6 +2,7 @@
 // Single translation unit: the kernels live in the .cuh files included below.
 #include "../../include/strata_b200.h"
 
+#include <math.h>
 #include <string.h>
 
 #include <atomic>
@@ -13,6 +14,7 @@
 #include "halo.cuh"
 #include "prepost.cuh"
 #include "adaln.cuh"
+#include "geometry.cuh"
 
 using namespace strata;
 
@@ -705,9 +707,57 @@ int64_t strata_adaln_cond_table_floats(int Cb, int factor, int ks) {
   return adaln_cond_table_floats(Cb, factor, ks);
 }
 
-int strata_adaln_cond_bf16(const void* tokens, int B, int D, int h, int w, int Cb, int factor,
+int strata_adaln_cond_table_f32(const float* w_dw, int Cb, int factor, int ks, float* table,
+                                void* stream) {
+  if (current_sm_count() <= 0) return STRATA_ERR_NO_DEVICE;
+  if (!w_dw || !table || !aligned16(table) || adaln_cond_table_floats(Cb, factor, ks) == 0)
+    return STRATA_ERR_ARG;
+  return launch_adaln_cond_table(w_dw, Cb, factor, ks, table, as_stream(stream));
+}
+
+int64_t strata_tile_tables_workspace_bytes(int B, int H, int W) {
+  if (B < 0 || H <= 0 || W <= 0) return -1;
+  return tile_tables_ws_bytes(B, H, W);
+}
+
+int strata_tile_tables(const float* lat, const float* lon, int B, int H, int W, float* lat0,
+                       float* lon0, int rope_mode, int patch, double length_scale, double rope_base,
+                       int head_dim, void* rope_cs, void* workspace, int64_t workspace_bytes,
+                       void* stream) {
+  if (current_sm_count() <= 0) return STRATA_ERR_NO_DEVICE;
+  if (B < 0 || B > 65535 || H <= 0 || W <= 0 || static_cast<int64_t>(H) * W > 0x7fffffffLL)
+    return STRATA_ERR_ARG;
+  if (rope_mode < STRATA_ROPE_NONE || rope_mode > STRATA_ROPE_STEREOGRAPHIC) return STRATA_ERR_UNSUPPORTED;
+  if ((lat0 == nullptr) != (lon0 == nullptr)) return STRATA_ERR_ARG;
+  const bool sums = lat0 != nullptr || rope_mode == STRATA_ROPE_STEREOGRAPHIC;
+  if (sums && (!lat || !lon)) return STRATA_ERR_ARG;
+  if (rope_mode != STRATA_ROPE_NONE &&
+      (!rope_cs || patch <= 0 || patch > H || patch > W || head_dim % 4 || head_dim <= 0 ||
+       head_dim > 128 || !(length_scale > 0.0) || !(rope_base > 0.0)))
+    return STRATA_ERR_ARG;
+  const int64_t need = tile_tables_ws_bytes(B, H, W);
+  if (sums && need > 0 && (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 7u)))
+    return STRATA_ERR_ARG;
+  if (B == 0 || (!sums && rope_mode == STRATA_ROPE_NONE)) return STRATA_OK;
+  TileTablesParams p{};
+  p.lat = lat; p.lon = lon; p.H = H; p.W = W;
+  p.mode = rope_mode;
+  p.lat0 = lat0; p.lon0 = lon0;
+  if (rope_mode != STRATA_ROPE_NONE) {
+    p.patch = patch; p.h = H / patch; p.w = W / patch;
+    p.pairs = head_dim / 2;
+    p.inv_scale = 1.0 / (length_scale * patch * patch);
+    const int n = head_dim / 4;
+    for (int i = 0; i < n; ++i) p.freq[i] = pow(rope_base, -static_cast<double>(i) / n);
+    p.table = static_cast<uint32_t*>(rope_cs);
+  }
+  return launch_tile_tables(p, B, static_cast<double*>(workspace), as_stream(stream));
+}
+
+// (the stencil table ready, or null)
+static int strata_adaln_cond_ready_bf16(const void* tokens, int B, int D, int h, int w, int Cb, int factor,
                            const float* w_dw, const float* b_dw, int ks, int64_t row0,
-                           int64_t n_rows, void* out, float* table_ws, void* stream) {
+                           int64_t n_rows, void* out, const float* table, void* stream) {
   const int sms = current_sm_count();
   if (sms <= 0) return STRATA_ERR_NO_DEVICE;
   if (n_rows == 0) return STRATA_OK;
@@ -723,9 +773,67 @@ int strata_adaln_cond_bf16(const void* tokens, int B, int D, int h, int w, int C
   p.out = static_cast<__nv_bfloat16*>(out);
   p.row0 = row0; p.n_rows = n_rows;
   p.D = D; p.h = h; p.w = w; p.Cb = Cb; p.factor = factor; p.ks = ks;
-  if (table_ws && !aligned16(table_ws)) return STRATA_ERR_ARG;
-  int r = launch_adaln_cond(p, table_ws, sms, as_stream(stream));
+  int r = launch_adaln_cond(p, table, sms, as_stream(stream));
   return r == -2 ? STRATA_ERR_ARG : r;
+}
+
+int strata_adaln_cond_bf16(const void* tokens, int B, int D, int h, int w, int Cb, int factor,
+                           const float* w_dw, const float* b_dw, int ks, int64_t row0,
+                           int64_t n_rows, void* out, float* table_ws, void* stream) {
+  if (table_ws && !aligned16(table_ws)) return STRATA_ERR_ARG;
+  if (n_rows == 0 || ks <= 0 || adaln_cond_table_floats(Cb, factor, ks) == 0) table_ws = nullptr;
+  if (table_ws) {
+    const int r = strata_adaln_cond_table_f32(w_dw, Cb, factor, ks, table_ws, stream);
+    if (r != 0) return r;
+  }
+  return strata_adaln_cond_ready_bf16(tokens, B, D, h, w, Cb, factor, w_dw, b_dw, ks, row0, n_rows, out,
+                                      table_ws, stream);
+}
+
+}  // extern "C"
+
+#include "network.cuh"
+
+extern "C" {
+
+static int network_check(const strata_backbone_desc* b, const strata_pixel_desc* px, int B, int D, int H,
+                         int W) {
+  if (!b || B < 0 || D <= 0 || H <= 0 || W <= 0) return STRATA_ERR_ARG;
+  if (b->patch_v <= 0 || b->patch_h <= 0 || b->patch_w <= 0 || D % b->patch_v || H % b->patch_h ||
+      W % b->patch_w)
+    return STRATA_ERR_ARG;
+  if (b->dim <= 0 || b->heads <= 0 || b->dim % b->heads || b->hidden <= 0 || b->n_blocks < 0 ||
+      b->k_embed <= 0 || (!px && b->n_head <= 0) || (b->n_blocks > 0 && (!b->h_blocks || !b->h_kernels)))
+    return STRATA_ERR_ARG;
+  if (b->rope_mode != STRATA_ROPE_NONE && b->patch_h != b->patch_w) return STRATA_ERR_UNSUPPORTED;
+  if (px) {
+    if (px->dim <= 0 || px->heads <= 0 || px->dim % px->heads || px->hidden <= 0 || px->n_blocks < 0 ||
+        px->k_embed <= 0 || px->n_head <= 0 || (px->n_blocks > 0 && (!px->h_blocks || !px->h_kernels)))
+      return STRATA_ERR_ARG;
+    if (b->patch_v != 1 || b->patch_h != b->patch_w) return STRATA_ERR_UNSUPPORTED;
+  }
+  return STRATA_OK;
+}
+
+int64_t strata_network_workspace_bytes(const strata_backbone_desc* b, const strata_pixel_desc* px, int B,
+                                       int D, int H, int W) {
+  NetworkPlan n;
+  if (network_check(b, px, B, D, H, W) != 0 || !network_plan(*b, px, B, D, H, W, nullptr, n)) return -1;
+  return n.bytes;
+}
+
+int strata_network_forward_f32(const strata_backbone_desc* b, const strata_pixel_desc* px, const float* x,
+                               const float* lat, const float* lon, int B, int D, int H, int W, float* out,
+                               void* workspace, int64_t workspace_bytes, void* stream) {
+  if (current_sm_count() <= 0) return STRATA_ERR_NO_DEVICE;
+  const int r = network_check(b, px, B, D, H, W);
+  if (r != 0) return r;
+  if (!x || !lat || !lon || !out || !workspace || (reinterpret_cast<uintptr_t>(workspace) & 255u))
+    return STRATA_ERR_ARG;
+  NetworkPlan n;
+  if (!network_plan(*b, px, B, D, H, W, workspace, n) || workspace_bytes < n.bytes) return STRATA_ERR_ARG;
+  if (B == 0) return STRATA_OK;
+  return network_forward(*b, px, x, lat, lon, B, D, H, W, out, n, stream);
 }
 
 }  // extern "C"

@@ -361,6 +361,46 @@ def postprocess_fields(y: torch.Tensor, shape, lat=None, lon=None, lat0=None, lo
     return out
 
 
+def _check_fields(x, lat, lon, channels, backbone) -> None:
+    """Shapes of a network call: fields [B, C, D, H, W] with lat / lon [B, H, W], patches that
+    divide the grid, and as many channels as the patch embedding has."""
+    B, _, D, H, W = x.shape
+    pv, ph, pw = backbone.patch_size
+    if D % pv or H % ph or W % pw:
+        raise ValueError(f"grid {(D, H, W)} is not divisible by the patch {(pv, ph, pw)}")
+    if tuple(lat.shape) != (B, H, W) or tuple(lon.shape) != (B, H, W):
+        raise ValueError(f"lat / lon must have shape {(B, H, W)}, got {tuple(lat.shape)}")
+    if channels != backbone.patch_embed.proj.in_channels:
+        raise ValueError(f"{channels} input channels, the patch embedding expects "
+                         f"{backbone.patch_embed.proj.in_channels}")
+
+
+def tile_tables(lat: torch.Tensor, lon: torch.Tensor, *, centre: bool = False, rope_mode: str = "none",
+                patch: int = 1, length_scale: float = 1.0, rope_base: float = 100.0, head_dim: int = 64):
+    """Tile centres and the packed rotary table of tiles given by per-pixel lat / lon [B, H, W]
+    (fp32 radians). Returns (lat0, lon0, rope_cs): lat0 / lon0 [B] or None; rope_cs the half table
+    [B, (H/patch)*(W/patch), head_dim/2, 2] (see rope.pack_rope_tables) or None."""
+    B, H, W = lat.shape
+    lat = _f32_dev(lat, "lat", (B, H, W))
+    lon = _f32_dev(lon, "lon", (B, H, W))
+    dev = lat.device
+    mode = {"none": 0, "axial": 1, "stereographic": 2}[rope_mode]
+    lat0 = torch.empty(B, device=dev) if centre else None
+    lon0 = torch.empty(B, device=dev) if centre else None
+    cs = None
+    if mode:
+        cs = torch.empty((B, (H // patch) * (W // patch), head_dim // 2, 2), dtype=torch.float16, device=dev)
+    lib = _lib.load()
+    need = int(lib.strata_tile_tables_workspace_bytes(B, H, W))
+    ws = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
+    p = lambda t: None if t is None else t.data_ptr()
+    with torch.cuda.device(dev):
+        _lib.check(lib.strata_tile_tables(lat.data_ptr(), lon.data_ptr(), B, H, W, p(lat0), p(lon0), mode,
+                                          int(patch), float(length_scale), float(rope_base), int(head_dim),
+                                          p(cs), p(ws), need, _stream_ptr(lat)), "strata_tile_tables")
+    return lat0, lon0, cs
+
+
 # ------------------------------------------------------------------ pixel stage (AdaLN blocks)
 def _rows_or_none(t, name, C):
     if t is None:

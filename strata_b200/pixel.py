@@ -19,6 +19,7 @@ import torch
 import torch.nn as nn
 
 from . import ops, rope
+from .network import NetworkHandle
 from .ops import EPI_BIAS, EPI_GATE, EPI_GELU
 from .strata import FinalLayer, Mlp, NeighborhoodAttention3D, PatchEmbed3D, StrataTransformer3D, _triple
 
@@ -58,6 +59,10 @@ class StrataPixel3DBlock(nn.Module):
             nn.init.zeros_(self.adaln_bilinear_dw_proj.bias)
         self._cache = None
         self._key = None
+
+    def _gelu_is_tanh(self) -> bool:
+        act = self.mlp.layers[1]
+        return isinstance(act, nn.GELU) and act.approximate == "tanh"
 
     @property
     def has_adaln(self) -> bool:
@@ -114,7 +119,7 @@ class StrataPixel3DBlock(nn.Module):
                 rope_cs: torch.Tensor | None = None) -> torch.Tensor:
         """x: bf16 rows [n_tiles * D*H*W, dim], updated in place and returned. rope_cs: packed
         half (cos, sin) table [n_tiles, H*W, 32, 2] or None."""
-        if not (isinstance(self.mlp.layers[1], nn.GELU) and self.mlp.layers[1].approximate == "tanh"):
+        if not self._gelu_is_tanh():
             raise RuntimeError("the fused MLP kernel implements the tanh GELU; this block's Mlp "
                                "still holds an exact GELU (the wrapper's tanh swap did not run)")
         C = self.dim
@@ -188,6 +193,7 @@ class Strata(nn.Module):
                                adaln_mode=adaln_mode, patch=self.backbone.patch_size)
             for i in range(num_layers_pixel)])
         self.pixel_final_layer = FinalLayer(embed_dim_pixel, self.out_channels)
+        self._network = NetworkHandle()
         if rope_mode_pixel == "axial":
             self._build_axial_rope_pixel()
 
@@ -200,25 +206,25 @@ class Strata(nn.Module):
         self.register_buffer("_rope_cos_pixel", cos[0].repeat(self.depth, 1), persistent=False)
         self.register_buffer("_rope_sin_pixel", sin[0].repeat(self.depth, 1), persistent=False)
 
-    def rope_tables_pixel(self, pos: torch.Tensor | None, n_tiles: int, grid_px):
+    def rope_tables_pixel(self, lat: torch.Tensor | None, lon: torch.Tensor | None, n_tiles: int, grid_px):
         """Packed half (cos, sin) table [n_tiles, H*W, head_dim/2, 2] of the pixel tokens, or None."""
         D, H, W = grid_px
         if self.rope_mode_pixel == "none":
             return None
         if self.rope_mode_pixel == "axial":
+            self._check_axial_rope_pixel(D * H * W)
             hw = H * W
-            if self._rope_cos_pixel.shape[0] != D * hw:
-                raise ValueError(f"axial pixel RoPE tables were built for {self._rope_cos_pixel.shape[0]} "
-                                 f"tokens, the input has {D * hw}; call set_tile_size first")
-            cos = self._rope_cos_pixel[:hw].expand(n_tiles, -1, -1).contiguous()
-            sin = self._rope_sin_pixel[:hw].expand(n_tiles, -1, -1).contiguous()
-        else:
-            if pos is None:
-                raise ValueError("stereographic RoPE needs pos=[B, 2, H, W] (lat, lon)")
-            cos, sin = rope.stereographic_rope_tables(pos, self.head_dim_pixel, 1,
-                                                      self.rope_length_scale_pixel,
-                                                      self.rope_base_pixel)
-        return rope.pack_rope_tables(cos, sin)
+            return rope.pack_rope_tables(self._rope_cos_pixel[:hw].expand(n_tiles, -1, -1),
+                                         self._rope_sin_pixel[:hw].expand(n_tiles, -1, -1))
+        if lat is None:
+            raise ValueError("stereographic RoPE needs the pixels' lat / lon [B, H, W]")
+        return ops.tile_tables(lat, lon, rope_mode="stereographic", length_scale=self.rope_length_scale_pixel,
+                               rope_base=self.rope_base_pixel, head_dim=self.head_dim_pixel)[2]
+
+    def _check_axial_rope_pixel(self, tokens: int) -> None:
+        if self._rope_cos_pixel.shape[0] != tokens:
+            raise ValueError(f"axial pixel RoPE tables were built for {self._rope_cos_pixel.shape[0]} "
+                             f"tokens, the input has {tokens}; call set_tile_size first")
 
     def pixel_stage(self, pixel_tokens: torch.Tensor, backbone_tokens: torch.Tensor, grid_px,
                     rope_cs: torch.Tensor | None = None):
@@ -240,17 +246,23 @@ class Strata(nn.Module):
         the un-patchify and inverse rotation one kernel on the way out."""
         bb = self.backbone
         B, _, D, H, W = x.shape
+        if self.rope_mode_pixel == "axial":
+            self._check_axial_rope_pixel(D * H * W)
+        if type(bb.patch_embed) is PatchEmbed3D and lat0 is None and lat is not None:
+            y = self._network.forward(bb, self, x, lat, lon, wind, concat_lat)
+            if y is not None:
+                return y
         grid = bb.token_grid(D, H, W)
+        lat0, lon0, cs = bb.fused_tables(lat, lon, lat0, lon0, wind)
         tokens = bb.embed_fused(x, lat, lon, lat0, lon0, wind, concat_lat)
-        cos, sin = bb.rope_tables(pos, B, grid)
-        tokens = bb.forward_tokens(tokens, grid, cos, sin)
+        tokens = bb._run_blocks(tokens, grid, cs)
         _, _, _, Kpp = self.pixel_patch_embed._gemm_weights()
         ap = ops.preprocess_patches(x, lat, lon, lat0, lon0, wind=wind, concat_lat=concat_lat,
                                     patch=(1, 1, 1), k_pad=Kpp)
         px = self.pixel_patch_embed.tokens_from_patches(ap, B)
         del ap
         px = self.pixel_stage(px, tokens.view(B, *grid, bb.embed_dim), (D, H, W),
-                              self.rope_tables_pixel(pos, B, (D, H, W)))
+                              self.rope_tables_pixel(lat, lon, B, (D, H, W)))
         y, _ = self.pixel_final_layer.matrix_bf16(px)
         return ops.postprocess_fields(y, (B, self.out_channels, D, H, W), lat, lon, lat0, lon0,
                                       wind=wind, patch=(1, 1, 1))

@@ -26,6 +26,7 @@ import torch
 import torch.nn as nn
 
 from . import ops, rope
+from .network import NetworkHandle
 
 
 def _triple(v):
@@ -307,6 +308,7 @@ class StrataTransformer3D(nn.Module):
         pv, ph, pw = self.patch_size
         self.final_layer = FinalLayer(embed_dim, pv * ph * pw * out_channels)
         self._workspace = None
+        self._network = NetworkHandle()
 
     # ---------------------------------------------------------------- geometry
     def set_tile_size(self, height: int, width: int) -> None:
@@ -341,8 +343,11 @@ class StrataTransformer3D(nn.Module):
     # ---------------------------------------------------------------- forward
     def forward_tokens(self, tokens: torch.Tensor, grid, rope_cos, rope_sin) -> torch.Tensor:
         """Runs the block stack on bf16 tokens [n_tiles, D*H*W, C]."""
-        ws = self._get_workspace(tokens.shape[0] * tokens.shape[1], tokens.device)
         cs = None if rope_cos is None else rope.pack_rope_tables(rope_cos, rope_sin)
+        return self._run_blocks(tokens, grid, cs)
+
+    def _run_blocks(self, tokens: torch.Tensor, grid, cs) -> torch.Tensor:
+        ws = self._get_workspace(tokens.shape[0] * tokens.shape[1], tokens.device)
         x = tokens
         for blk in self.blocks:
             x = blk(x, grid, cs, workspace=ws)
@@ -388,17 +393,31 @@ class StrataTransformer3D(nn.Module):
     def forward_fused(self, x: torch.Tensor, pos: torch.Tensor | None, *, lat=None, lon=None,
                       lat0=None, lon0=None, wind=None, concat_lat: bool = False) -> torch.Tensor:
         """Raw fields in, fields out, with the wrapper's pre- and post-processing inside:
-        x [B, C_raw, D, H, W] fp32 (before wind rotation and latitude channels) ->
-        [B, C_out, D, H, W] fp32 (wind channels rotated back). One kernel gathers, rotates,
-        appends and casts the patch rows, one un-patchifies and rotates back."""
+        x [B, C_raw, D, H, W] fp32 (before wind rotation and latitude channels), lat / lon [B, H, W]
+        -> [B, C_out, D, H, W] fp32 (wind channels rotated back). The tile centres lat0 / lon0 are
+        worked out from lat / lon unless given. One library call; a model with the de-aliased
+        embedding takes its steps one by one."""
+        if type(self.patch_embed) is PatchEmbed3D and lat0 is None and lat is not None:
+            y = self._network.forward(self, None, x, lat, lon, wind, concat_lat)
+            if y is not None:
+                return y
         B, _, D, H, W = x.shape
         grid = self.token_grid(D, H, W)
+        lat0, lon0, cs = self.fused_tables(lat, lon, lat0, lon0, wind)
         tokens = self.embed_fused(x, lat, lon, lat0, lon0, wind, concat_lat)
-        cos, sin = self.rope_tables(pos, B, grid)
-        tokens = self.forward_tokens(tokens, grid, cos, sin)
+        tokens = self._run_blocks(tokens, grid, cs)
         y, _ = self.final_layer.matrix_bf16(tokens)
         return ops.postprocess_fields(y, (B, self.out_channels, D, H, W), lat, lon, lat0, lon0,
                                       wind=wind, patch=self.patch_size)
+
+    def fused_tables(self, lat, lon, lat0, lon0, wind):
+        """(lat0, lon0, packed rotary table) of the tiles: centres only where a wind rotation
+        needs them and the caller has none."""
+        centre = wind is not None and lat0 is None
+        c_lat, c_lon, cs = ops.tile_tables(lat, lon, centre=centre, rope_mode=self.rope_mode,
+                                           patch=self.patch_size[1], length_scale=self.rope_length_scale,
+                                           rope_base=self.rope_base, head_dim=self.head_dim)
+        return (c_lat, c_lon, cs) if centre else (lat0, lon0, cs)
 
     def unpatchify(self, y: torch.Tensor, grid) -> torch.Tensor:
         B = y.shape[0]

@@ -185,6 +185,8 @@ class _StrataModelBase(nn.Module):
         behind it is one registered operator, so the module can be compiled whole
         (`torch.compile(network)`, also with fullgraph=True) and called under inference mode."""
         lat, lon = self.geometry.lat_lon_from_index(index)
+        if torch_ops.plain_call(x):
+            return self._forward_eager(x, lat, lon)
         return torch.ops.strata_b200.network_forward(x, lat, lon, self._op_handle)
 
     def _latlon_for(self, x: torch.Tensor, lat: torch.Tensor, lon: torch.Tensor):
@@ -337,12 +339,8 @@ class StrataBackboneModel(_StrataModelBase):
         lat, lon = self._latlon_for(x, lat, lon)
         lat = lat.to(device=x.device, dtype=torch.float32).contiguous()
         lon = lon.to(device=x.device, dtype=torch.float32).contiguous()
-        lat0 = lon0 = wind = None
-        if self._do_rotate_wind:
-            lat0, lon0 = TileGeometry.tile_center(lat, lon)
-            wind = self._wind_channel_indices
-        pos = torch.stack([lat, lon], dim=1)
-        return self.strata.forward_fused(x, pos, lat=lat, lon=lon, lat0=lat0, lon0=lon0, wind=wind,
+        return self.strata.forward_fused(x, None, lat=lat, lon=lon,
+                                         wind=self._wind_channel_indices if self._do_rotate_wind else None,
                                          concat_lat=self._do_concat_latitude)
 
 
@@ -492,10 +490,6 @@ class StrataModel(_StrataModelBase):
         lat, lon = self._latlon_for(x, lat, lon)
         lat = lat.to(device=x.device, dtype=torch.float32).contiguous()
         lon = lon.to(device=x.device, dtype=torch.float32).contiguous()
-        lat0 = lon0 = wind = None
-        if self._do_rotate_wind:
-            lat0, lon0 = TileGeometry.tile_center(lat, lon)
-            wind = self._wind_channel_indices
-        pos = torch.stack([lat, lon], dim=1)
-        return self.strata.forward_fused(x, pos, lat=lat, lon=lon, lat0=lat0, lon0=lon0, wind=wind,
+        return self.strata.forward_fused(x, None, lat=lat, lon=lon,
+                                         wind=self._wind_channel_indices if self._do_rotate_wind else None,
                                          concat_lat=self._do_concat_latitude)

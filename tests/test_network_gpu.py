@@ -1,0 +1,82 @@
+"""The one-call network forward and the tile-table kernels against the step-by-step path and the
+tensor formulas they replace."""
+import math
+
+import pytest
+import torch
+
+from oracle import block_oracle as bo
+from tests.util import tile_latlon
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B,H,W,patch", [(1, 8, 8, 4), (2, 33, 31, 1), (1, 32, 32, 1), (3, 36, 100, 4),
+                                         (1, 64, 264, 8), (2, 18, 6, 2)])
+def test_tile_tables_match_formulas(B, H, W, patch):
+    # 1024 pixels is where the tile's sums move to a kernel of their own
+    from strata_b200 import ops
+    from strata_b200.wrappers import TileGeometry
+    lat, lon = tile_latlon(B, H, W)
+    lon = lon + 5.9                                            # tiles across the 2 pi seam
+    scale = bo.default_rope_length_scale(patch) * 3
+    lat0, lon0, cs = ops.tile_tables(lat.cuda(), lon.cuda(), centre=True, rope_mode="stereographic",
+                                     patch=patch, length_scale=scale)
+    cos, sin = bo.stereographic_rope_tables(lat, lon, 64, patch, scale)
+    want = torch.stack([cos, sin], -1)
+    assert cs.shape == want.shape
+    assert (cs.float().cpu() - want).abs().max() < 6e-4        # half rounding of values up to 1
+    w0, w1 = TileGeometry.tile_center(lat.double(), lon.double())
+    assert torch.allclose(lat0.cpu().double(), w0.flatten(), atol=1e-6)
+    d = (lon0.cpu().double() - w1.flatten() + math.pi) % (2 * math.pi) - math.pi
+    assert d.abs().max() < 2e-6
+    _, _, ax = ops.tile_tables(lat.cuda(), lon.cuda(), rope_mode="axial", patch=patch)
+    cos, sin = bo.axial_rope_tables(H // patch, W // patch, 64)
+    assert (ax.float().cpu() - torch.stack([cos, sin], -1)).abs().max() < 6e-4
+
+
+def _randomised(m):
+    g = torch.Generator(device="cuda").manual_seed(3)
+    with torch.no_grad():
+        for p in m.parameters():
+            p.copy_(torch.randn(p.shape, generator=g, device="cuda") * (0.05 if p.dim() == 1 else p[0].numel() ** -0.5))
+    return m.eval()
+
+
+@pytest.mark.parametrize("two_stage,over", [
+    (False, dict()), (False, dict(do_rotate_wind=True, wind_channel_indices=(1, 0), gated_attention=True)),
+    (False, dict(do_rope_2d_stereographic=False, do_rope_2d=True, qk_norm=True, patch_size_vert=2,
+                 attn_kernel=(1, 3, 5))),
+    (True, dict(do_rotate_wind=True, wind_channel_indices=(0, 2), qk_norm_pixel=True)),
+    (True, dict(do_rope_2d_pixel=True, first_block_only_adaln_pixel=True)),
+    (True, dict(do_rope_2d_stereographic_pixel=True, gated_attention_pixel=True))])
+def test_one_call_equals_step_by_step(two_stage, over):
+    from strata_b200.wrappers import StrataBackboneModel, StrataModel
+    kw = dict(depth=4, height=40, width=24, n_layers=2, patch_size_horiz=4, in_chans=5, base_out_chans=4,
+              embed_dim=128, num_heads=2, attn_kernel=(3, 3, 5), do_rope_2d_stereographic=True,
+              index_is_latlon=True)
+    if two_stage:
+        kw.update(embed_dim_pixel=64, n_layers_pixel=2, attn_kernel_pixel=(3, 3, 3),
+                  use_bilinear_dw_gelu_project_adaln_pixel=True)
+    kw.update(over)
+    m = _randomised((StrataModel if two_stage else StrataBackboneModel)(**kw).cuda())
+    x = torch.randn(2, 5, 4, 40, 24, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    lat, lon = tile_latlon(2, 40, 24)
+    idx = {"lat": lat.cuda(), "lon": lon.cuda()}
+
+    class StepByStep:
+        def forward(self, *a):
+            return None
+    with torch.no_grad():
+        y = m(x, idx)
+        one_call, m.strata._network = m.strata._network, StepByStep()
+        assert torch.equal(m(x, idx), y)
+        # a changed weight, module or option reaches the next call
+        m.strata._network = one_call
+        bb = m.strata.backbone if two_stage else m.strata
+        bb.blocks[1].attn.proj.weight.mul_(1.5)
+        bb.blocks[0].mlp.layers[2] = torch.nn.Linear(512, 128).cuda()
+        bb.rope_length_scale *= 2.0
+        z = m(x, idx)
+        m.strata._network = StepByStep()
+        assert torch.equal(m(x, idx), z) and not torch.equal(y, z)
