@@ -327,218 +327,125 @@ __global__ void adaln_cond_table_kernel(const float* __restrict__ wdw, int Cb, i
   }
 }
 
-// acc = bias + sum_k w[k] * t[k] over the 3 x 3 token block; tb points at this thread's 8
-// channels of table entry k = 0, entries `stride` float4 apart.
-__device__ __forceinline__ void cond_stencil(const float4* tb, int stride, const uint4 (&tk)[9],
-                                             const float* bdw, int cv, float (&acc)[8]) {
-  if (bdw != nullptr) {
-    const float4 b0 = __ldg(reinterpret_cast<const float4*>(bdw) + cv * 2);
-    const float4 b1 = __ldg(reinterpret_cast<const float4*>(bdw) + cv * 2 + 1);
-    acc[0] = b0.x; acc[1] = b0.y; acc[2] = b0.z; acc[3] = b0.w;
-    acc[4] = b1.x; acc[5] = b1.y; acc[6] = b1.z; acc[7] = b1.w;
-  } else {
-#pragma unroll
-    for (int c = 0; c < 8; ++c) acc[c] = 0.f;
-  }
-#pragma unroll
-  for (int k = 0; k < 9; ++k) {
-    const float4 w0 = tb[k * stride];
-    const float4 w1 = tb[k * stride + 1];
-    float t[8];
-    unpack8(tk[k], t);
-    acc[0] = fmaf(w0.x, t[0], acc[0]); acc[1] = fmaf(w0.y, t[1], acc[1]);
-    acc[2] = fmaf(w0.z, t[2], acc[2]); acc[3] = fmaf(w0.w, t[3], acc[3]);
-    acc[4] = fmaf(w1.x, t[4], acc[4]); acc[5] = fmaf(w1.y, t[5], acc[5]);
-    acc[6] = fmaf(w1.z, t[6], acc[6]); acc[7] = fmaf(w1.w, t[7], acc[7]);
-  }
-}
-
-// The four corner cells of every plane (each has its own f x f block of table classes). One
-// thread: one cell (factor x factor pixels of one backbone token) x 8 channels, table entries
-// read from global memory (L2).
-constexpr int COND_CELLS_PER_ITEM = 256;   // interior kernel: cells a block walks per slab load
-constexpr int COND_BORDER_CELLS_PER_ITEM = 64;
+// GELU(stencil) of the cells of a row, through the table. One warp = a run of up to COND_RUN
+// neighbouring cells of one cell row x 64 channels: lane l owns channels 2l, 2l+1 of the group, so
+// a token read and a pixel write are 128 contiguous bytes per warp. The first and the last cell
+// of a row are runs of their own (their table classes differ), the cells between share one block
+// of classes; the row's own class follows from R. A lane keeps the 3 x (COND_RUN + 2) tokens its
+// cells touch as fp32 pairs in registers and reads the 9 table entries of a phase once for all
+// its cells (L1: a group's classes are 37 KB at factor 4).
+//
+// Bound: instruction issue and the FMA pipe - 9 packed multiply-adds for the stencil and 5 for
+// the GELU per pixel and channel pair. With 2 cells x 4 channels a lane the entries came from a
+// shared-memory slab, nine 16-byte reads per 36 multiply-adds, and those reads set the pace; a run
+// of 6 cells x 2 channels needs nine 8-byte reads per 54 with fewer token registers, because
+// neighbouring cells share six of their nine tokens (runs of 7 and 8 spill and are no faster).
+// No slab, so no block-wide item either: small images spread over the chip, and where the runs
+// alone are too few for it (psplit) the f phase rows of a run are separate warps. 2^18 pixels x 1024
+// channels: 0.40 -> 0.29 ms; 4 x 64 x 64 pixels x 128 channels: 88 -> 12 us (edges included).
+constexpr int COND_RUN = 6;
 
 __global__ void __launch_bounds__(256, 2)
-adaln_cond_border_kernel(const AdalnCondParams p, const float* __restrict__ table) {
-  const int nvec = p.Cb >> 3;
-  const int ncvg = nvec >> 2;
+adaln_cond_runs_kernel(const AdalnCondParams p, const float* __restrict__ table, int psplit) {
   const int f = p.factor;
   const int ncls = 3 * f;
   const int H = p.h * f, W = p.w * f;
+  const int groups = (p.Cb + 63) >> 6;
+  const int runs = 2 + (p.w - 2 + COND_RUN - 1) / COND_RUN;     // first cell, last cell, the rest
   const long long gR0 = p.row0 / W / f;
   const long long gR1 = (p.row0 + p.n_rows - 1) / W / f;
-  const long long ring = 4;                                  // the corner cells of one plane
-  const long long plane0 = gR0 / p.h;
-  const long long n_cells = (gR1 / p.h - plane0 + 1) * ring;
-  const long long n_chunks = (n_cells + COND_BORDER_CELLS_PER_ITEM - 1) / COND_BORDER_CELLS_PER_ITEM;
-  const long long n_items = n_chunks * ncvg;
+  const long long n_items = (gR1 - gR0 + 1) * runs * psplit;
   const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  for (long long item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int cvg = static_cast<int>(item / n_chunks);
-    const long long cell = (item % n_chunks) * COND_BORDER_CELLS_PER_ITEM + warp * 8 + (lane >> 2);
-    if (cell >= n_cells) continue;
-    const int cv = cvg * 4 + (lane & 3);
-    const long long plane = plane0 + cell / ring;
-    const int k = static_cast<int>(cell % ring);
-    const int R = (k & 2) ? p.h - 1 : 0, Cc = (k & 1) ? p.w - 1 : 0;
+  const int phys = psplit > 1 ? 1 : f;                          // phase rows of an item
+  // a block stays with one channel group, whose table entries then fit its L1; neighbouring blocks
+  // take the other groups of the same pixels, so that whole output rows are written at about one time
+  const int grp = static_cast<int>(blockIdx.x) % groups;
+  const int ch = grp * 64 + 2 * lane;
+  if (ch >= p.Cb) return;
+  const long long stride = static_cast<long long>(gridDim.x / groups) * 8;
+  for (long long item = static_cast<long long>(blockIdx.x / groups) * 8 + (threadIdx.x >> 5);
+       item < n_items; item += stride) {
+    long long t = item;
+    const int run = static_cast<int>(t % runs); t /= runs;
+    const int phy0 = psplit > 1 ? static_cast<int>(t % psplit) : 0;
+    if (psplit > 1) t /= psplit;
+    const long long gR = gR0 + t;
+    const long long plane = gR / p.h;
+    const int R = static_cast<int>(gR - plane * p.h);
+    // (the last full run ends at the last inner cell: it repeats some cells of the one before it
+    // rather than being a short run)
+    const int inner = p.w - 2;
+    const int c0 = run == 0 ? 0 : (run == 1 ? p.w - 1
+                                            : 1 + max(0, min((run - 2) * COND_RUN, inner - COND_RUN)));
+    const int n = run < 2 ? 1 : min(COND_RUN, inner);
     const int rb = R == 0 ? 0 : (R == p.h - 1 ? p.h - 3 : R - 1);
-    const int cb = Cc == 0 ? 0 : (Cc == p.w - 1 ? p.w - 3 : Cc - 1);
+    const int cb = run == 0 ? 0 : (run == 1 ? p.w - 3 : c0 - 1);
     const int ycls0 = R == 0 ? 0 : (R == p.h - 1 ? 2 * f : f);
-    const int xcls0 = Cc == 0 ? 0 : (Cc == p.w - 1 ? 2 * f : f);
-    const uint4* base = reinterpret_cast<const uint4*>(p.tok + plane * p.h * p.w * p.Cb) + cv;
-    uint4 tk[9];
+    const int xcls0 = run == 0 ? 0 : (run == 1 ? 2 * f : f);
+    uint64_t tk[3][COND_RUN + 2];
+    const __nv_bfloat16* base = p.tok + ((plane * p.h + rb) * p.w + cb) * static_cast<long long>(p.Cb) + ch;
 #pragma unroll
-    for (int t = 0; t < 9; ++t)
-      tk[t] = __ldg(base + (static_cast<long long>(rb + t / 3) * p.w + (cb + t % 3)) * nvec);
-    for (int phy = 0; phy < f; ++phy) {
-      const int y = R * f + phy;
-      for (int phx = 0; phx < f; ++phx) {
-        const int x = Cc * f + phx;
-        const long long pix = (plane * H + y) * W + x;
-        if (pix < p.row0 || pix >= p.row0 + p.n_rows) continue;
-        float acc[8];
-        const long long cls = static_cast<long long>(ycls0 + phy) * ncls + (xcls0 + phx);
-        cond_stencil(reinterpret_cast<const float4*>(table + cls * 9 * p.Cb) + cv * 2, p.Cb >> 2,
-                     tk, p.bdw, cv, acc);
-        gelu8(acc);
-        reinterpret_cast<uint4*>(p.out + (pix - p.row0) * p.Cb)[cv] = pack8(acc);
+    for (int j = 0; j < 3; ++j)
+#pragma unroll
+      for (int i = 0; i < COND_RUN + 2; ++i) {
+        const uint32_t v = i < n + 2 ? __ldg(reinterpret_cast<const uint32_t*>(
+                                           base + (static_cast<long long>(j) * p.w + i) * p.Cb)) : 0u;
+        tk[j][i] = pack2(bf16_lo(v), bf16_hi(v));
+        // keep the pair: the compiler would hold the bf16 word and convert it again at every use
+        asm volatile("" : "+l"(tk[j][i]));
       }
+    uint64_t bias = 0ull;
+    if (p.bdw != nullptr) {
+      const float2 b2 = __ldg(reinterpret_cast<const float2*>(p.bdw + ch));
+      bias = pack2(b2.x, b2.y);
     }
-  }
-}
-
-// Interior cells, second layout: one thread = TWO neighbouring cells x 4 channels. The table
-// entries of a phase (read from the shared-memory slab) serve both cells, which halves the
-// shared-memory reads per output - the interior kernel is paced by those reads and by
-// instruction issue in about equal parts. A warp holds 4 cell pairs x 8 channel quads (32
-// channels): a token read and a row write are still 64 contiguous bytes per cell.
-__global__ void __launch_bounds__(256, 2)
-adaln_cond_interior_kernel(const AdalnCondParams p, const float* __restrict__ table, int group0) {
-  extern __shared__ __align__(16) float slab[];
-  const int ncvg = p.Cb >> 5;
-  const int f = p.factor;
-  const int ncls = 3 * f;
-  const int H = p.h * f, W = p.w * f;
-  const long long gR0 = p.row0 / W / f;
-  const long long gR1 = (p.row0 + p.n_rows - 1) / W / f;
-  // blockIdx.y: which set of cells sharing one f x f block of table classes - 0: the interior,
-  // 1 / 2: first / last cell row without its corners, 3 / 4: first / last cell column without
-  // its corners (the four corner cells of a plane are left to the border kernel)
-  const int group = group0 + static_cast<int>(blockIdx.y);
-  const long long plane0 = gR0 / p.h;
-  const long long planes = gR1 / p.h - plane0 + 1;
-  const int per_plane = group == 0 ? 0 : (group <= 2 ? p.w - 2 : p.h - 2);
-  const long long n_cells = group == 0 ? (gR1 - gR0 + 1) * p.w : planes * per_plane;
-  const int ycls0 = group == 1 ? 0 : (group == 2 ? 2 * f : f);
-  const int xcls0 = group == 3 ? 0 : (group == 4 ? 2 * f : f);
-  const long long n_chunks = (n_cells + COND_CELLS_PER_ITEM - 1) / COND_CELLS_PER_ITEM;
-  const long long n_items = n_chunks * ncvg;
-  const int lane = threadIdx.x & 31;
-  const int warp = threadIdx.x >> 5;
-  const int cq = lane & 7;
-  const int slab_vec = f * f * 9 * 8;                      // float4 count of a slab
-  for (long long item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int cvg = static_cast<int>(item / n_chunks);
-    const long long cell0 = (item % n_chunks) * COND_CELLS_PER_ITEM;
-    __syncthreads();                                       // previous item's readers are done
-    for (int v = threadIdx.x; v < slab_vec; v += blockDim.x) {
-      const int e = v >> 3;                                // (phase, k)
-      const int phase = e / 9, k = e - phase * 9;
-      const int cls = (ycls0 + phase / f) * ncls + (xcls0 + phase % f);
-      reinterpret_cast<float4*>(slab)[v] = __ldg(
-          reinterpret_cast<const float4*>(table + (static_cast<long long>(cls) * 9 + k) * p.Cb +
-                                          cvg * 32) + (v & 7));
-    }
-    __syncthreads();
-    const int ch0 = cvg * 32 + 4 * cq;
-    float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (p.bdw != nullptr) bias = __ldg(reinterpret_cast<const float4*>(p.bdw + ch0));
-    for (int pass = 0; pass < COND_CELLS_PER_ITEM / 64; ++pass) {
-      uint64_t ta[9][2], tb[9][2];   // fp32 pairs (channels 0-1, 2-3): the stencil runs on packed fp32x2
-      long long pix_a = -1, pix_b = -1;     // first pixel of each cell; -1: the cell is skipped
-#pragma unroll
-      for (int s2 = 0; s2 < 2; ++s2) {
-        const long long cell = cell0 + pass * 64 + warp * 8 + 2 * (lane >> 3) + s2;
-        if (cell >= n_cells) continue;
-        long long plane;
-        int R, Cc;
-        if (group == 0) {
-          const long long gR = gR0 + cell / p.w;
-          Cc = static_cast<int>(cell % p.w);
-          plane = gR / p.h;
-          R = static_cast<int>(gR % p.h);
-          if (R < 1 || R > p.h - 2 || Cc < 1 || Cc > p.w - 2) continue;
-        } else {
-          plane = plane0 + cell / per_plane;
-          const int j = 1 + static_cast<int>(cell % per_plane);
-          R = group == 1 ? 0 : (group == 2 ? p.h - 1 : j);
-          Cc = group == 3 ? 0 : (group == 4 ? p.w - 1 : j);
-        }
-        // the 3 x 3 token block starts one cell before the cell, clamped into the plane
-        const int rb = R == 0 ? 0 : (R == p.h - 1 ? p.h - 3 : R - 1);
-        const int cb = Cc == 0 ? 0 : (Cc == p.w - 1 ? p.w - 3 : Cc - 1);
-        const __nv_bfloat16* base = p.tok + plane * p.h * p.w * p.Cb + ch0;
+    const float k0 = 0.7978845608028654f, k01 = 0.7978845608028654f * 0.044715f;
+    const uint64_t K0 = pack2(k0, k0), K01 = pack2(k01, k01), HALF = pack2(0.5f, 0.5f);
+    const int step = f * p.Cb;                                  // one cell to the right
+    for (int phy = phy0; phy < phy0 + phys; ++phy) {
+      // first pixel of the run in this image row, and the part of the run the call asks for
+      const long long pix0 = (plane * H + static_cast<long long>(R) * f + phy) * W +
+                             static_cast<long long>(c0) * f - p.row0;
+      if (pix0 >= p.n_rows || pix0 + static_cast<long long>(n) * f <= 0) continue;
+      const bool whole = pix0 >= 0 && pix0 + static_cast<long long>(n) * f <= p.n_rows;
+      const float* tb = table + (static_cast<long long>(ycls0 + phy) * ncls + xcls0) * 9 * p.Cb + ch;
+      __nv_bfloat16* op = p.out + pix0 * p.Cb + ch;
+      for (int phx = 0; phx < f; ++phx) {
+        uint64_t wt[9];
 #pragma unroll
         for (int k = 0; k < 9; ++k) {
-          const uint2 t2 = __ldg(reinterpret_cast<const uint2*>(
-              base + (static_cast<long long>(rb + k / 3) * p.w + (cb + k % 3)) * p.Cb));
-          if (s2 == 0) {
-            ta[k][0] = pack2(bf16_lo(t2.x), bf16_hi(t2.x)); ta[k][1] = pack2(bf16_lo(t2.y), bf16_hi(t2.y));
-          } else {
-            tb[k][0] = pack2(bf16_lo(t2.x), bf16_hi(t2.x)); tb[k][1] = pack2(bf16_lo(t2.y), bf16_hi(t2.y));
+          const float2 w2 = __ldg(reinterpret_cast<const float2*>(tb));
+          wt[k] = pack2(w2.x, w2.y);
+          tb += p.Cb;
+        }
+        auto pixel = [&](int i) -> uint32_t {
+          uint64_t x = bias;
+#pragma unroll
+          for (int k = 0; k < 9; ++k) x = ffma2(wt[k], tk[k / 3][i + k % 3], x);
+          // tanh GELU, the polynomial part on packed fp32x2
+          const uint64_t u = fmul2(x, ffma2(fmul2(x, x), K01, K0));
+          float u0, u1, v0, v1;
+          unpack2(u, u0, u1);
+          const uint64_t hx = fmul2(x, HALF);
+          unpack2(ffma2(hx, pack2(fast_tanh(u0), fast_tanh(u1)), hx), v0, v1);
+          return pack_bf16(v0, v1);
+        };
+        __nv_bfloat16* q = op;
+        if (whole && n == COND_RUN) {          // straight-line: the cells' chains overlap
+#pragma unroll
+          for (int i = 0; i < COND_RUN; ++i) {
+            *reinterpret_cast<uint32_t*>(q) = pixel(i);
+            q += step;
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < COND_RUN; ++i) {
+            const long long pix = pix0 + i * f + phx;
+            if (i < n && pix >= 0 && pix < p.n_rows) *reinterpret_cast<uint32_t*>(q) = pixel(i);
+            q += step;
           }
         }
-        const long long pix0 = (plane * H + static_cast<long long>(R) * f) * W + static_cast<long long>(Cc) * f;
-        if (s2 == 0) pix_a = pix0; else pix_b = pix0;
-      }
-      if (pix_a < 0 && pix_b < 0) continue;
-      if (pix_a < 0) {
-#pragma unroll
-        for (int k = 0; k < 9; ++k) ta[k][0] = ta[k][1] = 0ull;
-      }
-      if (pix_b < 0) {
-#pragma unroll
-        for (int k = 0; k < 9; ++k) tb[k][0] = tb[k][1] = 0ull;
-      }
-      for (int phy = 0; phy < f; ++phy) {
-        for (int phx = 0; phx < f; ++phx) {
-          const float4* wv = reinterpret_cast<const float4*>(slab) + (phy * f + phx) * 72 + cq;
-          uint64_t a[2] = {pack2(bias.x, bias.y), pack2(bias.z, bias.w)};
-          uint64_t b[2] = {a[0], a[1]};
-#pragma unroll
-          for (int k = 0; k < 9; ++k) {
-            const float4 w4 = wv[k * 8];
-            const uint64_t w01 = pack2(w4.x, w4.y), w23 = pack2(w4.z, w4.w);
-            a[0] = ffma2(w01, ta[k][0], a[0]); a[1] = ffma2(w23, ta[k][1], a[1]);
-            b[0] = ffma2(w01, tb[k][0], b[0]); b[1] = ffma2(w23, tb[k][1], b[1]);
-          }
-          const long long off = static_cast<long long>(phy) * W + phx;
-          auto finish = [&](const uint64_t (&v2)[2], long long pix0) {
-            const long long pix = pix0 + off;
-            if (pix0 < 0 || pix < p.row0 || pix >= p.row0 + p.n_rows) return;
-            // tanh GELU, the polynomial part on packed fp32x2
-            const float k0 = 0.7978845608028654f, k01 = 0.7978845608028654f * 0.044715f;
-            const uint64_t K0 = pack2(k0, k0), K01 = pack2(k01, k01), HALF = pack2(0.5f, 0.5f);
-            float v[4];
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-              const uint64_t x = v2[j];
-              const uint64_t u = fmul2(x, ffma2(fmul2(x, x), K01, K0));
-              float u0, u1;
-              unpack2(u, u0, u1);
-              const uint64_t hx = fmul2(x, HALF);
-              unpack2(ffma2(hx, pack2(fast_tanh(u0), fast_tanh(u1)), hx), v[2 * j], v[2 * j + 1]);
-            }
-            uint2 o;
-            o.x = pack_bf16(v[0], v[1]);
-            o.y = pack_bf16(v[2], v[3]);
-            *reinterpret_cast<uint2*>(p.out + (pix - p.row0) * p.Cb + ch0) = o;
-          };
-          finish(a, pix_a);
-          finish(b, pix_b);
-        }
+        op += p.Cb;
       }
     }
   }
@@ -547,7 +454,7 @@ adaln_cond_interior_kernel(const AdalnCondParams p, const float* __restrict__ ta
 // Number of floats of the table the cell kernel needs, or 0 when the geometry takes the
 // direct kernel (small factor, wide conv kernel, channel count not a multiple of 32).
 inline long long adaln_cond_table_floats(int Cb, int factor, int ks) {
-  if (factor < 4 || factor > 8 || ks > 5 || Cb % 32 != 0) return 0;   // slab <= 72 KB of smem
+  if (factor < 4 || factor > 8 || ks > 5 || Cb % 32 != 0) return 0;
   return 9LL * factor * factor * 9 * Cb;
 }
 
@@ -571,30 +478,16 @@ inline int launch_adaln_cond(const AdalnCondParams& p, const float* table, int s
       adaln_cond_table_floats(p.Cb, p.factor, p.ks) > 0) {
     const long long W = static_cast<long long>(p.w) * p.factor;
     const long long cell_rows = (p.row0 + p.n_rows - 1) / W / p.factor - p.row0 / W / p.factor + 1;
-    const long long items =
-        (cell_rows * p.w + COND_CELLS_PER_ITEM - 1) / COND_CELLS_PER_ITEM * (p.Cb / 32);
-    long long blocks = items;
-    const long long cap = static_cast<long long>(sm_count) * 24;
+    const int groups = (p.Cb + 63) / 64;
+    long long warps = cell_rows * (2 + (p.w - 2 + COND_RUN - 1) / COND_RUN);
+    // 16 warps of this kernel fill an SM; below two such waves a run's phase rows go to separate warps
+    const int psplit = warps * groups < 32LL * sm_count ? p.factor : 1;
+    warps *= psplit;
+    long long blocks = (warps + 7) / 8;
+    const long long cap = (static_cast<long long>(sm_count) * 16 + groups - 1) / groups;
     if (blocks > cap) blocks = cap;
-    const int slab_bytes = p.factor * p.factor * 9 * 32 * 4;
-    if (slab_bytes > 48 * 1024) {
-      cudaError_t ea = cudaFuncSetAttribute(adaln_cond_interior_kernel,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, slab_bytes);
-      if (ea != cudaSuccess) return -static_cast<int>(ea) - 1000;
-    }
-    adaln_cond_interior_kernel<<<static_cast<int>(blocks), 256, slab_bytes, stream>>>(p, table, 0);
-    {
-      const long long H = static_cast<long long>(p.h) * p.factor;
-      const long long planes = (p.row0 + p.n_rows - 1) / (H * W) - p.row0 / (H * W) + 1;
-      // the first / last cell rows and columns (groups 1-4), then the four corners per plane
-      const long long edge = planes * ((p.w > p.h ? p.w : p.h) - 2);
-      long long be = (edge + COND_CELLS_PER_ITEM - 1) / COND_CELLS_PER_ITEM * (p.Cb / 32);
-      if (be > cap) be = cap;
-      adaln_cond_interior_kernel<<<dim3(static_cast<unsigned>(be), 4), 256, slab_bytes, stream>>>(p, table, 1);
-      long long bb = (planes * 4 + COND_BORDER_CELLS_PER_ITEM - 1) / COND_BORDER_CELLS_PER_ITEM * (p.Cb / 32);
-      if (bb > cap) bb = cap;
-      adaln_cond_border_kernel<<<static_cast<int>(bb), 256, 0, stream>>>(p, table);
-    }
+    blocks *= groups;
+    adaln_cond_runs_kernel<<<static_cast<int>(blocks), 256, 0, stream>>>(p, table, psplit);
   } else {
     const long long total = p.n_rows * (p.Cb / 8);
     long long blocks = (total + 255) / 256;
