@@ -150,6 +150,30 @@ def load() -> ctypes.CDLL:
     return lib
 
 
+class _Nothing:
+    def __enter__(self):
+        return None
+
+    def __exit__(self, *exc):
+        return False
+
+
+_NOTHING = _Nothing()
+
+
+def on_device(t):
+    """Context in which t's device is current; free when it already is (torch's own guard costs
+    3 us of a call that takes 10)."""
+    import torch
+    return _NOTHING if t.device.index == torch.cuda.current_device() else torch.cuda.device(t.device)
+
+
+def stream_of(t) -> int:
+    """Raw handle of the current stream of t's device."""
+    import torch
+    return torch._C._cuda_getCurrentRawStream(t.device.index)
+
+
 def exported_names() -> list[str]:
     return sorted(_SIGNATURES)
 

@@ -451,14 +451,8 @@ int strata_halo_gather_fields_f32(float* out, const void* const* h_peer_src, int
   const long long ocells = static_cast<long long>(tiles_per_rank) * P * P;
   if (cells * world > 0x7fffffffLL || ocells > 0x7fffffffLL || L > 0x7fffffffLL)
     return STRATA_ERR_ARG;
-  long long bx = (ocells + 255) / 256;
-  if (bx > 4096) bx = 4096;
-  long long by = L;
-  const long long want = static_cast<long long>(sms) * 16;  // enough CTAs for two waves
-  if (bx * by > want) by = (want + bx - 1) / bx;
-  if (by < 1) by = 1;
-  if (by > 65535) by = 65535;
-  dim3 grid(static_cast<unsigned>(bx), static_cast<unsigned>(by));
+  const long long bx = (ocells + 255) / 256;
+  dim3 grid(static_cast<unsigned>(bx), field_grid_y(L, FIELD_UL_COPY));
   halo_gather_fields_kernel<<<grid, 256, 0, as_stream(stream)>>>(
       out, pp, src_a, src_b, static_cast<int>(ocells), static_cast<int>(cells),
       static_cast<int>(L));
@@ -486,14 +480,8 @@ int strata_halo_gather_knn_fields_f32(float* out, const void* const* h_peer_src,
   const long long ocells = static_cast<long long>(tiles_per_rank) * P * P;
   if (cells * world > 0x7fffffffLL || ocells > 0x7fffffffLL || L > 0x7fffffffLL)
     return STRATA_ERR_ARG;
-  long long bx = (ocells + 255) / 256;
-  if (bx > 4096) bx = 4096;
-  long long by = L;
-  const long long want = static_cast<long long>(sms) * 16;
-  if (bx * by > want) by = (want + bx - 1) / bx;
-  if (by < 1) by = 1;
-  if (by > 65535) by = 65535;
-  dim3 grid(static_cast<unsigned>(bx), static_cast<unsigned>(by));
+  const long long bx = (ocells + 255) / 256;
+  dim3 grid(static_cast<unsigned>(bx), field_grid_y(L, FIELD_UL_KNN));
   cudaStream_t st = as_stream(stream);
   const int no = static_cast<int>(ocells), nc = static_cast<int>(cells), nl = static_cast<int>(L);
   switch (k) {
@@ -526,14 +514,8 @@ int strata_halo_adjoint_fields_f32(float* out, const void* const* h_peer_padded,
   const long long cells = static_cast<long long>(tiles_per_rank) * T * T;
   const long long pcells = static_cast<long long>(tiles_per_rank) * P * P;
   if (pcells * world > 0x7fffffffLL || L > 0x7fffffffLL) return STRATA_ERR_ARG;
-  long long bx = (cells + 255) / 256;
-  if (bx > 4096) bx = 4096;
-  long long by = L;
-  const long long want = static_cast<long long>(sms) * 16;
-  if (bx * by > want) by = (want + bx - 1) / bx;
-  if (by < 1) by = 1;
-  if (by > 65535) by = 65535;
-  dim3 grid(static_cast<unsigned>(bx), static_cast<unsigned>(by));
+  const long long bx = (cells + 255) / 256;
+  dim3 grid(static_cast<unsigned>(bx), field_grid_y(L, FIELD_UL_ADJ));
   halo_adjoint_fields_kernel<<<grid, 256, 0, as_stream(stream)>>>(
       out, pp, offsets, cell, coef, window, weights, static_cast<int>(cells),
       static_cast<int>(pcells), P * P, static_cast<int>(L));

@@ -123,44 +123,65 @@ halo_gather_tokens_kernel(__nv_bfloat16* __restrict__ out, const PeerPtrs src,
   }
 }
 
+// Field kernels: one thread per cell, FIELD_ROUNDS groups of UL consecutive leading indices (grid:
+// x over 256 cells, y over the leading index), a cell's index work done once for all of them.
+// Bound: HBM, through the bytes in flight - with a 4-byte access per thread it takes all of an
+// SM's threads and several loads each to cover ~1 us of latency at 6.5 TB/s (44 KB per SM); UL
+// independent loads stand before a thread's first use. Measured on 24 tiles of 64 x 64, halo 8, 512
+// leading indices (516 MB read + written), before -> now, four loads in flight and a walk over
+// the whole leading index before: copy 153 -> 99 us, 4 neighbours 291 -> 192, overlap-add
+// 365 -> 136 (its transposed 4-neighbour form 1578 -> 316). One round per block: copy 136, the index
+// loads then delay every group; UL 8 / 12 / 16: copy 99 / 101 / 104, 4 neighbours 230 / 228 / 192,
+// overlap-add 164 / 136 / 153.
+constexpr int FIELD_ROUNDS = 2;
+constexpr int FIELD_UL_COPY = 8, FIELD_UL_KNN = 16, FIELD_UL_ADJ = 12;
+inline unsigned field_grid_y(int64_t L, int ul) {
+  const int64_t per = static_cast<int64_t>(ul) * FIELD_ROUNDS;
+  return static_cast<unsigned>((L + per - 1) / per < 65535 ? (L + per - 1) / per : 65535);
+}
+
+// Pointer to a cell (global id, in the owning rank's memory).
+__device__ __forceinline__ const float* field_cell(const PeerPtrs& src, int id, int cells_per_rank) {
+  int rank = 0;
+  if (id >= cells_per_rank) {      // never taken on one rank
+    rank = id / cells_per_rank;
+    id -= rank * cells_per_rank;
+  }
+  return static_cast<const float*>(src.p[rank]) + id;
+}
+
 // Field layout: source buffers [L, tiles_per_rank*T*T] fp32 (L = product of leading dims),
-// output [L, tiles_per_rank*P*P]. grid: x over padded cells, y over leading index.
+// output [L, tiles_per_rank*P*P].
 __global__ void __launch_bounds__(256)
-halo_gather_fields_kernel(float* __restrict__ out, const PeerPtrs src,
+halo_gather_fields_kernel(float* __restrict__ out, const __grid_constant__ PeerPtrs src,
                           const int* __restrict__ src_a, const int* __restrict__ src_b,
                           int n_out_cells, int cells_per_rank, int L) {
+  const int oc = blockIdx.x * 256 + threadIdx.x;
+  if (oc >= n_out_cells) return;
   const bool failed = halo_exchange_failed();
-  for (int oc = blockIdx.x * blockDim.x + threadIdx.x; oc < n_out_cells;
-       oc += gridDim.x * blockDim.x) {
-    const int a = __ldg(src_a + oc);
-    const int b = __ldg(src_b + oc);
-    const int ra = a / cells_per_rank, la = a - ra * cells_per_rank;
-    const float* pa = static_cast<const float*>(src.p[ra]) + la;
-    const float* pb = nullptr;
+  const float* pa = field_cell(src, __ldg(src_a + oc), cells_per_rank);
+  const int b = __ldg(src_b + oc);
+  for (int l0 = blockIdx.y * FIELD_UL_COPY; l0 < L; l0 += gridDim.y * FIELD_UL_COPY) {
+    const float* qa = pa + static_cast<long long>(l0) * cells_per_rank;
+    float v[FIELD_UL_COPY];
+#pragma unroll
+    for (int u = 0; u < FIELD_UL_COPY; ++u) {
+      v[u] = l0 + u < L ? *qa : 0.f;
+      qa += cells_per_rank;
+    }
     if (b >= 0) {
-      const int rb = b / cells_per_rank, lb = b - rb * cells_per_rank;
-      pb = static_cast<const float*>(src.p[rb]) + lb;
-    }
-    constexpr int UL = 4;   // leading indices in flight per thread (independent loads)
-    int l = blockIdx.y;
-    for (; l + (UL - 1) * static_cast<int>(gridDim.y) < L; l += UL * gridDim.y) {
-      float v[UL];
+      const float* qb = field_cell(src, b, cells_per_rank) + static_cast<long long>(l0) * cells_per_rank;
 #pragma unroll
-      for (int u = 0; u < UL; ++u) {
-        const long long so = static_cast<long long>(l + u * gridDim.y) * cells_per_rank;
-        v[u] = pa[so];
-        if (pb) v[u] = (v[u] + pb[so]) / 2.0f;
+      for (int u = 0; u < FIELD_UL_COPY; ++u) {
+        if (l0 + u < L) v[u] = (v[u] + *qb) / 2.0f;
+        qb += cells_per_rank;
       }
-#pragma unroll
-      for (int u = 0; u < UL; ++u)
-        out[static_cast<long long>(l + u * gridDim.y) * n_out_cells + oc] =
-            failed ? __int_as_float(0x7fc00000) : v[u];
     }
-    for (; l < L; l += gridDim.y) {
-      const long long so = static_cast<long long>(l) * cells_per_rank;
-      float v = pa[so];
-      if (pb) v = (v + pb[so]) / 2.0f;
-      out[static_cast<long long>(l) * n_out_cells + oc] = failed ? __int_as_float(0x7fc00000) : v;
+    float* op = out + static_cast<long long>(l0) * n_out_cells + oc;
+#pragma unroll
+    for (int u = 0; u < FIELD_UL_COPY; ++u) {
+      if (l0 + u < L) *op = failed ? __int_as_float(0x7fc00000) : v[u];
+      op += n_out_cells;
     }
   }
 }
@@ -173,27 +194,36 @@ halo_gather_fields_kernel(float* __restrict__ out, const PeerPtrs src,
 // Source buffers [L, cells_per_rank] fp32 per rank; out [L, n_out_cells].
 template <int K>
 __global__ void __launch_bounds__(256)
-halo_gather_knn_fields_kernel(float* __restrict__ out, const PeerPtrs src,
+halo_gather_knn_fields_kernel(float* __restrict__ out, const __grid_constant__ PeerPtrs src,
                               const int* __restrict__ idx, const float* __restrict__ w,
                               int n_out_cells, int cells_per_rank, int L) {
+  const int oc = blockIdx.x * 256 + threadIdx.x;
+  if (oc >= n_out_cells) return;
   const bool failed = halo_exchange_failed();
-  for (int oc = blockIdx.x * blockDim.x + threadIdx.x; oc < n_out_cells;
-       oc += gridDim.x * blockDim.x) {
-    const float* sp[K];
-    float wk[K];
+  const float* sp[K];
+  float wk[K];
+#pragma unroll
+  for (int j = 0; j < K; ++j) {
+    sp[j] = field_cell(src, __ldg(idx + static_cast<long long>(oc) * K + j), cells_per_rank);
+    wk[j] = __ldg(w + static_cast<long long>(oc) * K + j);
+  }
+  for (int l0 = blockIdx.y * FIELD_UL_KNN; l0 < L; l0 += gridDim.y * FIELD_UL_KNN) {
+    float acc[FIELD_UL_KNN];
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-      const int id = __ldg(idx + static_cast<long long>(oc) * K + j);
-      const int rank = id / cells_per_rank;
-      sp[j] = static_cast<const float*>(src.p[rank]) + (id - rank * cells_per_rank);
-      wk[j] = __ldg(w + static_cast<long long>(oc) * K + j);
-    }
-    for (int l = blockIdx.y; l < L; l += gridDim.y) {
-      const long long so = static_cast<long long>(l) * cells_per_rank;
-      float acc = 0.f;
+      const float* q = sp[j] + static_cast<long long>(l0) * cells_per_rank;
 #pragma unroll
-      for (int j = 0; j < K; ++j) acc = __fadd_rn(acc, __fmul_rn(wk[j], sp[j][so]));
-      out[static_cast<long long>(l) * n_out_cells + oc] = failed ? __int_as_float(0x7fc00000) : acc;
+      for (int u = 0; u < FIELD_UL_KNN; ++u) {
+        const float t = __fmul_rn(wk[j], l0 + u < L ? *q : 0.f);
+        acc[u] = __fadd_rn(j == 0 ? 0.f : acc[u], t);
+        q += cells_per_rank;
+      }
+    }
+    float* op = out + static_cast<long long>(l0) * n_out_cells + oc;
+#pragma unroll
+    for (int u = 0; u < FIELD_UL_KNN; ++u) {
+      if (l0 + u < L) *op = failed ? __int_as_float(0x7fc00000) : acc[u];
+      op += n_out_cells;
     }
   }
 }
@@ -207,76 +237,42 @@ halo_gather_knn_fields_kernel(float* __restrict__ out, const PeerPtrs src,
 // the result is bit-identical to the same loop on the host for normal-range values (the library
 // is built with flush-to-zero, so a denormal operand or result is zero here and not there).
 // Padded sources: [L, tiles_per_rank*P*P] fp32 per rank; out [L, tiles_per_rank*T*T].
+// An entry is worked out once per UL leading indices, whatever the length of a cell's list.
 __global__ void __launch_bounds__(256)
-halo_adjoint_fields_kernel(float* __restrict__ out, const PeerPtrs src,
+halo_adjoint_fields_kernel(float* __restrict__ out, const __grid_constant__ PeerPtrs src,
                            const int* __restrict__ offsets, const int* __restrict__ cell,
                            const float* __restrict__ coef, const float* __restrict__ window,
                            const float* __restrict__ weights, int n_cells,
                            int padded_cells_per_rank, int PP, int L) {
+  const int c = blockIdx.x * 256 + threadIdx.x;
+  if (c >= n_cells) return;
   const bool failed = halo_exchange_failed();
-  for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n_cells; c += gridDim.x * blockDim.x) {
-    const int e0 = __ldg(offsets + c), e1 = __ldg(offsets + c + 1);
-    // (after a failed barrier the divisor is NaN, and with it every output)
-    const float wsum = failed ? __int_as_float(0x7fc00000) : __ldg(weights + c);
-    // with the copy halo's coefficients (1 or 1/2) coef * (window * y) == (coef * window) * y bit
-    // for bit, so the per-entry factor and source pointer are set up once, outside the loop over
-    // the leading index (general coefficients - the k-nearest-neighbour lists - agree with the
-    // long-list branch below to rounding only)
-    constexpr int FAST = 4;
-    const int ne = e1 - e0;
-    if (ne <= FAST) {
-      const float* sp[FAST];
-      float wc[FAST];
+  const int e0 = __ldg(offsets + c), e1 = __ldg(offsets + c + 1);
+  // (after a failed barrier the divisor is NaN, and with it every output)
+  const float wsum = failed ? __int_as_float(0x7fc00000) : __ldg(weights + c);
+  for (int l0 = blockIdx.y * FIELD_UL_ADJ; l0 < L; l0 += gridDim.y * FIELD_UL_ADJ) {
+    float acc[FIELD_UL_ADJ];
 #pragma unroll
-      for (int j = 0; j < FAST; ++j) {
-        const int e = e0 + (j < ne ? j : 0);
-        const int p = __ldg(cell + e);
-        const int rank = p / padded_cells_per_rank;
-        const int local = p - rank * padded_cells_per_rank;
-        sp[j] = static_cast<const float*>(src.p[rank]) + local;
-        wc[j] = j < ne ? __fmul_rn(__ldg(coef + e), __ldg(window + local % PP)) : 0.f;
+    for (int u = 0; u < FIELD_UL_ADJ; ++u) acc[u] = 0.f;
+    for (int e = e0; e < e1; ++e) {
+      const int p = __ldg(cell + e);
+      const float cf = __ldg(coef + e), wn = __ldg(window + p % PP);
+      const float* q = field_cell(src, p, padded_cells_per_rank) +
+                       static_cast<long long>(l0) * padded_cells_per_rank;
+      float y[FIELD_UL_ADJ];
+#pragma unroll
+      for (int u = 0; u < FIELD_UL_ADJ; ++u) {
+        y[u] = l0 + u < L ? *q : 0.f;
+        q += padded_cells_per_rank;
       }
-      constexpr int UL = 4;   // leading indices in flight per thread (independent loads)
-      int l = blockIdx.y;
-      for (; l + (UL - 1) * static_cast<int>(gridDim.y) < L; l += UL * gridDim.y) {
-        float y[UL][FAST];
 #pragma unroll
-        for (int u = 0; u < UL; ++u) {
-          const long long so = static_cast<long long>(l + u * gridDim.y) * padded_cells_per_rank;
+      for (int u = 0; u < FIELD_UL_ADJ; ++u) acc[u] = __fadd_rn(acc[u], __fmul_rn(cf, __fmul_rn(wn, y[u])));
+    }
+    float* op = out + static_cast<long long>(l0) * n_cells + c;
 #pragma unroll
-          for (int j = 0; j < FAST; ++j) y[u][j] = j < ne ? sp[j][so] : 0.f;
-        }
-#pragma unroll
-        for (int u = 0; u < UL; ++u) {
-          float acc = 0.f;
-#pragma unroll
-          for (int j = 0; j < FAST; ++j)
-            if (j < ne) acc = __fadd_rn(acc, __fmul_rn(wc[j], y[u][j]));
-          out[static_cast<long long>(l + u * gridDim.y) * n_cells + c] = __fdiv_rn(acc, wsum);
-        }
-      }
-      for (; l < L; l += gridDim.y) {
-        const long long so = static_cast<long long>(l) * padded_cells_per_rank;
-        float acc = 0.f;
-#pragma unroll
-        for (int j = 0; j < FAST; ++j)
-          if (j < ne) acc = __fadd_rn(acc, __fmul_rn(wc[j], sp[j][so]));
-        out[static_cast<long long>(l) * n_cells + c] = __fdiv_rn(acc, wsum);
-      }
-    } else {
-      for (int l = blockIdx.y; l < L; l += gridDim.y) {
-        const long long so = static_cast<long long>(l) * padded_cells_per_rank;
-        float acc = 0.f;
-        for (int e = e0; e < e1; ++e) {
-          const int p = __ldg(cell + e);
-          const int rank = p / padded_cells_per_rank;
-          const int local = p - rank * padded_cells_per_rank;
-          const float y = static_cast<const float*>(src.p[rank])[so + local];
-          const float wy = __fmul_rn(__ldg(window + local % PP), y);
-          acc = __fadd_rn(acc, __fmul_rn(__ldg(coef + e), wy));
-        }
-        out[static_cast<long long>(l) * n_cells + c] = __fdiv_rn(acc, wsum);
-      }
+    for (int u = 0; u < FIELD_UL_ADJ; ++u) {
+      if (l0 + u < L) *op = __fdiv_rn(acc[u], wsum);
+      op += n_cells;
     }
   }
 }

@@ -22,6 +22,7 @@ as device status 105 (`check_status`).
 from __future__ import annotations
 
 import ctypes
+import math
 
 import numpy as np
 import torch
@@ -152,14 +153,13 @@ class DistributedTileCopyHaloPadding(torch.nn.Module):
         self._shared = PeerSharedBuffer(self.FLAG_BYTES + 2 * slot, group=self.group)
         self._epoch = 0
 
-    def _publish_and_sync(self, x_flat_bytes: torch.Tensor):
-        """Copy this rank's tiles into the current slot, run the flag barrier; returns the
-        per-rank source pointer array for the gather."""
+    def _publish_and_sync(self, x: torch.Tensor):
+        """Copy this rank's tiles (contiguous) into the current slot, run the flag barrier; returns
+        the per-rank source pointer array for the gather."""
         topo = self.topology
         if topo.world_size == 1:
-            arr = (ctypes.c_void_p * 1)()
-            arr[0] = x_flat_bytes.data_ptr()
-            return arr
+            return (ctypes.c_void_p * 1)(x.data_ptr())
+        x_flat_bytes = x.view(-1).view(torch.uint8)
         # The two alternating slots are safe only while every exchange through this module (the
         # un-pad adjoint shares its buffer) is issued on ONE stream, in the same order on all
         # ranks: a second stream could overwrite a slot a peer is still reading.
@@ -206,17 +206,17 @@ class DistributedTileCopyHaloPadding(torch.nn.Module):
         if x.dtype != torch.float32:
             raise TypeError(f"field-space halo exchange is float32, got {x.dtype}")
         P = topo.padded_tile_size
-        L = int(np.prod(shape)) if shape else 1
+        L = math.prod(shape)
         xc = x.contiguous()
         out = torch.empty(*shape, tpr, P, P, dtype=x.dtype, device=x.device)
         if L == 0:
             return out
-        with torch.cuda.device(x.device):
-            src = self._publish_and_sync(xc.view(-1).view(torch.uint8))
+        with _lib.on_device(x):
+            src = self._publish_and_sync(xc)
             _lib.check(_lib.load().strata_halo_gather_fields_f32(
                 out.data_ptr(), src, topo.world_size, self.src_a.data_ptr(), self.src_b.data_ptr(),
-                tpr, topo.tile_size, topo.halo_width, L,
-                torch.cuda.current_stream().cuda_stream), "strata_halo_gather_fields_f32")
+                tpr, topo.tile_size, topo.halo_width, L, _lib.stream_of(x)),
+                "strata_halo_gather_fields_f32")
         return out
 
     # ---------------------------------------------------------------- token space
@@ -237,8 +237,8 @@ class DistributedTileCopyHaloPadding(torch.nn.Module):
                 raise ValueError("only_halo needs a preallocated `out` holding the interiors")
             out = torch.empty(topo.tiles_per_rank, depth, P * P, C, dtype=torch.bfloat16,
                               device=tokens.device)
-        with torch.cuda.device(tokens.device):
-            src = self._publish_and_sync(tc.view(-1).view(torch.uint8))
+        with _lib.on_device(tokens):
+            src = self._publish_and_sync(tc)
             _lib.check(_lib.load().strata_halo_gather_tokens_bf16(
                 out.data_ptr(), src, topo.world_size, self.src_a.data_ptr(), self.src_b.data_ptr(),
                 topo.tiles_per_rank, depth, T, topo.halo_width, C, 1 if only_halo else 0,
@@ -308,17 +308,17 @@ class DistributedTileKNNHaloPadding(DistributedTileCopyHaloPadding):
         if x.dtype != torch.float32:
             raise TypeError(f"field-space halo exchange is float32, got {x.dtype}")
         P = topo.padded_tile_size
-        L = int(np.prod(shape)) if shape else 1
+        L = math.prod(shape)
         out = torch.empty(*shape, tpr, P, P, dtype=x.dtype, device=x.device)
         if L == 0:
             return out
         xc = x.contiguous()
-        with torch.cuda.device(x.device):
-            src = self._publish_and_sync(xc.view(-1).view(torch.uint8))
+        with _lib.on_device(x):
+            src = self._publish_and_sync(xc)
             _lib.check(_lib.load().strata_halo_gather_knn_fields_f32(
                 out.data_ptr(), src, topo.world_size, self.knn_idx.data_ptr(),
                 self.knn_weights.data_ptr(), self.k, tpr, topo.tile_size, topo.halo_width, L,
-                torch.cuda.current_stream().cuda_stream), "strata_halo_gather_knn_fields_f32")
+                _lib.stream_of(x)), "strata_halo_gather_knn_fields_f32")
         return out
 
 class DistributedTilePlanHaloPadding(DistributedTileKNNHaloPadding):
@@ -411,18 +411,17 @@ class NormalizedCopyHaloAdjoint(torch.nn.Module):
             raise _lib.StrataLibraryError("halo adjoint needs CUDA tensors (no CPU path)")
         if padded.dtype != torch.float32:
             raise TypeError(f"field-space halo adjoint is float32, got {padded.dtype}")
-        L = int(np.prod(shape)) if shape else 1
+        L = math.prod(shape)
         out = torch.empty(*shape, tpr, T, T, dtype=padded.dtype, device=padded.device)
         if L == 0:
             return out
         pc = padded.contiguous()
-        with torch.cuda.device(padded.device):
-            src = self.halo_exchange._publish_and_sync(pc.view(-1).view(torch.uint8))
+        with _lib.on_device(padded):
+            src = self.halo_exchange._publish_and_sync(pc)
             _lib.check(_lib.load().strata_halo_adjoint_fields_f32(
                 out.data_ptr(), src, topo.world_size, self._offsets.data_ptr(), self._cell.data_ptr(),
                 self._coef.data_ptr(), self.window.data_ptr(), self.weights.data_ptr(), tpr, T,
-                topo.halo_width, L, torch.cuda.current_stream().cuda_stream),
-                "strata_halo_adjoint_fields_f32")
+                topo.halo_width, L, _lib.stream_of(padded)), "strata_halo_adjoint_fields_f32")
         return out
 
 

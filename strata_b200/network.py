@@ -209,9 +209,9 @@ class NetworkHandle:
                              f"{backbone.patch_size})")
         out = torch.empty((B, backbone.out_channels, D, H, W), dtype=torch.float32, device=x.device)
         ws = torch.empty(max(need, 256), dtype=torch.uint8, device=x.device)
-        with torch.cuda.device(x.device):
+        with _lib.on_device(x):
             _lib.check(lib.strata_network_forward_f32(
                 dref, pref, x.data_ptr(), lat.data_ptr(), lon.data_ptr(), B, D, H, W, out.data_ptr(),
-                ws.data_ptr(), need, torch.cuda.current_stream().cuda_stream),
+                ws.data_ptr(), need, _lib.stream_of(x)),
                 "strata_network_forward_f32")
         return out

@@ -17,8 +17,7 @@ EPI_RESIDUAL = 2
 EPI_GATE = 4
 
 
-def _stream_ptr(t: torch.Tensor) -> int:
-    return torch.cuda.current_stream(t.device).cuda_stream
+_stream_ptr = _lib.stream_of
 
 
 def _require_cuda_bf16(t: torch.Tensor, name: str) -> None:
@@ -72,7 +71,7 @@ def layernorm(x: torch.Tensor, eps: float = 1e-6) -> torch.Tensor:
     _require_cuda_bf16(x, "x")
     x2, M, C, ld = _as_rows(x, "x")
     y = torch.empty((M, C), dtype=torch.bfloat16, device=x.device)
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x):
         _lib.check(_lib.load().strata_layernorm_bf16(x2.data_ptr(), ld, y.data_ptr(), C, M, C,
                                                      float(eps), _stream_ptr(x)),
                    "strata_layernorm_bf16")
@@ -106,7 +105,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
         _require_cuda_bf16(out, "out")
         if out.shape != (M, N) or out.stride(1) != 1:
             raise ValueError("out must be [M, N] with unit inner stride")
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x):
         _lib.check(_lib.load().strata_linear_bf16(
             x2.data_ptr(), ldx, w.data_ptr(), w.stride(0),
             None if bias is None else bias.data_ptr(), out.data_ptr(), out.stride(0), M, N, K,
@@ -131,7 +130,7 @@ def qkv_rope(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None, h
     n_tiles = M // max(tokens_per_tile, 1)
     cs = _rope_cs(rope_cos, rope_sin, rope_cs, (n_tiles, hw, head_dim // 2), x.device)
     out = torch.empty((M, 3 * C), dtype=torch.bfloat16, device=x.device)
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x):
         _lib.check(_lib.load().strata_qkv_rope_bf16(
             x2.data_ptr(), ldx, w.data_ptr(), w.stride(0),
             None if bias is None else bias.data_ptr(), out.data_ptr(), 3 * C, M, C, head_dim,
@@ -167,7 +166,7 @@ def na3d(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, kernel, scale: float
     if out is None:
         out = torch.empty((B, D, H, W, nh, hd), dtype=torch.bfloat16, device=q.device)
     ldo = _token_major(out, "out")
-    with torch.cuda.device(q.device):
+    with _lib.on_device(q):
         _lib.check(_lib.load().strata_na3d_fwd_bf16(
             q.data_ptr(), ldq, k.data_ptr(), ldk, v.data_ptr(), ldv, out.data_ptr(), ldo,
             B, D, H, W, nh, hd, kd, kh, kw, float(scale) if scale else 0.0, _stream_ptr(q)),
@@ -225,7 +224,7 @@ def block_forward(x: torch.Tensor, weights: dict, *, grid, num_heads: int, kerne
         setattr(wstruct, f"b_{name}", None if b is None else b.data_ptr())
     cs = _rope_cs(rope_cos, rope_sin, rope_cs, (n_tiles, H * W, (C // num_heads) // 2), x.device)
     import ctypes
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x):
         _lib.check(_lib.load().strata_block_forward_bf16(
             x.data_ptr(), out.data_ptr(), n_tiles, D, H, W, C, num_heads, hidden, kd, kh, kw,
             ctypes.byref(wstruct), None if cs is None else cs.data_ptr(),
@@ -252,7 +251,7 @@ def qkv_rope_padded(x: torch.Tensor, weight: torch.Tensor, bias, head_dim: int,
     w = weight if weight.stride(1) == 1 else weight.contiguous()
     bias = _f32_or_none(bias, "bias")
     cs = _rope_cs(None, None, rope_cs, (n_tiles, hw, head_dim // 2), x.device)
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x):
         _lib.check(_lib.load().strata_qkv_rope_padded_bf16(
             x2.data_ptr(), ldx, w.data_ptr(), w.stride(0),
             None if bias is None else bias.data_ptr(), out.data_ptr(), out.stride(0), M, C, head_dim,
@@ -283,7 +282,7 @@ def na3d_region(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, kernel, regio
         oh0, Ho, ow0, Wo = (int(t) for t in out_window)
         if tuple(out.shape) != (B, D, Ho, Wo, nh, hd) or not out.is_contiguous():
             raise ValueError("out must be a contiguous [B, D, Ho, Wo, heads, 64] tensor")
-    with torch.cuda.device(q.device):
+    with _lib.on_device(q):
         _lib.check(_lib.load().strata_na3d_fwd_region_bf16(
             q.data_ptr(), ldq, k.data_ptr(), ldk, v.data_ptr(), ldv, out.data_ptr(), nh * hd,
             B, D, H, W, nh, hd, kd, kh, kw, float(scale) if scale else 0.0, h0, Hq, w0, Wq,
@@ -326,7 +325,7 @@ def preprocess_patches(x: torch.Tensor, lat, lon, lat0=None, lon0=None, wind=Non
         raise ValueError(f"grid {(D, H, W)} is not divisible by the patch {(pv, ph, pw)}")
     a = torch.empty(B * (D // pv) * (H // ph) * (W // pw), Kp, dtype=torch.bfloat16, device=x.device)
     p = lambda t: None if t is None else t.data_ptr()
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x):
         _lib.check(_lib.load().strata_preprocess_patches_bf16(
             x.data_ptr(), B, C, D, H, W, p(lat), p(lon), p(lat0), p(lon0), u, v,
             1 if concat_lat else 0, pv, ph, pw, a.data_ptr(), Kp, _stream_ptr(x)),
@@ -354,7 +353,7 @@ def postprocess_fields(y: torch.Tensor, shape, lat=None, lon=None, lat0=None, lo
     lon0 = None if lon0 is None else _f32_dev(lon0.reshape(-1), "lon0", (B,))
     out = torch.empty(B, C, D, H, W, dtype=torch.float32, device=y.device)
     p = lambda t: None if t is None else t.data_ptr()
-    with torch.cuda.device(y.device):
+    with _lib.on_device(y):
         _lib.check(_lib.load().strata_postprocess_fields_f32(
             y.data_ptr(), y.stride(0), B, C, D, H, W, p(lat), p(lon), p(lat0), p(lon0), u, v,
             pv, ph, pw, out.data_ptr(), _stream_ptr(y)), "strata_postprocess_fields_f32")
@@ -394,7 +393,7 @@ def tile_tables(lat: torch.Tensor, lon: torch.Tensor, *, centre: bool = False, r
     need = int(lib.strata_tile_tables_workspace_bytes(B, H, W))
     ws = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
     p = lambda t: None if t is None else t.data_ptr()
-    with torch.cuda.device(dev):
+    with _lib.on_device(lat):
         _lib.check(lib.strata_tile_tables(lat.data_ptr(), lon.data_ptr(), B, H, W, p(lat0), p(lon0), mode,
                                           int(patch), float(length_scale), float(rope_base), int(head_dim),
                                           p(cs), p(ws), need, _stream_ptr(lat)), "strata_tile_tables")
@@ -433,7 +432,7 @@ def adaln_rows(x: torch.Tensor, *, y: torch.Tensor | None = None, gate: torch.Te
     if sp is not None and lds != ldc:
         raise ValueError("shift and scale must share a row stride")
     out = torch.empty((M, C), dtype=torch.bfloat16, device=x.device) if norm else None
-    with torch.cuda.device(x.device):
+    with _lib.on_device(x):
         _lib.check(_lib.load().strata_adaln_rows_bf16(
             x.data_ptr(), x.stride(0), yp, ldy, gp, ldg, x.data_ptr() if yp else None, x.stride(0),
             sp, cp, lds, None if out is None else out.data_ptr(), C, M, C, float(eps),
@@ -446,7 +445,7 @@ def qk_norm_rows_(qkv: torch.Tensor, C: int, eps: float = 1e-6) -> torch.Tensor:
     _require_cuda_bf16(qkv, "qkv")
     if qkv.dim() != 2 or qkv.shape[1] != 3 * C or qkv.stride(1) != 1:
         raise ValueError(f"qkv must be [M, {3 * C}] rows")
-    with torch.cuda.device(qkv.device):
+    with _lib.on_device(qkv):
         _lib.check(_lib.load().strata_qk_norm_rows_bf16(
             qkv.data_ptr(), qkv.stride(0), qkv.shape[0], int(C), float(eps), _stream_ptr(qkv)),
             "strata_qk_norm_rows_bf16")
@@ -479,7 +478,7 @@ def adaln_cond(tokens: torch.Tensor, w_dw: torch.Tensor, b_dw: torch.Tensor | No
     lib = _lib.load()
     n_table = 0 if direct else int(lib.strata_adaln_cond_table_floats(Cb, int(factor), ks))
     table = torch.empty(n_table, dtype=torch.float32, device=tokens.device) if n_table else None
-    with torch.cuda.device(tokens.device):
+    with _lib.on_device(tokens):
         _lib.check(lib.strata_adaln_cond_bf16(
             tokens.data_ptr(), B, D, h, w, Cb, int(factor), w_dw.data_ptr(),
             None if b_dw is None else b_dw.data_ptr(), ks, int(row0), int(n_rows), out.data_ptr(),
@@ -503,7 +502,7 @@ def dealias_patches(x_rows: torch.Tensor, shape, channels: int, patch, taps, k_p
     tokens = B * (D // pv) * (H // ph) * (W // pw)
     a = torch.empty((tokens, k_pad), dtype=torch.bfloat16, device=x_rows.device)
     t = (ctypes.c_float * len(taps))(*[float(v) for v in taps])
-    with torch.cuda.device(x_rows.device):
+    with _lib.on_device(x_rows):
         _lib.check(_lib.load().strata_dealias_patches_bf16(
             x_rows.data_ptr(), x_rows.stride(0), B, int(channels), D, H, W, pv, ph, pw,
             ctypes.cast(t, ctypes.c_void_p), len(taps), a.data_ptr(), k_pad, _stream_ptr(x_rows)),
