@@ -357,10 +357,11 @@ static int prepost_check(int B, int C, int D, int H, int W, int pv, int ph, int 
   return STRATA_OK;
 }
 
-int strata_preprocess_patches_bf16(const float* x, int B, int C_in, int D, int H, int W,
-                                   const float* lat, const float* lon, const float* lat0,
-                                   const float* lon0, int u_idx, int v_idx, int concat_lat, int pv,
-                                   int ph, int pw, void* a, int64_t lda, void* stream) {
+// (px_rot, px_lat: per-pixel geometry of tile_tables_kernel, or null)
+static int preprocess_impl(const float* x, int B, int C_in, int D, int H, int W, const float* lat,
+                           const float* lon, const float* lat0, const float* lon0, int u_idx,
+                           int v_idx, int concat_lat, int pv, int ph, int pw, void* a, int64_t lda,
+                           const float4* px_rot, const float2* px_lat, void* stream) {
   const int sms = current_sm_count();
   if (sms <= 0) return STRATA_ERR_NO_DEVICE;
   int r = prepost_check(B, C_in, D, H, W, pv, ph, pw, lat, lon, lat0, lon0, u_idx, v_idx, concat_lat);
@@ -370,12 +371,69 @@ int strata_preprocess_patches_bf16(const float* x, int B, int C_in, int D, int H
   if (lda < K) return STRATA_ERR_ARG;
   if (B == 0) return STRATA_OK;
   PrePostParams p{B, C_in, D, H, W, pv, ph, pw, u_idx < 0 ? -1 : u_idx, u_idx < 0 ? -1 : v_idx,
-                  concat_lat ? 1 : 0, lat, lon, lat0, lon0, lda};
-  const long long npix = static_cast<long long>(B) * H * W;
-  long long blocks = (npix + 255) / 256;
-  if (blocks > static_cast<long long>(sms) * 16) blocks = static_cast<long long>(sms) * 16;
-  preprocess_patches_kernel<<<static_cast<unsigned>(blocks), 256, 0, as_stream(stream)>>>(
+                  concat_lat ? 1 : 0, lat, lon, lat0, lon0, lda, 0, 0, 0, 0, 0, px_rot, px_lat};
+  if (pv == 1 && ph == 1 && pw == 1 && lda % 8 == 0 && aligned16(a)) {
+    const dim3 grid = pixels_grid(p, sms);
+    preprocess_pixels_kernel<<<grid, PREPOST_THREADS, 0, as_stream(stream)>>>(
+        x, static_cast<__nv_bfloat16*>(a), p);
+    const cudaError_t e1 = cudaGetLastError();
+    return e1 == cudaSuccess ? 0 : -static_cast<int>(e1) - 1000;
+  }
+  const int v = !aligned16(x) ? 1 : pw % 4 == 0 && W % 4 == 0 ? 4 : pw % 2 == 0 && W % 2 == 0 ? 2 : 1;
+  long long blocks;
+  int smem;
+  if (prepost_plan(p, pv * ph * pw, C_in + (concat_lat ? 2 : 0), v == 4 ? 8 : 4, concat_lat != 0, sms,
+                   &blocks, &smem) != 0)
+    return STRATA_ERR_UNSUPPORTED;
+  auto kern = v == 4 ? preprocess_patches_kernel<4> : v == 2 ? preprocess_patches_kernel<2> : preprocess_patches_kernel<1>;
+  if (smem > 48 * 1024) {
+    const cudaError_t ea = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (ea != cudaSuccess) return -static_cast<int>(ea) - 1000;
+  }
+  kern<<<static_cast<unsigned>(blocks), PREPOST_THREADS, smem, as_stream(stream)>>>(
       x, static_cast<__nv_bfloat16*>(a), p);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
+}
+
+int strata_preprocess_patches_bf16(const float* x, int B, int C_in, int D, int H, int W,
+                                   const float* lat, const float* lon, const float* lat0,
+                                   const float* lon0, int u_idx, int v_idx, int concat_lat, int pv,
+                                   int ph, int pw, void* a, int64_t lda, void* stream) {
+  return preprocess_impl(x, B, C_in, D, H, W, lat, lon, lat0, lon0, u_idx, v_idx, concat_lat, pv, ph, pw, a,
+                         lda, nullptr, nullptr, stream);
+}
+
+static int postprocess_impl(const void* y, int64_t ldy, int B, int C_out, int D, int H, int W,
+                            const float* lat, const float* lon, const float* lat0, const float* lon0,
+                            int u_idx, int v_idx, int pv, int ph, int pw, float* out,
+                            const float4* px_rot, void* stream) {
+  const int sms = current_sm_count();
+  if (sms <= 0) return STRATA_ERR_NO_DEVICE;
+  int r = prepost_check(B, C_out, D, H, W, pv, ph, pw, lat, lon, lat0, lon0, u_idx, v_idx, 0);
+  if (r != STRATA_OK) return r;
+  if (!y || !out || ldy < static_cast<long long>(C_out) * pv * ph * pw) return STRATA_ERR_ARG;
+  if (B == 0) return STRATA_OK;
+  PrePostParams p{B, C_out, D, H, W, pv, ph, pw, u_idx < 0 ? -1 : u_idx, u_idx < 0 ? -1 : v_idx, 0,
+                  lat, lon, lat0, lon0, ldy, 0, 0, 0, 0, 0, px_rot, nullptr};
+  if (pv == 1 && ph == 1 && pw == 1 && ldy % 8 == 0 && aligned16(y)) {
+    const dim3 grid = pixels_grid(p, sms);
+    postprocess_pixels_kernel<<<grid, PREPOST_THREADS, 0, as_stream(stream)>>>(
+        static_cast<const __nv_bfloat16*>(y), out, p);
+    const cudaError_t e1 = cudaGetLastError();
+    return e1 == cudaSuccess ? 0 : -static_cast<int>(e1) - 1000;
+  }
+  const int v = !aligned16(out) ? 1 : pw % 4 == 0 && W % 4 == 0 ? 4 : pw % 2 == 0 && W % 2 == 0 ? 2 : 1;
+  long long blocks;
+  int smem;
+  if (prepost_plan(p, pw * C_out, pv * ph, 4, false, sms, &blocks, &smem) != 0) return STRATA_ERR_UNSUPPORTED;
+  auto kern = v == 4 ? postprocess_fields_kernel<4> : v == 2 ? postprocess_fields_kernel<2> : postprocess_fields_kernel<1>;
+  if (smem > 48 * 1024) {
+    const cudaError_t ea = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (ea != cudaSuccess) return -static_cast<int>(ea) - 1000;
+  }
+  kern<<<static_cast<unsigned>(blocks), PREPOST_THREADS, smem, as_stream(stream)>>>(
+      static_cast<const __nv_bfloat16*>(y), out, p);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
 }
@@ -384,21 +442,8 @@ int strata_postprocess_fields_f32(const void* y, int64_t ldy, int B, int C_out, 
                                   const float* lat, const float* lon, const float* lat0,
                                   const float* lon0, int u_idx, int v_idx, int pv, int ph, int pw,
                                   float* out, void* stream) {
-  const int sms = current_sm_count();
-  if (sms <= 0) return STRATA_ERR_NO_DEVICE;
-  int r = prepost_check(B, C_out, D, H, W, pv, ph, pw, lat, lon, lat0, lon0, u_idx, v_idx, 0);
-  if (r != STRATA_OK) return r;
-  if (!y || !out || ldy < static_cast<long long>(C_out) * pv * ph * pw) return STRATA_ERR_ARG;
-  if (B == 0) return STRATA_OK;
-  PrePostParams p{B, C_out, D, H, W, pv, ph, pw, u_idx < 0 ? -1 : u_idx, u_idx < 0 ? -1 : v_idx, 0,
-                  lat, lon, lat0, lon0, ldy};
-  const long long npix = static_cast<long long>(B) * H * W;
-  long long blocks = (npix + 255) / 256;
-  if (blocks > static_cast<long long>(sms) * 16) blocks = static_cast<long long>(sms) * 16;
-  postprocess_fields_kernel<<<static_cast<unsigned>(blocks), 256, 0, as_stream(stream)>>>(
-      static_cast<const __nv_bfloat16*>(y), out, p);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
+  return postprocess_impl(y, ldy, B, C_out, D, H, W, lat, lon, lat0, lon0, u_idx, v_idx, pv, ph, pw, out,
+                          nullptr, stream);
 }
 
 int strata_halo_gather_tokens_bf16(void* out, const void* const* h_peer_src, int world,
@@ -702,10 +747,11 @@ int64_t strata_tile_tables_workspace_bytes(int B, int H, int W) {
   return tile_tables_ws_bytes(B, H, W);
 }
 
-int strata_tile_tables(const float* lat, const float* lon, int B, int H, int W, float* lat0,
-                       float* lon0, int rope_mode, int patch, double length_scale, double rope_base,
-                       int head_dim, void* rope_cs, void* workspace, int64_t workspace_bytes,
-                       void* stream) {
+static int tile_tables_impl(const float* lat, const float* lon, int B, int H, int W, float* lat0,
+                            float* lon0, int rope_mode, int patch, double length_scale,
+                            double rope_base, int head_dim, void* rope_cs, void* workspace,
+                            int64_t workspace_bytes, float4* px_fwd, float4* px_inv, float2* px_lat,
+                            void* stream) {
   if (current_sm_count() <= 0) return STRATA_ERR_NO_DEVICE;
   if (B < 0 || B > 65535 || H <= 0 || W <= 0 || static_cast<int64_t>(H) * W > 0x7fffffffLL)
     return STRATA_ERR_ARG;
@@ -720,8 +766,9 @@ int strata_tile_tables(const float* lat, const float* lon, int B, int H, int W, 
   const int64_t need = tile_tables_ws_bytes(B, H, W);
   if (sums && need > 0 && (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 7u)))
     return STRATA_ERR_ARG;
-  if (B == 0 || (!sums && rope_mode == STRATA_ROPE_NONE)) return STRATA_OK;
+  if (B == 0 || (!sums && rope_mode == STRATA_ROPE_NONE && !px_lat)) return STRATA_OK;
   TileTablesParams p{};
+  p.px_fwd = px_fwd; p.px_inv = px_inv; p.px_lat = px_lat;
   p.lat = lat; p.lon = lon; p.H = H; p.W = W;
   p.mode = rope_mode;
   p.lat0 = lat0; p.lon0 = lon0;
@@ -734,6 +781,14 @@ int strata_tile_tables(const float* lat, const float* lon, int B, int H, int W, 
     p.table = static_cast<uint32_t*>(rope_cs);
   }
   return launch_tile_tables(p, B, static_cast<double*>(workspace), as_stream(stream));
+}
+
+int strata_tile_tables(const float* lat, const float* lon, int B, int H, int W, float* lat0,
+                       float* lon0, int rope_mode, int patch, double length_scale, double rope_base,
+                       int head_dim, void* rope_cs, void* workspace, int64_t workspace_bytes,
+                       void* stream) {
+  return tile_tables_impl(lat, lon, B, H, W, lat0, lon0, rope_mode, patch, length_scale, rope_base, head_dim,
+                          rope_cs, workspace, workspace_bytes, nullptr, nullptr, nullptr, stream);
 }
 
 // (the stencil table ready, or null)

@@ -4,19 +4,21 @@
 //   tile_sums_kernel   partial sums over a tile's pixels (latitude, longitude circle, unit
 //                      vector); only launched when a tile has more pixels than one block of the
 //                      second kernel should walk by itself
-//   tile_tables_kernel tile centre from the sums; then one warp per token: stereographic
-//                      coordinates of the token's patch x patch pixels about the tile's spherical
+//   tile_tables_kernel tile centre from the sums; per pixel, where asked for, the wind rotation
+//                      about it and the latitude channels; per token the stereographic
+//                      coordinates of its patch x patch pixels about the tile's spherical
 //                      centroid, their mean, and the (cos, sin) half pair of every frequency
 //
 // Everything is evaluated in double precision and rounded once. Bound: launch and dependent
 // latency - the table is 4 * head_dim / 2 bytes per token, the arithmetic two sincos per pixel and
 // one per table entry. As ~45 tensor operations (each a launch of 2-4 us on the GPU and 5 us
 // on the host) the same tables took 150 us of GPU and 400 us of host time per model call at
-// 32 x 32 pixels; the two kernels take 14 us there and 25 us at 256 x 256.
+// 32 x 32 pixels; the two kernels take 7 us there and 17 us at 256 x 256.
 #pragma once
 #include <cuda_fp16.h>
 
 #include "common.cuh"
+#include "prepost.cuh"
 
 namespace strata {
 
@@ -78,14 +80,23 @@ struct TileTablesParams {
   float* lat0;               // [B] tile centre (nullable)
   float* lon0;
   uint32_t* table;           // [B, h*w, pairs] (cos, sin) half pairs; unused for ROPE_NONE
+  // per-pixel geometry for the pre- and post-processing kernels, each nullable: wind rotation
+  // into the tile frame and back (need lat0), (cos lat, sin lat)
+  float4 *px_fwd, *px_inv;   // [B, H, W]
+  float2* px_lat;
 };
+
+__host__ __device__ constexpr int geo_tokens_per_warp(int mode, int patch) {
+  return mode != ROPE_STEREO || patch > 4 || patch == 3 ? 1 : (patch == 1 ? 32 : (patch == 2 ? 8 : 2));
+}
 
 __global__ void __launch_bounds__(256) tile_tables_kernel(const TileTablesParams p) {
   __shared__ double sh[8][GEO_SUMS];
   __shared__ double centre[4];         // sin / cos of the centroid's latitude, of its longitude
+  __shared__ float wind0[2];           // tile centre of the wind rotation
   const int HW = p.H * p.W;
   const long long base = static_cast<long long>(blockIdx.y) * HW;
-  if (p.mode == ROPE_STEREO || (p.lat0 != nullptr && blockIdx.x == 0)) {
+  if (p.mode == ROPE_STEREO || (p.lat0 != nullptr && (blockIdx.x == 0 || p.px_fwd != nullptr))) {
     double s[GEO_SUMS] = {0, 0, 0, 0, 0, 0};
     if (p.parts == nullptr) {
       for (int i = threadIdx.x; i < HW; i += 256)
@@ -98,11 +109,15 @@ __global__ void __launch_bounds__(256) tile_tables_kernel(const TileTablesParams
     }
     geo_block_sum(s, sh);
     if (threadIdx.x == 0) {
-      if (p.lat0 != nullptr && blockIdx.x == 0) {
+      if (p.lat0 != nullptr) {
         double l = atan2(s[1] / HW, s[2] / HW);
         if (l < 0.0) l += 6.283185307179586476925;
-        p.lat0[blockIdx.y] = static_cast<float>(s[0] / HW);
-        p.lon0[blockIdx.y] = static_cast<float>(l);
+        wind0[0] = static_cast<float>(s[0] / HW);
+        wind0[1] = static_cast<float>(l);
+        if (blockIdx.x == 0) {
+          p.lat0[blockIdx.y] = wind0[0];
+          p.lon0[blockIdx.y] = wind0[1];
+        }
       }
       const double n = sqrt(s[3] * s[3] + s[4] * s[4] + s[5] * s[5]), r = sqrt(s[3] * s[3] + s[4] * s[4]);
       centre[0] = s[5] / n;
@@ -112,16 +127,40 @@ __global__ void __launch_bounds__(256) tile_tables_kernel(const TileTablesParams
     }
     __syncthreads();
   }
+  if (p.px_fwd != nullptr || p.px_lat != nullptr) {
+    Basis q0{};
+    if (p.px_fwd != nullptr) {
+      double s0, c0, so0, co0;
+      sincos(static_cast<double>(wind0[0]), &s0, &c0);
+      sincos(static_cast<double>(wind0[1]), &so0, &co0);
+      q0 = local_basis_enr(s0, c0, so0, co0);
+    }
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < HW; i += gridDim.x * 256) {
+      double sl, cl, so, co;
+      sincos(static_cast<double>(__ldg(p.lat + base + i)), &sl, &cl);
+      if (p.px_lat != nullptr) p.px_lat[base + i] = make_float2(static_cast<float>(cl), static_cast<float>(sl));
+      if (p.px_fwd == nullptr) continue;
+      sincos(static_cast<double>(__ldg(p.lon + base + i)), &so, &co);
+      const Basis q = local_basis_enr(sl, cl, so, co);
+      p.px_fwd[base + i] = wind_matrix(q, q0, true);
+      p.px_inv[base + i] = wind_matrix(q, q0, false);
+    }
+  }
   if (p.mode == ROPE_NONE) return;
   const int lane = threadIdx.x & 31;
   const int tokens = p.h * p.w, half = p.pairs >> 1;
-  for (int t = blockIdx.x * 8 + (threadIdx.x >> 5); t < tokens; t += gridDim.x * 8) {
+  // A warp takes TPW tokens at a time: first 32 / TPW lanes per token share its pixels, then all
+  // lanes write the tokens' rows one after the other. (One token per warp left 31 lanes waiting
+  // for the one pixel of a patch-1 token: 64 us for 24 tiles of 48 x 48, 24 now.)
+  const int tpw = geo_tokens_per_warp(p.mode, p.patch), lpt = 32 / tpw;
+  for (int t0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * tpw; t0 < tokens; t0 += gridDim.x * 8 * tpw) {
+    const int t = min(t0 + lane / lpt, tokens - 1);
     const int ti = t / p.w, tj = t - ti * p.w;
     double x = tj, y = ti;
     if (p.mode == ROPE_STEREO) {
       const double s0 = centre[0], c0 = centre[1];
       x = 0.0; y = 0.0;
-      for (int q = lane; q < p.patch * p.patch; q += 32) {
+      for (int q = lane % lpt; q < p.patch * p.patch; q += lpt) {
         const int dy = q / p.patch, dx = q - dy * p.patch;
         const long long pix = base + static_cast<long long>(ti * p.patch + dy) * p.W + tj * p.patch + dx;
         double sl, cl, so, co;
@@ -133,20 +172,23 @@ __global__ void __launch_bounds__(256) tile_tables_kernel(const TileTablesParams
         x += k * cl * sd;
         y += k * (c0 * sl - s0 * cl * cd);
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
+      for (int o = lpt >> 1; o > 0; o >>= 1) {
         x += __shfl_xor_sync(0xffffffffu, x, o);
         y += __shfl_xor_sync(0xffffffffu, y, o);
       }
       x *= p.inv_scale;
       y *= p.inv_scale;
     }
-    uint32_t* row = p.table + (static_cast<long long>(blockIdx.y) * tokens + t) * p.pairs;
-    for (int j = lane; j < p.pairs; j += 32) {
-      double s, c;
-      sincos(j < half ? x * p.freq[j] : y * p.freq[j - half], &s, &c);
-      const __half2 v = __floats2half2_rn(static_cast<float>(c), static_cast<float>(s));
-      row[j] = *reinterpret_cast<const uint32_t*>(&v);
+    const int n = min(tpw, tokens - t0);
+    uint32_t* row = p.table + (static_cast<long long>(blockIdx.y) * tokens + t0) * p.pairs;
+    for (int i = 0; i < n; ++i, row += p.pairs) {
+      const double xi = __shfl_sync(0xffffffffu, x, i * lpt), yi = __shfl_sync(0xffffffffu, y, i * lpt);
+      for (int j = lane; j < p.pairs; j += 32) {
+        double s, c;
+        sincos(j < half ? xi * p.freq[j] : yi * p.freq[j - half], &s, &c);
+        const __half2 v = __floats2half2_rn(static_cast<float>(c), static_cast<float>(s));
+        row[j] = *reinterpret_cast<const uint32_t*>(&v);
+      }
     }
   }
 }
@@ -168,8 +210,10 @@ inline int launch_tile_tables(TileTablesParams p, int B, double* ws, cudaStream_
     tile_sums_kernel<<<dim3(p.n_parts, B), 256, 0, stream>>>(p.lat, p.lon, p.H * p.W, ws);
     p.parts = ws;
   }
-  // one token per warp and pass; at most ~8 blocks a tile and SM's worth of them
-  int bx = p.mode == ROPE_NONE ? 1 : (p.h * p.w + 7) / 8;
+  // one round of tokens per warp, one pixel per thread
+  const int tpb = 8 * geo_tokens_per_warp(p.mode, p.patch);
+  int bx = p.mode == ROPE_NONE ? 1 : (p.h * p.w + tpb - 1) / tpb;
+  if (p.px_fwd != nullptr || p.px_lat != nullptr) bx = std::max(bx, (p.H * p.W + 255) / 256);
   if (bx > 1024) bx = 1024;
   tile_tables_kernel<<<dim3(bx, B), 256, 0, stream>>>(p);
   const cudaError_t e = cudaGetLastError();

@@ -36,6 +36,8 @@ struct NetworkPlan {
   // pieces
   float *lat0, *lon0;
   double* sums;
+  float4 *px_fwd, *px_inv;
+  float2* px_lat;
   void *rope, *rope_px;
   void *tokens, *patches, *block_ws;                   // backbone
   void *px, *px_patches, *mod, *cond, *xn, *qkv, *attn, *y, *hid;   // pixel stage
@@ -55,6 +57,12 @@ inline bool network_plan(const strata_backbone_desc& b, const strata_pixel_desc*
   n.lat0 = static_cast<float*>(s.take(4LL * B));
   n.lon0 = static_cast<float*>(s.take(4LL * B));
   n.sums = static_cast<double*>(s.take(strata_tile_tables_workspace_bytes(B, H, W)));
+  const int64_t columns = static_cast<int64_t>(B) * H * W;
+  if (b.u_idx >= 0) {
+    n.px_fwd = static_cast<float4*>(s.take(16 * columns));
+    n.px_inv = static_cast<float4*>(s.take(16 * columns));
+  }
+  if (b.concat_lat) n.px_lat = static_cast<float2*>(s.take(8 * columns));
   if (b.rope_mode != STRATA_ROPE_NONE) n.rope = s.take(4LL * B * n.h * n.w * (b.dim / b.heads / 2));
   n.tokens = s.take(2 * n.M * b.dim);
   // what follows is shared by phases that do not overlap in time
@@ -151,14 +159,14 @@ inline int network_forward(const strata_backbone_desc& b, const strata_pixel_des
                            const NetworkPlan& n, void* stream) {
   const bool wind = b.u_idx >= 0;
   const int hd = b.dim / b.heads, M = static_cast<int>(n.M);
-  STRATA_TRY(strata_tile_tables(lat, lon, B, H, W, wind ? n.lat0 : nullptr, wind ? n.lon0 : nullptr,
-                                b.rope_mode, b.patch_h, b.rope_length_scale, b.rope_base, hd, n.rope,
-                                n.sums, n.bytes, stream));
-  const float* lat0 = wind ? n.lat0 : nullptr;
-  const float* lon0 = wind ? n.lon0 : nullptr;
-  STRATA_TRY(strata_preprocess_patches_bf16(x, B, b.in_channels, D, H, W, lat, lon, lat0, lon0, b.u_idx,
-                                            b.v_idx, b.concat_lat, b.patch_v, b.patch_h, b.patch_w,
-                                            n.patches, b.k_embed, stream));
+  float* lat0 = wind ? n.lat0 : nullptr;
+  float* lon0 = wind ? n.lon0 : nullptr;
+  STRATA_TRY(tile_tables_impl(lat, lon, B, H, W, lat0, lon0, b.rope_mode, b.patch_h, b.rope_length_scale,
+                              b.rope_base, hd, n.rope, n.sums, n.bytes, n.px_fwd, n.px_inv, n.px_lat,
+                              stream));
+  STRATA_TRY(preprocess_impl(x, B, b.in_channels, D, H, W, lat, lon, lat0, lon0, b.u_idx, b.v_idx,
+                             b.concat_lat, b.patch_v, b.patch_h, b.patch_w, n.patches, b.k_embed, n.px_fwd,
+                             n.px_lat, stream));
   STRATA_TRY(strata_linear_bf16(n.patches, b.k_embed, b.w_embed, b.k_embed, b.b_embed, n.tokens, b.dim, M,
                                 b.dim, static_cast<int>(b.k_embed), STRATA_EPI_BIAS, nullptr, 0, stream));
   const int64_t ws_bytes = strata_block_workspace_bytes(n.M, b.dim, b.hidden);
@@ -176,9 +184,8 @@ inline int network_forward(const strata_backbone_desc& b, const strata_pixel_des
       STRATA_TRY(strata_tile_tables(lat, lon, B, H, W, nullptr, nullptr, px->rope_mode, 1,
                                     px->rope_length_scale, px->rope_base, px->dim / px->heads, n.rope_px,
                                     n.sums, n.bytes, stream));
-    STRATA_TRY(strata_preprocess_patches_bf16(x, B, b.in_channels, D, H, W, lat, lon, lat0, lon0, b.u_idx,
-                                              b.v_idx, b.concat_lat, 1, 1, 1, n.px_patches, px->k_embed,
-                                              stream));
+    STRATA_TRY(preprocess_impl(x, B, b.in_channels, D, H, W, lat, lon, lat0, lon0, b.u_idx, b.v_idx,
+                               b.concat_lat, 1, 1, 1, n.px_patches, px->k_embed, n.px_fwd, n.px_lat, stream));
     STRATA_TRY(strata_linear_bf16(n.px_patches, px->k_embed, px->w_embed, px->k_embed, px->b_embed, n.px,
                                   px->dim, static_cast<int>(n.Mp), px->dim, static_cast<int>(px->k_embed),
                                   STRATA_EPI_BIAS, nullptr, 0, stream));
@@ -189,8 +196,8 @@ inline int network_forward(const strata_backbone_desc& b, const strata_pixel_des
   STRATA_TRY(strata_layernorm_bf16(rows, C, n.head_n, C, R, C, 1e-6f, stream));
   STRATA_TRY(strata_linear_bf16(n.head_n, C, w_head, C, b_head, n.head_y, n_head, R, n_head, C,
                                 STRATA_EPI_BIAS, nullptr, 0, stream));
-  return strata_postprocess_fields_f32(n.head_y, n_head, B, b.out_channels, D, H, W, lat, lon, lat0, lon0,
-                                       b.u_idx, b.v_idx, pv, ph, pw, out, stream);
+  return postprocess_impl(n.head_y, n_head, B, b.out_channels, D, H, W, lat, lon, lat0, lon0, b.u_idx,
+                          b.v_idx, pv, ph, pw, out, n.px_inv, stream);
 }
 
 #undef STRATA_TRY

@@ -85,3 +85,32 @@ def test_argument_errors():
     with pytest.raises(ValueError):   # rotation without tile centres
         ops.preprocess_patches(x, torch.zeros(1, 8, 8, device="cuda"), torch.zeros(1, 8, 8, device="cuda"),
                                wind=(0, 1))
+
+
+# rows of tokens longer than a block's run (256 pixel columns), token rows larger than its tile
+# (pieces of them), widths and patches without four-pixel loads, a row stride without 16-byte stores
+@pytest.mark.parametrize("C,D,H,W,patch,k_pad", [(3, 3, 4, 264, (1, 4, 4), None), (5, 2, 3, 277, (1, 1, 1), None),
+                                                 (40, 4, 8, 24, (4, 8, 12), None), (4, 2, 6, 30, (1, 3, 5), 101),
+                                                 (2, 9, 1, 512, (1, 1, 1), None)])
+def test_round_trip_shapes(C, D, H, W, patch, k_pad):
+    from strata_b200 import ops
+    B = 2
+    pv, ph, pw = patch
+    x = torch.randn(B, C, D, H, W, generator=torch.Generator().manual_seed(3)).bfloat16().float().cuda()
+    lat, lon, lat0, lon0 = (t.cuda() for t in _geometry(B, H, W, 4))
+    a = ops.preprocess_patches(x, lat, lon, patch=patch, k_pad=k_pad)
+    rows = (B, D // pv, H // ph, W // pw)
+    want = x.view(B, C, D // pv, pv, H // ph, ph, W // pw, pw)
+    K = C * pv * ph * pw
+    assert torch.equal(a[:, :K].float(), want.permute(0, 2, 4, 6, 1, 3, 5, 7).reshape(-1, K))
+    assert torch.all(a[:, K:] == 0)
+    y = torch.zeros_like(a)
+    y[:, :K] = want.permute(0, 2, 4, 6, 3, 5, 7, 1).reshape(-1, K).bfloat16()
+    assert torch.equal(ops.postprocess_fields(y, x.shape, patch=patch), x)
+    # rotating into the tile frame and back is the identity up to the bf16 rounding of the rows
+    r = ops.preprocess_patches(x, lat, lon, lat0, lon0, wind=(1, 0), patch=patch, k_pad=k_pad)
+    r = r[:, :K].view(*rows, C, pv, ph, pw).permute(0, 1, 2, 3, 5, 6, 7, 4).reshape(-1, K)
+    y[:, :K] = r
+    back = ops.postprocess_fields(y, x.shape, lat, lon, lat0, lon0, wind=(1, 0), patch=patch)
+    assert torch.equal(back[:, 2:], x[:, 2:])
+    assert (back - x).abs().max() < 0.06
