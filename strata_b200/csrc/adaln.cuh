@@ -37,6 +37,7 @@ __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
 // LPR lanes (16 or 32) share one row; each holds VPL 16-byte vectors of it.
 template <int LPR, int VPL>
 __global__ void __launch_bounds__(256) adaln_rows_kernel(const AdalnRowsParams p) {
+  chain_begin();
   constexpr int ROWS_PER_WARP = 32 / LPR;
   const int lane = threadIdx.x & 31;
   const int sub = lane % LPR;
@@ -132,19 +133,18 @@ inline int launch_adaln_rows(const AdalnRowsParams& p, int sm_count, cudaStream_
   if (blocks > cap) blocks = cap;
   const int g = static_cast<int>(blocks);
   const int vpl = (nvec + lpr - 1) / lpr;
-  if (lpr == 16) adaln_rows_kernel<16, 1><<<g, threads, 0, stream>>>(p);
-  else if (vpl <= 1) adaln_rows_kernel<32, 1><<<g, threads, 0, stream>>>(p);
-  else if (vpl <= 2) adaln_rows_kernel<32, 2><<<g, threads, 0, stream>>>(p);
-  else if (vpl <= 4) adaln_rows_kernel<32, 4><<<g, threads, 0, stream>>>(p);
-  else adaln_rows_kernel<32, 8><<<g, threads, 0, stream>>>(p);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
+  auto kern = lpr == 16 ? adaln_rows_kernel<16, 1>
+              : vpl <= 1 ? adaln_rows_kernel<32, 1>
+              : vpl <= 2 ? adaln_rows_kernel<32, 2>
+              : vpl <= 4 ? adaln_rows_kernel<32, 4> : adaln_rows_kernel<32, 8>;
+  return launch_chained(kern, dim3(g), threads, 0, stream, 1, p);
 }
 
 // RMS norm of the q and k heads (64 channels each) of packed qkv rows [M, 3C], in place:
 // t <- t * rsqrt(mean(t^2) + eps). Eight lanes share a head (one 16-byte vector each).
 __global__ void __launch_bounds__(256)
 qk_norm_rows_kernel(__nv_bfloat16* __restrict__ qkv, long long ld, long long M, int C, float eps) {
+  chain_begin();
   const int heads2 = 2 * (C >> 6);                      // q heads then k heads: columns [0, 2C)
   const long long groups = M * heads2;                  // one 8-lane group per (row, head)
   const long long n_thr = static_cast<long long>(gridDim.x) * blockDim.x;
@@ -179,9 +179,7 @@ inline int launch_qk_norm_rows(__nv_bfloat16* qkv, long long ld, long long M, in
   long long blocks = (thr + 255) / 256;
   const long long cap = static_cast<long long>(sm_count) * 16;
   if (blocks > cap) blocks = cap;
-  qk_norm_rows_kernel<<<static_cast<int>(blocks), 256, 0, stream>>>(qkv, ld, M, C, eps);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
+  return launch_chained(qk_norm_rows_kernel, dim3(static_cast<unsigned>(blocks)), 256, 0, stream, 1, qkv, ld, M, C, eps);
 }
 
 // Source index and weights of a 1-D bilinear upsample by an integer factor (half-pixel
@@ -252,6 +250,7 @@ __device__ __forceinline__ void gelu8(float (&acc)[8]) {
 
 // One thread: one pixel x 8 channels, direct evaluation (any factor and kernel size).
 __global__ void __launch_bounds__(256) adaln_cond_kernel(const AdalnCondParams p) {
+  chain_begin();
   const int nvec = p.Cb >> 3;
   const int H = p.h * p.factor, W = p.w * p.factor;
   const long long total = p.n_rows * nvec;
@@ -287,6 +286,7 @@ __device__ __forceinline__ void cond_class_ref(int cls, int f, int& pos, int& ba
 
 __global__ void adaln_cond_table_kernel(const float* __restrict__ wdw, int Cb, int factor, int ks,
                                         float* __restrict__ table) {
+  chain_begin();
   const int ncls = 3 * factor;
   const int n = ncls * ncls * Cb;
   const int r = ks >> 1;
@@ -347,6 +347,7 @@ constexpr int COND_RUN = 6;
 
 __global__ void __launch_bounds__(256, 2)
 adaln_cond_runs_kernel(const AdalnCondParams p, const float* __restrict__ table, int psplit) {
+  chain_begin();
   const int f = p.factor;
   const int ncls = 3 * f;
   const int H = p.h * f, W = p.w * f;
@@ -461,9 +462,7 @@ inline long long adaln_cond_table_floats(int Cb, int factor, int ks) {
 inline int launch_adaln_cond_table(const float* wdw, int Cb, int factor, int ks, float* table,
                                    cudaStream_t stream) {
   const int n = 9 * factor * factor * Cb;
-  adaln_cond_table_kernel<<<(n + 255) / 256, 256, 0, stream>>>(wdw, Cb, factor, ks, table);
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
+  return launch_chained(adaln_cond_table_kernel, dim3((n + 255) / 256), 256, 0, stream, 1, wdw, Cb, factor, ks, table);
 }
 
 // table: what launch_adaln_cond_table wrote for these weights (adaln_cond_table_floats() floats),
@@ -487,16 +486,13 @@ inline int launch_adaln_cond(const AdalnCondParams& p, const float* table, int s
     const long long cap = (static_cast<long long>(sm_count) * 16 + groups - 1) / groups;
     if (blocks > cap) blocks = cap;
     blocks *= groups;
-    adaln_cond_runs_kernel<<<static_cast<int>(blocks), 256, 0, stream>>>(p, table, psplit);
-  } else {
-    const long long total = p.n_rows * (p.Cb / 8);
-    long long blocks = (total + 255) / 256;
-    const long long cap = static_cast<long long>(sm_count) * 32;
-    if (blocks > cap) blocks = cap;
-    adaln_cond_kernel<<<static_cast<int>(blocks), 256, 0, stream>>>(p);
+    return launch_chained(adaln_cond_runs_kernel, dim3(static_cast<unsigned>(blocks)), 256, 0, stream, 1, p, table, psplit);
   }
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
+  const long long total = p.n_rows * (p.Cb / 8);
+  long long blocks = (total + 255) / 256;
+  const long long cap = static_cast<long long>(sm_count) * 32;
+  if (blocks > cap) blocks = cap;
+  return launch_chained(adaln_cond_kernel, dim3(static_cast<unsigned>(blocks)), 256, 0, stream, 1, p);
 }
 
 }  // namespace strata

@@ -374,10 +374,7 @@ static int preprocess_impl(const float* x, int B, int C_in, int D, int H, int W,
                   concat_lat ? 1 : 0, lat, lon, lat0, lon0, lda, 0, 0, 0, 0, 0, px_rot, px_lat};
   if (pv == 1 && ph == 1 && pw == 1 && lda % 8 == 0 && aligned16(a)) {
     const dim3 grid = pixels_grid(p, sms);
-    preprocess_pixels_kernel<<<grid, PREPOST_THREADS, 0, as_stream(stream)>>>(
-        x, static_cast<__nv_bfloat16*>(a), p);
-    const cudaError_t e1 = cudaGetLastError();
-    return e1 == cudaSuccess ? 0 : -static_cast<int>(e1) - 1000;
+    return launch_chained(preprocess_pixels_kernel, grid, PREPOST_THREADS, 0, as_stream(stream), 1, x, static_cast<__nv_bfloat16*>(a), p);
   }
   const int v = !aligned16(x) ? 1 : pw % 4 == 0 && W % 4 == 0 ? 4 : pw % 2 == 0 && W % 2 == 0 ? 2 : 1;
   long long blocks;
@@ -385,15 +382,14 @@ static int preprocess_impl(const float* x, int B, int C_in, int D, int H, int W,
   if (prepost_plan(p, pv * ph * pw, C_in + (concat_lat ? 2 : 0), v == 4 ? 8 : 4, concat_lat != 0, sms,
                    &blocks, &smem) != 0)
     return STRATA_ERR_UNSUPPORTED;
+  static std::atomic<uint64_t> smem_set[3];
   auto kern = v == 4 ? preprocess_patches_kernel<4> : v == 2 ? preprocess_patches_kernel<2> : preprocess_patches_kernel<1>;
   if (smem > 48 * 1024) {
-    const cudaError_t ea = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t ea = allow_smem(reinterpret_cast<const void*>(kern), PREPOST_MAX_SMEM, smem_set[v >> 1]);
     if (ea != cudaSuccess) return -static_cast<int>(ea) - 1000;
   }
-  kern<<<static_cast<unsigned>(blocks), PREPOST_THREADS, smem, as_stream(stream)>>>(
-      x, static_cast<__nv_bfloat16*>(a), p);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
+  return launch_chained(kern, dim3(static_cast<unsigned>(blocks)), PREPOST_THREADS, smem, as_stream(stream), 1,
+                        x, static_cast<__nv_bfloat16*>(a), p);
 }
 
 int strata_preprocess_patches_bf16(const float* x, int B, int C_in, int D, int H, int W,
@@ -418,24 +414,20 @@ static int postprocess_impl(const void* y, int64_t ldy, int B, int C_out, int D,
                   lat, lon, lat0, lon0, ldy, 0, 0, 0, 0, 0, px_rot, nullptr};
   if (pv == 1 && ph == 1 && pw == 1 && ldy % 8 == 0 && aligned16(y)) {
     const dim3 grid = pixels_grid(p, sms);
-    postprocess_pixels_kernel<<<grid, PREPOST_THREADS, 0, as_stream(stream)>>>(
-        static_cast<const __nv_bfloat16*>(y), out, p);
-    const cudaError_t e1 = cudaGetLastError();
-    return e1 == cudaSuccess ? 0 : -static_cast<int>(e1) - 1000;
+    return launch_chained(postprocess_pixels_kernel, grid, PREPOST_THREADS, 0, as_stream(stream), 1, static_cast<const __nv_bfloat16*>(y), out, p);
   }
   const int v = !aligned16(out) ? 1 : pw % 4 == 0 && W % 4 == 0 ? 4 : pw % 2 == 0 && W % 2 == 0 ? 2 : 1;
   long long blocks;
   int smem;
   if (prepost_plan(p, pw * C_out, pv * ph, 4, false, sms, &blocks, &smem) != 0) return STRATA_ERR_UNSUPPORTED;
+  static std::atomic<uint64_t> smem_set[3];
   auto kern = v == 4 ? postprocess_fields_kernel<4> : v == 2 ? postprocess_fields_kernel<2> : postprocess_fields_kernel<1>;
   if (smem > 48 * 1024) {
-    const cudaError_t ea = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t ea = allow_smem(reinterpret_cast<const void*>(kern), PREPOST_MAX_SMEM, smem_set[v >> 1]);
     if (ea != cudaSuccess) return -static_cast<int>(ea) - 1000;
   }
-  kern<<<static_cast<unsigned>(blocks), PREPOST_THREADS, smem, as_stream(stream)>>>(
-      static_cast<const __nv_bfloat16*>(y), out, p);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
+  return launch_chained(kern, dim3(static_cast<unsigned>(blocks)), PREPOST_THREADS, smem, as_stream(stream), 1,
+                        static_cast<const __nv_bfloat16*>(y), out, p);
 }
 
 int strata_postprocess_fields_f32(const void* y, int64_t ldy, int B, int C_out, int D, int H, int W,
@@ -470,11 +462,9 @@ int strata_halo_gather_tokens_bf16(void* out, const void* const* h_peer_src, int
   if (bx > cap) bx = cap;
   dim3 grid(static_cast<unsigned>(bx), static_cast<unsigned>(tiles_per_rank * D));
   if (static_cast<long long>(tiles_per_rank) * D > 65535) return STRATA_ERR_UNSUPPORTED;
-  halo_gather_tokens_kernel<<<grid, 256, 0, as_stream(stream)>>>(
+  return launch_chained(halo_gather_tokens_kernel, grid, 256, 0, as_stream(stream), 1,
       static_cast<__nv_bfloat16*>(out), pp, src_a, src_b, P * P, T * T, D, C,
       static_cast<int>(cells), only_halo, halo, halo + T, P);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
 }
 
 int strata_halo_gather_fields_f32(float* out, const void* const* h_peer_src, int world,
@@ -498,11 +488,9 @@ int strata_halo_gather_fields_f32(float* out, const void* const* h_peer_src, int
     return STRATA_ERR_ARG;
   const long long bx = (ocells + 255) / 256;
   dim3 grid(static_cast<unsigned>(bx), field_grid_y(L, FIELD_UL_COPY));
-  halo_gather_fields_kernel<<<grid, 256, 0, as_stream(stream)>>>(
+  return launch_chained(halo_gather_fields_kernel, grid, 256, 0, as_stream(stream), 1,
       out, pp, src_a, src_b, static_cast<int>(ocells), static_cast<int>(cells),
       static_cast<int>(L));
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
 }
 
 int strata_halo_gather_knn_fields_f32(float* out, const void* const* h_peer_src, int world,
@@ -529,14 +517,10 @@ int strata_halo_gather_knn_fields_f32(float* out, const void* const* h_peer_src,
   dim3 grid(static_cast<unsigned>(bx), field_grid_y(L, FIELD_UL_KNN));
   cudaStream_t st = as_stream(stream);
   const int no = static_cast<int>(ocells), nc = static_cast<int>(cells), nl = static_cast<int>(L);
-  switch (k) {
-    case 1: halo_gather_knn_fields_kernel<1><<<grid, 256, 0, st>>>(out, pp, idx, weights, no, nc, nl); break;
-    case 2: halo_gather_knn_fields_kernel<2><<<grid, 256, 0, st>>>(out, pp, idx, weights, no, nc, nl); break;
-    case 4: halo_gather_knn_fields_kernel<4><<<grid, 256, 0, st>>>(out, pp, idx, weights, no, nc, nl); break;
-    default: halo_gather_knn_fields_kernel<8><<<grid, 256, 0, st>>>(out, pp, idx, weights, no, nc, nl); break;
-  }
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
+  auto kern = k == 1 ? halo_gather_knn_fields_kernel<1>
+              : k == 2 ? halo_gather_knn_fields_kernel<2>
+              : k == 4 ? halo_gather_knn_fields_kernel<4> : halo_gather_knn_fields_kernel<8>;
+  return launch_chained(kern, grid, 256, 0, st, 1, out, pp, idx, weights, no, nc, nl);
 }
 
 int strata_halo_adjoint_fields_f32(float* out, const void* const* h_peer_padded, int world,
@@ -561,11 +545,9 @@ int strata_halo_adjoint_fields_f32(float* out, const void* const* h_peer_padded,
   if (pcells * world > 0x7fffffffLL || L > 0x7fffffffLL) return STRATA_ERR_ARG;
   const long long bx = (cells + 255) / 256;
   dim3 grid(static_cast<unsigned>(bx), field_grid_y(L, FIELD_UL_ADJ));
-  halo_adjoint_fields_kernel<<<grid, 256, 0, as_stream(stream)>>>(
+  return launch_chained(halo_adjoint_fields_kernel, grid, 256, 0, as_stream(stream), 1,
       out, pp, offsets, cell, coef, window, weights, static_cast<int>(cells),
       static_cast<int>(pcells), P * P, static_cast<int>(L));
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
 }
 
 int strata_halo_gather_kv_bf16(void* qkv, const void* const* h_peer_qkv, int world,
@@ -596,12 +578,10 @@ int strata_halo_gather_kv_bf16(void* qkv, const void* const* h_peer_qkv, int wor
   if (bx > cap) bx = cap;
   if (bx < 1) return STRATA_OK;   // no halo
   dim3 grid(static_cast<unsigned>(bx), static_cast<unsigned>(tiles_per_rank * D));
-  halo_gather_kv_kernel<<<grid, 256, 0, as_stream(stream)>>>(
+  return launch_chained(halo_gather_kv_kernel, grid, 256, 0, as_stream(stream), 1,
       static_cast<__nv_bfloat16*>(qkv), pp, src_a, src_b, static_cast<const uint32_t*>(dcs_a),
       static_cast<const uint32_t*>(dcs_b), P, T, halo, D, C, head_dim, ldqkv,
       static_cast<int>(cells));
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
 }
 
 int strata_halo_barrier(int* const* h_flags, int me, int world, int epoch, int timeout_ms,
@@ -724,10 +704,8 @@ int strata_dealias_patches_bf16(const void* x_rows, int64_t ldx, int B, int C, i
   const long long total = static_cast<long long>(B) * (D / pv) * (H / ph) * (W / pw) * lda;
   long long blocks = (total + 255) / 256;
   if (blocks > static_cast<long long>(sms) * 32) blocks = static_cast<long long>(sms) * 32;
-  dealias_patches_kernel<<<static_cast<unsigned>(blocks), 256, 0, as_stream(stream)>>>(
+  return launch_chained(dealias_patches_kernel, dim3(static_cast<unsigned>(blocks)), 256, 0, as_stream(stream), 1,
       static_cast<const __nv_bfloat16*>(x_rows), static_cast<__nv_bfloat16*>(a), p);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
 }
 
 int64_t strata_adaln_cond_table_floats(int Cb, int factor, int ks) {

@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "launch.cuh"
+
 namespace strata {
 
 // Device status word: 0 = ok, otherwise the first error code a kernel recorded.

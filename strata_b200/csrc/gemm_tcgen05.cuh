@@ -285,6 +285,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   const int num_kb = (p.K + GEMM_BK - 1) / GEMM_BK;
 
   if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tmA);
+    tma_prefetch_desc(&tmB);
     for (int s = 0; s < S::STAGES; ++s) {
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
@@ -306,12 +308,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   if constexpr (PAIR) cluster_sync_all();   // the partner's barriers exist before anyone signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_begin();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      tma_prefetch_desc(&tmA);
-      tma_prefetch_desc(&tmB);
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -619,26 +620,11 @@ inline int launch_gemm_t(const __nv_bfloat16* A, long long lda, const __nv_bfloa
   }
   using S = GemmSmem<BN, PAIR>;
   auto kern = gemm_tcgen05_kernel<BN, EPI, PAIR>;
-  {
-    // Per-device attribute; setting it on every launch keeps the launcher stateless.
-    cudaError_t e =
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
-    if (e != cudaSuccess) return -static_cast<int>(e) - 1000;
-  }
+  static std::atomic<uint64_t> smem_set;
+  if (const cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), S::TOTAL, smem_set); e != cudaSuccess)
+    return -static_cast<int>(e) - 1000;
   if constexpr (PAIR) {
     const int tiles = ((p.M + 2 * GEMM_BM - 1) / (2 * GEMM_BM)) * ((p.N + BN - 1) / BN);
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(sm_count & ~1));
-    cfg.blockDim = dim3(GEMM_THREADS);
-    cfg.dynamicSmemBytes = S::TOTAL;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
     // A persistent grid must be resident at once: not every SM has a partner for a pair, so the
     // number of clusters that fit is asked for (once per kernel and device), not assumed.
     static std::atomic<int> max_clusters[64];   // per device; concurrent first calls store the same value
@@ -647,19 +633,28 @@ inline int launch_gemm_t(const __nv_bfloat16* A, long long lda, const __nv_bfloa
     if (dev < 0 || dev >= 64) return -24;
     int fit = max_clusters[dev].load(std::memory_order_relaxed);
     if (fit == 0) {
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(static_cast<unsigned>(sm_count & ~1));
+      cfg.blockDim = dim3(GEMM_THREADS);
+      cfg.dynamicSmemBytes = S::TOTAL;
+      cfg.stream = stream;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 2;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
       if (cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) != cudaSuccess || fit <= 0) return -24;
       max_clusters[dev].store(fit, std::memory_order_relaxed);
     }
     const int clusters = tiles < fit ? tiles : fit;
-    cfg.gridDim = dim3(static_cast<unsigned>(2 * clusters));
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tmA, tmB, tmOut, tmAux, p);
-    return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
+    return launch_chained(kern, dim3(static_cast<unsigned>(2 * clusters)), GEMM_THREADS, S::TOTAL, stream, 2,
+                          tmA, tmB, tmOut, tmAux, p);
   }
   const int tiles = ((p.M + GEMM_BM - 1) / GEMM_BM) * ((p.N + BN - 1) / BN);
   const int grid = tiles < sm_count ? tiles : sm_count;
-  kern<<<grid, GEMM_THREADS, S::TOTAL, stream>>>(tmA, tmB, tmOut, tmAux, p);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
+  return launch_chained(kern, dim3(grid), GEMM_THREADS, S::TOTAL, stream, 1, tmA, tmB, tmOut, tmAux, p);
 }
 
 template <int EPI>

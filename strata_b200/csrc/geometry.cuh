@@ -57,6 +57,7 @@ __device__ __forceinline__ void geo_block_sum(double (&s)[GEO_SUMS], double (*sh
 __global__ void __launch_bounds__(256)
 tile_sums_kernel(const float* __restrict__ lat, const float* __restrict__ lon, int HW,
                  double* __restrict__ parts) {
+  chain_begin();
   __shared__ double sh[8][GEO_SUMS];
   const long long base = static_cast<long long>(blockIdx.y) * HW;
   double s[GEO_SUMS] = {0, 0, 0, 0, 0, 0};
@@ -91,6 +92,7 @@ __host__ __device__ constexpr int geo_tokens_per_warp(int mode, int patch) {
 }
 
 __global__ void __launch_bounds__(256) tile_tables_kernel(const TileTablesParams p) {
+  chain_begin();
   __shared__ double sh[8][GEO_SUMS];
   __shared__ double centre[4];         // sin / cos of the centroid's latitude, of its longitude
   __shared__ float wind0[2];           // tile centre of the wind rotation
@@ -207,7 +209,8 @@ inline int launch_tile_tables(TileTablesParams p, int B, double* ws, cudaStream_
   p.n_parts = geo_parts(p.H * p.W);
   p.parts = nullptr;
   if (p.n_parts > 0 && (p.mode == ROPE_STEREO || p.lat0 != nullptr)) {
-    tile_sums_kernel<<<dim3(p.n_parts, B), 256, 0, stream>>>(p.lat, p.lon, p.H * p.W, ws);
+    const int r = launch_chained(tile_sums_kernel, dim3(p.n_parts, B), 256, 0, stream, 1, p.lat, p.lon, p.H * p.W, ws);
+    if (r != 0) return r;
     p.parts = ws;
   }
   // one round of tokens per warp, one pixel per thread
@@ -215,9 +218,7 @@ inline int launch_tile_tables(TileTablesParams p, int B, double* ws, cudaStream_
   int bx = p.mode == ROPE_NONE ? 1 : (p.h * p.w + tpb - 1) / tpb;
   if (p.px_fwd != nullptr || p.px_lat != nullptr) bx = std::max(bx, (p.H * p.W + 255) / 256);
   if (bx > 1024) bx = 1024;
-  tile_tables_kernel<<<dim3(bx, B), 256, 0, stream>>>(p);
-  const cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
+  return launch_chained(tile_tables_kernel, dim3(bx, B), 256, 0, stream, 1, p);
 }
 
 }  // namespace strata

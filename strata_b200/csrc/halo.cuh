@@ -52,6 +52,7 @@ halo_gather_tokens_kernel(__nv_bfloat16* __restrict__ out, const PeerPtrs src,
                           const int* __restrict__ src_a, const int* __restrict__ src_b, int PP,
                           int TT, int D, int C, int cells_per_rank, int only_halo,
                           int halo_lo, int halo_hi, int P) {
+  chain_begin();
   const int vpc = C >> 3;  // 16-byte vectors per cell
   const int tile = blockIdx.y / D;
   const int d = blockIdx.y - tile * D;
@@ -156,6 +157,7 @@ __global__ void __launch_bounds__(256)
 halo_gather_fields_kernel(float* __restrict__ out, const __grid_constant__ PeerPtrs src,
                           const int* __restrict__ src_a, const int* __restrict__ src_b,
                           int n_out_cells, int cells_per_rank, int L) {
+  chain_begin();
   const int oc = blockIdx.x * 256 + threadIdx.x;
   if (oc >= n_out_cells) return;
   const bool failed = halo_exchange_failed();
@@ -197,6 +199,7 @@ __global__ void __launch_bounds__(256)
 halo_gather_knn_fields_kernel(float* __restrict__ out, const __grid_constant__ PeerPtrs src,
                               const int* __restrict__ idx, const float* __restrict__ w,
                               int n_out_cells, int cells_per_rank, int L) {
+  chain_begin();
   const int oc = blockIdx.x * 256 + threadIdx.x;
   if (oc >= n_out_cells) return;
   const bool failed = halo_exchange_failed();
@@ -244,6 +247,7 @@ halo_adjoint_fields_kernel(float* __restrict__ out, const __grid_constant__ Peer
                            const float* __restrict__ coef, const float* __restrict__ window,
                            const float* __restrict__ weights, int n_cells,
                            int padded_cells_per_rank, int PP, int L) {
+  chain_begin();
   const int c = blockIdx.x * 256 + threadIdx.x;
   if (c >= n_cells) return;
   const bool failed = halo_exchange_failed();
@@ -291,6 +295,7 @@ halo_gather_kv_kernel(__nv_bfloat16* __restrict__ qkv, const PeerPtrs src,
                       const uint32_t* __restrict__ dcs_a, const uint32_t* __restrict__ dcs_b,
                       int P, int T, int halo, int D, int C, int head_dim, long long ld,
                       int cells_per_rank) {
+  chain_begin();
   const int PP = P * P, TT = T * T;
   const int vpc = (2 * C) >> 3;     // 16-byte vectors of k|v per cell
   const int kvec = C >> 3;          // the first kvec of them are K

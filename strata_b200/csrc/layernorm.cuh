@@ -14,6 +14,7 @@ template <int VEC_PER_LANE>  // number of 8-element (16-byte) vectors each lane 
 __global__ void __launch_bounds__(256)
 layernorm_rows_kernel(const __nv_bfloat16* __restrict__ x, long long ldx,
                       __nv_bfloat16* __restrict__ y, long long ldy, int M, int C, float eps) {
+  chain_begin();
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   const int nvec = C >> 3;
@@ -85,12 +86,10 @@ inline int launch_layernorm(const __nv_bfloat16* x, long long ldx, __nv_bfloat16
   const int nvec = C / 8;
   const int vpl = (nvec + 31) / 32;
   const int g = static_cast<int>(blocks);
-  if (vpl <= 1) layernorm_rows_kernel<1><<<g, threads, 0, stream>>>(x, ldx, y, ldy, M, C, eps);
-  else if (vpl <= 2) layernorm_rows_kernel<2><<<g, threads, 0, stream>>>(x, ldx, y, ldy, M, C, eps);
-  else if (vpl <= 4) layernorm_rows_kernel<4><<<g, threads, 0, stream>>>(x, ldx, y, ldy, M, C, eps);
-  else layernorm_rows_kernel<8><<<g, threads, 0, stream>>>(x, ldx, y, ldy, M, C, eps);
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
+  auto kern = vpl <= 1 ? layernorm_rows_kernel<1>
+              : vpl <= 2 ? layernorm_rows_kernel<2>
+              : vpl <= 4 ? layernorm_rows_kernel<4> : layernorm_rows_kernel<8>;
+  return launch_chained(kern, dim3(g), threads, 0, stream, 1, x, ldx, y, ldy, M, C, eps);
 }
 
 }  // namespace strata

@@ -346,6 +346,7 @@ na3d_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
   extern __shared__ __align__(1024) uint8_t smem[];
   const uint32_t sbase = smem_u32(smem);
   if ((sbase & 1023u) != 0) {  // the swizzled tiles need 1024-byte alignment
+    chain_begin();
     if (threadIdx.x == 0) atomicCAS(&g_status, 0, ST_BAD_TMEM);
     return;
   }
@@ -368,6 +369,9 @@ na3d_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
                    static_cast<int>(gridDim.x);
 
   if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tmQ);
+    tma_prefetch_desc(&tmK);
+    tma_prefetch_desc(&tmV);
     mbar_init(q_full, 1);
     mbar_init(q_empty, 1);
     mbar_init(s_full, 1);
@@ -388,13 +392,11 @@ na3d_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_begin();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      tma_prefetch_desc(&tmQ);
-      tma_prefetch_desc(&tmK);
-      tma_prefetch_desc(&tmV);
       bool ok = true;
       int st = 0;
       uint32_t ph = 0;
@@ -851,13 +853,11 @@ inline int launch_na3d_t(const __nv_bfloat16* q, long long ldq, const __nv_bfloa
   p.q = q; p.k = k; p.v = v;
   p.ldq = ldq; p.ldk = ldk; p.ldv = ldv;
   auto kern = na3d_fwd_kernel<KW, QW>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       Cfg::TOTAL);
-  if (e != cudaSuccess) return -static_cast<int>(e) - 1000;
+  static std::atomic<uint64_t> smem_set;
+  if (const cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), Cfg::TOTAL, smem_set); e != cudaSuccess)
+    return -static_cast<int>(e) - 1000;
   const int grid = p.n_items < 2 * sm_count ? p.n_items : 2 * sm_count;
-  kern<<<grid, Cfg::THREADS, Cfg::TOTAL, stream>>>(tmQ, tmK, tmV, p);
-  e = cudaGetLastError();
-  return e == cudaSuccess ? 0 : -static_cast<int>(e) - 1000;
+  return launch_chained(kern, dim3(grid), Cfg::THREADS, Cfg::TOTAL, stream, 1, tmQ, tmK, tmV, p);
 }
 
 inline int launch_na3d(const __nv_bfloat16* q, long long ldq, const __nv_bfloat16* k, long long ldk,

@@ -65,6 +65,7 @@ struct PrePostParams {
 };
 
 constexpr int PREPOST_THREADS = 256;
+constexpr int PREPOST_MAX_SMEM = 220 * 1024;
 
 // Position of a block: tokens [tw0, tw0 + nt) of token row th of batch entry b, levels [td0, td1).
 struct PrePostBlock {
@@ -185,6 +186,7 @@ template <int V>
 __global__ void __launch_bounds__(PREPOST_THREADS, 3)
 preprocess_patches_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ a,
                           const PrePostParams p) {
+  chain_begin();
   extern __shared__ __align__(16) uint8_t pp_smem[];
   constexpr int UR = 4;
   const PrePostBlock k = prepost_block(p);
@@ -309,6 +311,7 @@ template <int V>
 __global__ void __launch_bounds__(PREPOST_THREADS)
 postprocess_fields_kernel(const __nv_bfloat16* __restrict__ y, float* __restrict__ out,
                           const PrePostParams p) {
+  chain_begin();
   extern __shared__ __align__(16) uint8_t pp_smem[];
   const PrePostBlock k = prepost_block(p);
   const int npx = k.nt * p.pw, prow = p.pv * p.ph;
@@ -402,6 +405,7 @@ __device__ __forceinline__ void pixel_geometry(const PrePostParams& p, long long
 
 __global__ void __launch_bounds__(PREPOST_THREADS)
 preprocess_pixels_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ a, const PrePostParams p) {
+  chain_begin();
   const long long plane = static_cast<long long>(p.H) * p.W, cstep = p.D * plane;
   const long long pix = static_cast<long long>(blockIdx.x) * PREPOST_THREADS + threadIdx.x;
   if (pix >= p.B * plane) return;
@@ -442,6 +446,7 @@ preprocess_pixels_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict_
 
 __global__ void __launch_bounds__(PREPOST_THREADS)
 postprocess_pixels_kernel(const __nv_bfloat16* __restrict__ y, float* __restrict__ out, const PrePostParams p) {
+  chain_begin();
   const long long plane = static_cast<long long>(p.H) * p.W, cstep = p.D * plane;
   const long long pix = static_cast<long long>(blockIdx.x) * PREPOST_THREADS + threadIdx.x;
   if (pix >= p.B * plane) return;
@@ -518,7 +523,7 @@ inline int prepost_plan(PrePostParams& p, int unit, int n_units, int word, bool 
   p.DL = static_cast<int>(std::min<long long>(dl, d_tok));
   p.LT = static_cast<int>(std::max<long long>(1, std::min<long long>(p.DL, TILE / (2 * rs * p.NT))));
   const long long bytes = (static_cast<long long>(geo) * p.NT * p.pw + 15) / 16 * 16 + 2 * rs * p.NT * p.LT;
-  if (bytes > 220 * 1024) return -2;
+  if (bytes > PREPOST_MAX_SMEM) return -2;
   *smem = static_cast<int>(bytes);
   *blocks = base * ((d_tok + p.DL - 1) / p.DL);
   return *blocks > 0x7fffffffLL ? -2 : 0;
@@ -543,6 +548,7 @@ struct DealiasParams {
 __global__ void __launch_bounds__(256)
 dealias_patches_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ a,
                        const DealiasParams p) {
+  chain_begin();
   const int d_tok = p.D / p.pv, h_tok = p.H / p.ph, w_tok = p.W / p.pw;
   const int pvol = p.pv * p.ph * p.pw;
   const int K = p.C * pvol;
