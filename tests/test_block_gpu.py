@@ -429,3 +429,22 @@ def test_qkv_without_rope_but_with_qk_norm(ops, C, hd):
     ref_b = bo.block_forward(xb.bfloat16().float(), p, grid=(D, H, W), num_heads=heads,
                              kernel=(1, 3, 3), rope_cos=None, rope_sin=None, qk_norm=True, gated=False)
     assert rel_max_err(yb, ref_b) < TOL_BF16
+
+
+@pytest.mark.parametrize("B,D,H,W,nh,kernel", [
+    (1, 3, 9, 17, 2, (3, 3, 3)), (1, 1, 8, 8, 1, (1, 1, 1)), (2, 5, 15, 5, 1, (5, 15, 5)), (1, 4, 40, 33, 3, (3, 1, 1)),
+    (1, 15, 11, 6, 1, (15, 7, 3)), (2, 9, 50, 70, 12, (3, 3, 3)), (1, 7, 60, 90, 8, (5, 5, 5)), (1, 4, 31, 20, 2, (2, 9, 1)),
+    (1, 3, 12, 13, 1, (3, 4, 5)),
+])
+def test_na3d_narrow_windows(ops, B, D, H, W, nh, kernel):
+    # windows of at most five columns: planes of 8 x 8 queries with ragged edges, single and odd depths, window
+    # = axis, several key-row chunks, blocks with one and with many items (the ring of planes wraps
+    # inside an item and across items), a score range that moves the reference; an even height
+    # stays with the wide kernel
+    g = torch.Generator().manual_seed(D * 100 + H)
+    q, k = ((torch.randn(B, D, H, W, nh, 64, generator=g) * 3).bfloat16() for _ in range(2))
+    v = torch.randn(B, D, H, W, nh, 64, generator=g).bfloat16()
+    out = torch.full((B, D, H, W, nh, 64), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.na3d(q.cuda(), k.cuda(), v.cuda(), kernel, out=out)
+    assert _status() == 0
+    assert rel_max_err(out, bo.na3d(q.float(), k.float(), v.float(), kernel)) < TOL_BF16
