@@ -80,26 +80,26 @@ __device__ __forceinline__ int gemm_out_row(int m, const GemmParams& p) {
   return (t * P + i + p.pad_h) * P + j + p.pad_h;
 }
 
-#ifndef GEMM_USE_PAIRS
-#define GEMM_USE_PAIRS 1
-#endif
-
 constexpr int GEMM_BM = 128;
 constexpr int GEMM_BK = 64;
 constexpr int GEMM_EPI_WARPS = 16;
 constexpr int GEMM_THREADS = 64 + 32 * GEMM_EPI_WARPS;
 
-template <int BN, bool PAIR = false>
+template <int BN, bool PAIR, bool TABLE>
 struct GemmSmem {
   static constexpr int A_BYTES = GEMM_BM * GEMM_BK * 2;
   static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * GEMM_BK * 2;   // a pair splits the W tile
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = (BN == 256 && !PAIR) ? 4 : 6;
+  static constexpr int STAGES = BN == 256 && !PAIR ? (TABLE ? 3 : 4) : (TABLE ? 5 : 6);
   static constexpr int STAGING_BYTES = 32 * 32 * 2;             // one 32-row x 32-col bf16 box
+  // the rotary table rows of a tile's 128 output rows (TABLE: QKV epilogue), 128 bytes each, twice
+  static constexpr int TABLE_BYTES = TABLE ? 2 * GEMM_BM * 128 : 0;
   static constexpr int STAGING_OFF = STAGES * STAGE_BYTES;      // per epilogue warp
-  static constexpr int BAR_OFF = STAGING_OFF + GEMM_EPI_WARPS * STAGING_BYTES;
+  static constexpr int TABLE_OFF = STAGING_OFF + GEMM_EPI_WARPS * STAGING_BYTES;
+  static constexpr int BAR_OFF = TABLE_OFF + TABLE_BYTES;
   static constexpr int BAR_BYTES = 512;
   static constexpr int TOTAL = BAR_OFF + BAR_BYTES + 1024;      // + alignment slack
+  static_assert(TOTAL <= 232448, "shared memory of an SM");
 };
 
 // TMA store of a shared-memory box to global memory (bulk async group of the issuing thread).
@@ -247,12 +247,30 @@ __device__ __forceinline__ bool gemm_wait(uint32_t bar, uint32_t parity, volatil
   return gemm_wait_slow(bar, parity, abort_flag, code);
 }
 
-template <int BN, int EPI, bool PAIR = false>
+// Requests one warp's eight rows [r0, r0 + 8) of the rotary table part of a lane quarter (the 32
+// output rows from m_warp) into shared memory at `tab`, 128 bytes a row, 16-byte chunks swizzled over the
+// banks: one cp.async group.
+__device__ __forceinline__ void gemm_fetch_table(const GemmParams& p, int m_warp, int r0, uint32_t tab) {
+  const int lane = threadIdx.x & 31;
+  const int half = p.head_dim >> 1;
+  const int r = r0 + (lane >> 2);           // a row's chunks: four lanes, two each
+  const int m = min(m_warp + r, p.M - 1);
+  const uint32_t* src = p.rope_cs + (static_cast<long long>(m / p.tokens_per_tile) * p.hw + m % p.hw) * half;
+#pragma unroll
+  for (int ch = lane & 3; ch < 8; ch += 4)
+    if (ch * 4 < half)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tab + r * 128u + ((ch ^ (r & 7)) << 4)),
+                   "l"(src + ch * 4) : "memory");
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+template <int BN, int EPI, bool PAIR>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmOut,
                     const __grid_constant__ CUtensorMap tmAux, const GemmParams p) {
-  using S = GemmSmem<BN, PAIR>;
+  constexpr bool TABLE = EPI == EPI_QKV_ROPE;
+  using S = GemmSmem<BN, PAIR, TABLE>;
   // PAIR: this CTA is rank 0 or 1 of a cluster of two that computes 256 x BN tiles together
   const uint32_t pair_rank = PAIR ? cluster_ctarank() : 0u;
   const int unit = PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
@@ -266,12 +284,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
 
   const uint32_t bar_base = smem_base + S::BAR_OFF;
-  // barriers (8 bytes each): full[STAGES], empty[STAGES], acc_full[2], acc_empty[2], aux[8]
+  // barriers (8 bytes each): full[STAGES], empty[STAGES], acc_full[2], acc_empty[2], aux[warps]; the QKV
+  // epilogue has no aux operand and uses four of those for its table, one per lane quarter
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (S::STAGES + s); };
   auto accf_bar = [&](int b) { return bar_base + 8u * (2 * S::STAGES + b); };
   auto acce_bar = [&](int b) { return bar_base + 8u * (2 * S::STAGES + 2 + b); };
   auto aux_bar = [&](int w) { return bar_base + 8u * (2 * S::STAGES + 4 + w); };
+  [[maybe_unused]] auto tabf_bar = [&](int q) { return aux_bar(q); };
   uint8_t* tail = smem_gen + S::BAR_OFF + 8 * (2 * S::STAGES + 4 + GEMM_EPI_WARPS);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 8);
@@ -282,6 +302,19 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   const int tiles_m = (p.M + TILE_M - 1) / TILE_M;
   const int tiles_n = (p.N + BN - 1) / BN;
   const int num_tiles = tiles_m * tiles_n;
+  // Tile t of the order (row block, then column tile), walked t = unit, unit + n_units, ...: units side by
+  // side share their row block's A and their column tile's W while both are on their way through L2
+  // (one contiguous range per unit, A kept in shared memory over a row block's column tiles, ran 5 %
+  // slower at K = 512, and 10 to 30 % at K = 2048 and 3072 without the keeping). Where the last column
+  // tile is narrower, the column order turns with every round, so that no unit gets only wide ones.
+  const bool ragged = p.N % BN != 0;
+  auto tile_of = [&](int t, int& mt, int& jt) {
+    mt = t / tiles_n;
+    jt = t - mt * tiles_n;
+    if (ragged) jt = (jt + static_cast<int>(static_cast<long long>(mt) * tiles_n / n_units)) % tiles_n;
+  };
+  // columns of column tile j that the MMA computes (the last tile may be narrower)
+  auto tile_cols = [&](int j) { return min(BN, (p.N - j * BN + 31) / 32 * 32); };
   const int num_kb = (p.K + GEMM_BK - 1) / GEMM_BK;
 
   if (threadIdx.x == 0) {
@@ -295,7 +328,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       mbar_init(accf_bar(b), 1);
       mbar_init(acce_bar(b), PAIR ? 2 * GEMM_EPI_WARPS : GEMM_EPI_WARPS);
     }
-    for (int w = 0; w < GEMM_EPI_WARPS; ++w) mbar_init(aux_bar(w), 1);
+    // (a rotary table part is written by the four warps of a lane quarter)
+    for (int w = 0; w < GEMM_EPI_WARPS; ++w) mbar_init(aux_bar(w), TABLE ? 4 : 1);
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -317,8 +351,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       uint32_t phase = 0;
       bool ok = true;
       for (int t = unit; t < num_tiles && ok; t += n_units) {
-        const int m0 = (t / tiles_n) * TILE_M + static_cast<int>(pair_rank) * GEMM_BM;
-        const int n0 = (t % tiles_n) * BN + (PAIR ? static_cast<int>(pair_rank) * (BN / 2) : 0);
+        int mt, jt;
+        tile_of(t, mt, jt);
+        const int m0 = mt * TILE_M + static_cast<int>(pair_rank) * GEMM_BM;
+        // the pair's CTAs supply half of the MMA's columns each
+        const int n0 = jt * BN + (PAIR ? static_cast<int>(pair_rank) * (tile_cols(jt) / 2) : 0);
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(empty_bar(stage), phase ^ 1u, abort_flag, ST_TIMEOUT_PRODUCER)) {
             ok = false;
@@ -351,12 +388,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
     if (lane == 0 && pair_rank == 0) {
-      constexpr uint32_t idesc = umma_idesc_bf16(TILE_M, BN, false, false);
+      constexpr uint32_t idesc0 = umma_idesc_bf16(TILE_M, 0, false, false);
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
       bool ok = true;
       for (int t = unit; t < num_tiles && ok; t += n_units, ++it) {
+        int mt, jt;
+        tile_of(t, mt, jt);
+        const uint32_t idesc = idesc0 | (static_cast<uint32_t>(tile_cols(jt) >> 3) << 17);
         const int buf = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1u;
         if (!mbar_wait(acce_bar(buf), acc_phase ^ 1u, abort_flag, ST_TIMEOUT_MMA)) break;
@@ -408,29 +448,48 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     uint32_t aux_phase = 0;
     int it = 0;
     bool ok = true;
+    // EPI_QKV_ROPE: the rotation table rows (one 4-byte (cos, sin) pair per channel pair of a head: 128
+    // bytes for head_dim 64) are the same for every q / k head. The four warps of a lane quarter bring
+    // the 32 rows of a tile into shared memory together, eight each, while they work on the tile
+    // before; a row is then read by its lane, 16 bytes at a time. (Read from global memory, 32
+    // lanes with 32 different rows take 32 L1 cycles per 16 bytes, over a tile as many as its whole
+    // matrix work: 262144 x 1536, K = 512 took 0.50 ms instead of 0.45.)
+    const uint32_t tab_quarter = smem_base + S::TABLE_OFF + static_cast<uint32_t>(quarter) * 32u * 128u;
+    const bool rope = TABLE && p.rope_cs != nullptr;
+    auto tile_rows = [&](int t) {        // first output row of this warp's quarter in tile t
+      int mt, jt;
+      tile_of(t, mt, jt);
+      return mt * TILE_M + static_cast<int>(pair_rank) * GEMM_BM + quarter * 32;
+    };
+    if (rope && unit < num_tiles) gemm_fetch_table(p, tile_rows(unit), cg * 8, tab_quarter);
     for (int t = unit; t < num_tiles && ok; t += n_units, ++it) {
       const int buf = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1u;
-      const int m0 = (t / tiles_n) * TILE_M + static_cast<int>(pair_rank) * GEMM_BM;
-      const int n_tile0 = (t % tiles_n) * BN;
+      int mt, jt;
+      tile_of(t, mt, jt);
+      const int m0 = mt * TILE_M + static_cast<int>(pair_rank) * GEMM_BM;
+      const int n_tile0 = jt * BN;
       const int m_warp = m0 + quarter * 32;
       const int m = m_warp + lane;
       const bool row_ok = m < p.M;
       const int n_warp0 = n_tile0 + cg * WARP_COLS;
-      // EPI_QKV_ROPE: this row's rotation table (one 4-byte (cos, sin) pair per channel pair of
-      // a head: a single 128-byte line for head_dim 64) is the same for every q / k head. It is
-      // pulled into L1 here, before the accumulator is waited for, and read 32 bytes at a time
-      // where a 16-column group needs it.
-      const uint4* cs_src = nullptr;
       bool rope_tile = false;
-      if constexpr (EPI == EPI_QKV_ROPE) {
-        rope_tile = (p.rope_cs != nullptr) && (n_warp0 < p.rope_cols) && row_ok;
-        if (rope_tile) {
-          const int half = p.head_dim >> 1;
-          const long long trow =
-              static_cast<long long>(m / p.tokens_per_tile) * p.hw + (m % p.hw);
-          cs_src = reinterpret_cast<const uint4*>(p.rope_cs + trow * half);
-          asm volatile("prefetch.global.L1 [%0];" ::"l"(cs_src));
+      [[maybe_unused]] uint32_t tab_row = 0;
+      if constexpr (TABLE) {
+        if (rope) {
+          rope_tile = n_warp0 < p.rope_cols && row_ok;
+          tab_row = tab_quarter + static_cast<uint32_t>(buf) * (GEMM_BM * 128u) + lane * 128u;
+          // this warp's part of the tile's table has arrived; when all four warps say so, the whole has,
+          // and none of them reads the tile before's any more: the next tile's goes there
+          asm volatile("cp.async.wait_group 0;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) mbar_arrive(tabf_bar(quarter));
+          if (!gemm_wait(tabf_bar(quarter), it & 1u, abort_flag, ST_TIMEOUT_EPILOGUE)) {
+            ok = false;
+            break;
+          }
+          if (t + n_units < num_tiles)
+            gemm_fetch_table(p, tile_rows(t + n_units), cg * 8, tab_quarter + static_cast<uint32_t>(buf ^ 1) * (GEMM_BM * 128u));
         }
       }
       bool acc_ready = false;
@@ -497,11 +556,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           if constexpr (EPI == EPI_QKV_ROPE) {
             if (rotate && chunk_live) {
               const int pair0 = ((p.head_dim == 64) ? (n0 & 63) >> 1 : 0) + 8 * g;
-              const uint4* src = cs_src + (pair0 >> 2);
 #pragma unroll
               for (int q = 0; q < 2; ++q) {
-                const uint4 t4 = __ldg(src + q);
-                cs[4 * q] = t4.x; cs[4 * q + 1] = t4.y; cs[4 * q + 2] = t4.z; cs[4 * q + 3] = t4.w;
+                const uint32_t addr = tab_row + ((static_cast<uint32_t>((pair0 >> 2) + q) ^ (lane & 7u)) << 4);
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(cs[4 * q]), "=r"(cs[4 * q + 1]), "=r"(cs[4 * q + 2]), "=r"(cs[4 * q + 3])
+                             : "r"(addr) : "memory");
               }
             }
           }
@@ -585,7 +645,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 
 // Host launcher. A: [M,K] bf16 row-major with row stride lda (elements); W: [N,K] bf16
 // row-major with row stride ldw. Returns 0, or a negative argument error / CUDA error code.
-template <int BN, int EPI, bool PAIR = false>
+template <int BN, int EPI, bool PAIR>
 inline int launch_gemm_t(const __nv_bfloat16* A, long long lda, const __nv_bfloat16* W,
                          long long ldw, const GemmParams& p, int sm_count, cudaStream_t stream) {
   CUtensorMap tmA, tmB;
@@ -618,7 +678,7 @@ inline int launch_gemm_t(const __nv_bfloat16* A, long long lda, const __nv_bfloa
       if (make_tmap_bf16(&tmAux, p.aux, 2, dims, astr, box, TMAP_SWIZZLE_64B) != 0) return -23;
     }
   }
-  using S = GemmSmem<BN, PAIR>;
+  using S = GemmSmem<BN, PAIR, EPI == EPI_QKV_ROPE>;
   auto kern = gemm_tcgen05_kernel<BN, EPI, PAIR>;
   static std::atomic<uint64_t> smem_set;
   if (const cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), S::TOTAL, smem_set); e != cudaSuccess)
@@ -660,16 +720,20 @@ inline int launch_gemm_t(const __nv_bfloat16* A, long long lda, const __nv_bfloa
 template <int EPI>
 inline int launch_gemm(const __nv_bfloat16* A, long long lda, const __nv_bfloat16* W, long long ldw,
                        const GemmParams& p, int sm_count, cudaStream_t stream) {
-  // 128x256 tiles when the output is wide enough to fill the machine with them.
+  // CTA pairs share each MMA (less shared-memory traffic per SM) from 1024 rows on, for every N that
+  // one 128-wide tile does not cover; the last column tile is as narrow as it needs to be.
+  // (With one or two k-blocks a tile is all epilogue, and a ragged N runs faster as 128-wide
+  // tiles of one CTA: 1572864 x 384, K = 128 in 0.34 ms instead of 0.37.)
+  if (p.M >= 1024 && (p.N > 128 || EPI == EPI_QKV_ROPE) &&
+      !(EPI != EPI_QKV_ROPE && p.K <= 128 && p.N < 512 && p.N % 256 != 0 && p.N % 128 == 0)) {
+    return launch_gemm_t<256, EPI, true>(A, lda, W, ldw, p, sm_count, stream);
+  }
   // (the QKV epilogue always takes 256-wide tiles: a warp's 64 columns are then one whole
   // 64-channel head, which the qk norm needs)
-  if ((p.N >= 256 && (p.N % 256 == 0 || p.N > 512)) || EPI == EPI_QKV_ROPE) {
-    // large problems: CTA pairs share each MMA (less shared-memory traffic per SM)
-    if (GEMM_USE_PAIRS && p.M >= 1024)
-      return launch_gemm_t<256, EPI, true>(A, lda, W, ldw, p, sm_count, stream);
-    return launch_gemm_t<256, EPI>(A, lda, W, ldw, p, sm_count, stream);
-  }
-  return launch_gemm_t<128, EPI>(A, lda, W, ldw, p, sm_count, stream);
+  if (EPI == EPI_QKV_ROPE || (p.N >= 256 && (p.N % 256 == 0 || p.N > 512)))
+    return launch_gemm_t<256, EPI, false>(A, lda, W, ldw, p, sm_count, stream);
+  if constexpr (EPI != EPI_QKV_ROPE) return launch_gemm_t<128, EPI, false>(A, lda, W, ldw, p, sm_count, stream);
+  return -24;
 }
 
 }  // namespace strata

@@ -448,3 +448,43 @@ def test_na3d_narrow_windows(ops, B, D, H, W, nh, kernel):
     ops.na3d(q.cuda(), k.cuda(), v.cuda(), kernel, out=out)
     assert _status() == 0
     assert rel_max_err(out, bo.na3d(q.float(), k.float(), v.float(), kernel)) < TOL_BF16
+
+
+@pytest.mark.parametrize("epi", ["none", "residual"])
+@pytest.mark.parametrize("M,N,K", [(1024, 136, 64), (1500, 320, 200), (1025, 640, 512), (41000, 208, 72),
+                                   (22000, 1160, 64), (2560, 384, 128), (1024, 512, 128), (1023, 520, 64)])
+def test_linear_ragged_columns(ops, epi, M, N, K):
+    # the last column tile at its own width, in pairs of CTAs: a few columns, one tile of less than 256, a
+    # wide and a narrow one, and enough tiles that every pair walks several (the column order turns)
+    g = torch.Generator().manual_seed(M + N)
+    x = torch.randn(M, K, generator=g).bfloat16()
+    w = (torch.randn(N, K, generator=g) * 0.05).bfloat16()
+    b = torch.randn(N, generator=g)
+    a = torch.randn(M, N, generator=g).bfloat16()
+    args = (ops.EPI_RESIDUAL, a.cuda()) if epi == "residual" else ()
+    y = ops.linear(x.cuda(), w.cuda(), b.cuda(), *args)
+    assert _status() == 0
+    assert rel_max_err(y, x.float() @ w.float().T + b + (a.float() if args else 0.0)) < TOL_BF16
+
+
+@pytest.mark.parametrize("n_tiles,D,H,W,C,hd,qk_norm", [
+    (3, 5, 23, 60, 192, 64, True), (1, 7, 61, 96, 128, 64, False), (2, 3, 50, 70, 128, 32, False), (1, 1, 5, 7, 64, 64, False),
+])
+def test_qkv_rope_table_over_many_tiles(ops, n_tiles, D, H, W, C, hd, qk_norm):
+    # the rotary table rows are fetched one output tile ahead into two buffers: CTAs with several tiles
+    # (parities wrap), rows whose table index wraps at plane and tile ends inside a tile, 32-wide heads
+    heads = C // hd
+    g = torch.Generator().manual_seed(H)
+    x = torch.randn(n_tiles * D * H * W, C, generator=g).bfloat16()
+    w = (torch.randn(3 * C, C, generator=g) * 0.08).bfloat16()
+    b = torch.randn(3 * C, generator=g) * 0.1
+    lat, lon = tile_latlon(n_tiles, H, W)
+    cos, sin = bo.stereographic_rope_tables(lat, lon, hd, 1, bo.default_rope_length_scale(1))
+    y = ops.qkv_rope(x.cuda(), w.cuda(), b.cuda(), hd, cos.cuda(), sin.cuda(), D * H * W, H * W, qk_norm=qk_norm)
+    assert _status() == 0
+    qkv = (x.float() @ w.float().T + b).reshape(n_tiles, D, H * W, 3, heads, hd)
+    q, k, v = qkv[:, :, :, 0], qkv[:, :, :, 1], qkv[:, :, :, 2]
+    if qk_norm:
+        q, k = bo.rms_norm(q), bo.rms_norm(k)
+    ref = torch.stack([bo.apply_rope(q, cos, sin), bo.apply_rope(k, cos, sin), v], dim=3).reshape(-1, 3 * C)
+    assert rel_max_err(y, ref) < TOL_BF16
