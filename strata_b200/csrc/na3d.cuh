@@ -857,6 +857,8 @@ inline int launch_na3d_t(const __nv_bfloat16* q, long long ldq, const __nv_bfloa
   if (const cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), Cfg::TOTAL, smem_set); e != cudaSuccess)
     return -static_cast<int>(e) - 1000;
   const int grid = p.n_items < 2 * sm_count ? p.n_items : 2 * sm_count;
+  // (more than eight items a CTA are some 100 us: nothing to gain from an early start)
+  if (p.n_items > 8 * grid) return launch_plain(kern, dim3(grid), Cfg::THREADS, Cfg::TOTAL, stream, 1, tmQ, tmK, tmV, p);
   return launch_chained(kern, dim3(grid), Cfg::THREADS, Cfg::TOTAL, stream, 1, tmQ, tmK, tmV, p);
 }
 
