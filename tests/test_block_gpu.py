@@ -488,3 +488,18 @@ def test_qkv_rope_table_over_many_tiles(ops, n_tiles, D, H, W, C, hd, qk_norm):
         q, k = bo.rms_norm(q), bo.rms_norm(k)
     ref = torch.stack([bo.apply_rope(q, cos, sin), bo.apply_rope(k, cos, sin), v], dim=3).reshape(-1, 3 * C)
     assert rel_max_err(y, ref) < TOL_BF16
+
+
+@pytest.mark.parametrize("B,D,H,W,nh,kernel", [
+    (1, 8, 32, 32, 2, (3, 7, 7)), (1, 1, 37, 33, 9, (1, 7, 7)), (1, 5, 19, 18, 2, (3, 9, 9)), (1, 9, 13, 17, 1, (9, 9, 9)),
+    (1, 4, 21, 20, 4, (3, 13, 13)), (1, 6, 18, 31, 1, (5, 15, 15)), (1, 2, 40, 13, 3, (1, 5, 11)),
+])
+def test_na3d_half_tiles(ops, B, D, H, W, nh, kernel):
+    # launches of fewer items than SMs take half query tiles where that shortens the chain of key blocks
+    g = torch.Generator().manual_seed(D * 100 + W)
+    q, k = ((torch.randn(B, D, H, W, nh, 64, generator=g) * 2).bfloat16() for _ in range(2))
+    v = torch.randn(B, D, H, W, nh, 64, generator=g).bfloat16()
+    out = torch.full((B, D, H, W, nh, 64), float("nan"), dtype=torch.bfloat16, device="cuda")
+    ops.na3d(q.cuda(), k.cuda(), v.cuda(), kernel, out=out)
+    assert _status() == 0
+    assert rel_max_err(out, bo.na3d(q.float(), k.float(), v.float(), kernel)) < TOL_BF16
