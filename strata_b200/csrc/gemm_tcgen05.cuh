@@ -249,8 +249,8 @@ __device__ __forceinline__ bool gemm_wait(uint32_t bar, uint32_t parity, volatil
 
 // Requests one warp's eight rows [r0, r0 + 8) of the rotary table part of a lane quarter (the 32
 // output rows from m_warp) into shared memory at `tab`, 128 bytes a row, 16-byte chunks swizzled over the
-// banks: one cp.async group.
-__device__ __forceinline__ void gemm_fetch_table(const GemmParams& p, int m_warp, int r0, uint32_t tab) {
+// banks: one cp.async group. one_row: every row reads the same line, through L1.
+__device__ __forceinline__ void gemm_fetch_table(const GemmParams& p, int m_warp, int r0, uint32_t tab, bool one_row) {
   const int lane = threadIdx.x & 31;
   const int half = p.head_dim >> 1;
   const int r = r0 + (lane >> 2);           // a row's chunks: four lanes, two each
@@ -258,9 +258,11 @@ __device__ __forceinline__ void gemm_fetch_table(const GemmParams& p, int m_warp
   const uint32_t* src = p.rope_cs + (static_cast<long long>(m / p.tokens_per_tile) * p.hw + m % p.hw) * half;
 #pragma unroll
   for (int ch = lane & 3; ch < 8; ch += 4)
-    if (ch * 4 < half)
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tab + r * 128u + ((ch ^ (r & 7)) << 4)),
-                   "l"(src + ch * 4) : "memory");
+    if (ch * 4 < half) {
+      const uint32_t dst = tab + r * 128u + ((ch ^ (r & 7)) << 4);
+      if (one_row) asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src + ch * 4) : "memory");
+      else asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src + ch * 4) : "memory");
+    }
   asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
@@ -456,12 +458,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     // matrix work: 262144 x 1536, K = 512 took 0.50 ms instead of 0.45.)
     const uint32_t tab_quarter = smem_base + S::TABLE_OFF + static_cast<uint32_t>(quarter) * 32u * 128u;
     const bool rope = TABLE && p.rope_cs != nullptr;
+    // (a table of one row - the identity that a q/k norm without rotation runs with - is fetched into both
+    // buffers once: every SM asking L2 for the same line, tile after tile, made QKV of 393216 x 256 take
+    // 0.74 ms instead of 0.27)
+    const bool one_row = p.hw == 1 && p.tokens_per_tile >= p.M;
     auto tile_rows = [&](int t) {        // first output row of this warp's quarter in tile t
       int mt, jt;
       tile_of(t, mt, jt);
       return mt * TILE_M + static_cast<int>(pair_rank) * GEMM_BM + quarter * 32;
     };
-    if (rope && unit < num_tiles) gemm_fetch_table(p, tile_rows(unit), cg * 8, tab_quarter);
+    if (rope && unit < num_tiles) gemm_fetch_table(p, tile_rows(unit), cg * 8, tab_quarter, one_row);
     for (int t = unit; t < num_tiles && ok; t += n_units, ++it) {
       const int buf = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1u;
@@ -488,8 +494,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             ok = false;
             break;
           }
-          if (t + n_units < num_tiles)
-            gemm_fetch_table(p, tile_rows(t + n_units), cg * 8, tab_quarter + static_cast<uint32_t>(buf ^ 1) * (GEMM_BM * 128u));
+          if (t + n_units < num_tiles && !(one_row && it != 0))
+            gemm_fetch_table(p, tile_rows(t + n_units), cg * 8, tab_quarter + static_cast<uint32_t>(buf ^ 1) * (GEMM_BM * 128u), one_row);
         }
       }
       bool acc_ready = false;

@@ -503,3 +503,16 @@ def test_na3d_half_tiles(ops, B, D, H, W, nh, kernel):
     ops.na3d(q.cuda(), k.cuda(), v.cuda(), kernel, out=out)
     assert _status() == 0
     assert rel_max_err(out, bo.na3d(q.float(), k.float(), v.float(), kernel)) < TOL_BF16
+
+
+def test_qk_norm_without_rope_over_many_tiles(ops):
+    # the one-row identity table stays in both buffers while a CTA walks several tiles
+    M, C = 20000, 256
+    g = torch.Generator().manual_seed(17)
+    x = torch.randn(M, C, generator=g).bfloat16()
+    w = (torch.randn(3 * C, C, generator=g) * 0.08).bfloat16()
+    y = ops.qkv_rope(x.cuda(), w.cuda(), None, 64, None, None, M, 1, qk_norm=True)
+    assert _status() == 0
+    qkv = (x.float() @ w.float().T).reshape(M, 3, C // 64, 64)
+    ref = torch.stack([bo.rms_norm(qkv[:, 0]), bo.rms_norm(qkv[:, 1]), qkv[:, 2]], dim=1).reshape(M, 3 * C)
+    assert rel_max_err(y, ref) < TOL_BF16
