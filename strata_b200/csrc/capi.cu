@@ -11,7 +11,6 @@
 #include "gemm_tcgen05.cuh"
 #include "layernorm.cuh"
 #include "na3d.cuh"
-#include "na3d_narrow.cuh"
 #include "halo.cuh"
 #include "prepost.cuh"
 #include "adaln.cuh"
@@ -259,30 +258,6 @@ static int na3d_impl(const void* q, int64_t ldq, const void* k, int64_t ldk, con
   if (kd < 1 || kh < 1 || kw < 1 || kd > D || kh > H || kw > W) return STRATA_ERR_ARG;
   if (B == 0) return STRATA_OK;
   const float sc = scale > 0.f ? scale : 1.0f / sqrtf(static_cast<float>(head_dim));
-  // Narrow windows: why the line lies at five columns is told at the kernel. An even kh would have P V
-  // read half a pair of key rows from behind the box.
-  if (kw <= NA_NARROW_MAX_KW && (kw & 1) && (kh & 1) && kh <= 15 && kd <= 15) {
-    NaNarrowParams p{};
-    p.B = B; p.D = D; p.H = H; p.W = W; p.heads = heads;
-    p.kd = kd; p.kh = kh;
-    p.q_h0 = q_h0; p.q_w0 = q_w0;
-    p.q_H = q_H < 0 ? H : q_H;
-    p.q_W = q_W < 0 ? W : q_W;
-    if (q_h0 < 0 || q_w0 < 0 || p.q_H < 1 || p.q_W < 1 || q_h0 + p.q_H > H || q_w0 + p.q_W > W)
-      return STRATA_ERR_ARG;
-    const bool own = o_H < 0 || o_W < 0;      // the query region itself, stored compactly
-    p.o_h0 = own ? q_h0 : o_h0; p.o_H = own ? p.q_H : o_H;
-    p.o_w0 = own ? q_w0 : o_w0; p.o_W = own ? p.q_W : o_W;
-    if (p.o_h0 > q_h0 || p.o_w0 > q_w0 || p.o_h0 + p.o_H < q_h0 + p.q_H || p.o_w0 + p.o_W < q_w0 + p.q_W)
-      return STRATA_ERR_ARG;
-    p.tiles_d = (D + 1) / 2; p.tiles_h = (p.q_H + 7) / 8; p.tiles_w = (p.q_W + 7) / 8;
-    p.q = static_cast<const __nv_bfloat16*>(q); p.ldq = ldq;
-    p.out = static_cast<__nv_bfloat16*>(out); p.ldo = ldo;
-    p.scale_log2e = sc * 1.4426950408889634f;
-    const int rn = launch_na3d_narrow(static_cast<const __nv_bfloat16*>(k), ldk,
-                                      static_cast<const __nv_bfloat16*>(v), ldv, kw, p, sms, as_stream(stream));
-    return rn == -2 ? STRATA_ERR_UNSUPPORTED : rn;
-  }
   int r = launch_na3d(static_cast<const __nv_bfloat16*>(q), ldq,
                       static_cast<const __nv_bfloat16*>(k), ldk,
                       static_cast<const __nv_bfloat16*>(v), ldv, static_cast<__nv_bfloat16*>(out),

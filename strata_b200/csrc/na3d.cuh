@@ -905,6 +905,8 @@ inline int launch_na3d(const __nv_bfloat16* q, long long ldq, const __nv_bfloat1
     }
     if (best_units == (1 << 30)) return -2;
   }
+  p.q_rows = p.QD * p.QH * p.QW;
+  if (p.QH + kh - 1 > 31) return -2;
   p.q_h0 = q_h0; p.q_w0 = q_w0;
   p.q_H = q_H < 0 ? H : q_H;
   p.q_W = q_W < 0 ? W : q_W;
@@ -918,31 +920,10 @@ inline int launch_na3d(const __nv_bfloat16* q, long long ldq, const __nv_bfloat1
     if (o_h0 > p.q_h0 || o_w0 > p.q_w0 || o_h0 + o_H < p.q_h0 + p.q_H || o_w0 + o_W < p.q_w0 + p.q_W)
       return -1;   // the output window must contain the query region
   }
-  p.tiles_w = (p.q_W + p.QW - 1) / p.QW;
-  auto items_of = [&](int qd, int qh) {
-    return static_cast<long long>((D + qd - 1) / qd) * ((p.q_H + qh - 1) / qh) * p.tiles_w * heads * B;
-  };
-  // Fewer items than SMs: a launch is then one item's chain of key blocks long, and half a tile has fewer
-  // of them (its box is smaller) while the second CTA of an SM, which would be idle, takes the
-  // other half; two CTAs slow each other by a sixth. (2 heads of 4 x 32 x 32 tokens, 3 x 13 x 13:
-  // 18.0 -> 14.6 us; 8 x 20 x 20, 7 x 7 x 7: 18.3 -> 13.7; 8 x 32 x 32, 3 x 7 x 7: 11.4 either way.)
-  if (items_of(p.QD, p.QH) <= sm_count) {
-    auto blocks_of = [&](int qd, int qh) { return ((qd + kd - 1) * ((qh + kh + 2) / 4) + 1) / 2; };
-    int best = 6 * blocks_of(p.QD, p.QH);
-    const int rows = p.QD * p.QH / 2;
-    int bd = p.QD, bh = p.QH;
-    for (int qd = 1; qd <= p.QD && qd <= rows; qd <<= 1) {
-      const int qh = rows / qd;
-      if (qd * qh != rows || qh + kh - 1 > 31 || items_of(qd, qh) > 2 * sm_count) continue;
-      if (7 * blocks_of(qd, qh) < best) { best = 7 * blocks_of(qd, qh); bd = qd; bh = qh; }
-    }
-    p.QD = bd; p.QH = bh;
-  }
-  p.q_rows = p.QD * p.QH * p.QW;
-  if (p.QH + kh - 1 > 31) return -2;
   p.tiles_d = (D + p.QD - 1) / p.QD;
   p.tiles_h = (p.q_H + p.QH - 1) / p.QH;
-  const long long items = items_of(p.QD, p.QH);
+  p.tiles_w = (p.q_W + p.QW - 1) / p.QW;
+  const long long items = static_cast<long long>(p.tiles_d) * p.tiles_h * p.tiles_w * heads * B;
   if (items > 0x7fffffffLL) return -2;
   p.n_items = static_cast<int>(items);
   if (na_build_blocks(p) != 0) return -2;

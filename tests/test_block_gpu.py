@@ -431,25 +431,6 @@ def test_qkv_without_rope_but_with_qk_norm(ops, C, hd):
     assert rel_max_err(yb, ref_b) < TOL_BF16
 
 
-@pytest.mark.parametrize("B,D,H,W,nh,kernel", [
-    (1, 3, 9, 17, 2, (3, 3, 3)), (1, 1, 8, 8, 1, (1, 1, 1)), (2, 5, 15, 5, 1, (5, 15, 5)), (1, 4, 40, 33, 3, (3, 1, 1)),
-    (1, 15, 11, 6, 1, (15, 7, 3)), (2, 9, 50, 70, 12, (3, 3, 3)), (1, 7, 60, 90, 8, (5, 5, 5)), (1, 4, 31, 20, 2, (2, 9, 1)),
-    (1, 3, 12, 13, 1, (3, 4, 5)),
-])
-def test_na3d_narrow_windows(ops, B, D, H, W, nh, kernel):
-    # windows of at most five columns: planes of 8 x 8 queries with ragged edges, single and odd depths, window
-    # = axis, several key-row chunks, blocks with one and with many items (the ring of planes wraps
-    # inside an item and across items), a score range that moves the reference; an even height
-    # stays with the wide kernel
-    g = torch.Generator().manual_seed(D * 100 + H)
-    q, k = ((torch.randn(B, D, H, W, nh, 64, generator=g) * 3).bfloat16() for _ in range(2))
-    v = torch.randn(B, D, H, W, nh, 64, generator=g).bfloat16()
-    out = torch.full((B, D, H, W, nh, 64), float("nan"), dtype=torch.bfloat16, device="cuda")
-    ops.na3d(q.cuda(), k.cuda(), v.cuda(), kernel, out=out)
-    assert _status() == 0
-    assert rel_max_err(out, bo.na3d(q.float(), k.float(), v.float(), kernel)) < TOL_BF16
-
-
 @pytest.mark.parametrize("epi", ["none", "residual"])
 @pytest.mark.parametrize("M,N,K", [(1024, 136, 64), (1500, 320, 200), (1025, 640, 512), (41000, 208, 72),
                                    (22000, 1160, 64), (2560, 384, 128), (1024, 512, 128), (1023, 520, 64)])
@@ -488,21 +469,6 @@ def test_qkv_rope_table_over_many_tiles(ops, n_tiles, D, H, W, C, hd, qk_norm):
         q, k = bo.rms_norm(q), bo.rms_norm(k)
     ref = torch.stack([bo.apply_rope(q, cos, sin), bo.apply_rope(k, cos, sin), v], dim=3).reshape(-1, 3 * C)
     assert rel_max_err(y, ref) < TOL_BF16
-
-
-@pytest.mark.parametrize("B,D,H,W,nh,kernel", [
-    (1, 8, 32, 32, 2, (3, 7, 7)), (1, 1, 37, 33, 9, (1, 7, 7)), (1, 5, 19, 18, 2, (3, 9, 9)), (1, 9, 13, 17, 1, (9, 9, 9)),
-    (1, 4, 21, 20, 4, (3, 13, 13)), (1, 6, 18, 31, 1, (5, 15, 15)), (1, 2, 40, 13, 3, (1, 5, 11)),
-])
-def test_na3d_half_tiles(ops, B, D, H, W, nh, kernel):
-    # launches of fewer items than SMs take half query tiles where that shortens the chain of key blocks
-    g = torch.Generator().manual_seed(D * 100 + W)
-    q, k = ((torch.randn(B, D, H, W, nh, 64, generator=g) * 2).bfloat16() for _ in range(2))
-    v = torch.randn(B, D, H, W, nh, 64, generator=g).bfloat16()
-    out = torch.full((B, D, H, W, nh, 64), float("nan"), dtype=torch.bfloat16, device="cuda")
-    ops.na3d(q.cuda(), k.cuda(), v.cuda(), kernel, out=out)
-    assert _status() == 0
-    assert rel_max_err(out, bo.na3d(q.float(), k.float(), v.float(), kernel)) < TOL_BF16
 
 
 def test_qk_norm_without_rope_over_many_tiles(ops):
