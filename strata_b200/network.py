@@ -9,6 +9,7 @@ from __future__ import annotations
 import ctypes
 
 import torch
+from torch.nn.modules import module as _nn_module
 
 from . import _lib, ops
 
@@ -26,6 +27,69 @@ def _block_struct(weights: dict, out) -> None:
         setattr(out, f"b_{name}", _ptr(weights.get(f"b_{name}")))
 
 
+class Stock:
+    """A module class whose step the library call stands in for, with the methods that step goes
+    through. The call may do so only where nothing else would have run: no subclass, no method replaced
+    on the object or on the class and, for a module that the step calls (`called`), no hook."""
+
+    HOOKS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
+
+    def __init__(self, cls, *methods, called=False):
+        self.cls = cls
+        self._lookup = vars(cls).get
+        self._functions = {n: vars(cls)[n] for n in methods}
+        self._stock = list(self._functions.values())
+        # (_call_impl and _compiled_call_impl: what Module.__call__ and Module.compile() go through)
+        self._names = (*methods, "_call_impl", "_compiled_call_impl") if called else methods
+        self._hooks = self.HOOKS if called else ()
+
+    def class_intact(self) -> bool:
+        return list(map(self._lookup, self._functions)) == self._stock
+
+    def holds(self, m) -> bool:
+        if type(m) is not self.cls:
+            return False
+        v = vars(m)
+        for n in self._names:
+            if n in v:
+                return False
+        for h in self._hooks:
+            if v[h]:
+                return False
+        return True
+
+    def replaced(self, m, *methods) -> bool:
+        """Whether m has one of these methods from somewhere else than the class."""
+        return any(n in vars(m) or getattr(type(m), n) is not self._functions[n] for n in methods)
+
+
+def _stock_parts(backbone, pixel):
+    """(module, Stock) of every module whose own code a step-by-step pass would run."""
+    out = [(backbone, STOCK["backbone"]), (backbone.patch_embed, STOCK["patch_embed"])]
+    out += [(b, STOCK["block"]) for b in backbone.blocks]
+    head = backbone.final_layer
+    if pixel is not None:
+        out += [(pixel, STOCK["pixel"]), (pixel.pixel_patch_embed, STOCK["patch_embed"])]
+        out += [(b, STOCK["pixel_block"]) for b in pixel.pixel_blocks]
+        head = pixel.pixel_final_layer
+    return out + [(head, STOCK["final_layer"])]
+
+
+_GLOBAL_HOOKS = tuple("_global" + h for h in Stock.HOOKS)
+
+
+def _global_hooks() -> bool:
+    """Hooks registered for every module (they run when a block is called)."""
+    for name in _GLOBAL_HOOKS:
+        if getattr(_nn_module, name, None):
+            return True
+    return False
+
+
+# filled in by the modules that define the classes
+STOCK: dict[str, Stock] = {}
+
+
 class NetworkHandle:
     """Descriptors for one `StrataTransformer3D` (and, for the two-stage model, the `Strata` module
     around it). Belongs to the module that owns it; a copy of the module starts with an empty one."""
@@ -37,6 +101,7 @@ class NetworkHandle:
         self._modules = self._params = self._attrs = None
         self._desc = self._pixel = None
         self._keep = None
+        self._parts = self._classes = ()
 
     def __deepcopy__(self, memo):
         return NetworkHandle()
@@ -68,9 +133,25 @@ class NetworkHandle:
                 return False
         return True
 
+    def _take_parts(self, backbone, pixel) -> None:
+        self._parts = _stock_parts(backbone, pixel)
+        self._classes = {s for _, s in self._parts}
+
+    def _all_stock(self) -> bool:
+        for s in self._classes:
+            if not s.class_intact():
+                return False
+        for m, s in self._parts:
+            if not s.holds(m):
+                return False
+        return not _global_hooks()
+
     # ---------------------------------------------------------------- descriptors
     def _build(self, backbone, pixel) -> None:
         self._clear()
+        self._take_parts(backbone, pixel)
+        if not self._all_stock():
+            return          # looked at again on the next call
         attrs = []
         keep = []
 
@@ -182,7 +263,7 @@ class NetworkHandle:
     def forward(self, backbone, pixel, x, lat, lon, wind, concat_lat):
         """x [B, C, D, H, W] fp32, lat / lon [B, H, W] fp32 on x's device -> fields, or None when
         the model has a part that only the step-by-step path runs."""
-        if not self._unchanged():
+        if not (self._unchanged() and self._all_stock()):
             self._build(backbone, pixel)
         d, px = self._desc, self._pixel
         if d is None:

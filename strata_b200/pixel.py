@@ -19,7 +19,7 @@ import torch
 import torch.nn as nn
 
 from . import ops, rope
-from .network import NetworkHandle
+from .network import STOCK, NetworkHandle, Stock
 from .ops import EPI_BIAS, EPI_GATE, EPI_GELU
 from .strata import FinalLayer, Mlp, NeighborhoodAttention3D, PatchEmbed3D, StrataTransformer3D, _triple
 
@@ -255,7 +255,7 @@ class Strata(nn.Module):
         grid = bb.token_grid(D, H, W)
         lat0, lon0, cs = bb.fused_tables(lat, lon, lat0, lon0, wind)
         tokens = bb.embed_fused(x, lat, lon, lat0, lon0, wind, concat_lat)
-        tokens = bb._run_blocks(tokens, grid, cs)
+        tokens = bb._through_blocks(tokens, grid, pos, lat, lon, cs)
         _, _, _, Kpp = self.pixel_patch_embed._gemm_weights()
         ap = ops.preprocess_patches(x, lat, lon, lat0, lon0, wind=wind, concat_lat=concat_lat,
                                     patch=(1, 1, 1), k_pad=Kpp)
@@ -266,3 +266,9 @@ class Strata(nn.Module):
         y, _ = self.pixel_final_layer.matrix_bf16(px)
         return ops.postprocess_fields(y, (B, self.out_channels, D, H, W), lat, lon, lat0, lon0,
                                       wind=wind, patch=(1, 1, 1))
+
+
+STOCK.update(
+    pixel=Stock(Strata, "pixel_stage", "rope_tables_pixel"),
+    pixel_block=Stock(StrataPixel3DBlock, "forward", "modulation", "device_weights", "_gelu_is_tanh",
+                      called=True))

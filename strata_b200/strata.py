@@ -26,7 +26,7 @@ import torch
 import torch.nn as nn
 
 from . import ops, rope
-from .network import NetworkHandle
+from .network import STOCK, NetworkHandle, Stock
 
 
 def _triple(v):
@@ -405,10 +405,19 @@ class StrataTransformer3D(nn.Module):
         grid = self.token_grid(D, H, W)
         lat0, lon0, cs = self.fused_tables(lat, lon, lat0, lon0, wind)
         tokens = self.embed_fused(x, lat, lon, lat0, lon0, wind, concat_lat)
-        tokens = self._run_blocks(tokens, grid, cs)
+        tokens = self._through_blocks(tokens, grid, pos, lat, lon, cs)
         y, _ = self.final_layer.matrix_bf16(tokens)
         return ops.postprocess_fields(y, (B, self.out_channels, D, H, W), lat, lon, lat0, lon0,
                                       wind=wind, patch=self.patch_size)
+
+    def _through_blocks(self, tokens, grid, pos, lat, lon, cs):
+        """The block stack of the step-by-step pass: with the packed table cs, or through `rope_tables`
+        and `forward_tokens` where a subclass brings its own."""
+        if not STOCK["backbone"].replaced(self, "rope_tables", "forward_tokens"):
+            return self._run_blocks(tokens, grid, cs)
+        if pos is None and lat is not None:
+            pos = torch.stack([lat, lon], dim=1)
+        return self.forward_tokens(tokens, grid, *self.rope_tables(pos, tokens.shape[0], grid))
 
     def fused_tables(self, lat, lon, lat0, lon0, wind):
         """(lat0, lon0, packed rotary table) of the tiles: centres only where a wind rotation
@@ -427,3 +436,11 @@ class StrataTransformer3D(nn.Module):
         y = y.reshape(B, d, h, w, pv, ph, pw, c)
         y = y.permute(0, 7, 1, 4, 2, 5, 3, 6)
         return y.reshape(B, c, d * pv, h * ph, w * pw)
+
+
+STOCK.update(
+    backbone=Stock(StrataTransformer3D, "token_grid", "rope_tables", "forward_tokens", "fused_tables",
+                   "embed_fused", "_run_blocks"),
+    patch_embed=Stock(PatchEmbed3D, "tokens_from_patches", "_gemm_weights"),
+    block=Stock(StrataTransformer3DBlock, "forward", "device_weights", "_gelu_is_tanh", called=True),
+    final_layer=Stock(FinalLayer, "matrix_bf16", "_refresh"))

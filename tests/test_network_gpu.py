@@ -80,3 +80,58 @@ def test_one_call_equals_step_by_step(two_stage, over):
         z = m(x, idx)
         m.strata._network = StepByStep()
         assert torch.equal(m(x, idx), z) and not torch.equal(y, z)
+
+
+def _own_block_code(m, seen):
+    """Replaces parts of a model's blocks; every replaced part reports itself in `seen`."""
+    import types
+    bb = getattr(m.strata, "backbone", m.strata)
+    blocks = list(bb.blocks) + list(getattr(m.strata, "pixel_blocks", []))
+    for i, b in enumerate(blocks):
+        b.register_forward_pre_hook(lambda mod, a, i=i: seen.append(("pre", i)))
+        b.register_forward_hook(lambda mod, a, out, i=i: seen.append(("post", i)))
+
+    class Scaled(type(bb.blocks[1])):
+        def forward(self, x, *a, **k):
+            seen.append("subclass")
+            return super().forward(x, *a, **k) * 0.5
+    bb.blocks[1].__class__ = Scaled
+    stock = bb.blocks[0].forward
+
+    def patched(self, *a, **k):
+        seen.append("object")
+        return stock(*a, **k)
+    bb.blocks[0].forward = types.MethodType(patched, bb.blocks[0])
+    return len(blocks)
+
+
+@pytest.mark.parametrize("two_stage", [False, True])
+def test_hooks_and_own_blocks_run(two_stage):
+    from tests.test_network_host import small_model
+    m = _randomised(small_model(two_stage).cuda())
+    x = torch.randn(2, 5, 4, 16, 16, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    lat, lon = tile_latlon(2, 16, 16)
+    idx = {"lat": lat.cuda(), "lon": lon.cuda()}
+    seen = []
+    with torch.no_grad():
+        plain = m(x, idx)
+        n = _own_block_code(m, seen)
+        y = m(x, idx)
+    assert seen.count("subclass") == 1 and seen.count("object") == 1
+    assert [s for s in seen if isinstance(s, tuple)] == [(w, i) for i in range(n) for w in ("pre", "post")]
+    assert torch.isfinite(y).all() and not torch.equal(y, plain)
+
+
+def test_a_hook_that_only_looks_changes_nothing():
+    from tests.test_network_host import small_model
+    m = _randomised(small_model().cuda())
+    x = torch.randn(1, 5, 4, 16, 16, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    lat, lon = tile_latlon(1, 16, 16)
+    idx = {"lat": lat.cuda(), "lon": lon.cuda()}
+    got = []
+    with torch.no_grad():
+        y = m(x, idx)
+        handle = m.strata.blocks[0].register_forward_hook(lambda mod, a, out: got.append(out.clone()))
+        assert torch.equal(m(x, idx), y) and len(got) == 1 and got[0].shape == (1, 64, 128)
+        handle.remove()
+        assert torch.equal(m(x, idx), y) and len(got) == 1
