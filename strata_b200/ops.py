@@ -374,15 +374,27 @@ def _check_fields(x, lat, lon, channels, backbone) -> None:
                          f"{backbone.patch_embed.proj.in_channels}")
 
 
-def tile_tables(lat: torch.Tensor, lon: torch.Tensor, *, centre: bool = False, rope_mode: str = "none",
-                patch: int = 1, length_scale: float = 1.0, rope_base: float = 100.0, head_dim: int = 64):
+def tile_tables(lat: torch.Tensor | None, lon: torch.Tensor | None, *, centre: bool = False,
+                rope_mode: str = "none", patch: int = 1, length_scale: float = 1.0, rope_base: float = 100.0,
+                head_dim: int = 64, shape=None, device=None):
     """Tile centres and the packed rotary table of tiles given by per-pixel lat / lon [B, H, W]
     (fp32 radians). Returns (lat0, lon0, rope_cs): lat0 / lon0 [B] or None; rope_cs the half table
-    [B, (H/patch)*(W/patch), head_dim/2, 2] (see rope.pack_rope_tables) or None."""
-    B, H, W = lat.shape
-    lat = _f32_dev(lat, "lat", (B, H, W))
-    lon = _f32_dev(lon, "lon", (B, H, W))
-    dev = lat.device
+    [B, (H/patch)*(W/patch), head_dim/2, 2] (see rope.pack_rope_tables) or None. The axial table depends
+    on the shape alone: lat and lon may then be None, with shape = (B, H, W) and the device instead."""
+    if not centre and rope_mode == "none":
+        return None, None, None
+    if lat is None or lon is None:
+        if centre or rope_mode != "axial":
+            raise ValueError("tile centres and the stereographic RoPE table need the pixels' lat / lon "
+                             "[B, H, W] (or pos=[B, 2, H, W])")
+        B, H, W = shape
+        dev = torch.device(device)
+        lat = lon = None
+    else:
+        B, H, W = lat.shape
+        lat = _f32_dev(lat, "lat", (B, H, W))
+        lon = _f32_dev(lon, "lon", (B, H, W))
+        dev = lat.device
     mode = {"none": 0, "axial": 1, "stereographic": 2}[rope_mode]
     lat0 = torch.empty(B, device=dev) if centre else None
     lon0 = torch.empty(B, device=dev) if centre else None
@@ -393,10 +405,11 @@ def tile_tables(lat: torch.Tensor, lon: torch.Tensor, *, centre: bool = False, r
     need = int(lib.strata_tile_tables_workspace_bytes(B, H, W))
     ws = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
     p = lambda t: None if t is None else t.data_ptr()
-    with _lib.on_device(lat):
-        _lib.check(lib.strata_tile_tables(lat.data_ptr(), lon.data_ptr(), B, H, W, p(lat0), p(lon0), mode,
+    on = lat0 if cs is None else cs
+    with _lib.on_device(on):
+        _lib.check(lib.strata_tile_tables(p(lat), p(lon), B, H, W, p(lat0), p(lon0), mode,
                                           int(patch), float(length_scale), float(rope_base), int(head_dim),
-                                          p(cs), p(ws), need, _stream_ptr(lat)), "strata_tile_tables")
+                                          p(cs), p(ws), need, _stream_ptr(on)), "strata_tile_tables")
     return lat0, lon0, cs
 
 

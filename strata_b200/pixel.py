@@ -206,8 +206,9 @@ class Strata(nn.Module):
         self.register_buffer("_rope_cos_pixel", cos[0].repeat(self.depth, 1), persistent=False)
         self.register_buffer("_rope_sin_pixel", sin[0].repeat(self.depth, 1), persistent=False)
 
-    def rope_tables_pixel(self, lat: torch.Tensor | None, lon: torch.Tensor | None, n_tiles: int, grid_px):
-        """Packed half (cos, sin) table [n_tiles, H*W, head_dim/2, 2] of the pixel tokens, or None."""
+    def rope_tables_pixel(self, pos: torch.Tensor | None, n_tiles: int, grid_px):
+        """Packed half (cos, sin) table [n_tiles, H*W, head_dim/2, 2] of the pixel tokens, or None;
+        pos [B, 2, H, W] are the pixels' latitudes and longitudes."""
         D, H, W = grid_px
         if self.rope_mode_pixel == "none":
             return None
@@ -216,10 +217,11 @@ class Strata(nn.Module):
             hw = H * W
             return rope.pack_rope_tables(self._rope_cos_pixel[:hw].expand(n_tiles, -1, -1),
                                          self._rope_sin_pixel[:hw].expand(n_tiles, -1, -1))
-        if lat is None:
-            raise ValueError("stereographic RoPE needs the pixels' lat / lon [B, H, W]")
-        return ops.tile_tables(lat, lon, rope_mode="stereographic", length_scale=self.rope_length_scale_pixel,
-                               rope_base=self.rope_base_pixel, head_dim=self.head_dim_pixel)[2]
+        if pos is None:
+            raise ValueError("stereographic RoPE needs pos=[B, 2, H, W] (lat, lon)")
+        return ops.tile_tables(*pos.unbind(1), rope_mode="stereographic",
+                               length_scale=self.rope_length_scale_pixel, rope_base=self.rope_base_pixel,
+                               head_dim=self.head_dim_pixel)[2]
 
     def _check_axial_rope_pixel(self, tokens: int) -> None:
         if self._rope_cos_pixel.shape[0] != tokens:
@@ -243,17 +245,18 @@ class Strata(nn.Module):
                       lat0=None, lon0=None, wind=None, concat_lat: bool = False) -> torch.Tensor:
         """Raw fields [B, C_raw, D, H, W] fp32 in, fields [B, C_out, D, H, W] fp32 out; the wind
         rotation, latitude channels and patch gathering are one kernel per stage on the way in,
-        the un-patchify and inverse rotation one kernel on the way out."""
+        the un-patchify and inverse rotation one kernel on the way out. pos, lat / lon and lat0 / lon0
+        as in `StrataTransformer3D.forward_fused`."""
         bb = self.backbone
         B, _, D, H, W = x.shape
         if self.rope_mode_pixel == "axial":
             self._check_axial_rope_pixel(D * H * W)
-        if type(bb.patch_embed) is PatchEmbed3D and lat0 is None and lat is not None:
+        if pos is None and lat is not None and lat0 is None and type(bb.patch_embed) is PatchEmbed3D:
             y = self._network.forward(bb, self, x, lat, lon, wind, concat_lat)
             if y is not None:
                 return y
         grid = bb.token_grid(D, H, W)
-        lat0, lon0, cs = bb.fused_tables(lat, lon, lat0, lon0, wind)
+        lat0, lon0, cs = bb.fused_tables(pos, lat, lon, lat0, lon0, wind, (B, H, W), x.device)
         tokens = bb.embed_fused(x, lat, lon, lat0, lon0, wind, concat_lat)
         tokens = bb._through_blocks(tokens, grid, pos, lat, lon, cs)
         _, _, _, Kpp = self.pixel_patch_embed._gemm_weights()
@@ -261,8 +264,12 @@ class Strata(nn.Module):
                                     patch=(1, 1, 1), k_pad=Kpp)
         px = self.pixel_patch_embed.tokens_from_patches(ap, B)
         del ap
+        if pos is not None:
+            pos = pos.to(x.device, torch.float32)
+        elif lat is not None:
+            pos = torch.stack([lat, lon], dim=1)
         px = self.pixel_stage(px, tokens.view(B, *grid, bb.embed_dim), (D, H, W),
-                              self.rope_tables_pixel(lat, lon, B, (D, H, W)))
+                              self.rope_tables_pixel(pos, B, (D, H, W)))
         y, _ = self.pixel_final_layer.matrix_bf16(px)
         return ops.postprocess_fields(y, (B, self.out_channels, D, H, W), lat, lon, lat0, lon0,
                                       wind=wind, patch=(1, 1, 1))

@@ -395,15 +395,17 @@ class StrataTransformer3D(nn.Module):
         """Raw fields in, fields out, with the wrapper's pre- and post-processing inside:
         x [B, C_raw, D, H, W] fp32 (before wind rotation and latitude channels), lat / lon [B, H, W]
         -> [B, C_out, D, H, W] fp32 (wind channels rotated back). The tile centres lat0 / lon0 are
-        worked out from lat / lon unless given. One library call; a model with the de-aliased
-        embedding takes its steps one by one."""
-        if type(self.patch_embed) is PatchEmbed3D and lat0 is None and lat is not None:
+        worked out from lat / lon unless given; the rotary table is that of pos [B, 2, H, W] where it
+        is given, else of lat / lon, which only a wind rotation, latitude channels or that table need.
+        One library call from lat / lon alone; otherwise, and for a model with the de-aliased embedding,
+        the steps one by one."""
+        if pos is None and lat is not None and lat0 is None and type(self.patch_embed) is PatchEmbed3D:
             y = self._network.forward(self, None, x, lat, lon, wind, concat_lat)
             if y is not None:
                 return y
         B, _, D, H, W = x.shape
         grid = self.token_grid(D, H, W)
-        lat0, lon0, cs = self.fused_tables(lat, lon, lat0, lon0, wind)
+        lat0, lon0, cs = self.fused_tables(pos, lat, lon, lat0, lon0, wind, (B, H, W), x.device)
         tokens = self.embed_fused(x, lat, lon, lat0, lon0, wind, concat_lat)
         tokens = self._through_blocks(tokens, grid, pos, lat, lon, cs)
         y, _ = self.final_layer.matrix_bf16(tokens)
@@ -419,13 +421,17 @@ class StrataTransformer3D(nn.Module):
             pos = torch.stack([lat, lon], dim=1)
         return self.forward_tokens(tokens, grid, *self.rope_tables(pos, tokens.shape[0], grid))
 
-    def fused_tables(self, lat, lon, lat0, lon0, wind):
-        """(lat0, lon0, packed rotary table) of the tiles: centres only where a wind rotation
-        needs them and the caller has none."""
+    def fused_tables(self, pos, lat, lon, lat0, lon0, wind, shape, device):
+        """(lat0, lon0, packed rotary table) of tiles of shape (B, H, W): centres only where a wind
+        rotation needs them and the caller has none; the table from pos, or from lat / lon."""
         centre = wind is not None and lat0 is None
-        c_lat, c_lon, cs = ops.tile_tables(lat, lon, centre=centre, rope_mode=self.rope_mode,
-                                           patch=self.patch_size[1], length_scale=self.rope_length_scale,
-                                           rope_base=self.rope_base, head_dim=self.head_dim)
+        table = dict(rope_mode=self.rope_mode, patch=self.patch_size[1], length_scale=self.rope_length_scale,
+                     rope_base=self.rope_base, head_dim=self.head_dim, shape=shape, device=device)
+        if pos is None:
+            c_lat, c_lon, cs = ops.tile_tables(lat, lon, centre=centre, **table)
+        else:
+            c_lat, c_lon, _ = ops.tile_tables(lat, lon, centre=centre)
+            cs = ops.tile_tables(*(t.to(device, torch.float32) for t in pos.unbind(1)), **table)[2]
         return (c_lat, c_lon, cs) if centre else (lat0, lon0, cs)
 
     def unpatchify(self, y: torch.Tensor, grid) -> torch.Tensor:

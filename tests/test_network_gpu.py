@@ -135,3 +135,60 @@ def test_a_hook_that_only_looks_changes_nothing():
         assert torch.equal(m(x, idx), y) and len(got) == 1 and got[0].shape == (1, 64, 128)
         handle.remove()
         assert torch.equal(m(x, idx), y) and len(got) == 1
+
+
+@pytest.mark.parametrize("two_stage", [False, True])
+@pytest.mark.parametrize("rope", ["none", "axial", "stereographic"])
+def test_forward_fused_without_latitudes(two_stage, rope):
+    """lat / lon are needed for the wind rotation, the latitude channels and the stereographic table only,
+    and pos may bring the table's."""
+    from tests.test_network_host import small_model
+    over = dict(do_rope_2d_stereographic=rope == "stereographic", do_rope_2d=rope == "axial",
+                do_concat_latitude=False)
+    if two_stage and rope != "none":
+        over["do_rope_2d_stereographic_pixel" if rope == "stereographic" else "do_rope_2d_pixel"] = True
+    net = _randomised(small_model(two_stage, **over).cuda()).strata
+    x = torch.randn(2, 5, 4, 16, 16, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    lat, lon = (t.cuda() for t in tile_latlon(2, 16, 16))
+    pos = torch.stack([lat, lon], 1)
+    with torch.no_grad():
+        want = net.forward_fused(x, None, lat=lat, lon=lon)
+        assert torch.equal(net.forward_fused(x, pos), want)
+        # pos, not lat / lon, is the table's
+        assert torch.equal(net.forward_fused(x, pos, lat=lat + 0.1, lon=lon), want)
+        if rope == "stereographic":
+            with pytest.raises(ValueError, match="lat"):
+                net.forward_fused(x, None)
+        else:
+            assert torch.equal(net.forward_fused(x, None), want)
+        with pytest.raises(ValueError):
+            net.forward_fused(x, None if rope != "stereographic" else pos, wind=(0, 1))
+        moved = net.forward_fused(x, None, lat=lat + 0.3 * torch.rand_like(lat), lon=lon)
+        assert torch.equal(moved, want) == (rope != "stereographic")
+
+
+def test_own_tables_and_block_loop_run():
+    """A subclass's rope_tables and forward_tokens are what its pass goes through."""
+    from strata_b200.strata import StrataTransformer3D
+    from tests.test_network_host import small_model
+    seen = []
+
+    class Own(StrataTransformer3D):
+        def rope_tables(self, pos, n_tiles, grid):
+            seen.append(("tables", tuple(pos.shape)))
+            return super().rope_tables(pos, n_tiles, grid)
+
+        def forward_tokens(self, tokens, grid, rope_cos, rope_sin):
+            seen.append(("tokens", rope_cos.dtype))
+            return super().forward_tokens(tokens, grid, rope_cos, rope_sin)
+    m = _randomised(small_model().cuda())
+    x = torch.randn(1, 5, 4, 16, 16, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    lat, lon = tile_latlon(1, 16, 16)
+    idx = {"lat": lat.cuda(), "lon": lon.cuda()}
+    with torch.no_grad():
+        want = m(x, idx)
+        m.strata.__class__ = Own
+        y = m(x, idx)
+    assert seen == [("tables", (1, 2, 16, 16)), ("tokens", torch.float32)]
+    # the table of tensor operations in fp32 against the kernel's in fp64: a few half values differ by one
+    assert (y - want).norm() < 5e-3 * want.norm()
