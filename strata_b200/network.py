@@ -14,17 +14,44 @@ from torch.nn.modules import module as _nn_module
 from . import _lib, ops
 
 _ROPE_MODES = {"none": 0, "axial": 1, "stereographic": 2}
-_BLOCK_KEYS = ("qkv", "proj", "gate", "fc1", "fc2")
 
 
-def _ptr(t):
-    return None if t is None else t.data_ptr()
+class _Weights:
+    """The tensors a descriptor points to, kept with it; each has the shape the kernels will read and
+    is on the device they run on."""
 
+    def __init__(self, device):
+        self.device = device
+        self.keep = []
 
-def _block_struct(weights: dict, out) -> None:
-    for name in _BLOCK_KEYS:
-        setattr(out, f"w_{name}", _ptr(weights.get(f"w_{name}")))
-        setattr(out, f"b_{name}", _ptr(weights.get(f"b_{name}")))
+    def ptr(self, t, shape, name):
+        if t is None:
+            return None
+        if tuple(t.shape) != shape:
+            raise ValueError(f"{name} must have shape {shape}, got {tuple(t.shape)}")
+        if t.device != self.device:
+            raise _lib.StrataLibraryError(f"{name} is on {t.device}, the input on {self.device}")
+        self.keep.append(t)
+        return t.data_ptr()
+
+    def block(self, w: dict, dim: int, hidden: int, name: str, out) -> None:
+        shapes = {"qkv": (3 * dim, dim), "proj": (dim, dim), "gate": (dim, dim), "fc1": (hidden, dim),
+                  "fc2": (dim, hidden)}
+        for key, shape in shapes.items():
+            setattr(out, f"w_{key}", self.ptr(w.get(f"w_{key}"), shape, f"{name} {key} weight"))
+            setattr(out, f"b_{key}", self.ptr(w.get(f"b_{key}"), shape[:1], f"{name} {key} bias"))
+
+    def embed(self, layer, dim: int, name: str):
+        """(weight, bias, columns of the patch rows) of a patch embedding."""
+        wm, bias, _, kp = layer._gemm_weights()
+        return (self.ptr(wm, (dim, kp), f"{name} weight"), self.ptr(bias, (dim,), f"{name} bias"), kp)
+
+    def head(self, layer, dim: int, name: str):
+        """(weight, bias, output columns) of a final layer."""
+        layer._refresh()
+        wm, b, _ = layer._gemm_cache
+        n = wm.shape[0]
+        return self.ptr(wm, (n, dim), f"{name} weight"), self.ptr(b, (n,), f"{name} bias"), n
 
 
 class Stock:
@@ -100,7 +127,7 @@ class NetworkHandle:
     def _clear(self):
         self._modules = self._params = self._attrs = None
         self._desc = self._pixel = None
-        self._keep = None
+        self._keep = self._device = None
         self._parts = self._classes = ()
 
     def __deepcopy__(self, memo):
@@ -116,8 +143,8 @@ class NetworkHandle:
                         for m in root.modules() for k, p in m._parameters.items() if p is not None]
         self._attrs = attrs
 
-    def _unchanged(self) -> bool:
-        if self._modules is None:
+    def _unchanged(self, device) -> bool:
+        if self._modules is None or self._device != device:
             return False
         for d, items in self._modules:
             if len(d) != len(items):
@@ -147,13 +174,14 @@ class NetworkHandle:
         return not _global_hooks()
 
     # ---------------------------------------------------------------- descriptors
-    def _build(self, backbone, pixel) -> None:
+    def _build(self, backbone, pixel, device) -> None:
         self._clear()
         self._take_parts(backbone, pixel)
         if not self._all_stock():
             return          # looked at again on the next call
         attrs = []
-        keep = []
+        weights = _Weights(device)
+        keep = weights.keep
 
         def kernels_of(blocks):
             attrs.extend((b, "kernel", b.kernel) for b in blocks)
@@ -182,20 +210,17 @@ class NetworkHandle:
         d.hidden = blocks[0].mlp.layers[0].out_features if blocks else bb.embed_dim
         ok = ok and all(b.mlp.layers[0].out_features == d.hidden for b in blocks)
         d.qk_norm = 1 if qk_norm else 0
-        wm, bias, _, kp = bb.patch_embed._gemm_weights()
-        keep += [wm, bias]
-        d.w_embed, d.b_embed, d.k_embed = _ptr(wm), _ptr(bias), kp
+        d.w_embed, d.b_embed, d.k_embed = weights.embed(bb.patch_embed, bb.embed_dim, "patch embedding")
         structs = (_lib.BlockWeights * max(len(blocks), 1))()
-        for s, b in zip(structs, blocks):
-            w = b.device_weights()
-            keep.append(w)
-            _block_struct(w, s)
+        if ok:
+            for i, (s, b) in enumerate(zip(structs, blocks)):
+                weights.block(b.device_weights(), d.dim, d.hidden, f"block {i}:", s)
         kern = kernels_of(blocks)
         d.h_blocks = ctypes.cast(structs, ctypes.POINTER(_lib.BlockWeights))
         d.h_kernels = ctypes.cast(kern, ctypes.POINTER(ctypes.c_int32))
         keep += [structs, kern]
         if bb.final_layer is not None:
-            d.w_head, d.b_head, d.n_head = self._head(bb.final_layer, keep)
+            d.w_head, d.b_head, d.n_head = weights.head(bb.final_layer, bb.embed_dim, "final layer")
         px = None
         if pixel is not None:
             pblocks = list(pixel.pixel_blocks)
@@ -207,51 +232,46 @@ class NetworkHandle:
             px.hidden = pblocks[0].mlp.layers[0].out_features if pblocks else pixel.embed_dim_pixel
             ok = ok and all(b.mlp.layers[0].out_features == px.hidden for b in pblocks)
             px.qk_norm = 1 if pqk else 0
-            wm, bias, _, kp = pixel.pixel_patch_embed._gemm_weights()
-            keep += [wm, bias]
-            px.w_embed, px.b_embed, px.k_embed = _ptr(wm), _ptr(bias), kp
+            px.w_embed, px.b_embed, px.k_embed = weights.embed(pixel.pixel_patch_embed, px.dim,
+                                                               "pixel patch embedding")
             if ok:
-                px.cond_ks = self._pixel_blocks(pblocks, bb, px, keep)
+                px.cond_ks = self._pixel_blocks(pblocks, bb, px, weights)
                 ok = px.cond_ks is not None
             kern = kernels_of(pblocks)
             px.h_kernels = ctypes.cast(kern, ctypes.POINTER(ctypes.c_int32))
             keep.append(kern)
-            px.w_head, px.b_head, px.n_head = self._head(pixel.pixel_final_layer, keep)
-        self._keep = keep
+            px.w_head, px.b_head, px.n_head = weights.head(pixel.pixel_final_layer, px.dim,
+                                                           "pixel final layer")
+        self._keep, self._device = keep, device
         if ok:
             self._desc, self._pixel = d, px
         self._watch(backbone if pixel is None else pixel, attrs)
 
     @staticmethod
-    def _head(layer, keep):
-        layer._refresh()
-        wm, b, _ = layer._gemm_cache
-        keep += [wm, b]
-        return _ptr(wm), _ptr(b), wm.shape[0]
-
-    @staticmethod
-    def _pixel_blocks(pblocks, bb, px, keep):
+    def _pixel_blocks(pblocks, bb, px, weights):
         """Fills px.h_blocks; returns the depthwise kernel size (0: no block is modulated, None:
         the blocks disagree)."""
         lib = _lib.load()
         structs = (_lib.PixelBlockWeights * max(len(pblocks), 1))()
         sizes = set()
-        for s, b in zip(structs, pblocks):
-            w = b.device_weights()
-            keep.append(w)
-            _block_struct(w, s.block)
+        keep, Cb = weights.keep, bb.embed_dim
+        for i, (s, b) in enumerate(zip(structs, pblocks)):
+            w, name = b.device_weights(), f"pixel block {i}:"
+            weights.block(w, px.dim, px.hidden, name, s.block)
             if "w_mod" not in w:
                 continue
             ks = w["w_dw"].shape[-1]
             sizes.add(ks)
-            s.w_dw, s.b_dw = _ptr(w["w_dw"]), _ptr(w["b_dw"])
-            s.w_mod, s.b_mod = _ptr(w["w_mod"]), _ptr(w["b_mod"])
-            n = int(lib.strata_adaln_cond_table_floats(bb.embed_dim, bb.patch_size[1], ks))
+            s.w_dw = weights.ptr(w["w_dw"], (Cb, ks, ks), f"{name} depthwise weight")
+            s.b_dw = weights.ptr(w["b_dw"], (Cb,), f"{name} depthwise bias")
+            s.w_mod = weights.ptr(w["w_mod"], (6 * px.dim, Cb), f"{name} modulation weight")
+            s.b_mod = weights.ptr(w["b_mod"], (6 * px.dim,), f"{name} modulation bias")
+            n = int(lib.strata_adaln_cond_table_floats(Cb, bb.patch_size[1], ks))
             if n:
                 table = torch.empty(n, dtype=torch.float32, device=w["w_dw"].device)
                 with torch.cuda.device(table.device):
                     _lib.check(lib.strata_adaln_cond_table_f32(
-                        w["w_dw"].data_ptr(), bb.embed_dim, bb.patch_size[1], ks, table.data_ptr(),
+                        w["w_dw"].data_ptr(), Cb, bb.patch_size[1], ks, table.data_ptr(),
                         torch.cuda.current_stream().cuda_stream), "strata_adaln_cond_table_f32")
                 keep.append(table)
                 s.cond_table = table.data_ptr()
@@ -261,16 +281,15 @@ class NetworkHandle:
 
     # ---------------------------------------------------------------- one pass
     def forward(self, backbone, pixel, x, lat, lon, wind, concat_lat):
-        """x [B, C, D, H, W] fp32, lat / lon [B, H, W] fp32 on x's device -> fields, or None when
+        """x [B, C, D, H, W], lat / lon [B, H, W], CUDA fp32 on one device -> fields, or None when
         the model has a part that only the step-by-step path runs."""
-        if not (self._unchanged() and self._all_stock()):
-            self._build(backbone, pixel)
+        x, lat, lon = ops.network_inputs(x, lat, lon, x.shape[1] + (2 if concat_lat else 0), backbone)
+        if not (self._unchanged(x.device) and self._all_stock()):
+            self._build(backbone, pixel, x.device)
         d, px = self._desc, self._pixel
         if d is None:
             return None
-        x = x if x.is_contiguous() else x.contiguous()
         B, C, D, H, W = x.shape
-        ops._check_fields(x, lat, lon, C + (2 if concat_lat else 0), backbone)
         d.in_channels = C
         d.concat_lat = 1 if concat_lat else 0
         d.u_idx, d.v_idx = (-1, -1) if wind is None else (int(wind[0]), int(wind[1]))

@@ -360,18 +360,24 @@ def postprocess_fields(y: torch.Tensor, shape, lat=None, lon=None, lat0=None, lo
     return out
 
 
-def _check_fields(x, lat, lon, channels, backbone) -> None:
-    """Shapes of a network call: fields [B, C, D, H, W] with lat / lon [B, H, W], patches that
-    divide the grid, and as many channels as the patch embedding has."""
+def network_inputs(x, lat, lon, channels, backbone):
+    """The inputs of a network call, checked, as the kernels read them (fp32, packed): fields
+    [B, C, D, H, W] and lat / lon [B, H, W] on one CUDA device, patches that divide the grid, and as
+    many channels as the patch embedding has."""
+    if x.dtype != torch.float32 or not x.is_cuda or x.dim() != 5:
+        raise TypeError("x must be a CUDA float32 [B, C, D, H, W] tensor")
     B, _, D, H, W = x.shape
     pv, ph, pw = backbone.patch_size
     if D % pv or H % ph or W % pw:
         raise ValueError(f"grid {(D, H, W)} is not divisible by the patch {(pv, ph, pw)}")
-    if tuple(lat.shape) != (B, H, W) or tuple(lon.shape) != (B, H, W):
-        raise ValueError(f"lat / lon must have shape {(B, H, W)}, got {tuple(lat.shape)}")
+    lat = _f32_dev(lat, "lat", (B, H, W))
+    lon = _f32_dev(lon, "lon", (B, H, W))
+    if lat.device != x.device or lon.device != x.device:
+        raise ValueError(f"lat / lon are on {lat.device} / {lon.device}, the fields on {x.device}")
     if channels != backbone.patch_embed.proj.in_channels:
         raise ValueError(f"{channels} input channels, the patch embedding expects "
                          f"{backbone.patch_embed.proj.in_channels}")
+    return x.contiguous(), lat, lon
 
 
 def tile_tables(lat: torch.Tensor | None, lon: torch.Tensor | None, *, centre: bool = False,

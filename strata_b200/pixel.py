@@ -251,7 +251,8 @@ class Strata(nn.Module):
         B, _, D, H, W = x.shape
         if self.rope_mode_pixel == "axial":
             self._check_axial_rope_pixel(D * H * W)
-        if pos is None and lat is not None and lat0 is None and type(bb.patch_embed) is PatchEmbed3D:
+        if (pos is None and lat is not None and lon is not None and lat0 is None
+                and type(bb.patch_embed) is PatchEmbed3D):
             y = self._network.forward(bb, self, x, lat, lon, wind, concat_lat)
             if y is not None:
                 return y

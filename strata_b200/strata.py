@@ -399,7 +399,8 @@ class StrataTransformer3D(nn.Module):
         is given, else of lat / lon, which only a wind rotation, latitude channels or that table need.
         One library call from lat / lon alone; otherwise, and for a model with the de-aliased embedding,
         the steps one by one."""
-        if pos is None and lat is not None and lat0 is None and type(self.patch_embed) is PatchEmbed3D:
+        if (pos is None and lat is not None and lon is not None and lat0 is None
+                and type(self.patch_embed) is PatchEmbed3D):
             y = self._network.forward(self, None, x, lat, lon, wind, concat_lat)
             if y is not None:
                 return y

@@ -192,3 +192,40 @@ def test_own_tables_and_block_loop_run():
     assert seen == [("tables", (1, 2, 16, 16)), ("tokens", torch.float32)]
     # the table of tensor operations in fp32 against the kernel's in fp64: a few half values differ by one
     assert (y - want).norm() < 5e-3 * want.norm()
+
+
+@pytest.mark.parametrize("two_stage", [False, True])
+def test_inputs_are_checked_and_packed(two_stage):
+    from strata_b200 import _lib
+    from tests.test_network_host import small_model
+    m = _randomised(small_model(two_stage).cuda())
+    net = m.strata
+    x = torch.randn(2, 5, 4, 16, 16, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    lat, lon = (t.cuda() for t in tile_latlon(2, 16, 16))
+    call = lambda x, lat, lon: net.forward_fused(x, None, lat=lat, lon=lon, concat_lat=True)
+    with torch.no_grad():
+        want = call(x, lat, lon)
+        # strided inputs are packed first
+        wide = torch.stack([x, x], -1)[..., 0]
+        rows = lat[:1, :, :1].expand(2, 16, 16)
+        assert not wide.is_contiguous() and not rows.is_contiguous()
+        assert torch.equal(call(wide, lat, lon), want)
+        assert torch.equal(call(x, rows, lon), call(x, rows.contiguous(), lon))
+        for bad in (x.bfloat16(), x.double(), x[0], x.cpu()):
+            with pytest.raises((TypeError, ValueError)):
+                call(bad, lat, lon)
+        for bad in (lat.double(), lat.bfloat16(), lat.cpu()):
+            with pytest.raises(TypeError):
+                call(x, bad, lon)
+        for bad in (lat[:1], lat[:, :8], lat.flatten()):
+            with pytest.raises(ValueError):
+                call(x, lat, bad)
+        with pytest.raises(ValueError, match="input channels"):
+            call(x[:, :4], lat, lon)
+        with pytest.raises(ValueError, match="divisible"):
+            call(x[..., :15], lat[..., :15], lon[..., :15])
+        m.cpu()
+        with pytest.raises(_lib.StrataLibraryError):
+            m(x, {"lat": lat, "lon": lon})
+        m.cuda()
+        assert torch.equal(call(x, lat, lon), want)

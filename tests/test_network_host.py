@@ -5,6 +5,7 @@ import types
 import pytest
 import torch
 
+from strata_b200 import _lib
 from strata_b200.pixel import StrataPixel3DBlock
 from strata_b200.strata import FinalLayer, PatchEmbed3D, StrataTransformer3D, StrataTransformer3DBlock
 from strata_b200.wrappers import StrataBackboneModel, StrataModel
@@ -96,3 +97,55 @@ def test_hooks_on_all_modules_are_seen():
     finally:
         handle.remove()
     assert is_stock(m)
+
+
+# ------------------------------------------------------------------ what the library call is handed
+@pytest.mark.parametrize("two_stage", [False, True])
+def test_host_fields_never_reach_the_library(two_stage):
+    net = small_model(two_stage).strata
+    x, lat = torch.zeros(1, 5, 4, 16, 16), torch.zeros(1, 16, 16)
+    with pytest.raises(TypeError, match="CUDA float32"):
+        net.forward_fused(x, None, lat=lat, lon=lat, concat_lat=True)
+
+
+def build(m, device="cpu"):
+    h = m.strata._network
+    h._build(*parts(m), torch.device(device))
+    return h
+
+
+@pytest.mark.parametrize("two_stage", [False, True])
+def test_weights_on_another_device_are_refused(two_stage):
+    with pytest.raises(_lib.StrataLibraryError, match="is on cpu, the input on meta"):
+        build(small_model(two_stage), "meta")
+
+
+def _linear(n, k):
+    return torch.nn.Linear(k, n)
+
+
+WRONG = {
+    "block 1: proj weight": lambda bb, px: setattr(bb.blocks[1].attn, "proj", _linear(64, 128)),
+    "block 0: fc2 weight": lambda bb, px: bb.blocks[0].mlp.layers.__setitem__(2, _linear(128, 256)),
+    "block 0: qkv weight": lambda bb, px: setattr(bb.blocks[0].attn, "qkv", _linear(256, 128)),
+    "patch embedding weight": lambda bb, px: setattr(bb.patch_embed, "proj",
+                                                     torch.nn.Conv3d(7, 64, (1, 4, 4), (1, 4, 4))),
+    "final layer weight": lambda bb, px: setattr(px.pixel_final_layer if px else bb.final_layer, "linear",
+                                                 _linear(64, 96)),
+    "pixel block 1: fc1 weight": lambda bb, px: px.pixel_blocks[1].mlp.layers.__setitem__(0, _linear(256, 128)),
+    "pixel block 0: modulation weight": lambda bb, px: setattr(px.pixel_blocks[0], "adaln_bilinear_dw_proj",
+                                                               _linear(320, 128)),
+}
+
+
+@pytest.mark.parametrize("two_stage,what", [(t, w) for w in WRONG for t in (False, True)
+                                            if t or not w.startswith("pixel")])
+def test_weights_of_another_shape_are_refused(two_stage, what, monkeypatch):
+    # (laying out the conditioning table is the one step of the build that needs the GPU)
+    monkeypatch.setattr(_lib, "load", lambda: types.SimpleNamespace(
+        strata_adaln_cond_table_floats=lambda *a: 0))
+    m = small_model(two_stage)
+    assert build(m)._desc is not None
+    WRONG[what](*parts(m))
+    with pytest.raises(ValueError, match=what + " must have shape"):
+        build(m)
