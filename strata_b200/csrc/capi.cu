@@ -726,7 +726,7 @@ int64_t strata_tile_tables_workspace_bytes(int B, int H, int W) {
 }
 
 static int tile_tables_impl(const float* lat, const float* lon, int B, int H, int W, float* lat0,
-                            float* lon0, int rope_mode, int patch, double length_scale,
+                            float* lon0, int rope_mode, int patch_h, int patch_w, double length_scale,
                             double rope_base, int head_dim, void* rope_cs, void* workspace,
                             int64_t workspace_bytes, float4* px_fwd, float4* px_inv, float2* px_lat,
                             void* stream) {
@@ -737,8 +737,10 @@ static int tile_tables_impl(const float* lat, const float* lon, int B, int H, in
   if ((lat0 == nullptr) != (lon0 == nullptr)) return STRATA_ERR_ARG;
   const bool sums = lat0 != nullptr || rope_mode == STRATA_ROPE_STEREOGRAPHIC;
   if (sums && (!lat || !lon)) return STRATA_ERR_ARG;
+  // (the stereographic table takes the mean over a square patch; the axial one knows only the token grid)
+  if (rope_mode == STRATA_ROPE_STEREOGRAPHIC && patch_h != patch_w) return STRATA_ERR_UNSUPPORTED;
   if (rope_mode != STRATA_ROPE_NONE &&
-      (!rope_cs || patch <= 0 || patch > H || patch > W || head_dim % 4 || head_dim <= 0 ||
+      (!rope_cs || patch_h <= 0 || patch_w <= 0 || patch_h > H || patch_w > W || head_dim % 4 || head_dim <= 0 ||
        head_dim > 128 || !(length_scale > 0.0) || !(rope_base > 0.0)))
     return STRATA_ERR_ARG;
   const int64_t need = tile_tables_ws_bytes(B, H, W);
@@ -751,9 +753,9 @@ static int tile_tables_impl(const float* lat, const float* lon, int B, int H, in
   p.mode = rope_mode;
   p.lat0 = lat0; p.lon0 = lon0;
   if (rope_mode != STRATA_ROPE_NONE) {
-    p.patch = patch; p.h = H / patch; p.w = W / patch;
+    p.patch = patch_h; p.h = H / patch_h; p.w = W / patch_w;
     p.pairs = head_dim / 2;
-    p.inv_scale = 1.0 / (length_scale * patch * patch);
+    p.inv_scale = 1.0 / (length_scale * patch_h * patch_h);
     const int n = head_dim / 4;
     for (int i = 0; i < n; ++i) p.freq[i] = pow(rope_base, -static_cast<double>(i) / n);
     p.table = static_cast<uint32_t*>(rope_cs);
@@ -765,8 +767,8 @@ int strata_tile_tables(const float* lat, const float* lon, int B, int H, int W, 
                        float* lon0, int rope_mode, int patch, double length_scale, double rope_base,
                        int head_dim, void* rope_cs, void* workspace, int64_t workspace_bytes,
                        void* stream) {
-  return tile_tables_impl(lat, lon, B, H, W, lat0, lon0, rope_mode, patch, length_scale, rope_base, head_dim,
-                          rope_cs, workspace, workspace_bytes, nullptr, nullptr, nullptr, stream);
+  return tile_tables_impl(lat, lon, B, H, W, lat0, lon0, rope_mode, patch, patch, length_scale, rope_base,
+                          head_dim, rope_cs, workspace, workspace_bytes, nullptr, nullptr, nullptr, stream);
 }
 
 // (the stencil table ready, or null)
@@ -820,7 +822,7 @@ static int network_check(const strata_backbone_desc* b, const strata_pixel_desc*
   if (b->dim <= 0 || b->heads <= 0 || b->dim % b->heads || b->hidden <= 0 || b->n_blocks < 0 ||
       b->k_embed <= 0 || (!px && b->n_head <= 0) || (b->n_blocks > 0 && (!b->h_blocks || !b->h_kernels)))
     return STRATA_ERR_ARG;
-  if (b->rope_mode != STRATA_ROPE_NONE && b->patch_h != b->patch_w) return STRATA_ERR_UNSUPPORTED;
+  if (b->rope_mode == STRATA_ROPE_STEREOGRAPHIC && b->patch_h != b->patch_w) return STRATA_ERR_UNSUPPORTED;
   if (px) {
     if (px->dim <= 0 || px->heads <= 0 || px->dim % px->heads || px->hidden <= 0 || px->n_blocks < 0 ||
         px->k_embed <= 0 || px->n_head <= 0 || (px->n_blocks > 0 && (!px->h_blocks || !px->h_kernels)))

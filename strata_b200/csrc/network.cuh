@@ -161,8 +161,8 @@ inline int network_forward(const strata_backbone_desc& b, const strata_pixel_des
   const int hd = b.dim / b.heads, M = static_cast<int>(n.M);
   float* lat0 = wind ? n.lat0 : nullptr;
   float* lon0 = wind ? n.lon0 : nullptr;
-  STRATA_TRY(tile_tables_impl(lat, lon, B, H, W, lat0, lon0, b.rope_mode, b.patch_h, b.rope_length_scale,
-                              b.rope_base, hd, n.rope, n.sums, n.bytes, n.px_fwd, n.px_inv, n.px_lat,
+  STRATA_TRY(tile_tables_impl(lat, lon, B, H, W, lat0, lon0, b.rope_mode, b.patch_h, b.patch_w,
+                              b.rope_length_scale, b.rope_base, hd, n.rope, n.sums, n.bytes, n.px_fwd, n.px_inv, n.px_lat,
                               stream));
   STRATA_TRY(preprocess_impl(x, B, b.in_channels, D, H, W, lat, lon, lat0, lon0, b.u_idx, b.v_idx,
                              b.concat_lat, b.patch_v, b.patch_h, b.patch_w, n.patches, b.k_embed, n.px_fwd,

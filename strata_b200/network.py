@@ -287,7 +287,7 @@ class NetworkHandle:
         if not (self._unchanged(x.device) and self._all_stock()):
             self._build(backbone, pixel, x.device)
         d, px = self._desc, self._pixel
-        if d is None:
+        if d is None or (backbone.rope_mode == "stereographic" and d.patch_h != d.patch_w):
             return None
         B, C, D, H, W = x.shape
         d.in_channels = C

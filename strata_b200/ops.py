@@ -381,12 +381,22 @@ def network_inputs(x, lat, lon, channels, backbone):
 
 
 def tile_tables(lat: torch.Tensor | None, lon: torch.Tensor | None, *, centre: bool = False,
-                rope_mode: str = "none", patch: int = 1, length_scale: float = 1.0, rope_base: float = 100.0,
+                rope_mode: str = "none", patch=1, length_scale: float = 1.0, rope_base: float = 100.0,
                 head_dim: int = 64, shape=None, device=None):
     """Tile centres and the packed rotary table of tiles given by per-pixel lat / lon [B, H, W]
     (fp32 radians). Returns (lat0, lon0, rope_cs): lat0 / lon0 [B] or None; rope_cs the half table
     [B, (H/patch)*(W/patch), head_dim/2, 2] (see rope.pack_rope_tables) or None. The axial table depends
-    on the shape alone: lat and lon may then be None, with shape = (B, H, W) and the device instead."""
+    on the shape alone: lat and lon may then be None, with shape = (B, H, W) and the device instead, and
+    patch may be a pair (height, width)."""
+    ph, pw = (patch, patch) if isinstance(patch, int) else patch
+    if ph != pw and rope_mode == "axial":
+        B, H, W = shape if lat is None else lat.shape
+        c_lat, c_lon, _ = tile_tables(lat, lon, centre=centre)
+        return c_lat, c_lon, tile_tables(None, None, rope_mode="axial", rope_base=rope_base, head_dim=head_dim,
+                                         shape=(B, H // ph, W // pw),
+                                         device=device if lat is None else lat.device)[2]
+    if ph != pw and rope_mode == "stereographic":
+        raise ValueError(f"the stereographic RoPE table needs square patches, got {ph} x {pw}")
     if not centre and rope_mode == "none":
         return None, None, None
     if lat is None or lon is None:
@@ -406,7 +416,7 @@ def tile_tables(lat: torch.Tensor | None, lon: torch.Tensor | None, *, centre: b
     lon0 = torch.empty(B, device=dev) if centre else None
     cs = None
     if mode:
-        cs = torch.empty((B, (H // patch) * (W // patch), head_dim // 2, 2), dtype=torch.float16, device=dev)
+        cs = torch.empty((B, (H // ph) * (W // pw), head_dim // 2, 2), dtype=torch.float16, device=dev)
     lib = _lib.load()
     need = int(lib.strata_tile_tables_workspace_bytes(B, H, W))
     ws = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
@@ -414,7 +424,7 @@ def tile_tables(lat: torch.Tensor | None, lon: torch.Tensor | None, *, centre: b
     on = lat0 if cs is None else cs
     with _lib.on_device(on):
         _lib.check(lib.strata_tile_tables(p(lat), p(lon), B, H, W, p(lat0), p(lon0), mode,
-                                          int(patch), float(length_scale), float(rope_base), int(head_dim),
+                                          int(ph), float(length_scale), float(rope_base), int(head_dim),
                                           p(cs), p(ws), need, _stream_ptr(on)), "strata_tile_tables")
     return lat0, lon0, cs
 

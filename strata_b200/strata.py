@@ -426,7 +426,7 @@ class StrataTransformer3D(nn.Module):
         """(lat0, lon0, packed rotary table) of tiles of shape (B, H, W): centres only where a wind
         rotation needs them and the caller has none; the table from pos, or from lat / lon."""
         centre = wind is not None and lat0 is None
-        table = dict(rope_mode=self.rope_mode, patch=self.patch_size[1], length_scale=self.rope_length_scale,
+        table = dict(rope_mode=self.rope_mode, patch=self.patch_size[1:], length_scale=self.rope_length_scale,
                      rope_base=self.rope_base, head_dim=self.head_dim, shape=shape, device=device)
         if pos is None:
             c_lat, c_lon, cs = ops.tile_tables(lat, lon, centre=centre, **table)

@@ -229,3 +229,41 @@ def test_inputs_are_checked_and_packed(two_stage):
             m(x, {"lat": lat, "lon": lon})
         m.cuda()
         assert torch.equal(call(x, lat, lon), want)
+
+
+@pytest.mark.parametrize("rope,wind", [("axial", None), ("axial", (0, 1)), ("none", (1, 2))])
+@pytest.mark.parametrize("patch", [(1, 4, 2), (2, 2, 8)])
+def test_rectangular_patches(rope, wind, patch):
+    """The axial table is one of the token grid: patches need not be square (one call, steps, and the
+    oracle)."""
+    from strata_b200.strata import StrataTransformer3D
+    from strata_b200.wrappers import _use_tanh_gelu
+    net = StrataTransformer3D(in_channels=7, out_channels=5, input_shape=(4, 16, 24), patch_size=patch,
+                              embed_dim=128, num_heads=2, num_layers=2, attn_kernel=(1, 3, 3),
+                              rope_mode=rope).cuda()
+    _use_tanh_gelu(net)
+    _randomised(net)
+    x = torch.randn(2, 5, 4, 16, 24, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    lat, lon = (t.cuda() for t in tile_latlon(2, 16, 24))
+    with torch.no_grad():
+        y = net.forward_fused(x, None, lat=lat, lon=lon, wind=wind, concat_lat=True)
+        assert y.shape == x.shape and net._network._desc is not None
+        handle = net.blocks[0].register_forward_hook(lambda *a: None)
+        assert torch.equal(net.forward_fused(x, None, lat=lat, lon=lon, wind=wind, concat_lat=True), y)
+        handle.remove()
+        if wind is None:     # the same table by tensor operations, through the plain forward
+            e = lat.view(2, 1, 1, 16, 24).expand(-1, 1, 4, -1, -1)
+            z = net(torch.cat([x, e.cos(), e.sin()], 1), torch.stack([lat, lon], 1))
+            assert (y - z).norm() < 5e-3 * z.norm()
+
+
+def test_rectangular_patches_have_no_stereographic_table():
+    from strata_b200.strata import StrataTransformer3D
+    from strata_b200.wrappers import _use_tanh_gelu
+    net = StrataTransformer3D(in_channels=5, out_channels=5, input_shape=(4, 16, 24), patch_size=(1, 4, 2),
+                              embed_dim=128, num_heads=2, num_layers=1, rope_mode="stereographic").cuda()
+    _use_tanh_gelu(net)
+    x = torch.zeros(1, 5, 4, 16, 24, device="cuda")
+    lat, lon = (t.cuda() for t in tile_latlon(1, 16, 24))
+    with torch.no_grad(), pytest.raises(ValueError, match="square patches"):
+        net.forward_fused(x, None, lat=lat, lon=lon)
