@@ -117,53 +117,23 @@ def _global_hooks() -> bool:
 STOCK: dict[str, Stock] = {}
 
 
-class NetworkHandle:
-    """Descriptors for one `StrataTransformer3D` (and, for the two-stage model, the `Strata` module
-    around it). Belongs to the module that owns it; a copy of the module starts with an empty one."""
+class Described:
+    """The descriptors of a model as it is, and what they were read from. Complete when the constructor
+    returns and never written afterwards, so threads that share the model may share it; a change of the
+    model makes a new one (`current`). desc is None where only the step-by-step path will do."""
 
-    def __init__(self):
-        self._clear()
-
-    def _clear(self):
-        self._modules = self._params = self._attrs = None
-        self._desc = self._pixel = None
-        self._keep = self._device = None
-        self._parts = self._classes = ()
-
-    def __deepcopy__(self, memo):
-        return NetworkHandle()
-
-    def __reduce__(self):
-        return (NetworkHandle, ())
-
-    # ---------------------------------------------------------------- what may change
-    def _watch(self, root, attrs) -> None:
-        self._modules = [(m._modules, tuple(m._modules.items())) for m in root.modules() if m._modules]
-        self._params = [(m._parameters, k, p, p.data_ptr(), p._version)
-                        for m in root.modules() for k, p in m._parameters.items() if p is not None]
-        self._attrs = attrs
-
-    def _unchanged(self, device) -> bool:
-        if self._modules is None or self._device != device:
-            return False
-        for d, items in self._modules:
-            if len(d) != len(items):
-                return False
-            for k, m in items:
-                if d.get(k) is not m:
-                    return False
-        for d, k, p, ptr, version in self._params:
-            if d.get(k) is not p or p._version != version or p.data_ptr() != ptr:
-                return False
-        for obj, name, value in self._attrs:
-            if getattr(obj, name, None) != value:
-                return False
-        return True
-
-    def _take_parts(self, backbone, pixel) -> None:
+    def __init__(self, backbone, pixel, device):
+        self.device = device
+        self.desc = self.pixel = None
+        self.keep = None            # owns what the descriptors point to
+        self._modules = self._owners = self._params = self._ptrs = self._versions = self._attrs = ()
         self._parts = _stock_parts(backbone, pixel)
         self._classes = {s for _, s in self._parts}
+        self.stock = self._all_stock()
+        if self.stock:
+            self._describe(backbone, pixel)
 
+    # ---------------------------------------------------------------- what may change
     def _all_stock(self) -> bool:
         for s in self._classes:
             if not s.class_intact():
@@ -173,14 +143,37 @@ class NetworkHandle:
                 return False
         return not _global_hooks()
 
+    def _watch(self, root, attrs) -> None:
+        self._modules = [(m._modules, dict(m._modules)) for m in root.modules() if m._modules]
+        self._owners = [(m._parameters, k, p) for m in root.modules() for k, p in m._parameters.items()]
+        self._params = [p for _, _, p in self._owners if p is not None]
+        self._ptrs = [p.data_ptr() for p in self._params]
+        self._versions = [p._version for p in self._params]
+        self._attrs = attrs
+
+    def current(self, device) -> bool:
+        """Whether the model is still the one described, for inputs on `device`."""
+        if not self.stock or self.device != device or not self._all_stock():
+            return False
+        for d, was in self._modules:
+            if d != was:
+                return False
+        for d, k, p in self._owners:
+            if d.get(k) is not p:
+                return False
+        if [p._version for p in self._params] != self._versions or [p.data_ptr() for p in self._params] != self._ptrs:
+            return False
+        for obj, name, value in self._attrs:
+            if getattr(obj, name, None) != value:
+                return False
+        return True
+
     # ---------------------------------------------------------------- descriptors
-    def _build(self, backbone, pixel, device) -> None:
-        self._clear()
-        self._take_parts(backbone, pixel)
-        if not self._all_stock():
-            return          # looked at again on the next call
-        attrs = []
-        weights = _Weights(device)
+    def _describe(self, backbone, pixel) -> None:
+        attrs = [(backbone, n, getattr(backbone, n)) for n in ("out_channels", "patch_size", "embed_dim", "num_heads")]
+        if pixel is not None:
+            attrs += [(pixel, n, getattr(pixel, n)) for n in ("embed_dim_pixel", "num_heads_pixel")]
+        weights = _Weights(self.device)
         keep = weights.keep
 
         def kernels_of(blocks):
@@ -242,9 +235,8 @@ class NetworkHandle:
             keep.append(kern)
             px.w_head, px.b_head, px.n_head = weights.head(pixel.pixel_final_layer, px.dim,
                                                            "pixel final layer")
-        self._keep, self._device = keep, device
         if ok:
-            self._desc, self._pixel = d, px
+            self.desc, self.pixel, self.keep = d, px, keep
         self._watch(backbone if pixel is None else pixel, attrs)
 
     @staticmethod
@@ -279,16 +271,35 @@ class NetworkHandle:
         keep.append(structs)
         return None if len(sizes) > 1 else (sizes.pop() if sizes else 0)
 
+
+class NetworkHandle:
+    """The description of one `StrataTransformer3D` (and, for the two-stage model, the `Strata` module
+    around it) that the last pass found. Belongs to the module that owns it; a copy of the module
+    starts with an empty one."""
+
+    def __init__(self):
+        self._state = None      # read and replaced whole
+
+    def __deepcopy__(self, memo):
+        return NetworkHandle()
+
+    def __reduce__(self):
+        return (NetworkHandle, ())
+
     # ---------------------------------------------------------------- one pass
     def forward(self, backbone, pixel, x, lat, lon, wind, concat_lat):
         """x [B, C, D, H, W], lat / lon [B, H, W], CUDA fp32 on one device -> fields, or None when
         the model has a part that only the step-by-step path runs."""
         x, lat, lon = ops.network_inputs(x, lat, lon, x.shape[1] + (2 if concat_lat else 0), backbone)
-        if not (self._unchanged(x.device) and self._all_stock()):
-            self._build(backbone, pixel, x.device)
-        d, px = self._desc, self._pixel
-        if d is None or (backbone.rope_mode == "stereographic" and d.patch_h != d.patch_w):
+        s = self._state
+        if s is None or not s.current(x.device):
+            s = Described(backbone, pixel, x.device)
+            self._state = s
+        if s.desc is None or (backbone.rope_mode == "stereographic" and s.desc.patch_h != s.desc.patch_w):
             return None
+        # the call's own copy takes the values that differ from call to call
+        d = _lib.BackboneDesc.from_buffer_copy(s.desc)
+        px = None if s.pixel is None else _lib.PixelDesc.from_buffer_copy(s.pixel)
         B, C, D, H, W = x.shape
         d.in_channels = C
         d.concat_lat = 1 if concat_lat else 0

@@ -247,7 +247,7 @@ def test_rectangular_patches(rope, wind, patch):
     lat, lon = (t.cuda() for t in tile_latlon(2, 16, 24))
     with torch.no_grad():
         y = net.forward_fused(x, None, lat=lat, lon=lon, wind=wind, concat_lat=True)
-        assert y.shape == x.shape and net._network._desc is not None
+        assert y.shape == x.shape and net._network._state.desc is not None
         handle = net.blocks[0].register_forward_hook(lambda *a: None)
         assert torch.equal(net.forward_fused(x, None, lat=lat, lon=lon, wind=wind, concat_lat=True), y)
         handle.remove()

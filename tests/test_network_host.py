@@ -1,11 +1,12 @@
 """When a forward pass may be one library call: decided on the host, tested without a GPU (the passes
 themselves: tests/test_network_gpu.py)."""
+import sys
 import types
 
 import pytest
 import torch
 
-from strata_b200 import _lib
+from strata_b200 import _lib, network
 from strata_b200.pixel import StrataPixel3DBlock
 from strata_b200.strata import FinalLayer, PatchEmbed3D, StrataTransformer3D, StrataTransformer3DBlock
 from strata_b200.wrappers import StrataBackboneModel, StrataModel
@@ -26,10 +27,21 @@ def parts(m):
     return (m.strata.backbone, m.strata) if isinstance(m, StrataModel) else (m.strata, None)
 
 
+def described(m, device="cpu"):
+    return network.Described(*parts(m), torch.device(device))
+
+
+@pytest.fixture(autouse=True)
+def no_tables(monkeypatch):
+    # (laying out the conditioning table is the one step of a description that needs the GPU)
+    monkeypatch.setattr(_lib, "load", lambda: types.SimpleNamespace(
+        strata_adaln_cond_table_floats=lambda *a: 0))
+
+
 def is_stock(m):
-    h = m.strata._network
-    h._take_parts(*parts(m))
-    return h._all_stock()
+    s = described(m)
+    assert (s.desc is not None) == s.stock
+    return s.stock
 
 
 def _blocks(m):
@@ -108,16 +120,10 @@ def test_host_fields_never_reach_the_library(two_stage):
         net.forward_fused(x, None, lat=lat, lon=lat, concat_lat=True)
 
 
-def build(m, device="cpu"):
-    h = m.strata._network
-    h._build(*parts(m), torch.device(device))
-    return h
-
-
 @pytest.mark.parametrize("two_stage", [False, True])
 def test_weights_on_another_device_are_refused(two_stage):
     with pytest.raises(_lib.StrataLibraryError, match="is on cpu, the input on meta"):
-        build(small_model(two_stage), "meta")
+        described(small_model(two_stage), "meta")
 
 
 def _linear(n, k):
@@ -140,12 +146,80 @@ WRONG = {
 
 @pytest.mark.parametrize("two_stage,what", [(t, w) for w in WRONG for t in (False, True)
                                             if t or not w.startswith("pixel")])
-def test_weights_of_another_shape_are_refused(two_stage, what, monkeypatch):
-    # (laying out the conditioning table is the one step of the build that needs the GPU)
-    monkeypatch.setattr(_lib, "load", lambda: types.SimpleNamespace(
-        strata_adaln_cond_table_floats=lambda *a: 0))
+def test_weights_of_another_shape_are_refused(two_stage, what):
     m = small_model(two_stage)
-    assert build(m)._desc is not None
+    assert described(m).desc is not None
     WRONG[what](*parts(m))
     with pytest.raises(ValueError, match=what + " must have shape"):
-        build(m)
+        described(m)
+
+
+# ------------------------------------------------------------------ what a description was read from
+CHANGES = {
+    "weight in place": lambda bb: bb.blocks[1].attn.proj.weight.mul_(2),
+    "parameter": lambda bb: setattr(bb.blocks[0].attn.qkv, "weight", torch.nn.Parameter(torch.zeros(384, 128))),
+    "module": lambda bb: bb.blocks[0].mlp.layers.__setitem__(2, _linear(128, 512)),
+    "block gone": lambda bb: bb.blocks.__delitem__(1),
+    "window": lambda bb: setattr(bb.blocks[0], "kernel", (3, 5, 5)),
+    "q/k norm": lambda bb: setattr(bb.blocks[0], "qk_norm", True),
+    "exact GELU": lambda bb: setattr(bb.blocks[0].mlp.layers[1], "approximate", "none"),
+    "output channels": lambda bb: setattr(bb, "out_channels", 3),
+    "dtype": lambda bb: bb.double(),
+}
+
+
+@pytest.mark.parametrize("two_stage", [False, True])
+@pytest.mark.parametrize("what", CHANGES)
+def test_a_changed_model_is_described_again(what, two_stage):
+    m = small_model(two_stage)
+    s = described(m)
+    assert s.current(torch.device("cpu")) and not s.current(torch.device("meta"))
+    with torch.no_grad():
+        CHANGES[what](parts(m)[0])
+    assert not s.current(torch.device("cpu"))
+
+
+@pytest.mark.parametrize("two_stage", [False, True])
+def test_threads_share_a_model(two_stage, monkeypatch):
+    """First calls and calls after a change, from several threads at once: none sees half a description,
+    and none the sizes of another thread's call."""
+    import threading
+    m = small_model(two_stage)
+    sizes, seen, errors = {}, [], []
+
+    def forward_f32(dref, pref, x, lat, lon, B, D, H, W, *rest):
+        d = dref._obj
+        seen.append((threading.get_ident(), d.in_channels, d.concat_lat, d.u_idx, B))
+        return 0
+    monkeypatch.setattr(_lib, "load", lambda: types.SimpleNamespace(
+        strata_adaln_cond_table_floats=lambda *a: 0, strata_network_workspace_bytes=lambda *a: 256,
+        strata_network_forward_f32=forward_f32))
+    monkeypatch.setattr(_lib, "on_device", lambda t: _lib._NOTHING)
+    monkeypatch.setattr(_lib, "stream_of", lambda t: 0)
+    monkeypatch.setattr(network.ops, "network_inputs", lambda x, lat, lon, c, bb: (x, lat, lon))
+    bb, px = parts(m)
+    start = threading.Barrier(6)
+
+    def work(i):
+        try:
+            x, lat = torch.zeros(1 + i, 5 + 2 * (i % 2), 4, 16, 16), torch.zeros(1 + i, 16, 16)
+            sizes[threading.get_ident()] = (x.shape[1], (i + 1) % 2, i - 1, 1 + i)
+            for step in range(40):
+                start.wait(60)
+                if i == 0 and step % 4 == 0:
+                    m.strata._network = network.NetworkHandle()
+                y = m.strata._network.forward(bb, px, x, lat, lat, None if i == 0 else (i - 1, i), i % 2 == 0)
+                assert y.shape == (1 + i, 4, 4, 16, 16)
+        except BaseException as e:
+            errors.append(e)
+            start.abort()
+    switch = sys.getswitchinterval()
+    sys.setswitchinterval(1e-5)
+    try:
+        threads = [threading.Thread(target=work, args=(i,)) for i in range(6)]
+        [t.start() for t in threads]
+        [t.join() for t in threads]
+    finally:
+        sys.setswitchinterval(switch)
+    assert not errors, errors
+    assert len(seen) == 6 * 40 and all((s[1:]) == sizes[s[0]] for s in seen)
