@@ -174,6 +174,21 @@ def stream_of(t) -> int:
     return torch._C._cuda_getCurrentRawStream(t.device.index)
 
 
+def settle(device) -> bool:
+    """Called between filling tensors that a module will keep (weights cast for the kernels, tables) and
+    keeping them: waits for the device, after which any stream and thread may read them and nothing in
+    flight reads what they replace. False while a graph is being captured: nothing has run then, the
+    caller must use them in this call only."""
+    import torch
+    if device.type != "cuda":
+        return True
+    with torch.cuda.device(device):
+        if torch.cuda.is_current_stream_capturing():
+            return False
+        torch.cuda.synchronize()
+    return True
+
+
 def exported_names() -> list[str]:
     return sorted(_SIGNATURES)
 

@@ -48,8 +48,7 @@ class _Weights:
 
     def head(self, layer, dim: int, name: str):
         """(weight, bias, output columns) of a final layer."""
-        layer._refresh()
-        wm, b, _ = layer._gemm_cache
+        wm, b, _ = layer._gemm_weights()
         n = wm.shape[0]
         return self.ptr(wm, (n, dim), f"{name} weight"), self.ptr(b, (n,), f"{name} bias"), n
 
@@ -294,7 +293,9 @@ class NetworkHandle:
         s = self._state
         if s is None or not s.current(x.device):
             s = Described(backbone, pixel, x.device)
-            self._state = s
+            # (its conditioning tables are laid out on this call's stream)
+            if s.desc is None or _lib.settle(x.device):
+                self._state = s
         if s.desc is None or (backbone.rope_mode == "stereographic" and s.desc.patch_h != s.desc.patch_w):
             return None
         # the call's own copy takes the values that differ from call to call

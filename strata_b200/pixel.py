@@ -18,7 +18,7 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
-from . import ops, rope
+from . import _lib, ops, rope
 from .network import STOCK, NetworkHandle, Stock
 from .ops import EPI_BIAS, EPI_GATE, EPI_GELU
 from .strata import FinalLayer, Mlp, NeighborhoodAttention3D, PatchEmbed3D, StrataTransformer3D, _triple
@@ -88,7 +88,8 @@ class StrataPixel3DBlock(nn.Module):
             c["w_dw"] = conv.weight.detach().float().reshape(conv.out_channels, ks, ks).contiguous()
             c["b_dw"] = b(conv)
             c["w_mod"], c["b_mod"] = w(self.adaln_bilinear_dw_proj), b(self.adaln_bilinear_dw_proj)
-        self._cache, self._key = c, key
+        if _lib.settle(self.attn.qkv.weight.device):
+            self._cache, self._key = c, key
         return c
 
     def modulation(self, backbone_tokens: torch.Tensor, factor: int) -> torch.Tensor | None:

@@ -25,7 +25,7 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
-from . import ops, rope
+from . import _lib, ops, rope
 from .network import STOCK, NetworkHandle, Stock
 
 
@@ -62,8 +62,10 @@ class PatchEmbed3D(nn.Module):
         wm = torch.zeros(w.shape[0], Kp, dtype=torch.bfloat16, device=w.device)
         wm[:, :K] = w.reshape(w.shape[0], K)
         b = None if self.proj.bias is None else self.proj.bias.detach().float().contiguous()
-        self._gemm_cache, self._gemm_key = (wm, b, K, Kp), key
-        return self._gemm_cache
+        made = (wm, b, K, Kp)
+        if _lib.settle(w.device):
+            self._gemm_cache, self._gemm_key = made, key
+        return made
 
     def tokens_bf16(self, x: torch.Tensor) -> torch.Tensor:
         """[B, C_in, D, H, W] -> bf16 tokens [B, D'*H'*W', embed_dim] on the tensor cores: the
@@ -204,7 +206,8 @@ class StrataTransformer3DBlock(nn.Module):
                  "w_fc2": w(self.mlp.layers[2]), "b_fc2": b(self.mlp.layers[2])}
         if hasattr(self.attn, "gate_proj"):
             cache["w_gate"], cache["b_gate"] = w(self.attn.gate_proj), b(self.attn.gate_proj)
-        self._bf16_cache, self._bf16_key = cache, key
+        if _lib.settle(self.attn.qkv.weight.device):
+            self._bf16_cache, self._bf16_key = cache, key
         return cache
 
     def forward(self, x: torch.Tensor, grid, rope_cs, workspace=None) -> torch.Tensor:
@@ -236,25 +239,30 @@ class FinalLayer(nn.Module):
         y, N = self.matrix_bf16(tokens)
         return y[:, :N].float().view(*lead, N)
 
-    def _refresh(self) -> None:
+    def _gemm_weights(self):
+        """(weight [N padded to a multiple of 8, dim], bias, N) for the GEMM, re-cast when a parameter
+        changes."""
         key = tuple((p.data_ptr(), p._version, p.device) for p in self.linear.parameters())
-        if self._gemm_cache is None or key != self._gemm_key:
-            w = self.linear.weight.detach()
-            N = w.shape[0]
-            Np = (N + 7) // 8 * 8
-            wm = torch.zeros(Np, w.shape[1], dtype=torch.bfloat16, device=w.device)
-            wm[:N] = w
-            b = None
-            if self.linear.bias is not None:
-                b = torch.zeros(Np, dtype=torch.float32, device=w.device)
-                b[:N] = self.linear.bias.detach().float()
-            self._gemm_cache, self._gemm_key = (wm, b, N), key
+        if self._gemm_cache is not None and key == self._gemm_key:
+            return self._gemm_cache
+        w = self.linear.weight.detach()
+        N = w.shape[0]
+        Np = (N + 7) // 8 * 8
+        wm = torch.zeros(Np, w.shape[1], dtype=torch.bfloat16, device=w.device)
+        wm[:N] = w
+        b = None
+        if self.linear.bias is not None:
+            b = torch.zeros(Np, dtype=torch.float32, device=w.device)
+            b[:N] = self.linear.bias.detach().float()
+        made = (wm, b, N)
+        if _lib.settle(w.device):
+            self._gemm_cache, self._gemm_key = made, key
+        return made
 
     def matrix_bf16(self, tokens: torch.Tensor):
         """bf16 tokens [..., dim] -> (bf16 [rows, Np], N): the layer's output rows, N valid
         columns of a row stride padded to a multiple of 8."""
-        self._refresh()
-        wm, b, N = self._gemm_cache
+        wm, b, N = self._gemm_weights()
         return ops.linear(ops.layernorm(tokens.reshape(-1, tokens.shape[-1])), wm, b), N
 
 
@@ -450,4 +458,4 @@ STOCK.update(
                    "embed_fused", "_run_blocks"),
     patch_embed=Stock(PatchEmbed3D, "tokens_from_patches", "_gemm_weights"),
     block=Stock(StrataTransformer3DBlock, "forward", "device_weights", "_gelu_is_tanh", called=True),
-    final_layer=Stock(FinalLayer, "matrix_bf16", "_refresh"))
+    final_layer=Stock(FinalLayer, "matrix_bf16", "_gemm_weights"))

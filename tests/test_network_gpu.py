@@ -267,3 +267,51 @@ def test_rectangular_patches_have_no_stereographic_table():
     lat, lon = (t.cuda() for t in tile_latlon(1, 16, 24))
     with torch.no_grad(), pytest.raises(ValueError, match="square patches"):
         net.forward_fused(x, None, lat=lat, lon=lon)
+
+
+@pytest.mark.parametrize("two_stage", [False, True])
+def test_first_passes_on_two_streams(two_stage):
+    """Weights are cast and tables laid out by the first pass, on its stream; a pass on another stream
+    that is issued right behind it reads them whole."""
+    from tests.test_network_host import small_model
+    x = torch.randn(2, 5, 4, 16, 16, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    lat, lon = tile_latlon(2, 16, 16)
+    idx = {"lat": lat.cuda(), "lon": lon.cuda()}
+    m = _randomised(small_model(two_stage).cuda())
+    with torch.no_grad():
+        want = m(x, idx)
+        m.strata._network = type(m.strata._network)()
+        for mod in m.modules():
+            for name in ("_gemm_cache", "_bf16_cache", "_cache"):
+                if getattr(mod, name, None) is not None:
+                    setattr(mod, name, None)
+        torch.cuda.synchronize()
+        out = []
+        for _ in range(2):
+            with torch.cuda.stream(torch.cuda.Stream()):
+                torch.cuda._sleep(20_000_000)
+                out.append(m(x, idx))
+        torch.cuda.synchronize()
+        assert all(torch.equal(y, want) for y in out)
+
+
+@pytest.mark.parametrize("two_stage", [False, True])
+def test_first_pass_under_capture(two_stage):
+    """Casts that a capture records exist in its replays only; later calls make their own."""
+    from tests.test_network_host import small_model
+    x = torch.randn(2, 5, 4, 16, 16, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    lat, lon = tile_latlon(2, 16, 16)
+    idx = {"lat": lat.cuda(), "lon": lon.cuda()}
+    m = _randomised(small_model(two_stage).cuda())
+    with torch.no_grad():
+        want = m(x, idx)                              # (the library's kernels are loaded)
+        fresh = _randomised(small_model(two_stage).cuda())
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            y = fresh(x, idx)
+        assert fresh.strata._network._state is None
+        assert torch.equal(fresh(x, idx), want)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, want)
+        del graph

@@ -223,3 +223,18 @@ def test_threads_share_a_model(two_stage, monkeypatch):
         sys.setswitchinterval(switch)
     assert not errors, errors
     assert len(seen) == 6 * 40 and all((s[1:]) == sizes[s[0]] for s in seen)
+
+
+@pytest.mark.parametrize("settled", [True, False])
+def test_casts_are_kept_only_once_settled(settled, monkeypatch):
+    """What a module keeps for later calls was waited for; under capture (not settled) nothing is kept."""
+    calls = []
+    monkeypatch.setattr(_lib, "settle", lambda device: calls.append(device) or settled)
+    bb, px = parts(small_model(True))
+    makers = [bb.patch_embed._gemm_weights, px.pixel_final_layer._gemm_weights, bb.blocks[0].device_weights,
+              px.pixel_blocks[1].device_weights]
+    for make in makers:
+        n = len(calls)
+        first = make()
+        assert len(calls) == n + 1
+        assert (make() is first) == settled and len(calls) == n + (1 if settled else 2)
