@@ -315,7 +315,6 @@ class StrataTransformer3D(nn.Module):
         self.blocks = nn.ModuleList(blocks)
         pv, ph, pw = self.patch_size
         self.final_layer = FinalLayer(embed_dim, pv * ph * pw * out_channels)
-        self._workspace = None
         self._network = NetworkHandle()
 
     # ---------------------------------------------------------------- geometry
@@ -340,13 +339,11 @@ class StrataTransformer3D(nn.Module):
                                               self.rope_length_scale, self.rope_base)
 
     def _get_workspace(self, M: int, device) -> torch.Tensor:
+        """Scratch of one pass through the blocks. Each pass takes its own: the allocator hands it out by
+        stream, so passes on several streams or threads do not write into one another's."""
         hidden = self.blocks[0].mlp.layers[0].out_features
-        need = ops.block_workspace_bytes(M, self.embed_dim, hidden)
-        ws = self._workspace
-        if ws is None or ws.numel() < need or ws.device != device:
-            ws = torch.empty(need, dtype=torch.uint8, device=device)
-            self._workspace = ws
-        return ws
+        return torch.empty(ops.block_workspace_bytes(M, self.embed_dim, hidden), dtype=torch.uint8,
+                           device=device)
 
     # ---------------------------------------------------------------- forward
     def forward_tokens(self, tokens: torch.Tensor, grid, rope_cos, rope_sin) -> torch.Tensor:

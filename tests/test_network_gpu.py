@@ -315,3 +315,29 @@ def test_first_pass_under_capture(two_stage):
         torch.cuda.synchronize()
         assert torch.equal(y, want)
         del graph
+
+
+def test_step_by_step_passes_on_two_streams():
+    """Passes that are in flight at the same time have scratch of their own."""
+    from tests.test_network_host import small_model
+    m = _randomised(small_model().cuda())
+    m.strata.blocks[0].register_forward_hook(lambda *a: None)
+    g = torch.Generator("cuda").manual_seed(1)
+    xs = [torch.randn(2, 5, 4, 16, 16, device="cuda", generator=g) for _ in range(4)]
+    lat, lon = tile_latlon(2, 16, 16)
+    idx = {"lat": lat.cuda(), "lon": lon.cuda()}
+    with torch.no_grad():
+        want = [m(x, idx) for x in xs]
+        torch.cuda.synchronize()
+        spaces = []
+        for _ in xs:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                spaces.append(m.strata._get_workspace(512, xs[0].device))
+        assert len({t.data_ptr() for t in spaces}) == len(xs)
+        out = []
+        for x in xs:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                torch.cuda._sleep(10_000_000)
+                out.append(m(x, idx))
+        torch.cuda.synchronize()
+    assert all(torch.equal(y, w) for y, w in zip(out, want))
