@@ -43,12 +43,25 @@ def _module(handle: int) -> torch.nn.Module:
         raise RuntimeError(f"strata_b200::network_forward: no live module with handle {handle}") from None
 
 
+def _transform_probe():
+    """A function that says whether a dispatch mode or a functorch transform (vmap, grad, jvp) is
+    active. torch has no public call for either; without the private ones the answer is always yes."""
+    modes = getattr(torch._C, "_len_torch_dispatch_stack", None)
+    transforms = getattr(getattr(torch._C, "_functorch", None), "peek_interpreter_stack", None)
+    if modes is None or transforms is None:
+        return lambda: True
+    return lambda: modes() != 0 or transforms() is not None
+
+
+_transformed = _transform_probe()
+
+
 def plain_call(x: torch.Tensor) -> bool:
-    """Nothing is tracing this call - no compiler, no dispatch mode, a plain CUDA tensor that asks
-    for no gradient: the module's forward may then run directly, without the ~50 us the operator's
-    Python dispatch takes."""
+    """Nothing is tracing or transforming this call - no compiler, no dispatch mode, no functorch
+    transform, a plain CUDA tensor that asks for no gradient: the module's forward may then run
+    directly, without the ~50 us the operator's Python dispatch takes."""
     return (type(x) is torch.Tensor and x.is_cuda and not torch.compiler.is_compiling()
-            and torch._C._len_torch_dispatch_stack() == 0 and not (x.requires_grad and torch.is_grad_enabled()))
+            and not _transformed() and not (x.requires_grad and torch.is_grad_enabled()))
 
 
 @torch.library.custom_op("strata_b200::network_forward", mutates_args=())

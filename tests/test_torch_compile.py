@@ -97,6 +97,27 @@ def test_fine_grained_operators_have_fake_implementations():
                                                    False).shape == xb.shape
 
 
+def test_transforms_and_modes_are_noticed(monkeypatch):
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from strata_b200 import torch_ops
+    seen = []
+
+    def f(x):
+        seen.append(torch_ops._transform_probe()())
+        return x
+    f(torch.zeros(2))
+    torch.vmap(f)(torch.zeros(2, 3))
+    torch.func.grad(lambda x: f(x).sum())(torch.zeros(2))
+    with FakeTensorMode():
+        f(torch.zeros(2))
+    assert seen == [False, True, True, True]
+    # a torch without the private calls: every call goes through the operator
+    for holder, name in ((torch._C, "_len_torch_dispatch_stack"), (torch._C._functorch, "peek_interpreter_stack")):
+        with monkeypatch.context() as mp:
+            mp.delattr(holder, name)
+            assert torch_ops._transform_probe()()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("backend,fullgraph", [("eager", True), ("inductor", False)])
 def test_compiled_network_equals_eager(backend, fullgraph):
@@ -120,3 +141,21 @@ def test_compiled_network_equals_eager(backend, fullgraph):
     xb = torch.randn(256, 128, device="cuda").bfloat16()
     w = (torch.randn(64, 128, device="cuda") * 0.05).bfloat16()
     assert torch.equal(torch.ops.strata_b200.linear(xb, w, None, 0, None), ops.linear(xb, w))
+
+
+@pytest.mark.gpu
+def test_vmap_over_the_network():
+    """torch.vmap runs the operator sample by sample, as for any operator without a batching rule."""
+    m = _small_backbone().cuda().eval()
+    g = torch.Generator("cuda").manual_seed(0)
+    with torch.no_grad():
+        for p in m.parameters():
+            p.copy_(torch.randn(p.shape, generator=g, device="cuda") * 0.05)
+        x = torch.randn(3, 2, 5, 4, 16, 16, device="cuda", generator=g)
+        lat = torch.rand(3, 2, 16, 16, device="cuda", generator=g) * 0.5
+        lon = torch.rand(3, 2, 16, 16, device="cuda", generator=g) * 0.5
+        want = torch.stack([m(x[i], {"lat": lat[i], "lon": lon[i]}) for i in range(3)])
+        got = torch.vmap(lambda x, lat, lon: m(x, {"lat": lat, "lon": lon}))(x, lat, lon)
+        assert torch.equal(got, want)
+        got = torch.vmap(lambda lat: m(x[0], {"lat": lat, "lon": lon[0]}))(lat)
+    assert torch.equal(got[0], want[0])
