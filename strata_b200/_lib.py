@@ -168,10 +168,23 @@ def on_device(t):
     return _NOTHING if t.device.index == torch.cuda.current_device() else torch.cuda.device(t.device)
 
 
+def _stream_lookup():
+    """Device index -> raw handle of its current stream. torch's raw lookup is private; without it the
+    stream object is asked (4 us more a call)."""
+    import torch
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw if raw is not None else lambda index: torch.cuda.current_stream(index).cuda_stream
+
+
+_current_stream = None
+
+
 def stream_of(t) -> int:
     """Raw handle of the current stream of t's device."""
-    import torch
-    return torch._C._cuda_getCurrentRawStream(t.device.index)
+    global _current_stream
+    if _current_stream is None:
+        _current_stream = _stream_lookup()
+    return _current_stream(t.device.index)
 
 
 def settle(device) -> bool:

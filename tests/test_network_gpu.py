@@ -341,3 +341,13 @@ def test_step_by_step_passes_on_two_streams():
                 out.append(m(x, idx))
         torch.cuda.synchronize()
     assert all(torch.equal(y, w) for y, w in zip(out, want))
+
+
+def test_raw_stream_lookup_agrees(monkeypatch):
+    from strata_b200 import _lib
+    x = torch.zeros(1, device="cuda")
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        assert _lib.stream_of(x) == side.cuda_stream
+        monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
+        assert _lib._stream_lookup()(x.device.index) == side.cuda_stream

@@ -238,3 +238,12 @@ def test_casts_are_kept_only_once_settled(settled, monkeypatch):
         first = make()
         assert len(calls) == n + 1
         assert (make() is first) == settled and len(calls) == n + (1 if settled else 2)
+
+
+def test_streams_are_found_without_the_private_lookup(monkeypatch):
+    monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
+    monkeypatch.setattr(torch.cuda, "current_stream",
+                        lambda index: types.SimpleNamespace(cuda_stream=1000 + index))
+    monkeypatch.setattr(_lib, "_current_stream", None)
+    t = types.SimpleNamespace(device=torch.device("cuda", 3))
+    assert _lib.stream_of(t) == 1003
