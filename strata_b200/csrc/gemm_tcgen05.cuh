@@ -728,10 +728,18 @@ inline int launch_gemm(const __nv_bfloat16* A, long long lda, const __nv_bfloat1
                        const GemmParams& p, int sm_count, cudaStream_t stream) {
   // CTA pairs share each MMA (less shared-memory traffic per SM) from 1024 rows on, for every N that
   // one 128-wide tile does not cover; the last column tile is as narrow as it needs to be.
-  // (With one or two k-blocks a tile is all epilogue, and a ragged N runs faster as 128-wide
-  // tiles of one CTA: 1572864 x 384, K = 128 in 0.34 ms instead of 0.37.)
-  if (p.M >= 1024 && (p.N > 128 || EPI == EPI_QKV_ROPE) &&
-      !(EPI != EPI_QKV_ROPE && p.K <= 128 && p.N < 512 && p.N % 256 != 0 && p.N % 128 == 0)) {
+  // Except where the last tile is half one and a tile has two k-blocks at most: it is then all epilogue, the
+  // pair's two column tiles of 256 and 128 take turns at unequal lengths, and equal 128-wide tiles of one
+  // CTA run faster - as long as A's rows are whole pieces of a line (K = 32, 64, 128), for A is read once
+  // per column tile. Microseconds of pairs / of 128-wide tiles, at 1572864, 196608 and 24576 rows:
+  //   N = 384: K = 32 309 / 233, 51 / 40, 10.2 / 7.7; K = 64 314 / 231, 45 / 34, 10.0 / 7.3;
+  //            K = 128 318 / 293, 47 / 41, 10.6 / 8.3
+  //   N = 640: K = 64 487 / 378, 68 / 53, 12.0 / 10.1; K = 128 510 / 483, 69 / 64, 12.8 / 11.6
+  //   the other way: K = 8 N = 384 465 / 679, 76 / 85, 13.4 / 14.8; K = 120 395 / 630, 55 / 72, 12.7 / 11.6;
+  //            K = 192 372 / 388, 54 / 54, 12.3 / 10.2; N = 448 K = 128 339 / 458, 52 / 65, 11.8 / 12.3
+  if (p.M >= 1024 && (p.N > 128 || EPI == EPI_QKV_ROPE)) {
+    if (EPI != EPI_QKV_ROPE && p.N % 256 == 128 && p.K >= 32 && 128 % p.K == 0)
+      return launch_gemm_t<128, EPI, false>(A, lda, W, ldw, p, sm_count, stream);
     return launch_gemm_t<256, EPI, true>(A, lda, W, ldw, p, sm_count, stream);
   }
   // Few rows: a launch is one tile's latency long, and a 128-wide tile has half the epilogue of a 256-wide

@@ -482,3 +482,18 @@ def test_qk_norm_without_rope_over_many_tiles(ops):
     qkv = (x.float() @ w.float().T).reshape(M, 3, C // 64, 64)
     ref = torch.stack([bo.rms_norm(qkv[:, 0]), bo.rms_norm(qkv[:, 1]), qkv[:, 2]], dim=1).reshape(M, 3 * C)
     assert rel_max_err(y, ref) < TOL_BF16
+
+
+@pytest.mark.parametrize("M,N,K", [(m, n, k) for m, n in ((1024, 384), (1155, 640), (20001, 384), (4100, 896))
+                                   for k in (8, 24, 32, 64, 96, 128, 136)])
+def test_linear_half_last_tile(ops, M, N, K):
+    # a last column tile of 128 behind tiles of 256: 128-wide tiles of one CTA at K = 32, 64 and 128, pairs
+    # otherwise; both sum the k-blocks in the same order, so columns do not depend on the route
+    g = torch.Generator().manual_seed(M + N + K)
+    x = torch.randn(M, K, generator=g).bfloat16().cuda()
+    w = (torch.randn(N + 128, K, generator=g) * 0.05).bfloat16().cuda()
+    b = torch.randn(N + 128, generator=g).cuda()
+    y = ops.linear(x, w[:N], b[:N])
+    assert _status() == 0
+    assert rel_max_err(y, x.float() @ w[:N].float().T + b[:N]) < TOL_BF16
+    assert torch.equal(y, ops.linear(x, w, b)[:, :N])          # N + 128 is a multiple of 256: pairs
