@@ -128,14 +128,22 @@ halo_gather_tokens_kernel(__nv_bfloat16* __restrict__ out, const PeerPtrs src,
 // x over 256 cells, y over the leading index), a cell's index work done once for all of them.
 // Bound: HBM, through the bytes in flight - with a 4-byte access per thread it takes all of an
 // SM's threads and several loads each to cover ~1 us of latency at 6.5 TB/s (44 KB per SM); UL
-// independent loads stand before a thread's first use. Measured on 24 tiles of 64 x 64, halo 8, 512
-// leading indices (516 MB read + written), before -> now, four loads in flight and a walk over
-// the whole leading index before: copy 153 -> 99 us, 4 neighbours 291 -> 192, overlap-add
-// 365 -> 136 (its transposed 4-neighbour form 1578 -> 316). One round per block: copy 136, the index
-// loads then delay every group; UL 8 / 12 / 16: copy 99 / 101 / 104, 4 neighbours 230 / 228 / 192,
-// overlap-add 164 / 136 / 153.
+// independent loads stand before a thread's first use, four times as many with four neighbours. With
+// few leading indices a launch is one thread's chain of loads long, and every load past the last
+// index is an instruction for nothing. Microseconds at UL 4 / 8 / 12 / 16 (24 tiles of 64 x 64, halo 8):
+//   leading indices   1             16             64             512 (516 MB read + written)
+//   copy              4/5/5/5       8/8/8/8        20/16/15/16    131/97/101/98
+//   4 neighbours      5/6/7/8       13/16/17/16    29/31/32/35    189/225/186/192
+//   overlap-add       7/7/9/10      13/17/17/12    29/28/27/29    194/162/139/152
+//   ... of 4 neigh.   9/12/18/19    26/29/34/23    61/58/59/61    402/333/313/336
+// 24 tiles of 96 x 96, halo 16, 512 of them: 330/246/262/257, 492/582/496/499, 451/411/346/390,
+// 922/800/750/808; 54 tiles of 64 x 64, halo 4: 234/181/188/182, 314/403/317/324, 380/293/257/284,
+// 782/596/572/614; six tiles of 16 x 16: 3 to 17 us throughout. So 8 for the copy, 4 for the neighbours
+// (no slower than 16 with many indices, faster with few), 12 for the overlap-add, which is up to twice
+// its time at 4 with one index (9 us) and 30 % faster with many. One round per block: copy 136 instead
+// of 99 us, the index loads then delay every group.
 constexpr int FIELD_ROUNDS = 2;
-constexpr int FIELD_UL_COPY = 8, FIELD_UL_KNN = 16, FIELD_UL_ADJ = 12;
+constexpr int FIELD_UL_COPY = 8, FIELD_UL_KNN = 4, FIELD_UL_ADJ = 12;
 inline unsigned field_grid_y(int64_t L, int ul) {
   const int64_t per = static_cast<int64_t>(ul) * FIELD_ROUNDS;
   return static_cast<unsigned>((L + per - 1) / per < 65535 ? (L + per - 1) / per : 65535);

@@ -169,6 +169,27 @@ def test_knn_halo_bit_exact_against_host_evaluation():
     with pytest.raises(TypeError):
         mod(x.cuda().double())
 
+def test_leading_indices_in_groups():
+    # a thread takes its leading indices in groups: each result is the one of its index alone, whatever
+    # the remainder of the group
+    from strata_b200.halo import (DistributedTileCopyHaloPadding, DistributedTileKNNHaloPadding,
+                                  NormalizedHaloAdjoint)
+    from strata_b200.rollout import padded_face_latlon
+    from strata_b200.topology import TileTopology
+    topo = TileTopology(1, 0, 24, 12, 3)
+    lat, lon = padded_face_latlon(24, 3)
+    copy = DistributedTileCopyHaloPadding(topology=topo, device="cuda")
+    knn = DistributedTileKNNHaloPadding.from_padded_face_grid(
+        topology=topo, lon=torch.from_numpy(lon), lat=torch.from_numpy(lat), pad_width_data=3, device="cuda")
+    x = torch.randn(33, topo.tiles_per_rank, 12, 12, device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+    for pad in (copy, knn):
+        back = NormalizedHaloAdjoint(pad)
+        one = torch.stack([pad(x[i]) for i in range(33)])
+        un = torch.stack([back(one[i]) for i in range(33)])
+        for n in (1, 3, 4, 5, 7, 8, 9, 12, 13, 16, 17, 24, 25, 33):
+            assert torch.equal(pad(x[:n]), one[:n]) and torch.equal(back(one[:n]), un[:n]), n
+
+
 def test_knn_halo_and_adjoint_equal_the_reference_modules(golden_dir):
     # the reference's DistributedTileKNNHaloPadding_AllGather / NormalizedHaloAdjoint outputs at
     # world_size 1 (tests/golden/make_plan_golden.py: the reference's modules, earth2grid's
