@@ -195,10 +195,14 @@ static int qkv_rope_impl(const void* x, int64_t ldx, const void* w, int64_t ldw,
   const auto* W = static_cast<const __nv_bfloat16*>(w);
   if (!rope_cs && !qk_norm) return launch_gemm<EPI_BIAS>(A, ldx, W, ldw, p, sms, as_stream(stream));
   if (!rope_cs && C < 256 && head_dim == 64) {
-    // qk norm without rotation at a small width (the pixel stage: C = 128): the projection is
-    // bound by its output traffic and the fused epilogue's extra arithmetic costs more than a
-    // second pass - plain projection, then the in-place row kernel normalises the q and k heads
-    // (measured at C = 128: 0.29 + 0.27 ms against 0.72 ms fused).
+    // qk norm without rotation at a small width: a plain projection and the in-place row kernel, which
+    // normalises the q and k heads, against the fused epilogue with an identity table. Two kernels / fused,
+    // microseconds: C = 128 at 1572864 rows (the pixel stage of one production tile) 599 / 558, 262144 114 /
+    // 114, 24576 16.9 / 17.4, 1024 7.7 / 9.2; C = 64 341 / 306, 62 / 69, 13.3 / 12.8, 8.2 / 8.7; C = 192 1113 /
+    // 1072, 202 / 210, 23.0 / 24.1, 9.7 / 9.7 - within 10 % either way, in favour of two kernels where a launch
+    // is short. From C = 256 on fused is ahead: 1263 / 947, 212 / 173, 24.6 / 21.9, 9.6 / 9.6; C = 512 at 262144
+    // rows 525 / 388. (Here the norm sees q and k rounded to bf16, there the fp32 accumulators: error against
+    // 64 bits 2.1e-3 and 1.7e-3 of the result.)
     int r = launch_gemm<EPI_BIAS>(A, ldx, W, ldw, p, sms, as_stream(stream));
     if (r != 0) return r;
     long long rows = M;

@@ -11,9 +11,8 @@
 //
 // Everything is evaluated in double precision and rounded once. Bound: launch and dependent
 // latency - the table is 4 * head_dim / 2 bytes per token, the arithmetic two sincos per pixel and
-// one per table entry. As ~45 tensor operations (each a launch of 2-4 us on the GPU and 5 us
-// on the host) the same tables took 150 us of GPU and 400 us of host time per model call at
-// 32 x 32 pixels; the two kernels take 7 us there and 17 us at 256 x 256.
+// one per table entry: 7 us for 32 x 32 pixels, 17 us for 256 x 256. (Written with tensor operations,
+// rope.py, the tables are some 45 launches: 150 us of the GPU and 400 us of the host at 32 x 32.)
 #pragma once
 #include <cuda_fp16.h>
 
@@ -152,8 +151,8 @@ __global__ void __launch_bounds__(256) tile_tables_kernel(const TileTablesParams
   const int lane = threadIdx.x & 31;
   const int tokens = p.h * p.w, half = p.pairs >> 1;
   // A warp takes TPW tokens at a time: first 32 / TPW lanes per token share its pixels, then all
-  // lanes write the tokens' rows one after the other. (One token per warp left 31 lanes waiting
-  // for the one pixel of a patch-1 token: 64 us for 24 tiles of 48 x 48, 24 now.)
+  // lanes write the tokens' rows one after the other. (With one token per warp 31 lanes wait for
+  // the one pixel of a patch-1 token: 64 us for 24 tiles of 48 x 48, 24 this way.)
   const int tpw = geo_tokens_per_warp(p.mode, p.patch), lpt = 32 / tpw;
   for (int t0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * tpw; t0 < tokens; t0 += gridDim.x * 8 * tpw) {
     const int t = min(t0 + lane / lpt, tokens - 1);

@@ -857,7 +857,13 @@ inline int launch_na3d_t(const __nv_bfloat16* q, long long ldq, const __nv_bfloa
   if (const cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), Cfg::TOTAL, smem_set); e != cudaSuccess)
     return -static_cast<int>(e) - 1000;
   const int grid = p.n_items < 2 * sm_count ? p.n_items : 2 * sm_count;
-  // (more than eight items a CTA are some 100 us: nothing to gain from an early start)
+  // An early start saves a launch about 3 us, whatever its length; of a launch of many items a CTA it is
+  // less than what it can cost (launch.cuh: CTAs that come in one by one). Between its QKV and projection
+  // GEMMs, chained / plain time at 7, 9, 14, 28, 42 and 55 items a CTA, 16 x 64 x 64 tokens of 512 channels:
+  // window 3 x 1 x 1 0.982 0.996 0.992 1.000 1.011 1.013; 3 x 3 x 3 0.979 0.983 0.988 0.996 1.001 1.001;
+  // 3 x 9 x 9 0.978 0.983 0.990 0.997 1.002 1.004; 9 x 9 x 9 0.987 1.042 0.995 0.999 1.003 1.009;
+  // 5 x 13 x 13 0.989 1.040 0.991 0.998 1.002 1.008. Fewer items a CTA gain more (0.88 to 0.94 at 0.1); above
+  // eight there is 1 % to gain and 4 % to lose, where the last round of long items is one more for some.
   if (p.n_items > 8 * grid) return launch_plain(kern, dim3(grid), Cfg::THREADS, Cfg::TOTAL, stream, 1, tmQ, tmK, tmV, p);
   return launch_chained(kern, dim3(grid), Cfg::THREADS, Cfg::TOTAL, stream, 1, tmQ, tmK, tmV, p);
 }

@@ -1,8 +1,8 @@
 // Whole forward passes: the launches of a network's kernels in order on one stream, issued from
 // C++. A pass over a small tile is paced by the host - a block is seven kernels of 3-10 us each -
 // so nothing but the launches is left between them: no Python call, allocation, weight cast or
-// table per kernel. (32 x 32 pixel tile, two 128-wide blocks: 785 us a pass when every launch
-// was a Python call of its own and the rotary table 45 tensor operations.)
+// table per kernel. 32 x 32 pixels, two 128-wide blocks: 20 launches in 90 us; the same kernels with a
+// Python call each, as for a model with hooks, take 260 us and more.
 #pragma once
 #include "../../include/strata_b200.h"
 

