@@ -49,7 +49,17 @@ def _randomised(m):
                  attn_kernel=(1, 3, 5))),
     (True, dict(do_rotate_wind=True, wind_channel_indices=(0, 2), qk_norm_pixel=True)),
     (True, dict(do_rope_2d_pixel=True, first_block_only_adaln_pixel=True)),
-    (True, dict(do_rope_2d_stereographic_pixel=True, gated_attention_pixel=True))])
+    (True, dict(do_rope_2d_stereographic_pixel=True, gated_attention_pixel=True)),
+    # what the pixel block's two forms (C and Python) could differ in: gate, norm and rotation together, no
+    # block modulated but the first, other widths, other factors and kernels (table and tap by tap), runs
+    # of rows that do not end with the image, more pixels than one piece of the conditioning
+    (True, dict(gated_attention_pixel=True, qk_norm_pixel=True, do_rope_2d_stereographic_pixel=True,
+                do_rotate_wind=True, wind_channel_indices=(3, 1))),
+    (True, dict(first_block_only_adaln_pixel=True, qk_norm_pixel=True, n_layers_pixel=3,
+                attn_kernel_pixel=(1, 5, 7))),
+    (True, dict(embed_dim_pixel=192, mlp_ratio_pixel=2.0, patch_size_horiz=8, attn_kernel=3)),
+    (True, dict(patch_size_horiz=2, gated_attention=True)),
+    (True, dict(depth=5, height=256, width=240, n_layers=1, n_layers_pixel=1))])
 def test_one_call_equals_step_by_step(two_stage, over):
     from strata_b200.wrappers import StrataBackboneModel, StrataModel
     kw = dict(depth=4, height=40, width=24, n_layers=2, patch_size_horiz=4, in_chans=5, base_out_chans=4,
@@ -60,8 +70,9 @@ def test_one_call_equals_step_by_step(two_stage, over):
                   use_bilinear_dw_gelu_project_adaln_pixel=True)
     kw.update(over)
     m = _randomised((StrataModel if two_stage else StrataBackboneModel)(**kw).cuda())
-    x = torch.randn(2, 5, 4, 40, 24, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
-    lat, lon = tile_latlon(2, 40, 24)
+    D, H, W = kw["depth"], kw["height"], kw["width"]
+    x = torch.randn(2, 5, D, H, W, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    lat, lon = tile_latlon(2, H, W)
     idx = {"lat": lat.cuda(), "lon": lon.cuda()}
 
     class StepByStep:
@@ -74,7 +85,7 @@ def test_one_call_equals_step_by_step(two_stage, over):
         # a changed weight, module or option reaches the next call
         m.strata._network = one_call
         bb = m.strata.backbone if two_stage else m.strata
-        bb.blocks[1].attn.proj.weight.mul_(1.5)
+        bb.blocks[-1].attn.proj.weight.mul_(1.5)
         bb.blocks[0].mlp.layers[2] = torch.nn.Linear(512, 128).cuda()
         bb.rope_length_scale *= 2.0
         z = m(x, idx)
@@ -351,3 +362,92 @@ def test_raw_stream_lookup_agrees(monkeypatch):
         assert _lib.stream_of(x) == side.cuda_stream
         monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream", raising=False)
         assert _lib._stream_lookup()(x.device.index) == side.cuda_stream
+
+
+def test_blocks_that_differ_take_the_steps():
+    """A model whose blocks have no common width of their hidden rows has no descriptors."""
+    from strata_b200.strata import Mlp
+    from tests.test_network_host import small_model
+    from tests.util import rel_max_err
+    m = small_model().cuda()
+    mlp = Mlp(128, 256).cuda()
+    mlp.layers[1] = torch.nn.GELU(approximate="tanh")
+    m.strata.blocks[1].mlp = mlp
+    x = torch.randn(2, 5, 4, 16, 16, generator=torch.Generator().manual_seed(1))
+    lat, lon = tile_latlon(2, 16, 16)
+    with torch.no_grad():
+        y = m(x.cuda(), {"lat": lat.cuda(), "lon": lon.cuda()})
+        assert m.strata._network._state.desc is None
+        ref = bo.backbone_forward(x, {k: v.cpu() for k, v in m.state_dict().items()}, patch=(1, 4, 4),
+                                  num_heads=2, kernel=3, num_layers=2, lat=lat, lon=lon)
+        assert rel_max_err(y, ref) < 2e-2
+        mlp.layers[1] = torch.nn.GELU()
+        with pytest.raises(RuntimeError, match="tanh GELU"):
+            m(x.cuda(), {"lat": lat.cuda(), "lon": lon.cuda()})
+
+
+@pytest.mark.parametrize("two_stage", [False, True])
+def test_threads_with_streams_of_their_own(two_stage):
+    """One model, four threads, each with its stream, its batch size and its fields."""
+    import threading
+    from tests.test_network_host import small_model
+    m = _randomised(small_model(two_stage).cuda())
+    g = torch.Generator("cuda").manual_seed(1)
+    calls = []
+    for i in range(4):
+        lat, lon = (t.cuda() for t in tile_latlon(1 + i, 16, 16))
+        calls.append((torch.randn(1 + i, 5, 4, 16, 16, device="cuda", generator=g), {"lat": lat, "lon": lon}))
+    with torch.no_grad():
+        want = [m(*c) for c in calls]
+    torch.cuda.synchronize()
+    m.strata._network = type(m.strata._network)()
+    bad, start = [], threading.Barrier(4)
+
+    def work(i):
+        try:
+            stream = torch.cuda.Stream()
+            start.wait(60)
+            with torch.no_grad(), torch.cuda.stream(stream):
+                out = [m(*calls[i]) for _ in range(30)]
+            stream.synchronize()
+            bad.extend(i for y in out if not torch.equal(y, want[i]))
+        except BaseException as e:
+            bad.append(e)
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not bad, bad
+
+
+@pytest.mark.parametrize("two_stage", [False, True])
+def test_whole_forward_with_wind_beside_64_bits(two_stage, monkeypatch):
+    """Against the oracle in 64 bits the model is as far off as the oracle that rounds to bf16 where the
+    kernels do (a quarter more is allowed: other sums, other roundings on the way)."""
+    from oracle import pixel_oracle as po
+    from tests.util import in_double
+    from tests.test_network_host import small_model
+    over = dict(height=32, width=32, in_chans=5, base_out_chans=5, gated_attention=True, qk_norm=True,
+                do_rotate_wind=True, wind_channel_indices=(0, 1))
+    if two_stage:
+        over.update(qk_norm_pixel=True, attn_kernel_pixel=(3, 5, 5))
+    m = _randomised(small_model(two_stage, **over).cuda())
+    if two_stage:
+        with torch.no_grad():
+            for n, p in m.named_parameters():
+                if n.endswith("adaln_bilinear_dw_proj.weight"):
+                    p.mul_(0.5)
+    x = torch.randn(2, 5, 4, 32, 32, generator=torch.Generator().manual_seed(0))
+    lat, lon = tile_latlon(2, 32, 32)
+    with torch.no_grad():
+        y = m(x.cuda(), {"lat": lat.cuda(), "lon": lon.cuda()}).cpu()
+    state = {k: v.detach().cpu() for k, v in m.state_dict().items()}
+    kw = dict(patch=(1, 4, 4), num_heads=2, kernel=3, num_layers=2, qk_norm=True, gated=True, wind_channels=(0, 1))
+    fn = bo.backbone_forward
+    if two_stage:
+        fn = po.two_stage_forward
+        kw.update(num_heads_pixel=1, kernel_pixel=(3, 5, 5), num_layers_pixel=2, qk_norm_pixel=True)
+    exact = in_double(monkeypatch, fn, x, state, lat=lat, lon=lon, **kw)
+    rounded = fn(x, state, lat=lat, lon=lon, emulate_bf16=True, **kw)
+    err = lambda t: float((t.double() - exact).norm() / exact.norm())
+    print(f"whole forward with wind vs 64 bits: model {err(y):.3e}, oracle with bf16 {err(rounded):.3e}")
+    assert err(y) < 1.25 * err(rounded)

@@ -30,3 +30,13 @@ def device_block_weights(p: dict, device):
             out[f"w_{short}"] = p[f"{name}.weight"].to(device=device, dtype=torch.bfloat16).contiguous()
             out[f"b_{short}"] = p[f"{name}.bias"].to(device=device, dtype=torch.float32).contiguous()
     return out
+
+
+def in_double(monkeypatch, oracle_fn, x, state, *, lat, lon, **kw):
+    """An oracle's forward pass in 64 bits: it converts whatever it is given with Tensor.float()."""
+    with monkeypatch.context() as mp:
+        mp.setattr(torch.Tensor, "float", torch.Tensor.double)
+        y = oracle_fn(x.double(), {k: v.double() for k, v in state.items()}, lat=lat.double(),
+                      lon=lon.double(), **kw)
+    assert y.dtype == torch.float64
+    return y
