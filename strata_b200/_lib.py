@@ -6,6 +6,7 @@ error, the call raises.
 from __future__ import annotations
 
 import ctypes
+import threading
 from ctypes import c_char_p, c_double, c_float, c_int, c_int32, c_int64, c_void_p, POINTER, Structure
 from pathlib import Path
 
@@ -188,10 +189,9 @@ def stream_of(t) -> int:
 
 
 def settle(device) -> bool:
-    """Called between filling tensors that a module will keep (weights cast for the kernels, tables) and
-    keeping them: waits for the device, after which any stream and thread may read them and nothing in
-    flight reads what they replace. False while a graph is being captured: nothing has run then, the
-    caller must use them in this call only."""
+    """Waits for the device: what was filled on it before may then be read by any stream and thread, and
+    nothing in flight reads what it replaces. False while a graph is being captured: nothing has run
+    then."""
     import torch
     if device.type != "cuda":
         return True
@@ -200,6 +200,43 @@ def settle(device) -> bool:
             return False
         torch.cuda.synchronize()
     return True
+
+
+_filling = threading.local()
+
+
+def keep(device, store) -> None:
+    """Called with tensors that were just filled on the current stream and that a module will keep for
+    later passes (weights cast for the kernels, tables): store() puts them where these look, once they are
+    settled; under capture it is not called, and the tensors serve this pass only."""
+    together = getattr(_filling, "stores", None)
+    if together is not None:
+        together.append(store)
+    elif settle(device):
+        store()
+
+
+class settled_together:
+    """Context in which this thread's keep() calls wait for the device once, at its end. `kept` then
+    says whether what was filled inside may be kept."""
+
+    def __init__(self, device):
+        self.device = device
+        self.kept = False
+
+    def __enter__(self):
+        self._outer = getattr(_filling, "stores", None)
+        _filling.stores = self._stores = []
+        return self
+
+    def __exit__(self, kind, *exc):
+        _filling.stores = self._outer
+        if kind is None:
+            self.kept = not self._stores or settle(self.device)
+            if self.kept:
+                for store in self._stores:
+                    store()
+        return False
 
 
 def exported_names() -> list[str]:

@@ -62,15 +62,12 @@ class Stock:
 
     def __init__(self, cls, *methods, called=False):
         self.cls = cls
-        self._lookup = vars(cls).get
         self._functions = {n: vars(cls)[n] for n in methods}
-        self._stock = list(self._functions.values())
+        # what the class has to hold for them, to be looked up again: (lookup, name), function
+        self.lookups = [((vars(cls).get, n), f) for n, f in self._functions.items()]
         # (_call_impl and _compiled_call_impl: what Module.__call__ and Module.compile() go through)
         self._names = (*methods, "_call_impl", "_compiled_call_impl") if called else methods
         self._hooks = self.HOOKS if called else ()
-
-    def class_intact(self) -> bool:
-        return list(map(self._lookup, self._functions)) == self._stock
 
     def holds(self, m) -> bool:
         if type(m) is not self.cls:
@@ -90,12 +87,12 @@ class Stock:
 
 
 def _stock_parts(backbone, pixel):
-    """(module, Stock) of every module whose own code a step-by-step pass would run."""
-    out = [(backbone, STOCK["backbone"]), (backbone.patch_embed, STOCK["patch_embed"])]
+    """(module, Stock) of every module below the two whose own code a step-by-step pass would run."""
+    out = [(backbone.patch_embed, STOCK["patch_embed"])]
     out += [(b, STOCK["block"]) for b in backbone.blocks]
     head = backbone.final_layer
     if pixel is not None:
-        out += [(pixel, STOCK["pixel"]), (pixel.pixel_patch_embed, STOCK["patch_embed"])]
+        out.append((pixel.pixel_patch_embed, STOCK["patch_embed"]))
         out += [(b, STOCK["pixel_block"]) for b in pixel.pixel_blocks]
         head = pixel.pixel_final_layer
     return out + [(head, STOCK["final_layer"])]
@@ -119,7 +116,11 @@ STOCK: dict[str, Stock] = {}
 class Described:
     """The descriptors of a model as it is, and what they were read from. Complete when the constructor
     returns and never written afterwards, so threads that share the model may share it; a change of the
-    model makes a new one (`current`). desc is None where only the step-by-step path will do."""
+    model makes a new one (`current`). desc is None where only the step-by-step path will do. The module
+    that owns it is not referred to: with such a cycle a model's memory would wait for the collector."""
+
+    OWN = ("out_channels", "patch_size", "embed_dim", "num_heads")
+    OWN_PIXEL = ("embed_dim_pixel", "num_heads_pixel")
 
     def __init__(self, backbone, pixel, device):
         self.device = device
@@ -127,16 +128,24 @@ class Described:
         self.keep = None            # owns what the descriptors point to
         self._modules = self._owners = self._params = self._ptrs = self._versions = self._attrs = ()
         self._parts = _stock_parts(backbone, pixel)
-        self._classes = {s for _, s in self._parts}
-        self.stock = self._all_stock()
+        classes = {s for _, s in self._parts} | {STOCK["backbone"]} | ({STOCK["pixel"]} if pixel is not None else set())
+        lookups = [e for s in classes for e in s.lookups]
+        self._lookups, self._functions = [k for k, _ in lookups], [f for _, f in lookups]
+        self._own = self._owned(backbone, pixel)
+        self.stock = self._all_stock(backbone, pixel)
         if self.stock:
             self._describe(backbone, pixel)
 
     # ---------------------------------------------------------------- what may change
-    def _all_stock(self) -> bool:
-        for s in self._classes:
-            if not s.class_intact():
-                return False
+    def _owned(self, backbone, pixel):
+        own = [getattr(backbone, n) for n in self.OWN]
+        return own if pixel is None else own + [getattr(pixel, n) for n in self.OWN_PIXEL]
+
+    def _all_stock(self, backbone, pixel) -> bool:
+        if not STOCK["backbone"].holds(backbone) or not (pixel is None or STOCK["pixel"].holds(pixel)):
+            return False
+        if [get(n) for get, n in self._lookups] != self._functions:
+            return False
         for m, s in self._parts:
             if not s.holds(m):
                 return False
@@ -150,9 +159,11 @@ class Described:
         self._versions = [p._version for p in self._params]
         self._attrs = attrs
 
-    def current(self, device) -> bool:
+    def current(self, backbone, pixel, device) -> bool:
         """Whether the model is still the one described, for inputs on `device`."""
-        if not self.stock or self.device != device or not self._all_stock():
+        if not self.stock or self.device != device or not self._all_stock(backbone, pixel):
+            return False
+        if self._owned(backbone, pixel) != self._own:
             return False
         for d, was in self._modules:
             if d != was:
@@ -162,32 +173,30 @@ class Described:
                 return False
         if [p._version for p in self._params] != self._versions or [p.data_ptr() for p in self._params] != self._ptrs:
             return False
-        for obj, name, value in self._attrs:
-            if getattr(obj, name, None) != value:
+        for own, name, value in self._attrs:
+            if own.get(name) != value:
                 return False
         return True
 
     # ---------------------------------------------------------------- descriptors
     def _describe(self, backbone, pixel) -> None:
-        attrs = [(backbone, n, getattr(backbone, n)) for n in ("out_channels", "patch_size", "embed_dim", "num_heads")]
-        if pixel is not None:
-            attrs += [(pixel, n, getattr(pixel, n)) for n in ("embed_dim_pixel", "num_heads_pixel")]
+        attrs = []
         weights = _Weights(self.device)
         keep = weights.keep
 
         def kernels_of(blocks):
-            attrs.extend((b, "kernel", b.kernel) for b in blocks)
+            attrs.extend((vars(b), "kernel", b.kernel) for b in blocks)
             flat = [v for b in blocks for v in b.kernel]
             return (ctypes.c_int32 * max(len(flat), 1))(*flat)
 
         def same(blocks, name, default):
-            attrs.extend((b, name, getattr(b, name)) for b in blocks)
+            attrs.extend((vars(b), name, getattr(b, name)) for b in blocks)
             values = {getattr(b, name) for b in blocks} or {default}
             return values.pop() if len(values) == 1 else None
 
         def usable(blocks):
             for b in blocks:
-                attrs.append((b.mlp.layers[1], "approximate", "tanh"))
+                attrs.append((vars(b.mlp.layers[1]), "approximate", "tanh"))
             return all(b._gelu_is_tanh() for b in blocks)
 
         bb = backbone
@@ -265,6 +274,7 @@ class Described:
                         w["w_dw"].data_ptr(), Cb, bb.patch_size[1], ks, table.data_ptr(),
                         torch.cuda.current_stream().cuda_stream), "strata_adaln_cond_table_f32")
                 keep.append(table)
+                _lib.keep(table.device, lambda: None)     # (kept by this description, which waits for it)
                 s.cond_table = table.data_ptr()
         px.h_blocks = ctypes.cast(structs, ctypes.POINTER(_lib.PixelBlockWeights))
         keep.append(structs)
@@ -291,10 +301,10 @@ class NetworkHandle:
         the model has a part that only the step-by-step path runs."""
         x, lat, lon = ops.network_inputs(x, lat, lon, x.shape[1] + (2 if concat_lat else 0), backbone)
         s = self._state
-        if s is None or not s.current(x.device):
-            s = Described(backbone, pixel, x.device)
-            # (its conditioning tables are laid out on this call's stream)
-            if s.desc is None or _lib.settle(x.device):
+        if s is None or not s.current(backbone, pixel, x.device):
+            with _lib.settled_together(x.device) as new:
+                s = Described(backbone, pixel, x.device)
+            if new.kept:
                 self._state = s
         if s.desc is None or (backbone.rope_mode == "stereographic" and s.desc.patch_h != s.desc.patch_w):
             return None

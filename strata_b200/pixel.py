@@ -21,7 +21,7 @@ import torch.nn as nn
 from . import _lib, ops, rope
 from .network import STOCK, NetworkHandle, Stock
 from .ops import EPI_BIAS, EPI_GATE, EPI_GELU
-from .strata import FinalLayer, Mlp, NeighborhoodAttention3D, PatchEmbed3D, StrataTransformer3D, _triple
+from .strata import FinalLayer, Mlp, NeighborhoodAttention3D, PatchEmbed3D, StrataTransformer3D, _store, _triple
 
 # pixel rows whose conditioning matrix [rows, C_backbone] is materialised at a time
 _COND_CHUNK_ROWS = 1 << 18
@@ -88,8 +88,7 @@ class StrataPixel3DBlock(nn.Module):
             c["w_dw"] = conv.weight.detach().float().reshape(conv.out_channels, ks, ks).contiguous()
             c["b_dw"] = b(conv)
             c["w_mod"], c["b_mod"] = w(self.adaln_bilinear_dw_proj), b(self.adaln_bilinear_dw_proj)
-        if _lib.settle(self.attn.qkv.weight.device):
-            self._cache, self._key = c, key
+        _lib.keep(self.attn.qkv.weight.device, lambda: _store(self, "", c, key))
         return c
 
     def modulation(self, backbone_tokens: torch.Tensor, factor: int) -> torch.Tensor | None:

@@ -33,6 +33,13 @@ def _triple(v):
     return (int(v),) * 3 if isinstance(v, int) else tuple(int(t) for t in v)
 
 
+def _store(module, name, made, key) -> None:
+    """Keeps what was made from the parameters that `key` names. The key goes last: a thread that finds
+    it finds what belongs to it."""
+    setattr(module, name + "_cache", made)
+    setattr(module, name + "_key", key)
+
+
 class PatchEmbed3D(nn.Module):
     """[B, C_in, D, H, W] -> tokens [B, D'*H'*W', embed_dim] (d, h, w order)."""
 
@@ -63,8 +70,7 @@ class PatchEmbed3D(nn.Module):
         wm[:, :K] = w.reshape(w.shape[0], K)
         b = None if self.proj.bias is None else self.proj.bias.detach().float().contiguous()
         made = (wm, b, K, Kp)
-        if _lib.settle(w.device):
-            self._gemm_cache, self._gemm_key = made, key
+        _lib.keep(w.device, lambda: _store(self, "_gemm", made, key))
         return made
 
     def tokens_bf16(self, x: torch.Tensor) -> torch.Tensor:
@@ -206,8 +212,7 @@ class StrataTransformer3DBlock(nn.Module):
                  "w_fc2": w(self.mlp.layers[2]), "b_fc2": b(self.mlp.layers[2])}
         if hasattr(self.attn, "gate_proj"):
             cache["w_gate"], cache["b_gate"] = w(self.attn.gate_proj), b(self.attn.gate_proj)
-        if _lib.settle(self.attn.qkv.weight.device):
-            self._bf16_cache, self._bf16_key = cache, key
+        _lib.keep(self.attn.qkv.weight.device, lambda: _store(self, "_bf16", cache, key))
         return cache
 
     def forward(self, x: torch.Tensor, grid, rope_cs, workspace=None) -> torch.Tensor:
@@ -255,8 +260,7 @@ class FinalLayer(nn.Module):
             b = torch.zeros(Np, dtype=torch.float32, device=w.device)
             b[:N] = self.linear.bias.detach().float()
         made = (wm, b, N)
-        if _lib.settle(w.device):
-            self._gemm_cache, self._gemm_key = made, key
+        _lib.keep(w.device, lambda: _store(self, "_gemm", made, key))
         return made
 
     def matrix_bf16(self, tokens: torch.Tensor):

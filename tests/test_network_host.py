@@ -173,10 +173,28 @@ CHANGES = {
 def test_a_changed_model_is_described_again(what, two_stage):
     m = small_model(two_stage)
     s = described(m)
-    assert s.current(torch.device("cpu")) and not s.current(torch.device("meta"))
+    assert s.current(*parts(m), torch.device("cpu")) and not s.current(*parts(m), torch.device("meta"))
     with torch.no_grad():
         CHANGES[what](parts(m)[0])
-    assert not s.current(torch.device("cpu"))
+    assert not s.current(*parts(m), torch.device("cpu"))
+
+
+@pytest.mark.parametrize("two_stage", [False, True])
+def test_a_described_model_is_freed_at_once(two_stage):
+    """Its weights and their copies do not wait for the garbage collector."""
+    import gc
+    import weakref
+    m = small_model(two_stage)
+    m.strata._network._state = described(m)
+    refs = [weakref.ref(t) for t in (m.strata, m.strata._network._state, parts(m)[0].blocks[0].attn.qkv.weight,
+                                     parts(m)[0].blocks[0]._bf16_cache["w_qkv"])]
+    gc.collect()
+    gc.disable()
+    try:
+        del m
+        assert [r() for r in refs] == [None] * 4
+    finally:
+        gc.enable()
 
 
 @pytest.mark.parametrize("two_stage", [False, True])
@@ -238,6 +256,28 @@ def test_casts_are_kept_only_once_settled(settled, monkeypatch):
         first = make()
         assert len(calls) == n + 1
         assert (make() is first) == settled and len(calls) == n + (1 if settled else 2)
+
+
+@pytest.mark.parametrize("settled", [True, False])
+@pytest.mark.parametrize("two_stage", [False, True])
+def test_a_description_waits_once(two_stage, settled, monkeypatch):
+    calls = []
+    monkeypatch.setattr(_lib, "settle", lambda device: calls.append(device) or settled)
+    m = small_model(two_stage)
+    with _lib.settled_together(torch.device("cpu")) as new:
+        assert described(m).desc is not None
+        kept = [b._bf16_cache for b in parts(m)[0].blocks]
+        assert not calls and kept == [None, None]
+    assert len(calls) == 1 and new.kept == settled
+    assert all((b._bf16_cache is not None) == settled for b in parts(m)[0].blocks)
+    with _lib.settled_together(torch.device("cpu")) as new:
+        described(m)
+    assert len(calls) == (1 if settled else 2)          # nothing new: nothing to wait for
+    with pytest.raises(KeyError):
+        with _lib.settled_together(torch.device("cpu")) as new:
+            small_model().strata.blocks[0].device_weights()
+            raise KeyError
+    assert not new.kept and len(calls) == (1 if settled else 2) and _lib._filling.stores is None
 
 
 def test_streams_are_found_without_the_private_lookup(monkeypatch):
