@@ -296,7 +296,7 @@ def _f32_dev(t, name, shape=None):
     if t.dtype != torch.float32 or not t.is_cuda:
         raise TypeError(f"{name} must be a CUDA float32 tensor")
     t = t.contiguous()
-    if shape is not None and tuple(t.shape) != tuple(shape):
+    if shape is not None and t.shape != shape:
         raise ValueError(f"{name} must have shape {tuple(shape)}, got {tuple(t.shape)}")
     return t
 

@@ -196,6 +196,15 @@ class _StrataModelBase(nn.Module):
             lon = lon.expand(B, -1, -1)
         return lat, lon
 
+    def _latlon_on(self, x: torch.Tensor, lat: torch.Tensor, lon: torch.Tensor):
+        """The same in fp32 on the fields' device, as the kernels take them (packing is theirs)."""
+        lat, lon = self._latlon_for(x, lat, lon)
+        if lat.dtype != torch.float32 or lat.device != x.device:
+            lat = lat.to(device=x.device, dtype=torch.float32)
+        if lon.dtype != torch.float32 or lon.device != x.device:
+            lon = lon.to(device=x.device, dtype=torch.float32)
+        return lat, lon
+
     def _preprocess(self, x, index):
         lat, lon = self.geometry.lat_lon_from_index(index)
         return self._preprocess_latlon(x, lat, lon)
@@ -336,9 +345,7 @@ class StrataBackboneModel(_StrataModelBase):
         """Same result as _preprocess -> strata -> _postprocess, with the wind rotation, the
         latitude channels and the patch gathering done by one kernel on the way in and the
         un-patchify and inverse rotation by one kernel on the way out."""
-        lat, lon = self._latlon_for(x, lat, lon)
-        lat = lat.to(device=x.device, dtype=torch.float32).contiguous()
-        lon = lon.to(device=x.device, dtype=torch.float32).contiguous()
+        lat, lon = self._latlon_on(x, lat, lon)
         return self.strata.forward_fused(x, None, lat=lat, lon=lon,
                                          wind=self._wind_channel_indices if self._do_rotate_wind else None,
                                          concat_lat=self._do_concat_latitude)
@@ -487,9 +494,7 @@ class StrataModel(_StrataModelBase):
         if not (x.is_cuda and x.dtype == torch.float32):
             raise RuntimeError("the two-stage model runs on CUDA fp32 fields only (its kernels "
                                "have no CPU fallback)")
-        lat, lon = self._latlon_for(x, lat, lon)
-        lat = lat.to(device=x.device, dtype=torch.float32).contiguous()
-        lon = lon.to(device=x.device, dtype=torch.float32).contiguous()
+        lat, lon = self._latlon_on(x, lat, lon)
         return self.strata.forward_fused(x, None, lat=lat, lon=lon,
                                          wind=self._wind_channel_indices if self._do_rotate_wind else None,
                                          concat_lat=self._do_concat_latitude)
