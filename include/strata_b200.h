@@ -306,7 +306,8 @@ int strata_dealias_patches_bf16(const void* x_rows, int64_t ldx, int B, int C, i
  * patch convolution in (channel, dv, dh, dw) order, columns zero-padded to k_embed (a multiple of
  * 8); w_head: [n_head, dim] bf16, rows in (dv, dh, dw, channel) order, zero-padded to n_head (a
  * multiple of 8; ignored in front of a pixel stage). in_channels counts the raw fields; two more
- * channels follow when concat_lat is set. u_idx = v_idx = -1: no wind rotation. */
+ * channels follow when concat_lat is set. u_idx = v_idx = -1: no wind rotation. The stereographic
+ * table takes the mean over square patches: patch_h == patch_w there. */
 typedef struct strata_backbone_desc {
   int32_t in_channels, out_channels, patch_v, patch_h, patch_w;
   int32_t dim, heads, hidden, n_blocks, qk_norm;
