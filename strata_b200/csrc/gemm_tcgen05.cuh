@@ -298,7 +298,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 8);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
 
   const int tiles_m = (p.M + TILE_M - 1) / TILE_M;
@@ -343,12 +343,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   __syncthreads();
   if constexpr (PAIR) cluster_sync_all();   // the partner's barriers exist before anyone signals them
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   chain_begin();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -389,7 +389,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0 && pair_rank == 0) {
+    if (pair_rank == 0 && elect_one()) {
       constexpr uint32_t idesc0 = umma_idesc_bf16(TILE_M, 0, false, false);
       int stage = 0;
       uint32_t phase = 0;
@@ -514,10 +514,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           if (chunk_live) {
             // staging box free again? (previous TMA store has finished reading it) - a
             // residual / gated operand is fetched into it right away
-            if (lane == 0) tma_store_wait_read0();
+            if (elect_one()) tma_store_wait_read0();
             __syncwarp();
             if constexpr (HAS_AUX) {
-              if (lane == 0) {
+              if (elect_one()) {
                 mbar_expect_tx(aux_bar(e), S::STAGING_BYTES);
                 tma_load_2d(stage_s, &tmAux, n0, m_warp, aux_bar(e));
               }
@@ -611,7 +611,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 // the previous sub-chunk's TMA store must have finished reading the staging
                 // box before it is overwritten; waiting only now lets that drain overlap with
                 // the TMEM load and the arithmetic above
-                if (lane == 0) tma_store_wait_read0();
+                if (elect_one()) tma_store_wait_read0();
                 __syncwarp();
               }
             }
@@ -630,13 +630,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         if (!chunk_live) continue;
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) {
+        if (elect_one()) {
           tma_store_2d(&tmOut, stage_s, n0, gemm_out_row(m_warp, p));
           tma_store_commit();
         }
       }
     }
-    if (lane == 0) tma_store_wait_all();
+    if (elect_one()) tma_store_wait_all();
   }
 
   tc_fence_before();

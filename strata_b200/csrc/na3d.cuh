@@ -361,7 +361,7 @@ na3d_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::BAR_OFF + 128);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + Cfg::BAR_OFF + 136);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
   const int nblk = p.nblk;
   // items of this CTA: blockIdx.x, blockIdx.x + gridDim.x, ... (the grid never exceeds n_items)
@@ -391,12 +391,12 @@ na3d_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   chain_begin();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       bool ok = true;
       int st = 0;
       uint32_t ph = 0;
@@ -437,7 +437,7 @@ na3d_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_qk = umma_idesc_bf16(128, NKEYS, false, false);
       constexpr uint32_t idesc_pv = umma_idesc_bf16(128, 64, false, true);
       constexpr int PV_STEPS = NKEYS / 16;
