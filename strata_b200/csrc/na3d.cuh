@@ -66,6 +66,22 @@ namespace strata {
 
 constexpr int NA_MAX_BLOCKS = 64;   // 16 planes x 8 chunks / 2
 
+// n / d for 0 <= n < 2^31 by a multiplication: (mulhi(n, mul) + n) >> shift.
+struct NaDiv {
+  uint32_t d, mul, shift;
+  __device__ __forceinline__ int operator()(int& n) const {   // returns n mod d, leaves n / d
+    const uint32_t u = static_cast<uint32_t>(n);
+    const uint32_t q = (__umulhi(u, mul) + u) >> shift;
+    n = static_cast<int>(q);
+    return static_cast<int>(u - q * d);
+  }
+};
+inline NaDiv na_make_div(int d) {
+  uint32_t s = 0;
+  while ((1ull << s) < static_cast<uint64_t>(d)) ++s;
+  return {static_cast<uint32_t>(d), static_cast<uint32_t>((((1ull << s) - d) << 32) / d + 1), s};
+}
+
 struct Na3dParams {
   int B, D, H, W, heads;
   int kd, kh;            // kernel extents along depth and rows (columns: template KW)
@@ -81,9 +97,10 @@ struct Na3dParams {
   int o_h0, o_H, o_w0, o_W;
   int n_items;           // tiles_d*tiles_h*tiles_w*heads*B
   int nblk;              // key blocks per item
-  // blk[i][s]: unit in slot s of block i: chunk (4 rows) in bits 0-3, plane in bits 4-7;
-  // bit 15: the slot only repeats another unit to keep the block full - ignore its keys.
-  unsigned short blk[NA_MAX_BLOCKS][2];
+  // blk[i]: the units in the two slots of block i (slot 0 in the low half): first key row (4 * chunk) in
+  // bits 0-7, plane in bits 8-11; bit 12: the slot only repeats another unit to keep the block full -
+  // ignore its keys (bits 8-12 as a shift then reach behind the plane masks).
+  uint32_t blk[NA_MAX_BLOCKS];
   __nv_bfloat16* out;    // [B, D, q_H, q_W, ldo] with head h at channel offset h*64
   long long ldo;
   // the operands as plain pointers (token-major, row strides in elements): only the
@@ -91,6 +108,7 @@ struct Na3dParams {
   const __nv_bfloat16 *q, *k, *v;
   long long ldq, ldk, ldv;
   float scale_log2e;
+  NaDiv div_w, div_h, div_d, div_heads;   // tiles_w, tiles_h, tiles_d, heads
 };
 
 __device__ __forceinline__ int na_window_start(int i, int L, int k) {
@@ -239,23 +257,60 @@ __device__ __noinline__ float na_scale_o_row(uint32_t o_taddr, int e) {
   return alpha;
 }
 
-// Reads this thread's row of the O accumulator, scales it by inv and stores it as 64 bf16 at op
-// (nullptr: the row carries no query). Called by a whole warp, once per item.
-__device__ __noinline__ void na_store_o_row(uint32_t o_taddr, float inv, __nv_bfloat16* op) {
-#pragma unroll
-  for (int hh = 0; hh < 2; ++hh) {
-    uint32_t ob[32];
-    tmem_ld_32x32(o_taddr + 32 * hh, ob);
+
+// Normalises and stores the warp's 32 rows of the O accumulator as 64 bf16 each: row l by lane l's inv, at lane
+// l's op (nullptr: the row carries no query). Read as matrix fragments (a quad of lanes holds a row's
+// 8-channel chunks, a word per lane), the four lanes exchange words so that each has 32 bytes of the row
+// and a store covers eight whole rows. (One row per lane, 16 bytes at a time, touches 32 lines per
+// store: the stores alone were 13 % of the 3 x 3 x 3 window over 24 x 64 x 64 tokens, 12 heads, 20 % of 3 x 1 x 1.)
+// Called by a whole warp, once per item.
+__device__ __noinline__ void na_store_o_rows(uint32_t o_taddr, float inv, __nv_bfloat16* op) {
+  const int lane = threadIdx.x & 31;
+  const unsigned long long opl = reinterpret_cast<unsigned long long>(op);
+#pragma unroll 1
+  for (int half = 0; half < 2; ++half) {   // rows 16 half ... + 15
+    const int row0 = 16 * half + (lane >> 2);
+    const float i0 = __shfl_sync(0xffffffffu, inv, row0), i1 = __shfl_sync(0xffffffffu, inv, row0 + 8);
+    const unsigned long long p0 = __shfl_sync(0xffffffffu, opl, row0), p1 = __shfl_sync(0xffffffffu, opl, row0 + 8);
+    uint32_t r[32];
+    // registers 4 j + {0, 1}: row lane / 4, columns 8 j + 2 (lane % 4) + {0, 1}; 4 j + {2, 3}: row lane / 4 + 8
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(o_taddr + (static_cast<uint32_t>(16 * half) << 16))
+        : "memory");
     tmem_ld_wait();
-    if (op != nullptr) {
+    const bool odd = lane & 1, hi = lane & 2;
 #pragma unroll
-      for (int j = 0; j < 32; j += 8) {
-        uint4 v4;
-        v4.x = pack_bf16(__uint_as_float(ob[j]) * inv, __uint_as_float(ob[j + 1]) * inv);
-        v4.y = pack_bf16(__uint_as_float(ob[j + 2]) * inv, __uint_as_float(ob[j + 3]) * inv);
-        v4.z = pack_bf16(__uint_as_float(ob[j + 4]) * inv, __uint_as_float(ob[j + 5]) * inv);
-        v4.w = pack_bf16(__uint_as_float(ob[j + 6]) * inv, __uint_as_float(ob[j + 7]) * inv);
-        *reinterpret_cast<uint4*>(op + 32 * hh + j) = v4;
+    for (int g = 0; g < 2; ++g) {          // row, row + 8
+      const float inv_g = g ? i1 : i0;
+      __nv_bfloat16* pg = reinterpret_cast<__nv_bfloat16*>(g ? p1 : p0);
+      uint32_t y[2][4];                    // chunks 2 (lane % 4) and the next of the row
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {        // chunks q, q + 2, q + 4, q + 6: a word of each per lane -> one chunk per lane
+        uint32_t w[4], x[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int c8 = 4 * (2 * i + q) + 2 * g;
+          w[i] = pack_bf16(__uint_as_float(r[c8]) * inv_g, __uint_as_float(r[c8 + 1]) * inv_g);
+        }
+        const uint32_t s0 = __shfl_xor_sync(0xffffffffu, odd ? w[0] : w[1], 1);
+        const uint32_t s1 = __shfl_xor_sync(0xffffffffu, odd ? w[2] : w[3], 1);
+        x[0] = odd ? s0 : w[0]; x[1] = odd ? w[1] : s0;
+        x[2] = odd ? s1 : w[2]; x[3] = odd ? w[3] : s1;
+        const uint32_t u0 = __shfl_xor_sync(0xffffffffu, hi ? x[0] : x[2], 2);
+        const uint32_t u1 = __shfl_xor_sync(0xffffffffu, hi ? x[1] : x[3], 2);
+        y[q][0] = hi ? u0 : x[0]; y[q][1] = hi ? u1 : x[1]; y[q][2] = hi ? x[2] : u0; y[q][3] = hi ? x[3] : u1;
+      }
+      if (pg != nullptr) {
+        __nv_bfloat16* dst = pg + (lane & 3) * 16;
+        reinterpret_cast<uint4*>(dst)[0] = make_uint4(y[0][0], y[0][1], y[0][2], y[0][3]);
+        reinterpret_cast<uint4*>(dst)[1] = make_uint4(y[1][0], y[1][1], y[1][2], y[1][3]);
       }
     }
   }
@@ -272,6 +327,11 @@ __device__ __forceinline__ bool na_wait(uint32_t bar, uint32_t parity, volatile 
   return na_wait_slow(bar, parity, abort_flag, code);
 }
 
+// One arrival for a converged warp (lane 0's), without a branch.
+__device__ __forceinline__ void na_arrive(uint32_t bar, int lane) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar), "r"(lane) : "memory");
+}
+
 struct NaItem {
   int b, head, d0, h0, w0, bd0, bh0, bw0;
 };
@@ -279,11 +339,11 @@ template <int KW, int QW>
 __device__ __forceinline__ NaItem na_decode_item(int item, const Na3dParams& p) {
   NaItem it;
   int t = item;
-  const int tw = t % p.tiles_w; t /= p.tiles_w;
-  const int th = t % p.tiles_h; t /= p.tiles_h;
-  const int td = t % p.tiles_d; t /= p.tiles_d;
-  it.head = t % p.heads;
-  it.b = t / p.heads;
+  const int tw = p.div_w(t);
+  const int th = p.div_h(t);
+  const int td = p.div_d(t);
+  it.head = p.div_heads(t);
+  it.b = t;
   it.d0 = td * p.QD; it.h0 = p.q_h0 + th * p.QH; it.w0 = p.q_w0 + tw * QW;
   // key box origin = window start of the tile's first query on each axis
   it.bd0 = na_window_start(it.d0, p.D, p.kd);
@@ -410,9 +470,9 @@ na3d_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
           mbar_expect_tx(kv_full(st), 2 * Cfg::KV_BYTES);
 #pragma unroll
           for (int s = 0; s < 2; ++s) {
-            const uint32_t u = p.blk[i][s];
-            const int kh0 = it.bh0 + 4 * static_cast<int>(u & 15u);
-            const int kd0 = it.bd0 + static_cast<int>((u >> 4) & 15u);
+            const uint32_t u = p.blk[i] >> (16 * s);
+            const int kh0 = it.bh0 + static_cast<int>(u & 255u);
+            const int kd0 = it.bd0 + static_cast<int>((u >> 8) & 15u);
             tma_load_5d(k_smem(st) + s * Cfg::UNIT_BYTES, &tmK, it.head * 64, it.bw0, kh0, kd0,
                         it.b, kv_full(st));
             tma_load_5d(v_smem(st) + s * Cfg::UNIT_BYTES, &tmV, it.head * 64, it.bw0, kh0, kd0,
@@ -530,12 +590,18 @@ na3d_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
       const int wd = na_window_start(id, p.D, p.kd) - it.bd0;
       const int wh = na_window_start(ih, p.H, p.kh) - it.bh0;
       const int ww = na_window_start(iw, p.W, KW) - it.bw0;
-      const uint32_t hmask_all = ((1u << p.kh) - 1u) << wh;   // bit = key row of the box
+      // the planes and key rows of the box in this query's window, and in that of some query of the warp (whose
+      // queries are a box of their own: a unit is seen by one of them if its plane and a row of it are)
+      const uint32_t planes = has_query ? ((1u << p.kd) - 1u) << wd : 0u;
+      const uint32_t rows = ((1u << p.kh) - 1u) << wh;
+      const uint32_t warp_planes = __reduce_or_sync(0xffffffffu, planes);
+      const uint32_t warp_rows = __reduce_or_sync(0xffffffffu, has_query ? rows : 0u);
 
       // Scores are handled in scaled form t = s*c - mc (c = scale*log2 e, mc the scaled
       // reference). nb2 holds, per pair of key columns, the addend of that form: -mc inside
       // the query's window, -1e30 outside (the column mask).
       float mc = 0.f, l_run = 0.f;
+      bool any_fresh = true;   // some row of the warp has no reference yet
       uint64_t nb2[EW / 2];
       auto set_nb = [&](float ref) {
 #pragma unroll
@@ -549,23 +615,9 @@ na3d_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
       const uint64_t c2 = pack2(c, c);
 
       for (int i = 0; i < nblk; ++i, ++gb) {
-        // this thread's 8 key rows of the block: bit rr set = row rr lies in the query's window
-        uint32_t rowmask = 0;
-        {
-#pragma unroll
-          for (int s = 0; s < 2; ++s) {
-            const uint32_t u = p.blk[i][s];
-            const bool pl_ok = (u >> 15) == 0u &&
-                               static_cast<unsigned>(static_cast<int>((u >> 4) & 15u) - wd) <
-                                   static_cast<unsigned>(p.kd);
-            const uint32_t m = pl_ok ? (hmask_all >> (4u * (u & 15u))) & 15u : 0u;
-            rowmask |= m << (4 * s);
-          }
-          if (!has_query) rowmask = 0u;
-        }
-        const uint32_t warp_rows = __reduce_or_sync(0xffffffffu, rowmask);
+        const uint32_t u2 = p.blk[i];
         bool p_free = false;      // the previous block's P V has completed: P may be overwritten
-        if (i != 0 && __any_sync(0xffffffffu, l_run >= SUM_LIMIT)) {
+        if (__any_sync(0xffffffffu, l_run >= SUM_LIMIT)) {
           // rare: some row's scores have risen far above its reference. Move that reference up
           // by e whole binades: what has been accumulated under the old one - O (complete once
           // the previous P V is) and the running sum - is multiplied by 2^-e, which is exact.
@@ -604,14 +656,18 @@ na3d_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
         // is the detector: once it has reached 2^16 a score lies far above the reference, and
         // at the start of the next block (see above) the reference moves up. Rows of the unit
         // that this query does not see are masked (zero P, left out of the sum).
+        auto unit_rows = [&](int u, uint32_t pl, uint32_t rw) {   // the unit's rows (bits 0-3) that masks select
+          const uint32_t code = u2 >> (16 * u);
+          return (pl >> ((code >> 8) & 31u)) & 1u ? (rw >> (code & 31u)) & 15u : 0u;
+        };
+        const bool need[2] = {unit_rows(0, warp_planes, warp_rows) != 0u, unit_rows(1, warp_planes, warp_rows) != 0u};
         bool s_released = false;
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-          const uint32_t need4 = (warp_rows >> (4 * u)) & 15u;   // rows some query of the warp sees
-          const uint32_t mine4 = (rowmask >> (4 * u)) & 15u;     // rows this query sees
-          const bool last_load = (u == 1) || ((warp_rows >> 4) == 0u);
+          const uint32_t mine4 = unit_rows(u, planes, rows);     // rows this query sees
+          const bool last_load = (u == 1) || !need[1];
           uint32_t pk[UNIT_PCOLS];
-          if (need4 != 0u) {
+          if (need[u]) {
             uint32_t a[4][EWP];
 #pragma unroll
             for (int rr = 0; rr < 4; ++rr) tmem_ld_keyrow<EWP>(s_taddr + (4 * u + rr) * EWP, a[rr]);
@@ -619,11 +675,11 @@ na3d_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
             if (last_load && !s_released) {
               tc_fence_before();
               __syncwarp();
-              if (lane == 0) mbar_arrive(s_free);
+              na_arrive(s_free, lane);
               s_released = true;
             }
-            const bool fresh = has_query && l_run == 0.f;
-            if (__any_sync(0xffffffffu, fresh)) {
+            if (any_fresh) {
+              const bool fresh = has_query && l_run == 0.f;
               // The first reference of a row: the largest of some scores it sees in this unit
               // (scaled form). Any visible score will do - whatever lies above it by less than
               // 2^100 is absorbed by the running sum and the moves of the reference that follow
@@ -676,18 +732,19 @@ na3d_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
               unpack2(rs2, r0, r1);
               l_run += r0 + r1;
             }
+            if (any_fresh) any_fresh = __any_sync(0xffffffffu, has_query && l_run == 0.f);
           } else {
 #pragma unroll
             for (int j = 0; j < UNIT_PCOLS; ++j) pk[j] = 0u;
             if (last_load && !s_released) {
               tc_fence_before();
               __syncwarp();
-              if (lane == 0) mbar_arrive(s_free);
+              na_arrive(s_free, lane);
               s_released = true;
             }
             // The zeros of a first unit the warp does not see are stored after the second
             // unit's exponentials: the wait for the previous P V must not come before them.
-            if (u == 0 && (warp_rows >> 4) != 0u) continue;
+            if (u == 0 && need[1]) continue;
           }
           if (!p_free) {
             if (!na_wait(pv_done(st_prev), ph_prev, abort_flag, ST_TIMEOUT_SOFTMAX)) ok = false;
@@ -696,7 +753,7 @@ na3d_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
             if (i == 0 && pend && ok) {
               // O still holds the previous item (this item's first P V has not been issued):
               // its rows are normalised and stored now
-              na_store_o_row(o_taddr, pend_inv, pend_op);
+              na_store_o_rows(o_taddr, pend_inv, pend_op);
               pend = false;
             }
           }
@@ -707,7 +764,7 @@ na3d_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
             tmem_st_x16(p_taddr + u * UNIT_PCOLS, &pk[0]);
           }
         }
-        if ((warp_rows & 15u) == 0u && (warp_rows >> 4) != 0u) {   // the postponed zeros of unit 0
+        if (!need[0] && need[1]) {   // the postponed zeros of unit 0
           uint32_t z[16];
 #pragma unroll
           for (int j = 0; j < 16; ++j) z[j] = 0u;
@@ -719,7 +776,7 @@ na3d_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(p_ready);
+        na_arrive(p_ready, lane);
         if (++st_prev == STAGES) { st_prev = 0; ph_prev ^= 1u; }
       }
       if (!ok) break;
@@ -741,7 +798,7 @@ na3d_fwd_kernel(const __grid_constant__ CUtensorMap tmQ,
     if (ok && pend) {
       if (na_wait(pv_done(st_prev), ph_prev, abort_flag, ST_TIMEOUT_SOFTMAX)) {
         tc_fence_after();
-        na_store_o_row(o_taddr, pend_inv, pend_op);
+        na_store_o_rows(o_taddr, pend_inv, pend_op);
       } else {
         ok = false;
       }
@@ -792,7 +849,7 @@ inline int na_build_blocks(Na3dParams& p) {
       used[pl * NC + ch] = false;
     }
   auto pop = [](unsigned m) { return __builtin_popcount(m); };
-  auto code = [&](int u) { return static_cast<unsigned short>((u % NC) | ((u / NC) << 4)); };
+  auto code = [&](int u) { return static_cast<uint32_t>(4 * (u % NC) | ((u / NC) << 8)); };
   int nb = 0;
   // pass 1: disjoint pairs, widest sets first
   for (int want = 4; want >= 1; --want)
@@ -805,8 +862,7 @@ inline int na_build_blocks(Na3dParams& p) {
           best = v;
       if (best < 0) continue;
       used[u] = used[best] = true;
-      p.blk[nb][0] = code(u);
-      p.blk[nb][1] = code(best);
+      p.blk[nb] = code(u) | code(best) << 16;
       ++nb;
     }
   // pass 2: whatever is left, in order
@@ -814,14 +870,12 @@ inline int na_build_blocks(Na3dParams& p) {
   for (int u = 0; u < n; ++u) {
     if (used[u]) continue;
     if (pending < 0) { pending = u; continue; }
-    p.blk[nb][0] = code(pending);
-    p.blk[nb][1] = code(u);
+    p.blk[nb] = code(pending) | code(u) << 16;
     ++nb;
     pending = -1;
   }
   if (pending >= 0) {
-    p.blk[nb][0] = code(pending);
-    p.blk[nb][1] = static_cast<unsigned short>(code(pending) | 0x8000u);
+    p.blk[nb] = code(pending) | (code(pending) | 0x1000u) << 16;
     ++nb;
   }
   p.nblk = nb;
@@ -932,6 +986,10 @@ inline int launch_na3d(const __nv_bfloat16* q, long long ldq, const __nv_bfloat1
   const long long items = static_cast<long long>(p.tiles_d) * p.tiles_h * p.tiles_w * heads * B;
   if (items > 0x7fffffffLL) return -2;
   p.n_items = static_cast<int>(items);
+  p.div_w = na_make_div(p.tiles_w);
+  p.div_h = na_make_div(p.tiles_h);
+  p.div_d = na_make_div(p.tiles_d);
+  p.div_heads = na_make_div(heads);
   if (na_build_blocks(p) != 0) return -2;
   p.out = out;
   p.ldo = ldo;
