@@ -61,6 +61,18 @@ int strata_linear_bf16(const void* x, int64_t ldx, const void* w, int64_t ldw, c
                        void* y, int64_t ldy, int M, int N, int K, int epilogue, const void* aux,
                        int64_t ldaux, void* stream);
 
+/* y[M,C] = aux + [gate *] (W2 gelu(W1 x + b1) + b2): the MLP of a narrow block in one kernel, same bits as
+ * strata_linear_bf16 with STRATA_EPI_GELU and then with STRATA_EPI_RESIDUAL (aux, no gate), STRATA_EPI_BIAS (neither) or
+ * STRATA_EPI_BIAS followed by the gated residual of strata_adaln_rows_bf16 (gate). W1 [hidden,C] and
+ * W2 [C,hidden] are contiguous. C = 64, 128, 192 or 256 and hidden a multiple of 128, otherwise
+ * STRATA_ERR_UNSUPPORTED. y may be aux. */
+int strata_mlp_bf16(const void* x, int64_t ldx, const void* w1, const float* b1, const void* w2,
+                    const float* b2, const void* aux, int64_t ldaux, const void* gate, int64_t ldgate,
+                    void* y, int64_t ldy, int M, int C, int hidden, void* stream);
+/* 1 where strata_mlp_bf16 is the faster way to run an MLP of these sizes, 0 where two strata_linear_bf16 are
+ * (or it has no kernel). */
+int strata_mlp_fused(int M, int C, int hidden);
+
 /* qkv[M,3C] = x[M,C] Wqkv[3C,C]^T + b with, fused in the epilogue, optional per-head RMS
  * norm of q and k and the 2-D rotary embedding of q and k by the token's (cos,sin) row.
  * rope_cs: [n_tiles, hw, head_dim/2] pairs (cos, sin) in IEEE half, 4 bytes per pair (channel

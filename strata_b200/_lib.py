@@ -60,6 +60,9 @@ _SIGNATURES = {
     "strata_linear_bf16": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p,
                                    c_int64, c_int, c_int, c_int, c_int, c_void_p, c_int64,
                                    c_void_p]),
+    "strata_mlp_fused": (c_int, [c_int, c_int, c_int]),
+    "strata_mlp_bf16": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64,
+                                c_void_p, c_int64, c_void_p, c_int64, c_int, c_int, c_int, c_void_p]),
     "strata_qkv_rope_bf16": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p,
                                      c_int64, c_int, c_int, c_int, c_void_p, c_int, c_int,
                                      c_int, c_float, c_void_p]),

@@ -10,6 +10,7 @@
 #include "common.cuh"
 #include "gemm_tcgen05.cuh"
 #include "layernorm.cuh"
+#include "mlp_tcgen05.cuh"
 #include "na3d.cuh"
 #include "halo.cuh"
 #include "prepost.cuh"
@@ -129,6 +130,32 @@ int strata_linear_bf16(const void* x, int64_t ldx, const void* w, int64_t ldw, c
     case STRATA_EPI_GATE: return launch_gemm<EPI_GATE>(A, ldx, W, ldw, p, sms, st);
     default: return STRATA_ERR_UNSUPPORTED;
   }
+}
+
+int strata_mlp_fused(int M, int C, int hidden) { return mlp_fused_pays(M, C, hidden) ? 1 : 0; }
+
+int strata_mlp_bf16(const void* x, int64_t ldx, const void* w1, const float* b1, const void* w2, const float* b2,
+                    const void* aux, int64_t ldaux, const void* gate, int64_t ldgate, void* y, int64_t ldy, int M,
+                    int C, int hidden, void* stream) {
+  const int sms = current_sm_count();
+  if (sms <= 0) return STRATA_ERR_NO_DEVICE;
+  if (M < 0 || C <= 0 || hidden <= 0) return STRATA_ERR_ARG;
+  if (!mlp_fused_sizes(C, hidden)) return STRATA_ERR_UNSUPPORTED;
+  if (M == 0) return STRATA_OK;
+  if (!x || !w1 || !w2 || !y || (gate && !aux)) return STRATA_ERR_ARG;
+  if (ldx < C || ldx % 8 || ldy < C || ldy % 8 || (aux && (ldaux < C || ldaux % 8)) ||
+      (gate && (ldgate < C || ldgate % 8)))
+    return STRATA_ERR_ARG;
+  if (!aligned16(x) || !aligned16(w1) || !aligned16(w2) || !aligned16(y) || (aux && !aligned16(aux)) ||
+      (gate && !aligned16(gate)) || (b1 && !aligned16(b1)) || (b2 && !aligned16(b2)))
+    return STRATA_ERR_ARG;
+  MlpParams p{};
+  p.M = M; p.H = hidden;
+  p.b1 = b1; p.b2 = b2;
+  p.aux = static_cast<const __nv_bfloat16*>(aux); p.ldaux = ldaux;
+  p.gate = static_cast<const __nv_bfloat16*>(gate); p.ldgate = ldgate;
+  return launch_mlp(C, static_cast<const __nv_bfloat16*>(x), ldx, static_cast<const __nv_bfloat16*>(w1),
+                    static_cast<const __nv_bfloat16*>(w2), static_cast<__nv_bfloat16*>(y), ldy, p, sms, as_stream(stream));
 }
 
 // One row of the packed (cos, sin) half table that rotates by nothing: 32 pairs of (1.0, 0.0).
@@ -340,6 +367,9 @@ int strata_block_forward_bf16(const void* x, void* y, int n_tiles, int D, int H,
                               STRATA_EPI_RESIDUAL, x, C, stream)) != 0)
     return r;
   if ((r = strata_layernorm_bf16(x1, C, xn, C, M, C, ln_eps, stream)) != 0) return r;
+  if (mlp_fused_pays(M, C, hidden))
+    return strata_mlp_bf16(xn, C, wts->w_fc1, wts->b_fc1, wts->w_fc2, wts->b_fc2, x1, C, nullptr, 0, y, C, M, C, hidden,
+                           stream);
   if ((r = strata_linear_bf16(xn, C, wts->w_fc1, C, wts->b_fc1, hbuf, hidden, M, hidden, C,
                               STRATA_EPI_GELU, nullptr, 0, stream)) != 0)
     return r;

@@ -119,6 +119,18 @@ __device__ __forceinline__ void tma_store_wait_all() {
   asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
+// tanh GELU of a pair: the polynomial part runs on packed fp32x2 instructions.
+__device__ __forceinline__ uint64_t gelu_pair(uint64_t x) {
+  const float k0 = 0.7978845608028654f, k01 = 0.7978845608028654f * 0.044715f;
+  const uint64_t K0 = pack2(k0, k0), K01 = pack2(k01, k01), HALF = pack2(0.5f, 0.5f);
+  const uint64_t u = fmul2(x, ffma2(fmul2(x, x), K01, K0));
+  float u0, u1;
+  unpack2(u, u0, u1);
+  const uint64_t t = pack2(fast_tanh(u0), fast_tanh(u1));
+  const uint64_t hx = fmul2(x, HALF);
+  return ffma2(hx, t, hx);
+}
+
 // Epilogue math on 16 consecutive columns of output row m, in place. Lane `src_lane0 + j` of
 // the warp holds the bias of column j of the group; `aux` holds the residual / gated operand of
 // the same columns (bf16 pairs) for the epilogues that use one; `qk_scale` is the RMS-norm
@@ -145,19 +157,8 @@ __device__ __forceinline__ void gemm_epilogue_16(float (&v)[16], bool rotate, fl
     }
   }
   if constexpr (EPI == EPI_GELU) {
-    // tanh GELU on pairs: the polynomial part runs on packed fp32x2 instructions
-    const float k0 = 0.7978845608028654f, k01 = 0.7978845608028654f * 0.044715f;
-    const uint64_t K0 = pack2(k0, k0), K01 = pack2(k01, k01), HALF = pack2(0.5f, 0.5f);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const uint64_t x = pack2(v[2 * j], v[2 * j + 1]);
-      const uint64_t u = fmul2(x, ffma2(fmul2(x, x), K01, K0));
-      float u0, u1;
-      unpack2(u, u0, u1);
-      const uint64_t t = pack2(fast_tanh(u0), fast_tanh(u1));
-      const uint64_t hx = fmul2(x, HALF);
-      unpack2(ffma2(hx, t, hx), v[2 * j], v[2 * j + 1]);
-    }
+    for (int j = 0; j < 8; ++j) unpack2(gelu_pair(pack2(v[2 * j], v[2 * j + 1])), v[2 * j], v[2 * j + 1]);
   } else if constexpr (EPI == EPI_RESIDUAL) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) {

@@ -1,0 +1,533 @@
+// The MLP of a block in one kernel for narrow models (C = 64, 128, 192, 256 channels):
+//
+//   y = aux + [gate *] (W2 gelu(W1 x + b1) + b2)        x, aux, gate, y: [M, C] bf16; W1 [H, C], W2 [C, H]
+//
+// As two GEMMs the hidden rows [M, H] are written and read again: at C = 256, H = 1024 that is 4 of every 5
+// bytes the two move, and they are bound by it. Here a CTA keeps 128 rows: the hidden channels are made 128 at a time in
+// tensor memory, leave it as bf16 through the GELU into shared memory and are multiplied on from there.
+//
+//   warp 0      TMA producer: the x tile, and the weights of every chunk of 128 hidden channels through two
+//               rings (W1: 128 x 64 boxes, W2: C x 64 boxes); the weights come from L2, 16 C^2 bytes per tile.
+//   warp 1      MMA issuer: chunk c + 1 of W1 x goes to one of two accumulators while the epilogue warps work on
+//               chunk c, then W2 times the bf16 chunk c accumulates into the output columns.
+//   warps 2-17  epilogue: each takes 32 rows x 32 hidden channels of a chunk (bias, GELU, bf16, into the 128-byte
+//               swizzled layout the second product reads), and at a tile's end 32 x 32 boxes of the output
+//               (bias, gate, aux) through 64-byte-swizzled staging boxes to TMA stores.
+//
+// Every element sees the arithmetic of the two GEMMs - products accumulated over k in the same order, the
+// hidden channels rounded to bf16, the output too before it meets a gate - so the results are the same bits.
+//
+// Tensor memory: two chunk accumulators of 128 columns and the output, for C <= 128 twice: the epilogue warps then
+// form two sets that take the chunks in turn (a hidden buffer each), and the GELU of a tile's first chunk comes
+// before the last tile's output is read, which hides the last product.
+// Bound: C <= 128 by the epilogue warps (tanh on the special-function unit alone: 128 x 512 per tile take
+// 4096 cycles at C = 128, the products as many; a tile takes 11000), C = 256 by shared memory (operands,
+// weights coming in and the hidden chunk: 1.5 times what it moves in the products' own time) and the same warps.
+// 442368 rows, two GEMMs -> this kernel: C = 64 132 -> 80 us, 128 232 -> 145, 192 345 -> 301, 256 480 -> 412; with
+// the gated residual of the pixel blocks, which was a third kernel, 1572864 x 128 1010 -> 570.
+#pragma once
+#include "gemm_tcgen05.cuh"
+
+namespace strata {
+
+struct MlpParams {
+  int M, H;
+  const float* b1;              // [H] or nullptr
+  const float* b2;              // [C] or nullptr
+  const __nv_bfloat16* aux;     // [M, C] or nullptr
+  long long ldaux;
+  const __nv_bfloat16* gate;    // [M, C] or nullptr: the output is rounded to bf16 and multiplied by it
+  long long ldgate;
+};
+
+constexpr int MLP_CHUNK = 128;             // hidden channels of a chunk
+constexpr int MLP_MAX_C = 256;
+
+template <int C>
+struct MlpSmem {
+  static constexpr bool AHEAD = C <= 128;                        // see the top: two outputs, staging boxes of their own
+  static constexpr int SETS = AHEAD ? 2 : 1;                     // sets of epilogue warps, taking chunks in turn
+  static constexpr int KB = C / 64;                              // k-blocks of the first product
+  static constexpr int X_BYTES = KB * 128 * 128;
+  static constexpr int X_BUFS = 1;
+  static constexpr int H_BYTES = 2 * 128 * 128;                  // one chunk, a buffer per set
+  static constexpr int W1_BYTES = 128 * 128, W2_BYTES = C * 128; // one stage
+  static constexpr int S1 = C == 256 ? 4 : 3, S2 = C == 256 ? 2 : 3;
+  static constexpr int STAGING_BYTES = 32 * 32 * 2;
+  static constexpr int H_OFF = X_BUFS * X_BYTES;
+  static constexpr int W1_OFF = H_OFF + SETS * H_BYTES;
+  static constexpr int W2_OFF = W1_OFF + S1 * W1_BYTES;
+  static constexpr int STAGING_OFF = AHEAD ? W2_OFF + S2 * W2_BYTES : H_OFF;
+  static constexpr int BAR_OFF = W2_OFF + S2 * W2_BYTES + (AHEAD ? GEMM_EPI_WARPS * STAGING_BYTES : 0);
+  static constexpr int TOTAL = BAR_OFF + 512 + 1024;             // + alignment slack
+  static constexpr int OUT_COL = 256, OUT_BUFS = AHEAD ? 2 : 1, OUT_STRIDE = 128;
+  static_assert(GEMM_EPI_WARPS * STAGING_BYTES <= H_BYTES, "the staging boxes fit the hidden chunk's buffer");
+  static_assert(TOTAL <= 232448, "shared memory of an SM");
+};
+
+// 16 lanes x 32 columns as matrix fragments: registers 4 i + {0, 1}: row lane / 4, columns 8 i + 2 (lane % 4) + {0, 1};
+// 4 i + {2, 3}: row lane / 4 + 8.
+__device__ __forceinline__ void tmem_ld_16x256_x4(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+
+template <int C>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW1,
+                   const __grid_constant__ CUtensorMap tmW2, const __grid_constant__ CUtensorMap tmOut,
+                   const __grid_constant__ CUtensorMap tmAux, const MlpParams p) {
+  using S = MlpSmem<C>;
+  constexpr bool AHEAD = S::AHEAD;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+  const uint32_t bar = smem_base + S::BAR_OFF;
+  const uint32_t x_full = bar, x_empty = bar + 8u;
+  auto w1_full = [&](int s) { return bar + 32u + 8u * s; };
+  auto w1_empty = [&](int s) { return bar + 64u + 8u * s; };
+  auto w2_full = [&](int s) { return bar + 96u + 8u * s; };
+  auto w2_empty = [&](int s) { return bar + 120u + 8u * s; };
+  auto acc_full = [&](int b) { return bar + 144u + 8u * b; };
+  auto acc_free = [&](int b) { return bar + 160u + 8u * b; };
+  auto out_full = [&](int b) { return bar + 176u + 8u * b; };
+  auto out_free = [&](int b) { return bar + 192u + 8u * b; };
+  auto h_full = [&](int b) { return bar + 208u + 8u * b; };
+  auto h_empty = [&](int b) { return bar + 224u + 8u * b; };
+  const uint32_t staged = bar + 240u;
+  auto aux_full = [&](int w) { return bar + 256u + 8u * w; };
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_gen + S::BAR_OFF + 384);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + S::BAR_OFF + 392);
+
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
+  const int lane = threadIdx.x & 31;
+  const int tiles = (p.M + 127) / 128;
+  const int nj = p.H / MLP_CHUNK;
+  const int n_my = (tiles - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
+  const int chunks = n_my * nj;              // of this CTA, numbered through its tiles
+
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tmX);
+    tma_prefetch_desc(&tmW1);
+    tma_prefetch_desc(&tmW2);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(acc_full(b), 1);
+      mbar_init(acc_free(b), GEMM_EPI_WARPS / S::SETS);
+      mbar_init(h_full(b), GEMM_EPI_WARPS / S::SETS);
+      mbar_init(h_empty(b), 1);
+      mbar_init(out_full(b), 1);
+      mbar_init(out_free(b), GEMM_EPI_WARPS);
+    }
+    for (int s = 0; s < S::S1; ++s) { mbar_init(w1_full(s), 1); mbar_init(w1_empty(s), 1); }
+    for (int s = 0; s < S::S2; ++s) { mbar_init(w2_full(s), 1); mbar_init(w2_empty(s), 1); }
+    mbar_init(x_full, 1);
+    mbar_init(x_empty, 1);
+    mbar_init(staged, GEMM_EPI_WARPS);
+    for (int w = 0; w < GEMM_EPI_WARPS; ++w) mbar_init(aux_full(w), 1);
+    *abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(tmem_slot), 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  chain_begin();
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ TMA producer
+    if (elect_one()) {
+      bool ok = true;
+      int s1 = 0, s2 = 0;
+      uint32_t ph1 = 0, ph2 = 0;
+      // in the order of use: W1 of chunk c, then W2 of chunk c - 1
+      for (int c = 0; c <= chunks && ok; ++c) {
+        const int t = c / nj, j = c - t * nj;
+        if (c < chunks) {
+          if (j == 0) {
+            if (!mbar_wait(x_empty, (t & 1u) ^ 1u, abort_flag, ST_TIMEOUT_PRODUCER)) break;
+            mbar_expect_tx(x_full, S::X_BYTES);
+            const int m0 = (static_cast<int>(blockIdx.x) + t * static_cast<int>(gridDim.x)) * 128;
+            for (int kb = 0; kb < S::KB; ++kb)
+              tma_load_2d(smem_base + kb * 16384, &tmX, kb * 64, m0, x_full);
+          }
+          for (int kb = 0; kb < S::KB && ok; ++kb) {
+            ok = mbar_wait(w1_empty(s1), ph1 ^ 1u, abort_flag, ST_TIMEOUT_PRODUCER);
+            if (!ok) break;
+            mbar_expect_tx(w1_full(s1), S::W1_BYTES);
+            tma_load_2d(smem_base + S::W1_OFF + s1 * S::W1_BYTES, &tmW1, kb * 64, j * MLP_CHUNK, w1_full(s1));
+            if (++s1 == S::S1) { s1 = 0; ph1 ^= 1u; }
+          }
+        }
+        if (c > 0) {
+          const int jp = j == 0 ? nj - 1 : j - 1;
+          for (int hb = 0; hb < 2 && ok; ++hb) {
+            ok = mbar_wait(w2_empty(s2), ph2 ^ 1u, abort_flag, ST_TIMEOUT_PRODUCER);
+            if (!ok) break;
+            mbar_expect_tx(w2_full(s2), S::W2_BYTES);
+            tma_load_2d(smem_base + S::W2_OFF + s2 * S::W2_BYTES, &tmW2, jp * MLP_CHUNK + hb * 64, 0, w2_full(s2));
+            if (++s2 == S::S2) { s2 = 0; ph2 ^= 1u; }
+          }
+        }
+      }
+      if (*abort_flag)   // loads in flight must land before the CTA retires
+#pragma unroll 1
+        for (int i = 0; i < 2000; ++i) __nanosleep(100);
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ MMA issuer
+    if (elect_one()) {
+      constexpr uint32_t idesc1 = umma_idesc_bf16(128, MLP_CHUNK, false, false);
+      constexpr uint32_t idesc2 = umma_idesc_bf16(128, C, false, false);
+      int s1 = 0, s2 = 0;
+      uint32_t ph1 = 0, ph2 = 0;
+      int t1 = 0, j1 = 0;                   // tile and chunk of the next first product
+      auto first = [&](int c) -> bool {     // W1 x of chunk c
+        if (j1 == 0 && !mbar_wait(x_full, t1 & 1u, abort_flag, ST_TIMEOUT_MMA)) return false;
+        if (!mbar_wait(acc_free(c & 1), ((c >> 1) & 1u) ^ 1u, abort_flag, ST_TIMEOUT_MMA)) return false;
+        tc_fence_after();
+        for (int kb = 0; kb < S::KB; ++kb) {
+          if (!mbar_wait(w1_full(s1), ph1, abort_flag, ST_TIMEOUT_MMA)) return false;
+          tc_fence_after();
+          const uint64_t a = umma_smem_desc_sw128(smem_base + kb * 16384);
+          const uint64_t b = umma_smem_desc_sw128(smem_base + S::W1_OFF + s1 * S::W1_BYTES);
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            umma_ss(tmem_base + (c & 1) * MLP_CHUNK, a + 2u * k, b + 2u * k, idesc1, (kb | k) != 0 ? 1u : 0u);
+          umma_commit(w1_empty(s1));
+          if (++s1 == S::S1) { s1 = 0; ph1 ^= 1u; }
+        }
+        umma_commit(acc_full(c & 1));
+        if (++j1 == nj) {                   // the x tile has been read
+          umma_commit(x_empty);
+          j1 = 0;
+          ++t1;
+        }
+        return true;
+      };
+      bool ok = chunks > 0 && first(0);
+      int t = 0, j = 0;
+      for (int c = 0; c < chunks && ok; ++c) {
+        if (c + 1 < chunks && !first(c + 1)) break;
+        const int ob = AHEAD ? t & 1 : 0;
+        if (j == 0 && !mbar_wait(out_free(ob), ((AHEAD ? t >> 1 : t) & 1u) ^ 1u, abort_flag, ST_TIMEOUT_MMA)) break;
+        const int hbuf = c % S::SETS;
+        if (!mbar_wait(h_full(hbuf), (c / S::SETS) & 1u, abort_flag, ST_TIMEOUT_MMA)) break;
+        tc_fence_after();
+        for (int hb = 0; hb < 2; ++hb) {
+          if (!mbar_wait(w2_full(s2), ph2, abort_flag, ST_TIMEOUT_MMA)) { ok = false; break; }
+          tc_fence_after();
+          const uint64_t a = umma_smem_desc_sw128(smem_base + S::H_OFF + hbuf * S::H_BYTES + hb * 16384);
+          const uint64_t b = umma_smem_desc_sw128(smem_base + S::W2_OFF + s2 * S::W2_BYTES);
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            umma_ss(tmem_base + S::OUT_COL + ob * S::OUT_STRIDE, a + 2u * k, b + 2u * k, idesc2,
+                    (j | hb | k) != 0 ? 1u : 0u);
+          umma_commit(w2_empty(s2));
+          if (++s2 == S::S2) { s2 = 0; ph2 ^= 1u; }
+        }
+        if (!ok) break;
+        umma_commit(h_empty(hbuf));
+        if (++j == nj) {
+          umma_commit(out_full(ob));
+          j = 0;
+          ++t;
+        }
+      }
+    }
+  } else {
+    // ------------------------------------------------------------ epilogue warps
+    const int e = warp - 2;
+    const int quarter = warp & 3;            // TMEM lane quarter this warp may read
+    constexpr int SETS = S::SETS;
+    const int set = SETS == 2 ? e >> 3 : 0;
+    const int cg = SETS == 2 ? (e >> 2) & 1 : e >> 2;   // which 32 * SETS hidden channels of a chunk
+    const int box0 = (e >> 2) * 32;          // output columns of its (first) box
+    const uint32_t lane_taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    const uint32_t stage_s = smem_base + S::STAGING_OFF + e * S::STAGING_BYTES;
+    const uint32_t my_row_s = stage_s + lane * 64;
+    const uint32_t sw = static_cast<uint32_t>((lane >> 1) & 3);   // 64-byte swizzle of a staging box's row
+    const uint32_t h_row0 = smem_base + S::H_OFF + set * S::H_BYTES + quarter * 32 * 128;   // the quarter's rows of the hidden chunk
+    auto tile_row = [&](int t) { return (static_cast<int>(blockIdx.x) + t * static_cast<int>(gridDim.x)) * 128 + quarter * 32; };
+
+    // A chunk's accumulator is read as matrix fragments (lane: rows lane / 4 and + 8, columns 2 (lane % 4) and + 1
+    // of every 8): a lane then needs two biases per 8 columns, eight for its 32 channels, which are asked for before
+    // the accumulator is ready - with a row per lane all 32, read when they were needed, which cost 16 % at
+    // C = 128 - and stmatrix puts the 8 x 8 pieces where the second product wants them.
+    const uint32_t st_row = h_row0 + static_cast<uint32_t>(((lane >> 3) & 1) * 8 + (lane & 7)) * 128;
+    auto gelu_chunk = [&](int c, int j) -> bool {
+      const int buf = c & 1, use = c / SETS;
+      uint64_t bias[SETS][4];
+#pragma unroll
+      for (int pc = 0; pc < SETS; ++pc)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          bias[pc][i] = p.b1 == nullptr ? 0ull
+                                        : __ldg(reinterpret_cast<const unsigned long long*>(
+                                              p.b1 + j * MLP_CHUNK + (cg * SETS + pc) * 32 + 8 * i + 2 * (lane & 3)));
+      if (!gemm_wait(acc_full(buf), (c >> 1) & 1u, abort_flag, ST_TIMEOUT_EPILOGUE)) return false;
+      tc_fence_after();
+#pragma unroll
+      for (int pc = 0; pc < SETS; ++pc) {    // 32 hidden channels at a time
+        const int col = (cg * SETS + pc) * 32;
+        uint32_t acc[2][16], h[2][8];
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) tmem_ld_16x256_x4(lane_taddr + (static_cast<uint32_t>(16 * hf) << 16) + buf * MLP_CHUNK + col, acc[hf]);
+        tmem_ld_wait();
+        if (pc == SETS - 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(acc_free(buf));
+        }
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {      // columns 8 (i / 2), rows + 8 (i % 2)
+            float g0, g1;
+            unpack2(gelu_pair(fadd2(pack2u(acc[hf][2 * i], acc[hf][2 * i + 1]), bias[pc][i >> 1])), g0, g1);
+            h[hf][i] = pack_bf16(g0, g1);
+          }
+        // the product of the chunk before that used this buffer has read it
+        if (pc == 0 && !gemm_wait(h_empty(set), (use & 1u) ^ 1u, abort_flag, ST_TIMEOUT_EPILOGUE)) return false;
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf)
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {      // columns 16 q: k-block col / 64, 16-byte pieces (col % 64) / 8 + 2 q and + 1
+            const uint32_t piece = static_cast<uint32_t>((col & 32) / 8 + 2 * q + (lane >> 4));
+            const uint32_t addr = st_row + hf * 2048 + (col >> 6) * 16384 + ((piece ^ (lane & 7u)) << 4);
+            asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(h[hf][4 * q]),
+                         "r"(h[hf][4 * q + 1]), "r"(h[hf][4 * q + 2]), "r"(h[hf][4 * q + 3]) : "memory");
+          }
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(h_full(set));
+      return true;
+    };
+
+    // 64 bytes of this thread's row (a box's columns from n0) of an [M, C] operand
+    auto fetch = [&](uint4 (&v)[4], const __nv_bfloat16* base, long long ld, int t, int n0) {
+      const long long m = tile_row(t) + lane;
+      if (base != nullptr && m < p.M && n0 < C) {
+        const uint4* src = reinterpret_cast<const uint4*>(base + m * ld + n0);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = src[q];
+      }
+    };
+    // AHEAD: aux of a tile's box waits in the staging box, fetched while the tile is computed
+    auto fetch_aux_box = [&](int t) {
+      if (AHEAD && p.aux != nullptr && box0 < C && tile_row(t) < p.M && elect_one()) {
+        tma_store_wait_read0();
+        mbar_expect_tx(aux_full(e), S::STAGING_BYTES);
+        tma_load_2d(stage_s, &tmAux, box0, tile_row(t), aux_full(e));
+      }
+    };
+
+    // The tile's output boxes, columns box0 + 128 i. pre: requested ahead of a chunk's work, the first box's gate
+    // (AHEAD) or aux.
+    int aux_uses = 0;
+    auto store_tile = [&](int t, uint4 (&pre)[4]) -> bool {
+      const int ob = AHEAD ? t & 1 : 0;
+      const int m_warp = tile_row(t);
+      bool ready = false;
+#pragma unroll 1
+      for (int n0 = box0; n0 < C; n0 += 128) {
+        uint4 aux[4], gate[4];
+        if constexpr (AHEAD) {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) gate[q] = pre[q];
+        } else {
+#pragma unroll
+          for (int q = 0; q < 4; ++q) aux[q] = pre[q];
+          fetch(gate, p.gate, p.ldgate, t, n0);
+          fetch(pre, p.aux, p.ldaux, t, n0 + 128);   // the next box's
+        }
+        if (!ready) {
+          if (!gemm_wait(out_full(ob), (AHEAD ? t >> 1 : t) & 1u, abort_flag, ST_TIMEOUT_EPILOGUE)) return false;
+          tc_fence_after();
+          ready = true;
+        }
+        if (m_warp >= p.M) break;             // (warp-uniform; the hand-over below is still owed)
+        if constexpr (AHEAD) {
+          if (p.aux != nullptr) {
+            if (!gemm_wait(aux_full(e), aux_uses & 1u, abort_flag, ST_TIMEOUT_EPILOGUE)) return false;
+            ++aux_uses;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const uint32_t addr = my_row_s + ((static_cast<uint32_t>(q) ^ sw) << 4);
+              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(aux[q].x), "=r"(aux[q].y), "=r"(aux[q].z), "=r"(aux[q].w)
+                           : "r"(addr) : "memory");
+            }
+          } else {
+            if (elect_one()) tma_store_wait_read0();
+            __syncwarp();
+          }
+        } else {
+          if (elect_one()) tma_store_wait_read0();   // the staging box has been read
+          __syncwarp();
+        }
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+          uint32_t acc[16];
+          tmem_ld_32x16(lane_taddr + S::OUT_COL + ob * S::OUT_STRIDE + n0 + 16 * g, acc);
+          tmem_ld_wait();
+          float v[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(acc[i]);
+          if (p.b2 != nullptr) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const float4 b4 = __ldg(reinterpret_cast<const float4*>(p.b2 + n0 + 16 * g) + q);
+              v[4 * q] += b4.x; v[4 * q + 1] += b4.y; v[4 * q + 2] += b4.z; v[4 * q + 3] += b4.w;
+            }
+          }
+          if (p.aux != nullptr) {
+            const uint32_t ax[8] = {aux[2 * g].x, aux[2 * g].y, aux[2 * g].z, aux[2 * g].w,
+                                    aux[2 * g + 1].x, aux[2 * g + 1].y, aux[2 * g + 1].z, aux[2 * g + 1].w};
+            if (p.gate != nullptr) {
+              const uint32_t gt[8] = {gate[2 * g].x, gate[2 * g].y, gate[2 * g].z, gate[2 * g].w,
+                                      gate[2 * g + 1].x, gate[2 * g + 1].y, gate[2 * g + 1].z, gate[2 * g + 1].w};
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const uint32_t yb = pack_bf16(v[2 * i], v[2 * i + 1]);
+                v[2 * i] = fmaf(bf16_lo(gt[i]), bf16_lo(yb), bf16_lo(ax[i]));
+                v[2 * i + 1] = fmaf(bf16_hi(gt[i]), bf16_hi(yb), bf16_hi(ax[i]));
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                v[2 * i] += bf16_lo(ax[i]);
+                v[2 * i + 1] += bf16_hi(ax[i]);
+              }
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < 2; ++q) {
+            const uint32_t addr = my_row_s + ((static_cast<uint32_t>(2 * g + q) ^ sw) << 4);
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr),
+                         "r"(pack_bf16(v[8 * q], v[8 * q + 1])), "r"(pack_bf16(v[8 * q + 2], v[8 * q + 3])),
+                         "r"(pack_bf16(v[8 * q + 4], v[8 * q + 5])), "r"(pack_bf16(v[8 * q + 6], v[8 * q + 7]))
+                         : "memory");
+          }
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (elect_one()) {
+          tma_store_2d(&tmOut, stage_s, n0, m_warp);
+          tma_store_commit();
+        }
+      }
+      // the output columns may be accumulated into again
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(out_free(ob));
+      if constexpr (!AHEAD) {
+        // the staging boxes lie in the hidden chunk's buffer: nobody writes there before all have been read
+        if (elect_one()) tma_store_wait_read0();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(staged);
+        if (!gemm_wait(staged, t & 1u, abort_flag, ST_TIMEOUT_EPILOGUE)) return false;
+      }
+      return true;
+    };
+
+    bool ok = true;
+    uint4 pre[4] = {};
+    if constexpr (AHEAD) {
+      // a set's first chunk of a tile comes before the store of the tile before
+      int c0 = 0;
+      for (int t = 0; t <= n_my && ok; ++t, c0 += nj) {
+        int j = (set + c0) & 1;              // the set's first chunk of this tile (chunk numbers run through the tiles)
+        if (t > 0) fetch(pre, p.gate, p.ldgate, t - 1, box0);
+        if (t < n_my && j < nj) {
+          ok = gelu_chunk(c0 + j, j);
+          j += 2;
+        }
+        if (t > 0 && ok) ok = store_tile(t - 1, pre);
+        if (t == n_my || !ok) break;
+        fetch_aux_box(t);
+        for (; j < nj && ok; j += 2) ok = gelu_chunk(c0 + j, j);
+      }
+    } else {
+      int c = 0;
+      for (int t = 0; t < n_my && ok; ++t) {
+        for (int j = 0; j < nj && ok; ++j, ++c) {
+          if (j == nj - 1) fetch(pre, p.aux, p.ldaux, t, box0);
+          ok = gelu_chunk(c, j);
+        }
+        if (ok) ok = store_tile(t, pre);
+      }
+    }
+    if (elect_one()) tma_store_wait_all();
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    __syncwarp();
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+template <int C>
+inline int launch_mlp_t(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w1, const __nv_bfloat16* w2,
+                        __nv_bfloat16* y, long long ldy, const MlpParams& p, int sm_count, cudaStream_t stream) {
+  using S = MlpSmem<C>;
+  CUtensorMap tmX, tmW1, tmW2, tmOut, tmAux;
+  auto make = [&](CUtensorMap* tm, const __nv_bfloat16* base, uint64_t cols, uint64_t rows, long long ld, uint32_t bc,
+                  uint32_t br, TmapSwizzle swz) {
+    const uint64_t dims[2] = {cols, rows}, str[1] = {static_cast<uint64_t>(ld) * 2};
+    const uint32_t box[2] = {bc, br};
+    return make_tmap_bf16(tm, base, 2, dims, str, box, swz);
+  };
+  const uint64_t M = static_cast<uint64_t>(p.M), H = static_cast<uint64_t>(p.H);
+  if (make(&tmX, x, C, M, ldx, 64, 128, TMAP_SWIZZLE_128B) != 0 ||
+      make(&tmW1, w1, C, H, C, 64, MLP_CHUNK, TMAP_SWIZZLE_128B) != 0 ||
+      make(&tmW2, w2, H, C, p.H, 64, C, TMAP_SWIZZLE_128B) != 0 ||
+      make(&tmOut, y, C, M, ldy, 32, 32, TMAP_SWIZZLE_64B) != 0)
+    return -20;
+  tmAux = tmOut;
+  if (p.aux != nullptr && make(&tmAux, p.aux, C, M, p.ldaux, 32, 32, TMAP_SWIZZLE_64B) != 0) return -20;
+  auto kern = mlp_tcgen05_kernel<C>;
+  static std::atomic<uint64_t> smem_set;
+  if (const cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), S::TOTAL, smem_set); e != cudaSuccess)
+    return -static_cast<int>(e) - 1000;
+  const int tiles = (p.M + 127) / 128;
+  return launch_chained(kern, dim3(static_cast<unsigned>(tiles < sm_count ? tiles : sm_count)), GEMM_THREADS, S::TOTAL,
+                        stream, 1, tmX, tmW1, tmW2, tmOut, tmAux, p);
+}
+
+// Whether the kernel takes these sizes (weights contiguous, everything else as the GEMMs want it).
+inline bool mlp_fused_sizes(int C, int H) { return C % 64 == 0 && C > 0 && C <= MLP_MAX_C && H % MLP_CHUNK == 0 && H > 0; }
+
+// Whether it is the faster way: two GEMMs / this kernel, microseconds with a residual, from a cold L2, at 256, 1024,
+// 8192, 24576, 131072 and 442368 rows, H = 4 C:
+//   C =  64: 13.1 / 11.0, 15.3 / 11.1, 17.3 / 11.2, 21.4 / 14.3, 46 / 31, 132 / 80
+//   C = 128: 13.3 / 14.3, 17.3 / 14.2, 17.4 / 14.3, 25.6 / 20.5, 79 / 51, 232 / 145
+//   C = 192: 15.3 / 20.4, 21.5 / 19.4, 23.6 / 20.5, 35.8 / 34.7, 116 / 100, 345 / 301
+//   C = 256: 17.4 / 24.5, 23.6 / 23.6, 27.6 / 24.5, 44.0 / 43.0, 155 / 129, 480 / 412
+// A few row blocks of a wide model leave most SMs idle through all of its chunks.
+inline bool mlp_fused_pays(int M, int C, int H) { return mlp_fused_sizes(C, H) && (C <= 128 || M >= 1024); }
+
+inline int launch_mlp(int C, const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w1, const __nv_bfloat16* w2,
+                      __nv_bfloat16* y, long long ldy, const MlpParams& p, int sm_count, cudaStream_t stream) {
+  switch (C) {
+    case 64: return launch_mlp_t<64>(x, ldx, w1, w2, y, ldy, p, sm_count, stream);
+    case 128: return launch_mlp_t<128>(x, ldx, w1, w2, y, ldy, p, sm_count, stream);
+    case 192: return launch_mlp_t<192>(x, ldx, w1, w2, y, ldy, p, sm_count, stream);
+    case 256: return launch_mlp_t<256>(x, ldx, w1, w2, y, ldy, p, sm_count, stream);
+    default: return -2;
+  }
+}
+
+}  // namespace strata

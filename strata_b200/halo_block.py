@@ -193,8 +193,8 @@ class TiledBlockRunner:
                 ac = ops.linear(ops.layernorm(xc), weights["w_gate"], weights.get("b_gate"),
                                 ops.EPI_GATE, ac)
             x1 = ops.linear(ac, weights["w_proj"], weights.get("b_proj"), ops.EPI_RESIDUAL, xc)
-            hmid = ops.linear(ops.layernorm(x1), weights["w_fc1"], weights.get("b_fc1"), ops.EPI_GELU)
-            ops.linear(hmid, weights["w_fc2"], weights.get("b_fc2"), ops.EPI_RESIDUAL, x1, out=y[sl])
+            ops.mlp(ops.layernorm(x1), weights["w_fc1"], weights.get("b_fc1"), weights["w_fc2"],
+                    weights.get("b_fc2"), x1, out=y[sl])
         return y.view(tpr, tokens, C)
 
     def check_status(self) -> None:

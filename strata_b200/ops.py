@@ -113,6 +113,31 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
     return out if x.dim() == 2 else out.reshape(*x.shape[:-1], N)
 
 
+def mlp(x: torch.Tensor, w1: torch.Tensor, b1: torch.Tensor | None, w2: torch.Tensor,
+        b2: torch.Tensor | None, residual: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+    """residual + linear(gelu(linear(x, w1, b1)), w2, b2) of rows [M, C]: one kernel for narrow models, the two
+    GEMMs otherwise; the same bits either way."""
+    M, C = x.shape
+    H = w1.shape[0]
+    rows = (x, residual) if out is None else (x, residual, out)
+    if not (x.is_cuda and _lib.load().strata_mlp_fused(M, C, H) and w1.is_contiguous() and w2.is_contiguous() and
+            tuple(w2.shape) == (C, H) and all(t.shape == x.shape and t.stride(1) == 1 for t in rows)):
+        return linear(linear(x, w1, b1, EPI_GELU), w2, b2, EPI_RESIDUAL, residual, out=out)
+    for t, n in ((x, "x"), (w1, "w1"), (w2, "w2"), (residual, "residual")):
+        _require_cuda_bf16(t, n)
+    b1, b2 = _f32_or_none(b1, "b1"), _f32_or_none(b2, "b2")
+    if out is None:
+        out = torch.empty((M, C), dtype=torch.bfloat16, device=x.device)
+    else:
+        _require_cuda_bf16(out, "out")
+    with _lib.on_device(x):
+        _lib.check(_lib.load().strata_mlp_bf16(
+            x.data_ptr(), x.stride(0), w1.data_ptr(), None if b1 is None else b1.data_ptr(), w2.data_ptr(),
+            None if b2 is None else b2.data_ptr(), residual.data_ptr(), residual.stride(0), None, 0,
+            out.data_ptr(), out.stride(0), M, C, H, _stream_ptr(x)), "strata_mlp_bf16")
+    return out
+
+
 def qkv_rope(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None, head_dim: int,
              rope_cos: torch.Tensor | None, rope_sin: torch.Tensor | None, tokens_per_tile: int,
              hw: int, qk_norm: bool = False, qk_eps: float = 1e-6,

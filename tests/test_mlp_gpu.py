@@ -1,0 +1,89 @@
+"""The one-kernel MLP of narrow blocks against the two GEMMs it stands for (same bits) and the fp32 result."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from strata_b200 import ops
+    return ops
+
+
+def _data(M, C, H, seed, pad=0):
+    g = torch.Generator("cuda").manual_seed(seed)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    rows = lambda: rnd(M, C + pad).bfloat16()[:, :C]       # pad: rows with a stride of their own
+    return dict(x=rows(), aux=rows(), gate=rows(), w1=(rnd(H, C) * C ** -0.5).bfloat16(),
+                w2=(rnd(C, H) * H ** -0.5).bfloat16(), b1=rnd(H) * 0.1, b2=rnd(C) * 0.1)
+
+
+def _fused(ops, d, aux, gate, bias, out):
+    from strata_b200 import _lib
+    ptr = lambda t: None if t is None else t.data_ptr()
+    ld = lambda t: 0 if t is None else t.stride(0)
+    M, C = d["x"].shape
+    H = d["w1"].shape[0]
+    b1, b2 = (d["b1"], d["b2"]) if bias else (None, None)
+    lib = _lib.load()
+    assert lib.strata_mlp_bf16(ptr(d["x"]), ld(d["x"]), ptr(d["w1"]), ptr(b1), ptr(d["w2"]), ptr(b2), ptr(aux), ld(aux),
+                               ptr(gate), ld(gate), ptr(out), ld(out), M, C, H,
+                               torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    assert _lib.device_status() == 0
+
+
+# rows: one, the edges of a 128-row tile and of a 32-row box, one tile more than the SMs, several tiles a CTA;
+# hidden: one chunk, an odd number of them, several
+@pytest.mark.parametrize("M,C,H,mode,pad", [
+    (1, 64, 128, "residual", 0), (127, 64, 256, "bias", 0), (129, 128, 128, "residual", 8), (31, 128, 512, "gate", 0),
+    (97, 192, 768, "gate", 8), (256, 192, 384, "residual", 0), (300, 256, 1024, "residual", 0), (160, 256, 128, "bias", 8),
+    (149 * 128 + 5, 128, 512, "gate", 0), (149 * 128 + 5, 256, 384, "residual", 0), (45001, 64, 128, "residual", 0),
+    (60007, 128, 384, "residual", 0), (60007, 192, 768, "gate", 0), (60007, 256, 1024, "bias", 0)])
+@pytest.mark.parametrize("bias", [True, False])
+def test_mlp_is_the_two_gemms(ops, M, C, H, mode, pad, bias):
+    from strata_b200 import _lib
+    d = _data(M, C, H, M + C + H, pad)
+    b1, b2 = (d["b1"], d["b2"]) if bias else (None, None)
+    aux = d["aux"] if mode != "bias" else None
+    gate = d["gate"] if mode == "gate" else None
+    out = torch.full((M, C + pad), float("nan"), device="cuda", dtype=torch.bfloat16)[:, :C]
+    _fused(ops, d, aux, gate, bias, out)
+    h = ops.linear(d["x"], d["w1"], b1, ops.EPI_GELU)
+    if mode == "residual":
+        want = ops.linear(h, d["w2"], b2, ops.EPI_RESIDUAL, aux)
+    else:
+        want = ops.linear(h, d["w2"], b2)
+        if mode == "gate":
+            y, want = want, torch.empty_like(want)
+            assert _lib.load().strata_adaln_rows_bf16(
+                aux.data_ptr(), aux.stride(0), y.data_ptr(), C, gate.data_ptr(), gate.stride(0), want.data_ptr(), C,
+                None, None, 0, None, 0, M, C, 1e-6, torch.cuda.current_stream().cuda_stream) == 0
+    assert torch.equal(out, want)
+    t = torch.nn.functional.gelu(d["x"].double() @ d["w1"].double().T + (b1.double() if bias else 0.0), approximate="tanh")
+    t = t @ d["w2"].double().T + (b2.double() if bias else 0.0)
+    if mode != "bias":
+        t = aux.double() + (gate.double() if gate is not None else 1.0) * t
+    # bf16 hidden channels and result: two roundings of 2^-9 relative rms at most, and bf16's own
+    assert float((out.double() - t).norm() / t.norm()) < 4e-3
+
+
+def test_mlp_in_place_and_through_ops(ops):
+    d = _data(5000, 128, 512, 3)
+    want = ops.linear(ops.linear(d["x"], d["w1"], d["b1"], ops.EPI_GELU), d["w2"], d["b2"], ops.EPI_RESIDUAL, d["aux"])
+    assert torch.equal(ops.mlp(d["x"], d["w1"], d["b1"], d["w2"], d["b2"], d["aux"]), want)
+    x = d["aux"].clone()
+    _fused(ops, d, x, None, True, x)            # the result goes over the residual
+    assert torch.equal(x, want)
+
+
+def test_mlp_refuses_what_it_has_no_kernel_for(ops):
+    from strata_b200 import _lib
+    x = torch.zeros(128, 320, device="cuda", dtype=torch.bfloat16)
+    f = _lib.load().strata_mlp_bf16
+    p = x.data_ptr()
+    assert f(p, 320, p, None, p, None, None, 0, None, 0, p, 320, 128, 320, 1280, 0) == -2     # too wide
+    assert f(p, 320, p, None, p, None, None, 0, None, 0, p, 320, 128, 128, 320, 0) == -2      # part of a chunk
+    assert f(p, 320, p, None, p, None, None, 0, p, 320, p, 320, 128, 128, 128, 0) == -1       # a gate without aux
+    assert f(p + 2, 320, p, None, p, None, None, 0, None, 0, p, 320, 128, 128, 128, 0) == -1  # alignment
