@@ -210,7 +210,6 @@ static int qkv_rope_impl(const void* x, int64_t ldx, const void* w, int64_t ldw,
   p.hw = hw > 0 ? hw : 1;
   p.head_dim = head_dim;
   p.rope_cols = 2 * C;
-  p.qk_norm = qk_norm;
   p.qk_eps = qk_eps;
   if (pad_T > 0) {
     if (pad_T % 32 != 0 || pad_halo < 0 || pad_D < 1 ||
@@ -224,12 +223,11 @@ static int qkv_rope_impl(const void* x, int64_t ldx, const void* w, int64_t ldw,
   if (!rope_cs && C < 256 && head_dim == 64) {
     // qk norm without rotation at a small width: a plain projection and the in-place row kernel, which
     // normalises the q and k heads, against the fused epilogue with an identity table. Two kernels / fused,
-    // microseconds: C = 128 at 1572864 rows (the pixel stage of one production tile) 599 / 558, 262144 114 /
-    // 114, 24576 16.9 / 17.4, 1024 7.7 / 9.2; C = 64 341 / 306, 62 / 69, 13.3 / 12.8, 8.2 / 8.7; C = 192 1113 /
-    // 1072, 202 / 210, 23.0 / 24.1, 9.7 / 9.7 - within 10 % either way, in favour of two kernels where a launch
-    // is short. From C = 256 on fused is ahead: 1263 / 947, 212 / 173, 24.6 / 21.9, 9.6 / 9.6; C = 512 at 262144
-    // rows 525 / 388. (Here the norm sees q and k rounded to bf16, there the fp32 accumulators: error against
-    // 64 bits 2.1e-3 and 1.7e-3 of the result.)
+    // microseconds at 1024, 24576, 262144 and 1572864 rows (the pixel stage of one production tile): C = 64 13.3 / 13.3,
+    // 17.4 / 17.4, 54 / 56, 327 / 282; C = 128 11.2 / 13.4, 19.5 / 20.5, 103 / 98, 570 / 520; C = 192 13.3 / 14.3, 25.6 /
+    // 26.6, 183 / 171, 1157 / 949 - in favour of two kernels where a launch is short. From C = 256 on fused is
+    // ahead: 212 / 173, 24.6 / 21.9, 9.6 / 9.6; C = 512 at 262144 rows 491 / 377. (Here the norm sees q and k rounded
+    // to bf16, there the fp32 accumulators: error against 64 bits 2.1e-3 and 1.7e-3 of the result.)
     int r = launch_gemm<EPI_BIAS>(A, ldx, W, ldw, p, sms, as_stream(stream));
     if (r != 0) return r;
     long long rows = M;
@@ -252,7 +250,8 @@ static int qkv_rope_impl(const void* x, int64_t ldx, const void* w, int64_t ldw,
     p.tokens_per_tile = M;
     p.hw = 1;
   }
-  return launch_gemm<EPI_QKV_ROPE>(A, ldx, W, ldw, p, sms, as_stream(stream));
+  return qk_norm ? launch_gemm<EPI_QKV_NORM>(A, ldx, W, ldw, p, sms, as_stream(stream))
+                 : launch_gemm<EPI_QKV_ROPE>(A, ldx, W, ldw, p, sms, as_stream(stream));
 }
 
 int strata_qkv_rope_bf16(const void* x, int64_t ldx, const void* w, int64_t ldw, const float* bias,

@@ -25,7 +25,8 @@
 //   EPI_BIAS           y = acc + b                                   (generic Linear)
 //   EPI_GELU           y = gelu_tanh(acc + b)                        (mlp.layers.0 + tanh GELU)
 //   EPI_RESIDUAL       y = acc + b + R[m,n]                          (attn.proj / mlp.layers.2)
-//   EPI_QKV_ROPE       y = rope(rmsnorm?(acc + b)) on q,k columns    (attn.qkv + RoPE + pack)
+//   EPI_QKV_ROPE       y = rope(acc + b) on q,k columns              (attn.qkv + RoPE + pack)
+//   EPI_QKV_NORM       y = rope(rmsnorm(acc + b)) on q,k columns     (the same with the q/k norm)
 //   EPI_GATE           y = G[m,n] * sigmoid(acc + b)                 (attn.gate_proj)
 #pragma once
 #include <cuda_fp16.h>
@@ -43,6 +44,7 @@ enum GemmEpilogue : int {
   EPI_RESIDUAL = 2,
   EPI_QKV_ROPE = 3,
   EPI_GATE = 4,
+  EPI_QKV_NORM = 5,   // EPI_QKV_ROPE with the q/k norm
 };
 
 struct GemmParams {
@@ -60,7 +62,6 @@ struct GemmParams {
   int hw;
   int head_dim;
   int rope_cols;   // columns [0, rope_cols) are q and k
-  int qk_norm;     // 1: RMS-normalise each head of q and k before the rotation
   float qk_eps;
   // Output row remap (pad_T > 0): the M input rows are the interior tokens of tiles
   // [tile, d, i, j] with i, j < pad_T (pad_T a multiple of 32), and row m is stored at row
@@ -131,16 +132,12 @@ __device__ __forceinline__ uint64_t gelu_pair(uint64_t x) {
   return ffma2(hx, t, hx);
 }
 
-// Epilogue math on 16 consecutive columns of output row m, in place. Lane `src_lane0 + j` of
-// the warp holds the bias of column j of the group; `aux` holds the residual / gated operand of
-// the same columns (bf16 pairs) for the epilogues that use one; `qk_scale` is the RMS-norm
-// factor of the head these columns belong to; cs: this row's (cos, sin) half pairs for the 8
-// channel pairs of these 16 columns.
+// Epilogue math of the row-per-lane form on 16 consecutive columns of output row m, in place. Lane `src_lane0 + j` of
+// the warp holds the bias of column j of the group; cs: this row's (cos, sin) half pairs for the 8 channel pairs of
+// these 16 columns.
 template <int EPI>
-__device__ __forceinline__ void gemm_epilogue_16(float (&v)[16], bool rotate, float b_lane,
-                                                 int src_lane0, const uint32_t (&aux)[8],
-                                                 float qk_scale, const uint32_t (&cs)[8],
-                                                 const GemmParams& p, const float* bias16) {
+__device__ __forceinline__ void gemm_epilogue_16(float (&v)[16], bool rotate, float b_lane, int src_lane0,
+                                                 const uint32_t (&cs)[8], const GemmParams& p, const float* bias16) {
   if (p.bias != nullptr) {
     if (bias16 != nullptr) {
       // the 16 biases of this column group, the same for every row: four 16-byte loads at an
@@ -156,27 +153,8 @@ __device__ __forceinline__ void gemm_epilogue_16(float (&v)[16], bool rotate, fl
       for (int j = 0; j < 16; ++j) v[j] += __shfl_sync(0xffffffffu, b_lane, src_lane0 + j);
     }
   }
-  if constexpr (EPI == EPI_GELU) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) unpack2(gelu_pair(pack2(v[2 * j], v[2 * j + 1])), v[2 * j], v[2 * j + 1]);
-  } else if constexpr (EPI == EPI_RESIDUAL) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      v[2 * j] += bf16_lo(aux[j]);
-      v[2 * j + 1] += bf16_hi(aux[j]);
-    }
-  } else if constexpr (EPI == EPI_GATE) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      v[2 * j] = bf16_lo(aux[j]) / (1.0f + __expf(-v[2 * j]));
-      v[2 * j + 1] = bf16_hi(aux[j]) / (1.0f + __expf(-v[2 * j + 1]));
-    }
-  } else if constexpr (EPI == EPI_QKV_ROPE) {
+  if constexpr (EPI == EPI_QKV_ROPE) {
     if (rotate) {
-      if (p.qk_norm) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] *= qk_scale;
-      }
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float2 t =
@@ -187,6 +165,75 @@ __device__ __forceinline__ void gemm_epilogue_16(float (&v)[16], bool rotate, fl
       }
     }
   }
+}
+
+// The other epilogues read the accumulator as matrix fragments, 16 rows x 32 columns a load: registers 4 i + {0, 1} hold row lane / 4,
+// columns 8 i + 2 (lane % 4) + {0, 1}, registers 4 i + {2, 3} the same of row lane / 4 + 8. A lane then needs eight
+// biases for 32 columns (with a row per lane all 32) and holds the pairs that the rotation turns, a row's
+// squares are summed within a quad, and 8 x 8 pieces go to the staging boxes and come from them with stmatrix and
+// ldmatrix.
+__device__ __forceinline__ void tmem_ld_16x256_x4(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void stmatrix_x4(uint32_t addr, const uint32_t* w) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w[0]), "r"(w[1]),
+               "r"(w[2]), "r"(w[3]) : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t* w) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(addr) : "memory");
+}
+
+// The biases of this lane's columns in the 32 from n0 (zero without a bias, and behind column N).
+__device__ __forceinline__ void gemm_lane_bias(const GemmParams& p, int n0, int lane, uint64_t (&bias)[4]) {
+  const int n = n0 + 2 * (lane & 3);
+  if (p.bias != nullptr && n0 + 32 <= p.N) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) bias[i] = __ldg(reinterpret_cast<const unsigned long long*>(p.bias + n + 8 * i));
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int k = n + 8 * i;
+      bias[i] = p.bias == nullptr ? 0ull : pack2(k < p.N ? __ldg(p.bias + k) : 0.f, k + 1 < p.N ? __ldg(p.bias + k + 1) : 0.f);
+    }
+  }
+}
+
+// Epilogue math on a pair of neighbouring columns of one row (bias added); aux: the residual / gated operand of the
+// pair (bf16); cs: its (cos, sin) half pair; scale: the RMS factor of the row's head.
+template <int EPI>
+__device__ __forceinline__ uint32_t gemm_epilogue_pair(uint64_t x, uint32_t aux, bool rotate, uint32_t cs, float scale) {
+  float a, b;
+  if constexpr (EPI == EPI_GELU) {
+    unpack2(gelu_pair(x), a, b);
+  } else {
+    unpack2(x, a, b);
+    if constexpr (EPI == EPI_RESIDUAL) {
+      a += bf16_lo(aux);
+      b += bf16_hi(aux);
+    } else if constexpr (EPI == EPI_GATE) {
+      a = bf16_lo(aux) / (1.0f + __expf(-a));
+      b = bf16_hi(aux) / (1.0f + __expf(-b));
+    } else if constexpr (EPI == EPI_QKV_NORM) {
+      if (rotate) {
+        a *= scale;
+        b *= scale;
+        const float2 t = __half22float2(*reinterpret_cast<const __half2*>(&cs));   // (cos, sin)
+        // (spelled out: the row form's contractions, so that both give the same bits)
+        const float r0 = __fmaf_rn(a, t.x, -__fmul_rn(b, t.y));
+        b = __fmaf_rn(a, t.y, __fmul_rn(b, t.x));
+        a = r0;
+      }
+    }
+  }
+  return pack_bf16(a, b);
 }
 
 // Per-head RMS factors of the q/k norm for one output row: one extra pass over the warp's
@@ -272,7 +319,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmOut,
                     const __grid_constant__ CUtensorMap tmAux, const GemmParams p) {
-  constexpr bool TABLE = EPI == EPI_QKV_ROPE;
+  constexpr bool TABLE = EPI == EPI_QKV_ROPE || EPI == EPI_QKV_NORM;
+  // The accumulator as matrix fragments (see above) or a row per lane. Fragments / rows, microseconds: residual
+  // 262144 x 512, K = 512 115 / 121, 442368 x 256, K = 256 91 / 101; GELU 442368 x 1024, K = 256 231 / 267, 103000 x 1536,
+  // K = 384 103 / 110, level from K = 512 on; q/k norm and rotation 262144 x 1536, K = 512 377 / 383, 98304 x 2304,
+  // K = 768 243 / 267, 103000 x 1152, K = 384 150 / 167. The other way: rotation alone 346 / 338, 252 / 246, 121 / 120
+  // (without the norm's code in the kernel rows take 324, 245, 121); bias alone 295 / 291, 171 / 166.
+  constexpr bool FRAG = EPI != EPI_BIAS && EPI != EPI_QKV_ROPE;
   using S = GemmSmem<BN, PAIR, TABLE>;
   // PAIR: this CTA is rank 0 or 1 of a cluster of two that computes 256 x BN tiles together
   const uint32_t pair_rank = PAIR ? cluster_ctarank() : 0u;
@@ -281,7 +334,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   constexpr int TILE_M = PAIR ? 2 * GEMM_BM : GEMM_BM;
   constexpr bool HAS_AUX = (EPI == EPI_RESIDUAL || EPI == EPI_GATE);
   // Epilogues without an operand to prefetch wait for the staging box as late as possible.
-  constexpr bool LATE_WAIT = (EPI == EPI_BIAS || EPI == EPI_GELU || EPI == EPI_QKV_ROPE);
+  constexpr bool LATE_WAIT = !HAS_AUX;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -444,8 +497,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     constexpr int WARP_COLS = BN / 4;
     constexpr int NSUB = WARP_COLS / 32;
     const uint32_t stage_s = smem_base + S::STAGING_OFF + e * S::STAGING_BYTES;
-    const uint32_t my_row_s = stage_s + lane * 64;
-    const uint32_t sw = static_cast<uint32_t>((lane >> 1) & 3);   // 64-byte swizzle of this row
+    [[maybe_unused]] const uint32_t my_row_s = stage_s + lane * 64;               // (row form: this lane's row, its swizzle)
+    [[maybe_unused]] const uint32_t sw = static_cast<uint32_t>((lane >> 1) & 3);
+    // this lane's row of the four 8 x 8 pieces (rows 16 hf + {0, 8}, columns 16 q + {0, 8}) of a staging box: 64-byte
+    // rows, 64-byte swizzle
+    const uint32_t box_row = stage_s + static_cast<uint32_t>(((lane >> 3) & 1) * 8 + (lane & 7)) * 64u;
+    auto box_addr = [&](int hf, int q) -> uint32_t {
+      return box_row + hf * 1024u + ((static_cast<uint32_t>(2 * q + (lane >> 4)) ^ static_cast<uint32_t>((lane >> 1) & 3)) << 4);
+    };
     const uint32_t acce_remote0 = PAIR ? map_to_cta(acce_bar(0), 0) : 0u;
     const uint32_t acce_remote1 = PAIR ? map_to_cta(acce_bar(1), 0) : 0u;
     uint32_t aux_phase = 0;
@@ -477,15 +536,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const int m0 = mt * TILE_M + static_cast<int>(pair_rank) * GEMM_BM;
       const int n_tile0 = jt * BN;
       const int m_warp = m0 + quarter * 32;
-      const int m = m_warp + lane;
-      const bool row_ok = m < p.M;
       const int n_warp0 = n_tile0 + cg * WARP_COLS;
-      bool rope_tile = false;
-      [[maybe_unused]] uint32_t tab_row = 0;
+      [[maybe_unused]] uint32_t tab_base = 0;   // the tile's table rows of this lane quarter
       if constexpr (TABLE) {
         if (rope) {
-          rope_tile = n_warp0 < p.rope_cols && row_ok;
-          tab_row = tab_quarter + static_cast<uint32_t>(buf) * (GEMM_BM * 128u) + lane * 128u;
+          tab_base = tab_quarter + static_cast<uint32_t>(buf) * (GEMM_BM * 128u);
           // this warp's part of the tile's table has arrived; when all four warps say so, the whole has,
           // and none of them reads the tile before's any more: the next tile's goes there
           asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -500,84 +555,65 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         }
       }
       bool acc_ready = false;
-      // per-head RMS factor (qk norm): one extra pass over the head's 64 (or 32) accumulator
-      // columns; with 64-wide heads the warp's 64 columns are exactly one head
-      float qk_scale[NSUB];
-#pragma unroll
-      for (int c = 0; c < NSUB; ++c) qk_scale[c] = 1.f;
+      float qk_scale[4] = {1.f, 1.f, 1.f, 1.f};   // RMS factors of this lane's four rows
+      [[maybe_unused]] float2 row_scale = make_float2(1.f, 1.f);   // of row `lane`, for the warp's two sub-chunks
 #pragma unroll 1
       for (int c = 0; c < NSUB; ++c) {
         const int n0 = n_warp0 + c * 32;
         const bool chunk_live = (n0 < p.N) && (m_warp < p.M);   // warp-uniform
-        float b_lane = 0.f;
-        if (p.bias != nullptr && n0 + lane < p.N) b_lane = __ldg(p.bias + n0 + lane);
-        if constexpr (!LATE_WAIT) {
-          if (chunk_live) {
-            // staging box free again? (previous TMA store has finished reading it) - a
-            // residual / gated operand is fetched into it right away
-            if (elect_one()) tma_store_wait_read0();
-            __syncwarp();
-            if constexpr (HAS_AUX) {
-              if (elect_one()) {
-                mbar_expect_tx(aux_bar(e), S::STAGING_BYTES);
-                tma_load_2d(stage_s, &tmAux, n0, m_warp, aux_bar(e));
+        if constexpr (FRAG) {
+          uint64_t bias[4];
+          gemm_lane_bias(p, n0, lane, bias);
+          if constexpr (!LATE_WAIT) {
+            if (chunk_live) {
+              // staging box free again? (previous TMA store has finished reading it) - a
+              // residual / gated operand is fetched into it right away
+              if (elect_one()) tma_store_wait_read0();
+              __syncwarp();
+              if constexpr (HAS_AUX) {
+                if (elect_one()) {
+                  mbar_expect_tx(aux_bar(e), S::STAGING_BYTES);
+                  tma_load_2d(stage_s, &tmAux, n0, m_warp, aux_bar(e));
+                }
               }
             }
           }
-        }
-        if (!acc_ready) {
-          if (!gemm_wait(accf_bar(buf), acc_phase, abort_flag, ST_TIMEOUT_EPILOGUE)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          acc_ready = true;
-        }
-        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
-                               static_cast<uint32_t>(buf * BN + cg * WARP_COLS + c * 32);
-        if constexpr (EPI == EPI_QKV_ROPE) {
-          if (c == 0 && p.qk_norm && m_warp < p.M && n_warp0 < p.rope_cols && n_warp0 < p.N) {
-            // (out of line: most models run without the q/k norm)
-            const float2 sc = gemm_qk_norm_scales<NSUB>(taddr, p.bias, n_warp0, p.N, lane, p.head_dim,
-                                                        p.qk_eps);
-            qk_scale[0] = sc.x;
-            qk_scale[NSUB - 1] = sc.y;
-          }
-        }
-        if constexpr (HAS_AUX) {
-          if (chunk_live) {
-            if (!gemm_wait(aux_bar(e), aux_phase, abort_flag, ST_TIMEOUT_EPILOGUE)) {
+          if (!acc_ready) {
+            if (!gemm_wait(accf_bar(buf), acc_phase, abort_flag, ST_TIMEOUT_EPILOGUE)) {
               ok = false;
               break;
             }
-            aux_phase ^= 1u;
+            tc_fence_after();
+            acc_ready = true;
           }
-        }
+          const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
+                                 static_cast<uint32_t>(buf * BN + cg * WARP_COLS + c * 32);
+          const bool rotate = rope && n0 < p.rope_cols;           // warp-uniform
+          if constexpr (EPI == EPI_QKV_NORM) {
+            // q/k norm: one extra pass over the warp's columns with a row per lane (a row's squares are then summed in
+            // column order by one lane); the factors of this lane's fragment rows come from the lanes that have them
+            if (c == 0 && rotate && chunk_live)
+              row_scale = gemm_qk_norm_scales<NSUB>(taddr, p.bias, n_warp0, p.N, lane, p.head_dim, p.qk_eps);
 #pragma unroll
-        for (int g = 0; g < 2; ++g) {
-          // head_dim 64: the 32-column sub-chunks of a head use table pairs [0,16) and
-          // [16,32); head_dim 32: each sub-chunk is a whole head and uses pairs [0,16).
-          // The table words are requested before the TMEM load so that the two latencies overlap.
-          const bool rotate = rope_tile && (n0 < p.rope_cols);
-          uint32_t cs[8];
-          if constexpr (EPI == EPI_QKV_ROPE) {
-            if (rotate && chunk_live) {
-              const int pair0 = ((p.head_dim == 64) ? (n0 & 63) >> 1 : 0) + 8 * g;
-#pragma unroll
-              for (int q = 0; q < 2; ++q) {
-                const uint32_t addr = tab_row + ((static_cast<uint32_t>((pair0 >> 2) + q) ^ (lane & 7u)) << 4);
-                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                             : "=r"(cs[4 * q]), "=r"(cs[4 * q + 1]), "=r"(cs[4 * q + 2]), "=r"(cs[4 * q + 3])
-                             : "r"(addr) : "memory");
+            for (int k = 0; k < 4; ++k)
+              qk_scale[k] = __shfl_sync(0xffffffffu, c == 0 ? row_scale.x : row_scale.y, 8 * k + (lane >> 2));
+          }
+          if constexpr (HAS_AUX) {
+            if (chunk_live) {
+              if (!gemm_wait(aux_bar(e), aux_phase, abort_flag, ST_TIMEOUT_EPILOGUE)) {
+                ok = false;
+                break;
               }
+              aux_phase ^= 1u;
             }
           }
-          uint32_t r[16];
+          uint32_t acc[2][16];
           if (chunk_live) {
-            tmem_ld_32x16(taddr + 16 * g, r);
+            tmem_ld_16x256_x4(taddr, acc[0]);
+            tmem_ld_16x256_x4(taddr + (16u << 16), acc[1]);
             tmem_ld_wait();
           }
-          if (g == 1 && c == NSUB - 1) {
+          if (c == NSUB - 1) {
             // the accumulator is in registers (or not needed): hand it back to the MMA warp
             tc_fence_before();
             __syncwarp();
@@ -587,27 +623,101 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             }
           }
           if (chunk_live) {
-            float v[16];
+            // head_dim 64: the 32-column sub-chunks of a head use table pairs [0, 16) and [16, 32); head_dim
+            // 32: each sub-chunk is a whole head and uses pairs [0, 16). The table's 16-byte pieces hold four pairs.
+            [[maybe_unused]] const uint32_t piece0 = p.head_dim == 64 ? static_cast<uint32_t>(n0 & 63) >> 3 : 0u;
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
-            uint32_t aux[8];
-            if constexpr (HAS_AUX) {
+            for (int hf = 0; hf < 2; ++hf) {
+              uint32_t aux[8], w[8];
+              if constexpr (HAS_AUX) {
 #pragma unroll
-              for (int q = 0; q < 2; ++q) {
-                const uint32_t addr = my_row_s + ((static_cast<uint32_t>(2 * g + q) ^ sw) << 4);
-                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                             : "=r"(aux[4 * q]), "=r"(aux[4 * q + 1]), "=r"(aux[4 * q + 2]),
-                               "=r"(aux[4 * q + 3])
-                             : "r"(addr)
-                             : "memory");
+                for (int q = 0; q < 2; ++q) ldmatrix_x4(box_addr(hf, q), &aux[4 * q]);
+              }
+              // (a pair of the table is four bytes, a piece four pairs: the words of an 8 x 8 matrix of halves)
+              uint32_t cs[8];
+              if constexpr (TABLE) {
+                if (rotate) {
+#pragma unroll
+                  for (int q = 0; q < 2; ++q)
+                    ldmatrix_x4(tab_base + (16 * hf + ((lane >> 3) & 1) * 8 + (lane & 7)) * 128u +
+                                    (((piece0 + 2 * q + (lane >> 4)) ^ (lane & 7u)) << 4),
+                                &cs[4 * q]);
+                }
+              }
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {       // columns 8 (i / 2), row + 8 (i % 2)
+                w[i] = gemm_epilogue_pair<EPI>(fadd2(pack2u(acc[hf][2 * i], acc[hf][2 * i + 1]), bias[i >> 1]),
+                                               HAS_AUX ? aux[i] : 0u, rotate, TABLE ? cs[i] : 0u,
+                                               qk_scale[2 * hf + (i & 1)]);
+              }
+              if constexpr (LATE_WAIT) {
+                if (hf == 0) {
+                  // the previous sub-chunk's TMA store must have finished reading the staging
+                  // box before it is overwritten; waiting only now lets that drain overlap with
+                  // the TMEM load and the arithmetic above
+                  if (elect_one()) tma_store_wait_read0();
+                  __syncwarp();
+                }
+              }
+#pragma unroll
+              for (int q = 0; q < 2; ++q) stmatrix_x4(box_addr(hf, q), &w[4 * q]);
+            }
+          }
+        } else {
+          float b_lane = 0.f;
+          if (p.bias != nullptr && n0 + lane < p.N) b_lane = __ldg(p.bias + n0 + lane);
+          if (!acc_ready) {
+            if (!gemm_wait(accf_bar(buf), acc_phase, abort_flag, ST_TIMEOUT_EPILOGUE)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            acc_ready = true;
+          }
+          const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
+                                 static_cast<uint32_t>(buf * BN + cg * WARP_COLS + c * 32);
+#pragma unroll
+          for (int g = 0; g < 2; ++g) {
+            // head_dim 64: the 32-column sub-chunks of a head use table pairs [0,16) and
+            // [16,32); head_dim 32: each sub-chunk is a whole head and uses pairs [0,16).
+            // The table words are requested before the TMEM load so that the two latencies overlap.
+            const bool rotate = rope && n0 < p.rope_cols;
+            uint32_t cs[8];
+            if constexpr (EPI == EPI_QKV_ROPE) {
+              if (rotate && chunk_live) {
+                const int pair0 = ((p.head_dim == 64) ? (n0 & 63) >> 1 : 0) + 8 * g;
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                  const uint32_t addr = tab_base + lane * 128u + ((static_cast<uint32_t>((pair0 >> 2) + q) ^ (lane & 7u)) << 4);
+                  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                               : "=r"(cs[4 * q]), "=r"(cs[4 * q + 1]), "=r"(cs[4 * q + 2]), "=r"(cs[4 * q + 3])
+                               : "r"(addr) : "memory");
+                }
               }
             }
-            // (the bias group is read directly when all its 16 columns exist; p.bias is
-            // 16-byte aligned and n0 a multiple of 32)
-            const float* bias16 = (p.bias != nullptr && n0 + 16 * g + 16 <= p.N)
-                                      ? p.bias + n0 + 16 * g : nullptr;
-            gemm_epilogue_16<EPI>(v, rotate, b_lane, 16 * g, aux, qk_scale[c], cs, p, bias16);
-            if constexpr (LATE_WAIT) {
+            uint32_t r[16];
+            if (chunk_live) {
+              tmem_ld_32x16(taddr + 16 * g, r);
+              tmem_ld_wait();
+            }
+            if (g == 1 && c == NSUB - 1) {
+              // the accumulator is in registers (or not needed): hand it back to the MMA warp
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) {
+                if constexpr (PAIR) mbar_arrive_cluster(buf ? acce_remote1 : acce_remote0);
+                else mbar_arrive(acce_bar(buf));
+              }
+            }
+            if (chunk_live) {
+              float v[16];
+#pragma unroll
+              for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+              // (the bias group is read directly when all its 16 columns exist; p.bias is
+              // 16-byte aligned and n0 a multiple of 32)
+              const float* bias16 = (p.bias != nullptr && n0 + 16 * g + 16 <= p.N)
+                                        ? p.bias + n0 + 16 * g : nullptr;
+              gemm_epilogue_16<EPI>(v, rotate, b_lane, 16 * g, cs, p, bias16);
               if (g == 0) {
                 // the previous sub-chunk's TMA store must have finished reading the staging
                 // box before it is overwritten; waiting only now lets that drain overlap with
@@ -615,16 +725,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 if (elect_one()) tma_store_wait_read0();
                 __syncwarp();
               }
-            }
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-              const uint32_t addr = my_row_s + ((static_cast<uint32_t>(2 * g + q) ^ sw) << 4);
-              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr),
-                           "r"(pack_bf16(v[8 * q], v[8 * q + 1])),
-                           "r"(pack_bf16(v[8 * q + 2], v[8 * q + 3])),
-                           "r"(pack_bf16(v[8 * q + 4], v[8 * q + 5])),
-                           "r"(pack_bf16(v[8 * q + 6], v[8 * q + 7]))
-                           : "memory");
+              for (int q = 0; q < 2; ++q) {
+                const uint32_t addr = my_row_s + ((static_cast<uint32_t>(2 * g + q) ^ sw) << 4);
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr),
+                             "r"(pack_bf16(v[8 * q], v[8 * q + 1])),
+                             "r"(pack_bf16(v[8 * q + 2], v[8 * q + 3])),
+                             "r"(pack_bf16(v[8 * q + 4], v[8 * q + 5])),
+                             "r"(pack_bf16(v[8 * q + 6], v[8 * q + 7]))
+                             : "memory");
+              }
             }
           }
         }
@@ -685,7 +795,7 @@ inline int launch_gemm_t(const __nv_bfloat16* A, long long lda, const __nv_bfloa
       if (make_tmap_bf16(&tmAux, p.aux, 2, dims, astr, box, TMAP_SWIZZLE_64B) != 0) return -23;
     }
   }
-  using S = GemmSmem<BN, PAIR, EPI == EPI_QKV_ROPE>;
+  using S = GemmSmem<BN, PAIR, EPI == EPI_QKV_ROPE || EPI == EPI_QKV_NORM>;
   auto kern = gemm_tcgen05_kernel<BN, EPI, PAIR>;
   static std::atomic<uint64_t> smem_set;
   if (const cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), S::TOTAL, smem_set); e != cudaSuccess)
@@ -738,17 +848,17 @@ inline int launch_gemm(const __nv_bfloat16* A, long long lda, const __nv_bfloat1
   //   N = 640: K = 64 487 / 378, 68 / 53, 12.0 / 10.1; K = 128 510 / 483, 69 / 64, 12.8 / 11.6
   //   the other way: K = 8 N = 384 465 / 679, 76 / 85, 13.4 / 14.8; K = 120 395 / 630, 55 / 72, 12.7 / 11.6;
   //            K = 192 372 / 388, 54 / 54, 12.3 / 10.2; N = 448 K = 128 339 / 458, 52 / 65, 11.8 / 12.3
-  if (p.M >= 1024 && (p.N > 128 || EPI == EPI_QKV_ROPE)) {
-    if (EPI != EPI_QKV_ROPE && p.N % 256 == 128 && p.K >= 32 && 128 % p.K == 0)
+  constexpr bool QKV = EPI == EPI_QKV_ROPE || EPI == EPI_QKV_NORM;
+  if (p.M >= 1024 && (p.N > 128 || QKV)) {
+    if (!QKV && p.N % 256 == 128 && p.K >= 32 && 128 % p.K == 0)
       return launch_gemm_t<128, EPI, false>(A, lda, W, ldw, p, sm_count, stream);
     return launch_gemm_t<256, EPI, true>(A, lda, W, ldw, p, sm_count, stream);
   }
   // Few rows: a launch is one tile's latency long, and a 128-wide tile has half the epilogue of a 256-wide
   // one, as long as there are SMs for twice as many (256 x 512, K = 128: 5.6 -> 4.1 us; 256 x 384 with rotation: 5.9 -> 4.3). The qk norm needs
   // 256-wide tiles: a warp's 64 columns are then one whole 64-channel head.
-  const bool norm = EPI == EPI_QKV_ROPE && p.qk_norm != 0;
   const int tiles128 = ((p.M + GEMM_BM - 1) / GEMM_BM) * ((p.N + 127) / 128);
-  if (norm || (tiles128 > sm_count && (EPI == EPI_QKV_ROPE || p.N % 256 == 0 || p.N > 512)))
+  if (EPI == EPI_QKV_NORM || (tiles128 > sm_count && (QKV || p.N % 256 == 0 || p.N > 512)))
     return launch_gemm_t<256, EPI, false>(A, lda, W, ldw, p, sm_count, stream);
   return launch_gemm_t<128, EPI, false>(A, lda, W, ldw, p, sm_count, stream);
 }

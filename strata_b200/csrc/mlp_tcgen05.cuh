@@ -65,19 +65,6 @@ struct MlpSmem {
   static_assert(TOTAL <= 232448, "shared memory of an SM");
 };
 
-// 16 lanes x 32 columns as matrix fragments: registers 4 i + {0, 1}: row lane / 4, columns 8 i + 2 (lane % 4) + {0, 1};
-// 4 i + {2, 3}: row lane / 4 + 8.
-__device__ __forceinline__ void tmem_ld_16x256_x4(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-}
-
 template <int C>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW1,
@@ -304,8 +291,7 @@ mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
           for (int q = 0; q < 2; ++q) {      // columns 16 q: k-block col / 64, 16-byte pieces (col % 64) / 8 + 2 q and + 1
             const uint32_t piece = static_cast<uint32_t>((col & 32) / 8 + 2 * q + (lane >> 4));
             const uint32_t addr = st_row + hf * 2048 + (col >> 6) * 16384 + ((piece ^ (lane & 7u)) << 4);
-            asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(h[hf][4 * q]),
-                         "r"(h[hf][4 * q + 1]), "r"(h[hf][4 * q + 2]), "r"(h[hf][4 * q + 3]) : "memory");
+            stmatrix_x4(addr, &h[hf][4 * q]);
           }
       }
       fence_proxy_async_smem();

@@ -401,6 +401,58 @@ def test_na3d_sweep_plane_size(ops, kernel, nh, D):
     assert rel_max_err(o, ref) < TOL_BF16
 
 
+# rows and columns at the edges of a 32 x 32 box, of a 128-row and a 256-column tile and of a CTA pair's 256 rows, one
+# k-block and a part of one; a bias of every kind
+@pytest.mark.parametrize("epi", ["bias", "gelu", "residual", "gate"])
+@pytest.mark.parametrize("M,N,K", [(1, 8, 8), (31, 40, 64), (33, 24, 72), (129, 136, 64), (300, 264, 136), (1024, 136, 64),
+                                   (1025, 520, 72), (1300, 264, 128), (2049, 248, 192)])
+@pytest.mark.parametrize("bias", [True, False])
+def test_linear_edges(ops, epi, M, N, K, bias):
+    g = torch.Generator().manual_seed(M + 3 * N + K)
+    x = torch.randn(M, K, generator=g).bfloat16()
+    w = (torch.randn(N, K, generator=g) * K ** -0.5).bfloat16()
+    b = torch.randn(N, generator=g) if bias else None
+    aux = torch.randn(M, N, generator=g).bfloat16()
+    acc = x.double() @ w.double().T + (b.double() if bias else 0.0)
+    ref = {"bias": lambda: acc, "gelu": lambda: torch.nn.functional.gelu(acc, approximate="tanh"),
+           "residual": lambda: acc + aux.double(), "gate": lambda: aux.double() * torch.sigmoid(acc)}[epi]()
+    out = torch.full((M + 1, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    ops.linear(x.cuda(), w.cuda(), b.cuda() if bias else None, getattr(ops, f"EPI_{epi.upper()}"),
+               aux.cuda() if epi in ("residual", "gate") else None, out=out[:M])
+    assert _status() == 0
+    assert bool((out[M] == 7.0).all())          # nothing behind the last row
+    # one bf16 rounding of the result (2^-9 relative), tanh.approx (2^-11) and the fast exponential besides
+    err = (out[:M].double().cpu() - ref).abs()
+    assert bool((err <= 2.0 ** -8 * ref.abs() + 2e-3).all())
+
+
+@pytest.mark.parametrize("M,C,hd,norm", [(1, 64, 64, True), (129, 128, 64, True), (129, 64, 32, True), (1100, 192, 64, True),
+                                         (1100, 320, 32, True), (2500, 576, 64, True), (1100, 192, 64, False),
+                                         (129, 192, 32, False)])
+def test_qkv_rotation_and_norm_edges(ops, M, C, hd, norm):
+    # a table row of its own for every token, rows and heads at the edges of tiles and of column tiles that
+    # hold q, k and v at once
+    g = torch.Generator().manual_seed(M + C)
+    x = torch.randn(M, C, generator=g).bfloat16()
+    w = (torch.randn(3 * C, C, generator=g) * C ** -0.5).bfloat16()
+    b = torch.randn(3 * C, generator=g) * 0.1
+    t = torch.rand(1, M, hd // 2, generator=g) * 6
+    cos, sin = t.cos().half().float(), t.sin().half().float()
+    y = ops.qkv_rope(x.cuda(), w.cuda(), b.cuda(), hd, cos.cuda(), sin.cuda(), M, M, qk_norm=norm)
+    assert _status() == 0
+    acc = (x.double() @ w.double().T + b.double()).reshape(M, 3, C // hd, hd)
+    qk = acc[:, :2]
+    if norm:
+        qk = qk * torch.rsqrt((qk * qk).mean(-1, keepdim=True) + 1e-6)
+    p = qk.reshape(M, 2, C // hd, hd // 2, 2)
+    co, si = cos[0].double()[:, None, None], sin[0].double()[:, None, None]
+    rot = torch.stack([p[..., 0] * co - p[..., 1] * si, p[..., 0] * si + p[..., 1] * co], -1).reshape(M, 2, C // hd, hd)
+    ref = torch.cat([rot, acc[:, 2:]], 1).reshape(M, 3 * C)
+    err = (y.double().cpu() - ref).abs()
+    # one bf16 rounding; the products of a pair are rounded in fp32
+    assert bool((err <= 2.0 ** -8 * ref.abs() + 1e-4).all())
+
+
 @pytest.mark.parametrize("C,hd", [(128, 64), (256, 64), (512, 64), (256, 32)])
 def test_qkv_without_rope_but_with_qk_norm(ops, C, hd):
     # rope_mode 'none' with qk_norm=True (accepted by the wrappers). Below C = 256: projection,
