@@ -134,9 +134,9 @@ int strata_linear_bf16(const void* x, int64_t ldx, const void* w, int64_t ldw, c
 
 int strata_mlp_fused(int M, int C, int hidden) { return mlp_fused_pays(M, C, hidden) ? 1 : 0; }
 
-int strata_mlp_bf16(const void* x, int64_t ldx, const void* w1, const float* b1, const void* w2, const float* b2,
-                    const void* aux, int64_t ldaux, const void* gate, int64_t ldgate, void* y, int64_t ldy, int M,
-                    int C, int hidden, void* stream) {
+static int mlp_impl(const void* x, int64_t ldx, const void* w1, const float* b1, const void* w2, const float* b2,
+                    const void* aux, int64_t ldaux, const void* gate, int64_t ldgate, void* y, int64_t ldy,
+                    void* ln_out, int64_t ldln, float ln_eps, int M, int C, int hidden, void* stream) {
   const int sms = current_sm_count();
   if (sms <= 0) return STRATA_ERR_NO_DEVICE;
   if (M < 0 || C <= 0 || hidden <= 0) return STRATA_ERR_ARG;
@@ -154,8 +154,15 @@ int strata_mlp_bf16(const void* x, int64_t ldx, const void* w1, const float* b1,
   p.b1 = b1; p.b2 = b2;
   p.aux = static_cast<const __nv_bfloat16*>(aux); p.ldaux = ldaux;
   p.gate = static_cast<const __nv_bfloat16*>(gate); p.ldgate = ldgate;
+  p.ln_out = static_cast<__nv_bfloat16*>(ln_out); p.ldln = ldln; p.ln_eps = ln_eps;
   return launch_mlp(C, static_cast<const __nv_bfloat16*>(x), ldx, static_cast<const __nv_bfloat16*>(w1),
                     static_cast<const __nv_bfloat16*>(w2), static_cast<__nv_bfloat16*>(y), ldy, p, sms, as_stream(stream));
+}
+
+int strata_mlp_bf16(const void* x, int64_t ldx, const void* w1, const float* b1, const void* w2, const float* b2,
+                    const void* aux, int64_t ldaux, const void* gate, int64_t ldgate, void* y, int64_t ldy, int M,
+                    int C, int hidden, void* stream) {
+  return mlp_impl(x, ldx, w1, b1, w2, b2, aux, ldaux, gate, ldgate, y, ldy, nullptr, 0, 0.f, M, C, hidden, stream);
 }
 
 // One row of the packed (cos, sin) half table that rotates by nothing: 32 pairs of (1.0, 0.0).
@@ -323,11 +330,20 @@ int64_t strata_block_workspace_bytes(int64_t M, int C, int hidden) {
   return r256(M * C * 2) * 3 + r256(M * 3 * C * 2) + r256(M * static_cast<int64_t>(hidden) * 2);
 }
 
-int strata_block_forward_bf16(const void* x, void* y, int n_tiles, int D, int H, int W, int C,
-                              int heads, int hidden, int kd, int kh, int kw,
-                              const strata_block_weights* wts, const void* rope_cs, int qk_norm,
-                              float ln_eps, float qk_eps, void* workspace,
-                              int64_t workspace_bytes, void* stream) {
+// Where the projection writes the block's second norm, and the MLP (C <= 128) the norm that comes next: up to 256 channels
+// (whole rows in a tile), a power of two, so that the division by their number is exact and the norm has the
+// bits of the kernel of its own. 442368 x 256: projection and norm 122 + 109 us, in one 178; a block on 8192 x 128
+// 39.7 -> 38.4 us, three on 18480 x 128 219 -> 206. A short launch's own norm is spread over all SMs and overlaps
+// its neighbours, here it is at the end of every CTA's chain: on 256 and 1024 rows of 128 level (0.99 - 1.01).
+static bool ln_fused_pays(int M, int C) { return M >= 4096 && (C == 64 || C == 128 || C == 256); }
+
+// One block. xn_ready: the workspace begins with layernorm(x) already. ln_out (or null): layernorm(y) goes there, which
+// may be the workspace's beginning; *ln_done says whether it did.
+static int block_impl(const void* x, void* y, int n_tiles, int D, int H, int W, int C, int heads, int hidden, int kd,
+                      int kh, int kw, const strata_block_weights* wts, const void* rope_cs, int qk_norm, float ln_eps,
+                      float qk_eps, void* workspace, int64_t workspace_bytes, bool xn_ready, void* ln_out, bool* ln_done,
+                      void* stream) {
+  if (ln_done) *ln_done = false;
   if (!x || !y || !wts || !workspace || n_tiles < 0 || D <= 0 || H <= 0 || W <= 0)
     return STRATA_ERR_ARG;
   if (heads <= 0 || C % heads != 0) return STRATA_ERR_ARG;
@@ -349,7 +365,7 @@ int strata_block_forward_bf16(const void* x, void* y, int n_tiles, int D, int H,
   void* hbuf = ws;
   const int tokens_per_tile = D * H * W;
   int r;
-  if ((r = strata_layernorm_bf16(x, C, xn, C, M, C, ln_eps, stream)) != 0) return r;
+  if (!xn_ready && (r = strata_layernorm_bf16(x, C, xn, C, M, C, ln_eps, stream)) != 0) return r;
   if ((r = strata_qkv_rope_bf16(xn, C, wts->w_qkv, C, wts->b_qkv, qkv, 3 * C, M, C, hd, rope_cs,
                                 tokens_per_tile, H * W, qk_norm, qk_eps, stream)) != 0)
     return r;
@@ -362,18 +378,44 @@ int strata_block_forward_bf16(const void* x, void* y, int n_tiles, int D, int H,
                                 STRATA_EPI_GATE, attn, C, stream)) != 0)
       return r;
   }
-  if ((r = strata_linear_bf16(attn, C, wts->w_proj, C, wts->b_proj, x1, C, M, C, C,
-                              STRATA_EPI_RESIDUAL, x, C, stream)) != 0)
+  if (ln_fused_pays(M, C)) {
+    GemmParams p{};
+    p.M = M; p.N = C; p.K = C;
+    p.out = static_cast<__nv_bfloat16*>(x1); p.ldo = C;
+    p.bias = wts->b_proj;
+    p.aux = static_cast<const __nv_bfloat16*>(x); p.ldaux = C;
+    p.ln_eps = ln_eps;
+    if (!aligned16(x) || !aligned16(wts->w_proj) || (wts->b_proj && !aligned16(wts->b_proj))) return STRATA_ERR_ARG;
+    if ((r = launch_gemm_residual_ln(static_cast<const __nv_bfloat16*>(attn), C, static_cast<const __nv_bfloat16*>(wts->w_proj), C,
+                                     static_cast<__nv_bfloat16*>(xn), C, p, current_sm_count(), as_stream(stream))) != 0)
+      return r;
+  } else {
+    if ((r = strata_linear_bf16(attn, C, wts->w_proj, C, wts->b_proj, x1, C, M, C, C,
+                                STRATA_EPI_RESIDUAL, x, C, stream)) != 0)
+      return r;
+    if ((r = strata_layernorm_bf16(x1, C, xn, C, M, C, ln_eps, stream)) != 0) return r;
+  }
+  if (mlp_fused_pays(M, C, hidden)) {
+    const bool ln = ln_out && ln_fused_pays(M, C) && C <= 128;
+    r = mlp_impl(xn, C, wts->w_fc1, wts->b_fc1, wts->w_fc2, wts->b_fc2, x1, C, nullptr, 0, y, C, ln ? ln_out : nullptr, C,
+                 ln_eps, M, C, hidden, stream);
+    if (ln_done) *ln_done = ln && r == 0;
     return r;
-  if ((r = strata_layernorm_bf16(x1, C, xn, C, M, C, ln_eps, stream)) != 0) return r;
-  if (mlp_fused_pays(M, C, hidden))
-    return strata_mlp_bf16(xn, C, wts->w_fc1, wts->b_fc1, wts->w_fc2, wts->b_fc2, x1, C, nullptr, 0, y, C, M, C, hidden,
-                           stream);
+  }
   if ((r = strata_linear_bf16(xn, C, wts->w_fc1, C, wts->b_fc1, hbuf, hidden, M, hidden, C,
                               STRATA_EPI_GELU, nullptr, 0, stream)) != 0)
     return r;
   return strata_linear_bf16(hbuf, hidden, wts->w_fc2, hidden, wts->b_fc2, y, C, M, C, hidden,
                             STRATA_EPI_RESIDUAL, x1, C, stream);
+}
+
+int strata_block_forward_bf16(const void* x, void* y, int n_tiles, int D, int H, int W, int C,
+                              int heads, int hidden, int kd, int kh, int kw,
+                              const strata_block_weights* wts, const void* rope_cs, int qk_norm,
+                              float ln_eps, float qk_eps, void* workspace,
+                              int64_t workspace_bytes, void* stream) {
+  return block_impl(x, y, n_tiles, D, H, W, C, heads, hidden, kd, kh, kw, wts, rope_cs, qk_norm, ln_eps, qk_eps,
+                    workspace, workspace_bytes, false, nullptr, nullptr, stream);
 }
 
 static int prepost_check(int B, int C, int D, int H, int W, int pv, int ph, int pw, const float* lat,

@@ -27,6 +27,7 @@
 //   EPI_RESIDUAL       y = acc + b + R[m,n]                          (attn.proj / mlp.layers.2)
 //   EPI_QKV_ROPE       y = rope(acc + b) on q,k columns              (attn.qkv + RoPE + pack)
 //   EPI_QKV_NORM       y = rope(rmsnorm(acc + b)) on q,k columns     (the same with the q/k norm)
+//   EPI_RESIDUAL_LN    the same, and layernorm(y) besides            (attn.proj and the norm behind it)
 //   EPI_GATE           y = G[m,n] * sigmoid(acc + b)                 (attn.gate_proj)
 #pragma once
 #include <cuda_fp16.h>
@@ -45,6 +46,7 @@ enum GemmEpilogue : int {
   EPI_QKV_ROPE = 3,
   EPI_GATE = 4,
   EPI_QKV_NORM = 5,   // EPI_QKV_ROPE with the q/k norm
+  EPI_RESIDUAL_LN = 6,   // EPI_RESIDUAL, and the LayerNorm of the result into a second matrix (N <= 256)
 };
 
 struct GemmParams {
@@ -63,6 +65,7 @@ struct GemmParams {
   int head_dim;
   int rope_cols;   // columns [0, rope_cols) are q and k
   float qk_eps;
+  float ln_eps;    // EPI_RESIDUAL_LN
   // Output row remap (pad_T > 0): the M input rows are the interior tokens of tiles
   // [tile, d, i, j] with i, j < pad_T (pad_T a multiple of 32), and row m is stored at row
   // ((tile*pad_D + d)*P + i + pad_h)*P + j + pad_h of the output, P = pad_T + 2*pad_h: the
@@ -93,7 +96,8 @@ struct GemmSmem {
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = BN == 256 && !PAIR ? (TABLE ? 3 : 4) : (TABLE ? 5 : 6);
   static constexpr int STAGING_BYTES = 32 * 32 * 2;             // one 32-row x 32-col bf16 box
-  // the rotary table rows of a tile's 128 output rows (TABLE: QKV epilogue), 128 bytes each, twice
+  // TABLE: the rotary table rows of a tile's 128 output rows, 128 bytes each, twice (QKV epilogues), or the
+  // LayerNorm's sums of 8 columns of every row, for the mean and the variance
   static constexpr int TABLE_BYTES = TABLE ? 2 * GEMM_BM * 128 : 0;
   static constexpr int STAGING_OFF = STAGES * STAGE_BYTES;      // per epilogue warp
   static constexpr int TABLE_OFF = STAGING_OFF + GEMM_EPI_WARPS * STAGING_BYTES;
@@ -283,6 +287,53 @@ __device__ __noinline__ float2 gemm_qk_norm_scales(uint32_t taddr, const float* 
   return make_float2(rsqrtf(ss[0] * (1.0f / 32.0f) + eps), rsqrtf(ss[NSUB - 1] * (1.0f / 32.0f) + eps));
 }
 
+// LayerNorm of a row that four warps (a lane quarter) hold in parts, a row per lane, bf16 in and out: what
+// layernorm_rows_kernel computes, with its order of additions - pairs, the four pairs of 8 columns in turn, then the 8-column
+// sums i with i ^ 16, i ^ 8, ... - so that the result is the same bits. Each warp leaves its 8-column sums in shared
+// memory ([groups][32 rows] of its quarter, one buffer for the mean and one for the variance) and reads all of them.
+__device__ __forceinline__ float ln_group_sum(const uint32_t* w) {   // 8 columns
+  float s = 0.f;
+#pragma unroll
+  for (int t = 0; t < 4; ++t) s += bf16_lo(w[t]) + bf16_hi(w[t]);
+  return s;
+}
+__device__ __forceinline__ float ln_group_squares(const uint32_t* w, float mean) {
+  float s = 0.f;
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    float d = bf16_lo(w[t]) - mean;
+    s += d * d;
+    d = bf16_hi(w[t]) - mean;
+    s += d * d;
+  }
+  return s;
+}
+__device__ __forceinline__ void ln_put(uint32_t buf, int group, int lane, float v) {
+  asm volatile("st.shared.f32 [%0], %1;" ::"r"(buf + static_cast<uint32_t>(group * 32 + lane) * 4u), "f"(v) : "memory");
+}
+// GROUPS: 32, or 16 where group i stands for the sum of i and i + 16 already.
+template <int GROUPS>
+__device__ __forceinline__ float ln_total(uint32_t buf, int lane) {
+  float g[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(g[i]) : "r"(buf + static_cast<uint32_t>(i * 32 + lane) * 4u) : "memory");
+    if constexpr (GROUPS == 32) {
+      float h;
+      asm volatile("ld.shared.f32 %0, [%1];" : "=f"(h) : "r"(buf + static_cast<uint32_t>((i + 16) * 32 + lane) * 4u) : "memory");
+      g[i] += h;
+    }
+  }
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+    for (int i = 0; i < o; ++i) g[i] += g[i + o];
+  return g[0];
+}
+__device__ __forceinline__ uint32_t ln_pair(uint32_t w, float mean, float rstd) {
+  return pack_bf16((bf16_lo(w) - mean) * rstd, (bf16_hi(w) - mean) * rstd);
+}
+
 // mbar_wait with the (bounded) polling loop out of line, for the epilogue warps: the phase has
 // usually completed, and rare code left inline in their loop costs registers and schedule.
 __device__ __noinline__ bool gemm_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag,
@@ -318,21 +369,23 @@ template <int BN, int EPI, bool PAIR>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ CUtensorMap tmOut,
-                    const __grid_constant__ CUtensorMap tmAux, const GemmParams p) {
+                    const __grid_constant__ CUtensorMap tmAux, const __grid_constant__ CUtensorMap tmLn,
+                    const GemmParams p) {
+  constexpr bool LN = EPI == EPI_RESIDUAL_LN;
   constexpr bool TABLE = EPI == EPI_QKV_ROPE || EPI == EPI_QKV_NORM;
   // The accumulator as matrix fragments (see above) or a row per lane. Fragments / rows, microseconds: residual
   // 262144 x 512, K = 512 115 / 121, 442368 x 256, K = 256 91 / 101; GELU 442368 x 1024, K = 256 231 / 267, 103000 x 1536,
   // K = 384 103 / 110, level from K = 512 on; q/k norm and rotation 262144 x 1536, K = 512 377 / 383, 98304 x 2304,
   // K = 768 243 / 267, 103000 x 1152, K = 384 150 / 167. The other way: rotation alone 346 / 338, 252 / 246, 121 / 120
   // (without the norm's code in the kernel rows take 324, 245, 121); bias alone 295 / 291, 171 / 166.
-  constexpr bool FRAG = EPI != EPI_BIAS && EPI != EPI_QKV_ROPE;
-  using S = GemmSmem<BN, PAIR, TABLE>;
+  constexpr bool FRAG = EPI != EPI_BIAS && EPI != EPI_QKV_ROPE && !LN;
+  using S = GemmSmem<BN, PAIR, TABLE || LN>;
   // PAIR: this CTA is rank 0 or 1 of a cluster of two that computes 256 x BN tiles together
   const uint32_t pair_rank = PAIR ? cluster_ctarank() : 0u;
   const int unit = PAIR ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
   const int n_units = PAIR ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
   constexpr int TILE_M = PAIR ? 2 * GEMM_BM : GEMM_BM;
-  constexpr bool HAS_AUX = (EPI == EPI_RESIDUAL || EPI == EPI_GATE);
+  constexpr bool HAS_AUX = (EPI == EPI_RESIDUAL || EPI == EPI_GATE || LN);
   // Epilogues without an operand to prefetch wait for the staging box as late as possible.
   constexpr bool LATE_WAIT = !HAS_AUX;
   extern __shared__ uint8_t smem_raw[];
@@ -351,6 +404,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   uint8_t* tail = smem_gen + S::BAR_OFF + 8 * (2 * S::STAGES + 4 + GEMM_EPI_WARPS);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 8);
+  [[maybe_unused]] const uint32_t ln_bar0 = bar_base + 8u * (2 * S::STAGES + 4 + GEMM_EPI_WARPS) + 16u;   // one per lane quarter
 
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
@@ -386,6 +440,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     }
     // (a rotary table part is written by the four warps of a lane quarter)
     for (int w = 0; w < GEMM_EPI_WARPS; ++w) mbar_init(aux_bar(w), TABLE ? 4 : 1);
+    if constexpr (LN)
+      for (int q = 0; q < 4; ++q) mbar_init(ln_bar0 + 8u * q, 4);
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -527,6 +583,115 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       tile_of(t, mt, jt);
       return mt * TILE_M + static_cast<int>(pair_rank) * GEMM_BM + quarter * 32;
     };
+    // EPI_RESIDUAL_LN: one tile (N <= BN: a tile has whole rows)
+    [[maybe_unused]] auto ln_tile = [&](int it_, int m_warp, int n_warp0) -> bool {
+      const int buf = it_ & 1;
+      const uint32_t sums = smem_base + S::TABLE_OFF + static_cast<uint32_t>(quarter) * 4096u, squares = sums + 16384u;
+      const uint32_t ln_bar = ln_bar0 + 8u * quarter;
+      uint32_t w[NSUB][16];
+#pragma unroll
+      for (int c = 0; c < NSUB; ++c) {
+        const int n0 = n_warp0 + c * 32;
+        const bool live = n0 < p.N && m_warp < p.M;           // warp-uniform
+        if (live && elect_one()) {
+          tma_store_wait_read0();
+          mbar_expect_tx(aux_bar(e), S::STAGING_BYTES);
+          tma_load_2d(stage_s, &tmAux, n0, m_warp, aux_bar(e));
+        }
+        if (c == 0) {
+          if (!gemm_wait(accf_bar(buf), (it_ >> 1) & 1u, abort_flag, ST_TIMEOUT_EPILOGUE)) return false;
+          tc_fence_after();
+        }
+        if (live) {
+          if (!gemm_wait(aux_bar(e), aux_phase, abort_flag, ST_TIMEOUT_EPILOGUE)) return false;
+          aux_phase ^= 1u;
+        }
+#pragma unroll
+        for (int g = 0; g < 2; ++g) {
+          uint32_t r[16];
+          if (live) {
+            tmem_ld_32x16(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
+                              static_cast<uint32_t>(buf * BN + cg * WARP_COLS + c * 32 + 16 * g), r);
+            tmem_ld_wait();
+          }
+          if (g == 1 && c == NSUB - 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+              if constexpr (PAIR) mbar_arrive_cluster(buf ? acce_remote1 : acce_remote0);
+              else mbar_arrive(acce_bar(buf));
+            }
+          }
+          if (live) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              const uint32_t addr = my_row_s + ((static_cast<uint32_t>(2 * g + q) ^ sw) << 4);
+              uint32_t ax[4];
+              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(ax[0]), "=r"(ax[1]), "=r"(ax[2]), "=r"(ax[3])
+                           : "r"(addr) : "memory");
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {       // four columns: N is a multiple of 64
+                float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (p.bias != nullptr) b4 = __ldg(reinterpret_cast<const float4*>(p.bias + n0 + 16 * g + 8 * q + 4 * h));
+                const int k = 8 * q + 4 * h;
+                w[c][8 * g + 4 * q + 2 * h] = pack_bf16(__uint_as_float(r[k]) + b4.x + bf16_lo(ax[2 * h]),
+                                                        __uint_as_float(r[k + 1]) + b4.y + bf16_hi(ax[2 * h]));
+                w[c][8 * g + 4 * q + 2 * h + 1] = pack_bf16(__uint_as_float(r[k + 2]) + b4.z + bf16_lo(ax[2 * h + 1]),
+                                                            __uint_as_float(r[k + 3]) + b4.w + bf16_hi(ax[2 * h + 1]));
+              }
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w[c][8 * g + 4 * q]),
+                           "r"(w[c][8 * g + 4 * q + 1]), "r"(w[c][8 * g + 4 * q + 2]), "r"(w[c][8 * g + 4 * q + 3]) : "memory");
+            }
+          }
+        }
+        if (live) {
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (elect_one()) {
+            tma_store_2d(&tmOut, stage_s, n0, m_warp);
+            tma_store_commit();
+          }
+        }
+        if (m_warp < p.M) {                        // (columns behind N count as zero)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) ln_put(sums, cg * (WARP_COLS / 8) + 4 * c + k, lane, live ? ln_group_sum(&w[c][4 * k]) : 0.f);
+        }
+      }
+      if (m_warp >= p.M) return true;              // all four warps of the quarter
+      __syncwarp();
+      if (lane == 0) mbar_arrive(ln_bar);
+      if (!gemm_wait(ln_bar, 0u, abort_flag, ST_TIMEOUT_EPILOGUE)) return false;
+      const float mean = ln_total<BN / 8>(sums, lane) / static_cast<float>(p.N);
+#pragma unroll
+      for (int c = 0; c < NSUB; ++c)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          ln_put(squares, cg * (WARP_COLS / 8) + 4 * c + k, lane, n_warp0 + 32 * c < p.N ? ln_group_squares(&w[c][4 * k], mean) : 0.f);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(ln_bar);
+      if (!gemm_wait(ln_bar, 1u, abort_flag, ST_TIMEOUT_EPILOGUE)) return false;
+      const float rstd = rsqrtf(ln_total<BN / 8>(squares, lane) / static_cast<float>(p.N) + p.ln_eps);
+#pragma unroll
+      for (int c = 0; c < NSUB; ++c) {
+        if (n_warp0 + 32 * c >= p.N) break;
+        if (elect_one()) tma_store_wait_read0();
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const uint32_t addr = my_row_s + ((static_cast<uint32_t>(q) ^ sw) << 4);
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(ln_pair(w[c][4 * q], mean, rstd)),
+                       "r"(ln_pair(w[c][4 * q + 1], mean, rstd)), "r"(ln_pair(w[c][4 * q + 2], mean, rstd)),
+                       "r"(ln_pair(w[c][4 * q + 3], mean, rstd)) : "memory");
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (elect_one()) {
+          tma_store_2d(&tmLn, stage_s, n_warp0 + 32 * c, m_warp);
+          tma_store_commit();
+        }
+      }
+      return true;
+    };
     if (rope && unit < num_tiles) gemm_fetch_table(p, tile_rows(unit), cg * 8, tab_quarter, one_row);
     for (int t = unit; t < num_tiles && ok; t += n_units, ++it) {
       const int buf = it & 1;
@@ -553,6 +718,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
           if (t + n_units < num_tiles && !(one_row && it != 0))
             gemm_fetch_table(p, tile_rows(t + n_units), cg * 8, tab_quarter + static_cast<uint32_t>(buf ^ 1) * (GEMM_BM * 128u), one_row);
         }
+      }
+      if constexpr (LN) {
+        if (!ln_tile(it, m_warp, n_warp0)) {
+          ok = false;
+          break;
+        }
+        continue;
       }
       bool acc_ready = false;
       float qk_scale[4] = {1.f, 1.f, 1.f, 1.f};   // RMS factors of this lane's four rows
@@ -764,7 +936,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 // row-major with row stride ldw. Returns 0, or a negative argument error / CUDA error code.
 template <int BN, int EPI, bool PAIR>
 inline int launch_gemm_t(const __nv_bfloat16* A, long long lda, const __nv_bfloat16* W,
-                         long long ldw, const GemmParams& p, int sm_count, cudaStream_t stream) {
+                         long long ldw, const GemmParams& p, int sm_count, cudaStream_t stream,
+                         __nv_bfloat16* ln_out = nullptr, long long ldln = 0) {
   CUtensorMap tmA, tmB;
   {
     uint64_t dims[2] = {static_cast<uint64_t>(p.K), static_cast<uint64_t>(p.M)};
@@ -778,7 +951,7 @@ inline int launch_gemm_t(const __nv_bfloat16* A, long long lda, const __nv_bfloa
     uint32_t box[2] = {GEMM_BK, static_cast<uint32_t>(PAIR ? BN / 2 : BN)};
     if (make_tmap_bf16(&tmB, W, 2, dims, str, box) != 0) return -21;
   }
-  CUtensorMap tmOut, tmAux;
+  CUtensorMap tmOut, tmAux, tmLn;
   {
     uint64_t dims[2] = {static_cast<uint64_t>(p.N), static_cast<uint64_t>(p.M)};
     uint64_t str[1] = {static_cast<uint64_t>(p.ldo) * 2};
@@ -790,12 +963,17 @@ inline int launch_gemm_t(const __nv_bfloat16* A, long long lda, const __nv_bfloa
     }
     if (make_tmap_bf16(&tmOut, p.out, 2, odims, str, box, TMAP_SWIZZLE_64B) != 0) return -22;
     tmAux = tmOut;
-    if (EPI == EPI_RESIDUAL || EPI == EPI_GATE) {
+    if (EPI == EPI_RESIDUAL || EPI == EPI_GATE || EPI == EPI_RESIDUAL_LN) {
       uint64_t astr[1] = {static_cast<uint64_t>(p.ldaux) * 2};
       if (make_tmap_bf16(&tmAux, p.aux, 2, dims, astr, box, TMAP_SWIZZLE_64B) != 0) return -23;
     }
+    tmLn = tmOut;
+    if (EPI == EPI_RESIDUAL_LN) {
+      uint64_t lstr[1] = {static_cast<uint64_t>(ldln) * 2};
+      if (make_tmap_bf16(&tmLn, ln_out, 2, dims, lstr, box, TMAP_SWIZZLE_64B) != 0) return -25;
+    }
   }
-  using S = GemmSmem<BN, PAIR, EPI == EPI_QKV_ROPE || EPI == EPI_QKV_NORM>;
+  using S = GemmSmem<BN, PAIR, EPI == EPI_QKV_ROPE || EPI == EPI_QKV_NORM || EPI == EPI_RESIDUAL_LN>;
   auto kern = gemm_tcgen05_kernel<BN, EPI, PAIR>;
   static std::atomic<uint64_t> smem_set;
   if (const cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), S::TOTAL, smem_set); e != cudaSuccess)
@@ -827,11 +1005,11 @@ inline int launch_gemm_t(const __nv_bfloat16* A, long long lda, const __nv_bfloa
     }
     const int clusters = tiles < fit ? tiles : fit;
     return launch_chained(kern, dim3(static_cast<unsigned>(2 * clusters)), GEMM_THREADS, S::TOTAL, stream, 2,
-                          tmA, tmB, tmOut, tmAux, p);
+                          tmA, tmB, tmOut, tmAux, tmLn, p);
   }
   const int tiles = ((p.M + GEMM_BM - 1) / GEMM_BM) * ((p.N + BN - 1) / BN);
   const int grid = tiles < sm_count ? tiles : sm_count;
-  return launch_chained(kern, dim3(grid), GEMM_THREADS, S::TOTAL, stream, 1, tmA, tmB, tmOut, tmAux, p);
+  return launch_chained(kern, dim3(grid), GEMM_THREADS, S::TOTAL, stream, 1, tmA, tmB, tmOut, tmAux, tmLn, p);
 }
 
 template <int EPI>
@@ -861,6 +1039,15 @@ inline int launch_gemm(const __nv_bfloat16* A, long long lda, const __nv_bfloat1
   if (EPI == EPI_QKV_NORM || (tiles128 > sm_count && (QKV || p.N % 256 == 0 || p.N > 512)))
     return launch_gemm_t<256, EPI, false>(A, lda, W, ldw, p, sm_count, stream);
   return launch_gemm_t<128, EPI, false>(A, lda, W, ldw, p, sm_count, stream);
+}
+
+// y = A W^T + bias + aux and layernorm(y) into ln_out, for whole rows in a tile: N a multiple of 64, at most 256.
+// For calls of many rows: pairs of CTAs where one 128-wide tile does not hold a row.
+inline int launch_gemm_residual_ln(const __nv_bfloat16* A, long long lda, const __nv_bfloat16* W, long long ldw,
+                                   __nv_bfloat16* ln_out, long long ldln, const GemmParams& p, int sm_count, cudaStream_t stream) {
+  if (p.N % 64 != 0 || p.N > 256) return -2;
+  if (p.N <= 128) return launch_gemm_t<128, EPI_RESIDUAL_LN, false>(A, lda, W, ldw, p, sm_count, stream, ln_out, ldln);
+  return launch_gemm_t<256, EPI_RESIDUAL_LN, true>(A, lda, W, ldw, p, sm_count, stream, ln_out, ldln);
 }
 
 }  // namespace strata

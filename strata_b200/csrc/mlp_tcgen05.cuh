@@ -12,7 +12,11 @@
 //               chunk c, then W2 times the bf16 chunk c accumulates into the output columns.
 //   warps 2-17  epilogue: each takes 32 rows x 32 hidden channels of a chunk (bias, GELU, bf16, into the 128-byte
 //               swizzled layout the second product reads), and at a tile's end 32 x 32 boxes of the output
-//               (bias, gate, aux) through 64-byte-swizzled staging boxes to TMA stores.
+//               (bias, gate, aux) through 64-byte-swizzled staging boxes to TMA stores, and for C <= 128, where a
+//               warp has one box of a tile, the LayerNorm of the rows besides (the next block begins with it:
+//               of one block on 8 x 32 x 32 tokens of 128 channels the two norms that the kernels before them write
+//               are 39.6 -> 38.3 us, of three blocks on 19000 220 -> 204; at C = 256 the second box and the
+//               wait for the sums cost more than the pass they save, 3.33 -> 3.48 ms in two blocks on 442368).
 //
 // Every element sees the arithmetic of the two GEMMs - products accumulated over k in the same order, the
 // hidden channels rounded to bf16, the output too before it meets a gate - so the results are the same bits.
@@ -38,12 +42,15 @@ struct MlpParams {
   long long ldaux;
   const __nv_bfloat16* gate;    // [M, C] or nullptr: the output is rounded to bf16 and multiplied by it
   long long ldgate;
+  __nv_bfloat16* ln_out;        // [M, C] or nullptr: layernorm(y), for C = 64 and 128 (may be x)
+  long long ldln;
+  float ln_eps;
 };
 
 constexpr int MLP_CHUNK = 128;             // hidden channels of a chunk
 constexpr int MLP_MAX_C = 256;
 
-template <int C>
+template <int C, bool LN>
 struct MlpSmem {
   static constexpr bool AHEAD = C <= 128;                        // see the top: two outputs, staging boxes of their own
   static constexpr int SETS = AHEAD ? 2 : 1;                     // sets of epilogue warps, taking chunks in turn
@@ -52,25 +59,28 @@ struct MlpSmem {
   static constexpr int X_BUFS = 1;
   static constexpr int H_BYTES = 2 * 128 * 128;                  // one chunk, a buffer per set
   static constexpr int W1_BYTES = 128 * 128, W2_BYTES = C * 128; // one stage
-  static constexpr int S1 = C == 256 ? 4 : 3, S2 = C == 256 ? 2 : 3;
+  static_assert(!LN || C == 64 || C == 128, "the norm of a tile's rows comes out of one box per warp");
+  static constexpr int S1 = C == 256 ? 4 : 3, S2 = C == 256 || (C == 128 && LN) ? 2 : 3;
   static constexpr int STAGING_BYTES = 32 * 32 * 2;
   static constexpr int H_OFF = X_BUFS * X_BYTES;
   static constexpr int W1_OFF = H_OFF + SETS * H_BYTES;
   static constexpr int W2_OFF = W1_OFF + S1 * W1_BYTES;
   static constexpr int STAGING_OFF = AHEAD ? W2_OFF + S2 * W2_BYTES : H_OFF;
-  static constexpr int BAR_OFF = W2_OFF + S2 * W2_BYTES + (AHEAD ? GEMM_EPI_WARPS * STAGING_BYTES : 0);
+  // LN: sums over 8 columns of every row, for the mean and the variance: [quarter][16 groups][32 rows] each
+  static constexpr int LN_OFF = W2_OFF + S2 * W2_BYTES + (AHEAD ? GEMM_EPI_WARPS * STAGING_BYTES : 0);
+  static constexpr int BAR_OFF = LN_OFF + (LN ? 2 * 4 * 16 * 32 * 4 : 0);
   static constexpr int TOTAL = BAR_OFF + 512 + 1024;             // + alignment slack
   static constexpr int OUT_COL = 256, OUT_BUFS = AHEAD ? 2 : 1, OUT_STRIDE = 128;
   static_assert(GEMM_EPI_WARPS * STAGING_BYTES <= H_BYTES, "the staging boxes fit the hidden chunk's buffer");
   static_assert(TOTAL <= 232448, "shared memory of an SM");
 };
 
-template <int C>
+template <int C, bool LN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW1,
                    const __grid_constant__ CUtensorMap tmW2, const __grid_constant__ CUtensorMap tmOut,
-                   const __grid_constant__ CUtensorMap tmAux, const MlpParams p) {
-  using S = MlpSmem<C>;
+                   const __grid_constant__ CUtensorMap tmAux, const __grid_constant__ CUtensorMap tmLn, const MlpParams p) {
+  using S = MlpSmem<C, LN>;
   constexpr bool AHEAD = S::AHEAD;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -89,6 +99,7 @@ mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   auto h_empty = [&](int b) { return bar + 224u + 8u * b; };
   const uint32_t staged = bar + 240u;
   auto aux_full = [&](int w) { return bar + 256u + 8u * w; };
+  [[maybe_unused]] auto ln_bar = [&](int q) { return bar + 400u + 8u * q; };
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem_gen + S::BAR_OFF + 384);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem_gen + S::BAR_OFF + 392);
 
@@ -117,9 +128,12 @@ mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     mbar_init(x_empty, 1);
     mbar_init(staged, GEMM_EPI_WARPS);
     for (int w = 0; w < GEMM_EPI_WARPS; ++w) mbar_init(aux_full(w), 1);
+    for (int q = 0; q < 4; ++q) mbar_init(ln_bar(q), C < 128 ? C / 32 : 4);   // the warps of a quarter that have columns
     *abort_flag = 0;
     fence_mbar_init();
   }
+  if constexpr (LN && C == 64)   // groups that no warp has
+    for (int i = threadIdx.x; i < 2 * 4 * 16 * 32; i += GEMM_THREADS) *reinterpret_cast<float*>(smem_gen + S::LN_OFF + 4 * i) = 0.f;
   if (warp == 1) {
     tmem_alloc(smem_u32(tmem_slot), 512);
     tmem_relinquish();
@@ -325,6 +339,8 @@ mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       const int ob = AHEAD ? t & 1 : 0;
       const int m_warp = tile_row(t);
       bool ready = false;
+      [[maybe_unused]] uint32_t keep[16];          // LN: the row's columns of this warp
+      [[maybe_unused]] const uint32_t sums = smem_base + S::LN_OFF + static_cast<uint32_t>(quarter) * 2048u, squares = sums + 8192u;
 #pragma unroll 1
       for (int n0 = box0; n0 < C; n0 += 128) {
         uint4 aux[4], gate[4];
@@ -399,10 +415,13 @@ mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
 #pragma unroll
           for (int q = 0; q < 2; ++q) {
             const uint32_t addr = my_row_s + ((static_cast<uint32_t>(2 * g + q) ^ sw) << 4);
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr),
-                         "r"(pack_bf16(v[8 * q], v[8 * q + 1])), "r"(pack_bf16(v[8 * q + 2], v[8 * q + 3])),
-                         "r"(pack_bf16(v[8 * q + 4], v[8 * q + 5])), "r"(pack_bf16(v[8 * q + 6], v[8 * q + 7]))
-                         : "memory");
+            uint32_t w[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              w[i] = pack_bf16(v[8 * q + 2 * i], v[8 * q + 2 * i + 1]);
+              if constexpr (LN) keep[8 * g + 4 * q + i] = w[i];
+            }
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
           }
         }
         fence_proxy_async_smem();
@@ -416,6 +435,37 @@ mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(out_free(ob));
+      if constexpr (LN) {
+        if (box0 < C && m_warp < p.M) {      // (the whole quarter has rows or none)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) ln_put(sums, box0 / 8 + k, lane, ln_group_sum(&keep[4 * k]));
+          __syncwarp();
+          if (lane == 0) mbar_arrive(ln_bar(quarter));
+          if (!gemm_wait(ln_bar(quarter), 0u, abort_flag, ST_TIMEOUT_EPILOGUE)) return false;
+          const float mean = ln_total<16>(sums, lane) / static_cast<float>(C);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) ln_put(squares, box0 / 8 + k, lane, ln_group_squares(&keep[4 * k], mean));
+          __syncwarp();
+          if (lane == 0) mbar_arrive(ln_bar(quarter));
+          if (!gemm_wait(ln_bar(quarter), 1u, abort_flag, ST_TIMEOUT_EPILOGUE)) return false;
+          const float rstd = rsqrtf(ln_total<16>(squares, lane) / static_cast<float>(C) + p.ln_eps);
+          if (elect_one()) tma_store_wait_read0();
+          __syncwarp();
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const uint32_t addr = my_row_s + ((static_cast<uint32_t>(q) ^ sw) << 4);
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(ln_pair(keep[4 * q], mean, rstd)),
+                         "r"(ln_pair(keep[4 * q + 1], mean, rstd)), "r"(ln_pair(keep[4 * q + 2], mean, rstd)),
+                         "r"(ln_pair(keep[4 * q + 3], mean, rstd)) : "memory");
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (elect_one()) {
+            tma_store_2d(&tmLn, stage_s, box0, m_warp);
+            tma_store_commit();
+          }
+        }
+      }
       if constexpr (!AHEAD) {
         // the staging boxes lie in the hidden chunk's buffer: nobody writes there before all have been read
         if (elect_one()) tma_store_wait_read0();
@@ -465,11 +515,11 @@ mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   }
 }
 
-template <int C>
+template <int C, bool LN>
 inline int launch_mlp_t(const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w1, const __nv_bfloat16* w2,
                         __nv_bfloat16* y, long long ldy, const MlpParams& p, int sm_count, cudaStream_t stream) {
-  using S = MlpSmem<C>;
-  CUtensorMap tmX, tmW1, tmW2, tmOut, tmAux;
+  using S = MlpSmem<C, LN>;
+  CUtensorMap tmX, tmW1, tmW2, tmOut, tmAux, tmLn;
   auto make = [&](CUtensorMap* tm, const __nv_bfloat16* base, uint64_t cols, uint64_t rows, long long ld, uint32_t bc,
                   uint32_t br, TmapSwizzle swz) {
     const uint64_t dims[2] = {cols, rows}, str[1] = {static_cast<uint64_t>(ld) * 2};
@@ -484,13 +534,15 @@ inline int launch_mlp_t(const __nv_bfloat16* x, long long ldx, const __nv_bfloat
     return -20;
   tmAux = tmOut;
   if (p.aux != nullptr && make(&tmAux, p.aux, C, M, p.ldaux, 32, 32, TMAP_SWIZZLE_64B) != 0) return -20;
-  auto kern = mlp_tcgen05_kernel<C>;
+  tmLn = tmOut;
+  if (LN && make(&tmLn, p.ln_out, C, M, p.ldln, 32, 32, TMAP_SWIZZLE_64B) != 0) return -20;
+  auto kern = mlp_tcgen05_kernel<C, LN>;
   static std::atomic<uint64_t> smem_set;
   if (const cudaError_t e = allow_smem(reinterpret_cast<const void*>(kern), S::TOTAL, smem_set); e != cudaSuccess)
     return -static_cast<int>(e) - 1000;
   const int tiles = (p.M + 127) / 128;
   return launch_chained(kern, dim3(static_cast<unsigned>(tiles < sm_count ? tiles : sm_count)), GEMM_THREADS, S::TOTAL,
-                        stream, 1, tmX, tmW1, tmW2, tmOut, tmAux, p);
+                        stream, 1, tmX, tmW1, tmW2, tmOut, tmAux, tmLn, p);
 }
 
 // Whether the kernel takes these sizes (weights contiguous, everything else as the GEMMs want it).
@@ -507,11 +559,16 @@ inline bool mlp_fused_pays(int M, int C, int H) { return mlp_fused_sizes(C, H) &
 
 inline int launch_mlp(int C, const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w1, const __nv_bfloat16* w2,
                       __nv_bfloat16* y, long long ldy, const MlpParams& p, int sm_count, cudaStream_t stream) {
+  if (p.ln_out != nullptr) switch (C) {
+    case 64: return launch_mlp_t<64, true>(x, ldx, w1, w2, y, ldy, p, sm_count, stream);
+    case 128: return launch_mlp_t<128, true>(x, ldx, w1, w2, y, ldy, p, sm_count, stream);
+    default: return -2;
+  }
   switch (C) {
-    case 64: return launch_mlp_t<64>(x, ldx, w1, w2, y, ldy, p, sm_count, stream);
-    case 128: return launch_mlp_t<128>(x, ldx, w1, w2, y, ldy, p, sm_count, stream);
-    case 192: return launch_mlp_t<192>(x, ldx, w1, w2, y, ldy, p, sm_count, stream);
-    case 256: return launch_mlp_t<256>(x, ldx, w1, w2, y, ldy, p, sm_count, stream);
+    case 64: return launch_mlp_t<64, false>(x, ldx, w1, w2, y, ldy, p, sm_count, stream);
+    case 128: return launch_mlp_t<128, false>(x, ldx, w1, w2, y, ldy, p, sm_count, stream);
+    case 192: return launch_mlp_t<192, false>(x, ldx, w1, w2, y, ldy, p, sm_count, stream);
+    case 256: return launch_mlp_t<256, false>(x, ldx, w1, w2, y, ldy, p, sm_count, stream);
     default: return -2;
   }
 }

@@ -172,11 +172,16 @@ inline int network_forward(const strata_backbone_desc& b, const strata_pixel_des
   STRATA_TRY(strata_linear_bf16(n.patches, b.k_embed, b.w_embed, b.k_embed, b.b_embed, n.tokens, b.dim, M,
                                 b.dim, static_cast<int>(b.k_embed), STRATA_EPI_BIAS, nullptr, 0, stream));
   const int64_t ws_bytes = strata_block_workspace_bytes(n.M, b.dim, b.hidden);
+  // a narrow block writes the norm that the next one, or the head, begins with
+  bool normed = false;
   for (int i = 0; i < b.n_blocks; ++i) {
     const int32_t* k3 = b.h_kernels + 3 * i;
-    STRATA_TRY(strata_block_forward_bf16(n.tokens, n.tokens, B, n.d, n.h, n.w, b.dim, b.heads, b.hidden,
-                                         k3[0], k3[1], k3[2], b.h_blocks + i, n.rope, b.qk_norm, 1e-6f,
-                                         1e-6f, n.block_ws, ws_bytes, stream));
+    void* next = i + 1 < b.n_blocks ? n.block_ws : (px ? nullptr : n.head_n);
+    bool done = false;
+    STRATA_TRY(block_impl(n.tokens, n.tokens, B, n.d, n.h, n.w, b.dim, b.heads, b.hidden, k3[0], k3[1], k3[2],
+                          b.h_blocks + i, n.rope, b.qk_norm, 1e-6f, 1e-6f, n.block_ws, ws_bytes, normed, next, &done,
+                          stream));
+    normed = done;
   }
   const void *rows = n.tokens, *w_head = b.w_head;
   const float* b_head = b.b_head;
@@ -192,10 +197,11 @@ inline int network_forward(const strata_backbone_desc& b, const strata_pixel_des
                                   px->dim, static_cast<int>(n.Mp), px->dim, static_cast<int>(px->k_embed),
                                   STRATA_EPI_BIAS, nullptr, 0, stream));
     for (int i = 0; i < px->n_blocks; ++i) STRATA_TRY(pixel_block(b, *px, i, B, D, H, W, n, stream));
+    normed = false;
     rows = n.px; w_head = px->w_head; b_head = px->b_head;
     C = px->dim; n_head = px->n_head; R = static_cast<int>(n.Mp); pv = ph = pw = 1;
   }
-  STRATA_TRY(strata_layernorm_bf16(rows, C, n.head_n, C, R, C, 1e-6f, stream));
+  if (!normed) STRATA_TRY(strata_layernorm_bf16(rows, C, n.head_n, C, R, C, 1e-6f, stream));
   STRATA_TRY(strata_linear_bf16(n.head_n, C, w_head, C, b_head, n.head_y, n_head, R, n_head, C,
                                 STRATA_EPI_BIAS, nullptr, 0, stream));
   return postprocess_impl(n.head_y, n_head, B, b.out_channels, D, H, W, lat, lon, lat0, lon0, b.u_idx,

@@ -549,3 +549,32 @@ def test_linear_half_last_tile(ops, M, N, K):
     assert _status() == 0
     assert rel_max_err(y, x.float() @ w[:N].float().T + b[:N]) < TOL_BF16
     assert torch.equal(y, ops.linear(x, w, b)[:, :N])          # N + 128 is a multiple of 256: pairs
+
+
+@pytest.mark.parametrize("C,grid,tiles,gated", [(64, (1, 5, 6), 1, False), (128, (2, 9, 13), 2, True), (192, (3, 8, 8), 3, False),
+                                                (256, (2, 7, 9), 1, True), (192, (4, 20, 53), 1, True), (256, (8, 24, 50), 2, False),
+                                                (128, (8, 40, 63), 2, False), (64, (3, 31, 67), 1, True)])
+def test_narrow_block_is_its_steps(ops, C, grid, tiles, gated):
+    # up to 256 channels the projection writes the norm behind it and the MLP is one kernel: the same bits as one
+    # operation after the other, for part tiles, several tiles a CTA, single CTAs and pairs
+    g = torch.Generator("cuda").manual_seed(C + grid[1])
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    D, H, W = grid
+    M, heads = tiles * D * H * W, C // 64
+    kernel = (1, 3, 3)
+    w = {}
+    for n, (o, i) in {"qkv": (3 * C, C), "gate": (C, C), "proj": (C, C), "fc1": (4 * C, C), "fc2": (C, 4 * C)}.items():
+        if n != "gate" or gated:
+            w[f"w_{n}"], w[f"b_{n}"] = (rnd(o, i) * i ** -0.5).bfloat16(), rnd(o) * 0.1
+    x = (rnd(M, C) * 2 + 0.5).bfloat16()
+    y = ops.block_forward(x.view(tiles, D * H * W, C), w, grid=grid, num_heads=heads, kernel=kernel, rope_cos=None, rope_sin=None)
+    assert _status() == 0
+    xn = ops.layernorm(x)
+    q6 = ops.qkv_rope(xn, w["w_qkv"], w["b_qkv"], 64, None, None, D * H * W, H * W).view(tiles, D, H, W, 3, heads, 64)
+    attn = ops.na3d(*(q6[..., i, :, :] for i in range(3)), kernel).reshape(M, C)
+    if gated:
+        attn = ops.linear(xn, w["w_gate"], w["b_gate"], ops.EPI_GATE, attn)
+    x1 = ops.linear(attn, w["w_proj"], w["b_proj"], ops.EPI_RESIDUAL, x)
+    h = ops.linear(ops.layernorm(x1), w["w_fc1"], w["b_fc1"], ops.EPI_GELU)
+    want = ops.linear(h, w["w_fc2"], w["b_fc2"], ops.EPI_RESIDUAL, x1)
+    assert torch.equal(y.view(M, C), want)

@@ -93,6 +93,31 @@ def test_one_call_equals_step_by_step(two_stage, over):
         assert torch.equal(m(x, idx), z) and not torch.equal(y, z)
 
 
+@pytest.mark.parametrize("dim,layers,size,gated", [(64, 3, (9, 72, 80), False), (128, 4, (5, 100, 92), True),
+                                                   (192, 3, (9, 60, 72), False), (256, 3, (5, 100, 92), False),
+                                                   (128, 1, (2, 12, 16), False), (320, 2, (3, 24, 40), False)])
+def test_norms_written_by_the_kernels_before_them(dim, layers, size, gated):
+    # up to 256 channels a block's second norm comes from its projection, up to 128 the next block's first and the
+    # head's from its MLP; step by step they are kernels of their own: the same bits
+    from strata_b200.wrappers import StrataBackboneModel
+    D, H, W = size
+    m = _randomised(StrataBackboneModel(depth=D, height=H, width=W, n_layers=layers, patch_size_vert=1, patch_size_horiz=4,
+                                        in_chans=5, base_out_chans=5, embed_dim=dim, num_heads=dim // 64, attn_kernel=(1, 3, 3),
+                                        do_rope_2d_stereographic=True, index_is_latlon=True, gated_attention=gated,
+                                        do_bf16_mixed=True).cuda())
+    x = torch.randn(2, 5, D, H, W, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    lat, lon = tile_latlon(2, H, W)
+    idx = {"lat": lat.cuda(), "lon": lon.cuda()}
+
+    class StepByStep:
+        def forward(self, *a):
+            return None
+    with torch.no_grad():
+        y = m(x, idx)
+        m.strata._network = StepByStep()
+        assert torch.equal(m(x, idx), y)
+
+
 def _own_block_code(m, seen):
     """Replaces parts of a model's blocks; every replaced part reports itself in `seen`."""
     import types
