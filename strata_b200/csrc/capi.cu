@@ -6,6 +6,7 @@
 #include <string.h>
 
 #include <atomic>
+#include <initializer_list>
 
 #include "common.cuh"
 #include "gemm_tcgen05.cuh"
@@ -542,6 +543,17 @@ int strata_halo_gather_tokens_bf16(void* out, const void* const* h_peer_src, int
       static_cast<int>(cells), only_halo, halo, halo + T, P);
 }
 
+// Four cells a thread in the field copy: tile and halo widths multiples of four (so that rows, tiles and ranks
+// start on a 16-byte boundary, and interior and halo meet on one) and every array 16-byte aligned. Elsewhere
+// few groups of four could be loaded as one.
+static bool field_four(int T, int halo, const PeerPtrs& src, int world, std::initializer_list<const void*> arrays) {
+  if (T % 4 != 0 || halo % 4 != 0) return false;
+  uintptr_t bits = 0;
+  for (const void* p : arrays) bits |= reinterpret_cast<uintptr_t>(p);
+  for (int r = 0; r < world; ++r) bits |= reinterpret_cast<uintptr_t>(src.p[r]);
+  return (bits & 15) == 0;
+}
+
 int strata_halo_gather_fields_f32(float* out, const void* const* h_peer_src, int world,
                                   const int32_t* src_a, const int32_t* src_b, int tiles_per_rank,
                                   int T, int halo, int64_t L, void* stream) {
@@ -561,11 +573,12 @@ int strata_halo_gather_fields_f32(float* out, const void* const* h_peer_src, int
   const long long ocells = static_cast<long long>(tiles_per_rank) * P * P;
   if (cells * world > 0x7fffffffLL || ocells > 0x7fffffffLL || L > 0x7fffffffLL)
     return STRATA_ERR_ARG;
-  const long long bx = (ocells + 255) / 256;
-  dim3 grid(static_cast<unsigned>(bx), field_grid_y(L, FIELD_UL_COPY));
-  return launch_chained(halo_gather_fields_kernel, grid, 256, 0, as_stream(stream), 1,
-      out, pp, src_a, src_b, static_cast<int>(ocells), static_cast<int>(cells),
-      static_cast<int>(L));
+  const bool four = field_four(T, halo, pp, world, {out, src_a, src_b});
+  const int v = four ? 4 : 1, ul = four ? FIELD_UL_COPY4 : FIELD_UL_COPY;
+  dim3 grid(static_cast<unsigned>((ocells / v + 255) / 256), field_grid_y(L, ul));
+  auto kern = four ? halo_gather_fields_kernel<4, FIELD_UL_COPY4> : halo_gather_fields_kernel<1, FIELD_UL_COPY>;
+  return launch_chained(kern, grid, 256, 0, as_stream(stream), 1, out, pp, src_a, src_b,
+      static_cast<int>(ocells), static_cast<int>(cells), static_cast<int>(L));
 }
 
 int strata_halo_gather_knn_fields_f32(float* out, const void* const* h_peer_src, int world,
@@ -618,11 +631,11 @@ int strata_halo_adjoint_fields_f32(float* out, const void* const* h_peer_padded,
   const long long cells = static_cast<long long>(tiles_per_rank) * T * T;
   const long long pcells = static_cast<long long>(tiles_per_rank) * P * P;
   if (pcells * world > 0x7fffffffLL || L > 0x7fffffffLL) return STRATA_ERR_ARG;
-  const long long bx = (cells + 255) / 256;
-  dim3 grid(static_cast<unsigned>(bx), field_grid_y(L, FIELD_UL_ADJ));
-  return launch_chained(halo_adjoint_fields_kernel, grid, 256, 0, as_stream(stream), 1,
-      out, pp, offsets, cell, coef, window, weights, static_cast<int>(cells),
-      static_cast<int>(pcells), P * P, static_cast<int>(L));
+  const int64_t bx = (cells + 255) / 256;
+  const int rounds = bx * field_grid_y(L, FIELD_UL_ADJ, 2) >= FIELD_ADJ_TWO ? 2 : 1;
+  dim3 grid(static_cast<unsigned>(bx), field_grid_y(L, FIELD_UL_ADJ, rounds));
+  return launch_chained(halo_adjoint_fields_kernel, grid, 256, 0, as_stream(stream), 1, out, pp, offsets,
+      cell, coef, window, weights, static_cast<int>(cells), static_cast<int>(pcells), P * P, static_cast<int>(L));
 }
 
 int strata_halo_gather_kv_bf16(void* qkv, const void* const* h_peer_qkv, int world,

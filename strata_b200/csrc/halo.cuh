@@ -124,28 +124,30 @@ halo_gather_tokens_kernel(__nv_bfloat16* __restrict__ out, const PeerPtrs src,
   }
 }
 
-// Field kernels: one thread per cell, FIELD_ROUNDS groups of UL consecutive leading indices (grid:
-// x over 256 cells, y over the leading index), a cell's index work done once for all of them.
-// Bound: HBM, through the bytes in flight - with a 4-byte access per thread it takes all of an
-// SM's threads and several loads each to cover ~1 us of latency at 6.5 TB/s (44 KB per SM); UL
-// independent loads stand before a thread's first use, four times as many with four neighbours. With
-// few leading indices a launch is one thread's chain of loads long, and every load past the last
-// index is an instruction for nothing. Microseconds at UL 4 / 8 / 12 / 16 (24 tiles of 64 x 64, halo 8):
-//   leading indices   1             16             64             512 (516 MB read + written)
-//   copy              4/5/5/5       8/8/8/8        20/16/15/16    131/97/101/98
-//   4 neighbours      5/6/7/8       13/16/17/16    29/31/32/35    189/225/186/192
-//   overlap-add       7/7/9/10      13/17/17/12    29/28/27/29    194/162/139/152
-//   ... of 4 neigh.   9/12/18/19    26/29/34/23    61/58/59/61    402/333/313/336
-// 24 tiles of 96 x 96, halo 16, 512 of them: 330/246/262/257, 492/582/496/499, 451/411/346/390,
-// 922/800/750/808; 54 tiles of 64 x 64, halo 4: 234/181/188/182, 314/403/317/324, 380/293/257/284,
-// 782/596/572/614; six tiles of 16 x 16: 3 to 17 us throughout. So 8 for the copy, 4 for the neighbours
-// (no slower than 16 with many indices, faster with few), 12 for the overlap-add, which is up to twice
-// its time at 4 with one index (9 us) and 30 % faster with many. One round per block: copy 136 instead
-// of 99 us, the index loads then delay every group.
+// Field kernels: one thread per cell (or four), `rounds` groups of UL consecutive leading indices (grid: x over
+// the cells, y over the leading index), a cell's index work done once for all of them.
+// Bound: HBM, through the bytes in flight - with a 4-byte access per thread it takes all of an SM's threads and
+// several loads each to cover ~1 us of latency at 6.5 TB/s (44 KB per SM); UL independent loads stand before a
+// thread's first use (2 UL in the overlap-add), four times as many with four neighbours. With few leading
+// indices a launch is one thread's chain of loads long, and every load past the last index is for nothing.
+// Measured, microseconds (24 tiles of 64 x 64, halo 8; 512 leading indices are 516 MB read + written):
+//   leading indices                     1     16    64    512    | 96 x 96, halo 16: 256 | 128 x 128, halo 32: 64
+//   copy, 1 cell a thread, UL 8         8     12    22    104    | 133                    | 84
+//   copy, 4 cells, UL 4                 8     11    20     93    | 121                    | 74   (UL 2: 100, UL 8: 98 at 512)
+//   4 neighbours, UL 4 (UL 8, 16)      10     18    29    196 (233, 199)
+//   overlap-add, UL 8                  12     16    29    128    | 162                    | 120
+//   ..., every entry in its turn, UL 12  14   23    37    145    | 195                    | 154
+//   ..., UL 12 (16)                    12     17    33 (31) 145  | 194 (182)              | 155 (137)
+//   ... of 4 neighbours, UL 8          15     25          301    (in turn, UL 12: 20, 35, 318)
+// Overlap-add, four cells a thread: 189 at 512 (four lists to walk, and both forms of load in most warps); the first
+// four entries in registers instead of two: 150. One round instead of two in the overlap-add: 139 at 512 but
+// 119 instead of 127 at 128 x 128, halo 32: two where that leaves FIELD_ADJ_TWO blocks. One round in the copy of one
+// cell a thread: 136 instead of 99, the index loads then delay every group.
 constexpr int FIELD_ROUNDS = 2;
-constexpr int FIELD_UL_COPY = 8, FIELD_UL_KNN = 4, FIELD_UL_ADJ = 12;
-inline unsigned field_grid_y(int64_t L, int ul) {
-  const int64_t per = static_cast<int64_t>(ul) * FIELD_ROUNDS;
+constexpr int FIELD_UL_COPY = 8, FIELD_UL_COPY4 = 4, FIELD_UL_KNN = 4, FIELD_UL_ADJ = 8;
+constexpr int64_t FIELD_ADJ_TWO = 8192;
+inline unsigned field_grid_y(int64_t L, int ul, int rounds = FIELD_ROUNDS) {
+  const int64_t per = static_cast<int64_t>(ul) * rounds;
   return static_cast<unsigned>((L + per - 1) / per < 65535 ? (L + per - 1) / per : 65535);
 }
 
@@ -159,38 +161,86 @@ __device__ __forceinline__ const float* field_cell(const PeerPtrs& src, int id, 
   return static_cast<const float*>(src.p[rank]) + id;
 }
 
+// V consecutive cells' values: one or four, the four on a 16-byte boundary. (Sources may be written by a peer
+// while an earlier kernel runs: ordinary loads, as everywhere in this file.)
+template <int V, class T>
+__device__ __forceinline__ void ld_cells(T* v, const T* p) {
+  static_assert((V == 1 || V == 4) && sizeof(T) == 4, "one cell or four");
+  if constexpr (V == 1) {
+    v[0] = *p;
+  } else {
+    const uint4 x = *reinterpret_cast<const uint4*>(p);
+    memcpy(v, &x, 16);
+  }
+}
+template <int V>
+__device__ __forceinline__ void st_cells(float* p, const float* v) {
+  if constexpr (V == 1) {
+    *p = v[0];
+  } else {
+    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  }
+}
+
 // Field layout: source buffers [L, tiles_per_rank*T*T] fp32 (L = product of leading dims),
-// output [L, tiles_per_rank*P*P].
+// output [L, tiles_per_rank*P*P]. V consecutive output cells per thread: with V = 4 they are one 16-byte
+// store, and one 16-byte load where the map names four consecutive cells on a 16-byte boundary.
+template <int V, int UL>
 __global__ void __launch_bounds__(256)
 halo_gather_fields_kernel(float* __restrict__ out, const __grid_constant__ PeerPtrs src,
                           const int* __restrict__ src_a, const int* __restrict__ src_b,
                           int n_out_cells, int cells_per_rank, int L) {
   chain_begin();
-  const int oc = blockIdx.x * 256 + threadIdx.x;
+  const int oc = (blockIdx.x * 256 + threadIdx.x) * V;
   if (oc >= n_out_cells) return;
   const bool failed = halo_exchange_failed();
-  const float* pa = field_cell(src, __ldg(src_a + oc), cells_per_rank);
-  const int b = __ldg(src_b + oc);
-  for (int l0 = blockIdx.y * FIELD_UL_COPY; l0 < L; l0 += gridDim.y * FIELD_UL_COPY) {
-    const float* qa = pa + static_cast<long long>(l0) * cells_per_rank;
-    float v[FIELD_UL_COPY];
+  int a[V], b[V];
+  ld_cells<V>(a, src_a + oc);
+  ld_cells<V>(b, src_b + oc);
+  bool wide = V > 1 && (a[0] & (V - 1)) == 0;   // (then all of them are one rank's: a multiple of V cells each)
 #pragma unroll
-    for (int u = 0; u < FIELD_UL_COPY; ++u) {
-      v[u] = l0 + u < L ? *qa : 0.f;
-      qa += cells_per_rank;
-    }
-    if (b >= 0) {
-      const float* qb = field_cell(src, b, cells_per_rank) + static_cast<long long>(l0) * cells_per_rank;
+  for (int k = 0; k < V; ++k) wide = wide && b[k] < 0 && a[k] == a[0] + k;
+  const float* pa[V];
 #pragma unroll
-      for (int u = 0; u < FIELD_UL_COPY; ++u) {
-        if (l0 + u < L) v[u] = (v[u] + *qb) / 2.0f;
-        qb += cells_per_rank;
+  for (int k = 0; k < V; ++k) pa[k] = field_cell(src, a[k], cells_per_rank);
+  for (int l0 = blockIdx.y * UL; l0 < L; l0 += gridDim.y * UL) {
+    const long long off = static_cast<long long>(l0) * cells_per_rank;
+    float v[UL][V];
+    if (wide) {
+      const float* q = pa[0] + off;
+#pragma unroll
+      for (int u = 0; u < UL; ++u) {
+        if (l0 + u < L) ld_cells<V>(v[u], q);
+        q += cells_per_rank;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        const float* q = pa[k] + off;
+#pragma unroll
+        for (int u = 0; u < UL; ++u) {
+          v[u][k] = l0 + u < L ? *q : 0.f;
+          q += cells_per_rank;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        if (b[k] < 0) continue;
+        const float* q = field_cell(src, b[k], cells_per_rank) + off;
+#pragma unroll
+        for (int u = 0; u < UL; ++u) {
+          if (l0 + u < L) v[u][k] = (v[u][k] + *q) / 2.0f;
+          q += cells_per_rank;
+        }
       }
     }
     float* op = out + static_cast<long long>(l0) * n_out_cells + oc;
 #pragma unroll
-    for (int u = 0; u < FIELD_UL_COPY; ++u) {
-      if (l0 + u < L) *op = failed ? __int_as_float(0x7fc00000) : v[u];
+    for (int u = 0; u < UL; ++u) {
+      if (failed)
+#pragma unroll
+        for (int k = 0; k < V; ++k) v[u][k] = __int_as_float(0x7fc00000);
+      if (l0 + u < L) st_cells<V>(op, v[u]);
       op += n_out_cells;
     }
   }
@@ -248,41 +298,61 @@ halo_gather_knn_fields_kernel(float* __restrict__ out, const __grid_constant__ P
 // the result is bit-identical to the same loop on the host for normal-range values (the library
 // is built with flush-to-zero, so a denormal operand or result is zero here and not there).
 // Padded sources: [L, tiles_per_rank*P*P] fp32 per rank; out [L, tiles_per_rank*T*T].
-// An entry is worked out once per UL leading indices, whatever the length of a cell's list.
+// A cell's first two entries (most cells have no more) stand in registers for all leading indices and their
+// loads are issued together.
 __global__ void __launch_bounds__(256)
 halo_adjoint_fields_kernel(float* __restrict__ out, const __grid_constant__ PeerPtrs src,
                            const int* __restrict__ offsets, const int* __restrict__ cell,
                            const float* __restrict__ coef, const float* __restrict__ window,
                            const float* __restrict__ weights, int n_cells,
                            int padded_cells_per_rank, int PP, int L) {
+  constexpr int UL = FIELD_UL_ADJ;
   chain_begin();
   const int c = blockIdx.x * 256 + threadIdx.x;
   if (c >= n_cells) return;
   const bool failed = halo_exchange_failed();
-  const int e0 = __ldg(offsets + c), e1 = __ldg(offsets + c + 1);
+  const int e0 = __ldg(offsets + c), n = __ldg(offsets + c + 1) - e0;
   // (after a failed barrier the divisor is NaN, and with it every output)
   const float wsum = failed ? __int_as_float(0x7fc00000) : __ldg(weights + c);
-  for (int l0 = blockIdx.y * FIELD_UL_ADJ; l0 < L; l0 += gridDim.y * FIELD_UL_ADJ) {
-    float acc[FIELD_UL_ADJ];
+  struct Entry {
+    const float* q;
+    float cf, wn;
+  };
+  auto entry = [&](int j) {
+    const int p = __ldg(cell + e0 + j);
+    return Entry{field_cell(src, p, padded_cells_per_rank), __ldg(coef + e0 + j), __ldg(window + p % PP)};
+  };
+  auto term = [](const Entry& e, float y) { return __fmul_rn(e.cf, __fmul_rn(e.wn, y)); };
+  Entry ea{}, eb{};
+  if (n > 0) ea = entry(0);
+  if (n > 1) eb = entry(1);
+  for (int l0 = blockIdx.y * UL; l0 < L; l0 += gridDim.y * UL) {
+    const long long off = static_cast<long long>(l0) * padded_cells_per_rank;
+    float acc[UL], ya[UL], yb[UL];
+    auto load = [&](float (&y)[UL], const Entry& e, bool there) {
+      const float* q = e.q + off;
 #pragma unroll
-    for (int u = 0; u < FIELD_UL_ADJ; ++u) acc[u] = 0.f;
-    for (int e = e0; e < e1; ++e) {
-      const int p = __ldg(cell + e);
-      const float cf = __ldg(coef + e), wn = __ldg(window + p % PP);
-      const float* q = field_cell(src, p, padded_cells_per_rank) +
-                       static_cast<long long>(l0) * padded_cells_per_rank;
-      float y[FIELD_UL_ADJ];
-#pragma unroll
-      for (int u = 0; u < FIELD_UL_ADJ; ++u) {
-        y[u] = l0 + u < L ? *q : 0.f;
+      for (int u = 0; u < UL; ++u) {
+        y[u] = there && l0 + u < L ? *q : 0.f;
         q += padded_cells_per_rank;
       }
+    };
+    load(ya, ea, n > 0);
+    load(yb, eb, n > 1);
 #pragma unroll
-      for (int u = 0; u < FIELD_UL_ADJ; ++u) acc[u] = __fadd_rn(acc[u], __fmul_rn(cf, __fmul_rn(wn, y[u])));
+    for (int u = 0; u < UL; ++u) {
+      acc[u] = n > 0 ? __fadd_rn(0.f, term(ea, ya[u])) : 0.f;
+      if (n > 1) acc[u] = __fadd_rn(acc[u], term(eb, yb[u]));
+    }
+    for (int j = 2; j < n; ++j) {
+      const Entry e = entry(j);
+      load(ya, e, true);
+#pragma unroll
+      for (int u = 0; u < UL; ++u) acc[u] = __fadd_rn(acc[u], term(e, ya[u]));
     }
     float* op = out + static_cast<long long>(l0) * n_cells + c;
 #pragma unroll
-    for (int u = 0; u < FIELD_UL_ADJ; ++u) {
+    for (int u = 0; u < UL; ++u) {
       if (l0 + u < L) *op = __fdiv_rn(acc[u], wsum);
       op += n_cells;
     }

@@ -357,3 +357,52 @@ def test_barrier_wait_runs_out_and_reports():
     assert _lib.device_status() == 0
     x = torch.ones(8, device="cuda")
     assert float((x * 2).sum()) == 16.0         # context still alive
+
+
+@pytest.mark.parametrize("world,fs,ts,hw,L,shift", [
+    (1, 16, 8, 4, 1, 0), (1, 16, 8, 4, 9, 0), (2, 16, 8, 4, 7, 0), (3, 12, 4, 4, 17, 0),   # four cells a thread
+    (1, 16, 8, 4, 5, 1), (2, 16, 8, 3, 8, 0), (1, 10, 5, 4, 33, 0), (1, 8, 4, 0, 4, 0),    # one
+    (1, 128, 64, 8, 350, 0),                                                              # two rounds a block
+])
+def test_field_gather_and_overlap_add_are_their_lists(world, fs, ts, hw, L, shift):
+    # Every rank's call on buffers of this GPU (world > 1: one per rank) against the maps and the lists applied in
+    # plain tensor arithmetic, every product and sum rounded on its own: the same bits. shift: elements by which
+    # the arrays miss a 16-byte boundary.
+    import ctypes
+    from strata_b200 import _lib
+    from strata_b200.topology import TileTopology, halo_adjoint_lists, halo_source_maps
+    lib, stream = _lib.load(), torch.cuda.current_stream().cuda_stream
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    gen = torch.Generator(device="cuda").manual_seed(fs + L)
+
+    def buffers(cells):
+        base = [torch.randn(L * cells + shift, device="cuda", generator=gen) for _ in range(world)]
+        return [b[shift:].view(L, cells) for b in base]
+
+    topos = [TileTopology(world, r, fs, ts, hw) for r in range(world)]
+    tpr, P = topos[0].tiles_per_rank, topos[0].padded_tile_size
+    x, y = buffers(tpr * ts * ts), buffers(tpr * P * P)
+    pointers = lambda bufs: (ctypes.c_void_p * world)(*(b.data_ptr() for b in bufs))
+    xa, ya = torch.cat(x, 1), torch.cat(y, 1)
+    win = np.random.default_rng(1).random((P, P), np.float32) + 0.5
+    window = dev(win).reshape(-1)
+    for topo in topos:
+        a, b = (dev(m).reshape(-1) for m in halo_source_maps(topo))
+        got = torch.full((L * a.numel() + shift,), 7.0, device="cuda")[shift:].view(L, -1)
+        _lib.check(lib.strata_halo_gather_fields_f32(got.data_ptr(), pointers(x), world, a.data_ptr(), b.data_ptr(),
+                                                     tpr, ts, hw, L, stream), "strata_halo_gather_fields_f32")
+        va = xa[:, a.long()]
+        assert torch.equal(got, torch.where(b >= 0, (va + xa[:, b.clamp(min=0).long()]) / 2, va))
+        off, cell, coef, weights = (dev(m) for m in halo_adjoint_lists(topo, win))
+        got = torch.full((L * weights.numel() + shift,), 7.0, device="cuda")[shift:].view(L, -1)
+        _lib.check(lib.strata_halo_adjoint_fields_f32(
+            got.data_ptr(), pointers(y), world, off.data_ptr(), cell.data_ptr(), coef.data_ptr(), window.data_ptr(),
+            weights.data_ptr(), tpr, ts, hw, L, stream), "strata_halo_adjoint_fields_f32")
+        n = (off[1:] - off[:-1]).long()
+        acc = torch.zeros_like(got)
+        for j in range(int(n.max())):
+            e = (off[:-1].long() + j).clamp(max=cell.numel() - 1)
+            p = cell[e].long()
+            acc = torch.where(n > j, acc + coef[e] * (window[p % (P * P)] * ya[:, p]), acc)
+        assert torch.equal(got, acc / weights)
+    assert _lib.device_status() == 0
