@@ -133,7 +133,10 @@ int strata_linear_bf16(const void* x, int64_t ldx, const void* w, int64_t ldw, c
   }
 }
 
-int strata_mlp_fused(int M, int C, int hidden) { return mlp_fused_pays(M, C, hidden) ? 1 : 0; }
+int strata_mlp_fused(int M, int C, int hidden) {
+  const int sms = current_sm_count();
+  return sms > 0 && mlp_fused_pays(M, C, hidden, sms) ? 1 : 0;
+}
 
 static int mlp_impl(const void* x, int64_t ldx, const void* w1, const float* b1, const void* w2, const float* b2,
                     const void* aux, int64_t ldaux, const void* gate, int64_t ldgate, void* y, int64_t ldy,
@@ -335,8 +338,12 @@ int64_t strata_block_workspace_bytes(int64_t M, int C, int hidden) {
 // (whole rows in a tile), a power of two, so that the division by their number is exact and the norm has the
 // bits of the kernel of its own. 442368 x 256: projection and norm 122 + 109 us, in one 178; a block on 8192 x 128
 // 39.7 -> 38.4 us, three on 18480 x 128 219 -> 206. A short launch's own norm is spread over all SMs and overlaps
-// its neighbours, here it is at the end of every CTA's chain: on 256 and 1024 rows of 128 level (0.99 - 1.01).
-static bool ln_fused_pays(int M, int C) { return M >= 4096 && (C == 64 || C == 128 || C == 256); }
+// its neighbours, here it is at the end of every CTA's chain: on 256 and 1024 rows of 128 level (0.99 - 1.01), and with
+// 256 channels, where one tile is all of a row's columns, a block on 8192 rows 52.9 -> 55.0 us, on 65536 213.7 -> 216.8,
+// on 131072 387 -> 386.
+static bool ln_fused_pays(int M, int C) {
+  return C == 256 ? M >= 131072 : M >= 4096 && (C == 64 || C == 128);
+}
 
 // One block. xn_ready: the workspace begins with layernorm(x) already. ln_out (or null): layernorm(y) goes there, which
 // may be the workspace's beginning; *ln_done says whether it did.
@@ -396,7 +403,7 @@ static int block_impl(const void* x, void* y, int n_tiles, int D, int H, int W, 
       return r;
     if ((r = strata_layernorm_bf16(x1, C, xn, C, M, C, ln_eps, stream)) != 0) return r;
   }
-  if (mlp_fused_pays(M, C, hidden)) {
+  if (mlp_fused_pays(M, C, hidden, current_sm_count())) {
     const bool ln = ln_out && ln_fused_pays(M, C) && C <= 128;
     r = mlp_impl(xn, C, wts->w_fc1, wts->b_fc1, wts->w_fc2, wts->b_fc2, x1, C, nullptr, 0, y, C, ln ? ln_out : nullptr, C,
                  ln_eps, M, C, hidden, stream);

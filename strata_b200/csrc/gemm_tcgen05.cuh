@@ -1015,7 +1015,7 @@ inline int launch_gemm_t(const __nv_bfloat16* A, long long lda, const __nv_bfloa
 template <int EPI>
 inline int launch_gemm(const __nv_bfloat16* A, long long lda, const __nv_bfloat16* W, long long ldw,
                        const GemmParams& p, int sm_count, cudaStream_t stream) {
-  // CTA pairs share each MMA (less shared-memory traffic per SM) from 1024 rows on, for every N that
+  // CTA pairs share each MMA (less shared-memory and L2 traffic per SM) from 1024 rows on, for every N that
   // one 128-wide tile does not cover; the last column tile is as narrow as it needs to be.
   // Except where the last tile is half one and a tile has two k-blocks at most: it is then all epilogue, the
   // pair's two column tiles of 256 and 128 take turns at unequal lengths, and equal 128-wide tiles of one
@@ -1026,16 +1026,28 @@ inline int launch_gemm(const __nv_bfloat16* A, long long lda, const __nv_bfloat1
   //   N = 640: K = 64 487 / 378, 68 / 53, 12.0 / 10.1; K = 128 510 / 483, 69 / 64, 12.8 / 11.6
   //   the other way: K = 8 N = 384 465 / 679, 76 / 85, 13.4 / 14.8; K = 120 395 / 630, 55 / 72, 12.7 / 11.6;
   //            K = 192 372 / 388, 54 / 54, 12.3 / 10.2; N = 448 K = 128 339 / 458, 52 / 65, 11.8 / 12.3
+  // And except where the chip is not filled: a launch that is a few turns of the persistent CTAs long costs what its
+  // longest CTA does, and a CTA's 128-wide tile is half a pair's share. Times as fast, by turns with 128-wide tiles /
+  // with pairs (M = 1024 ... 24576, C = 192 ... 1024, a block's four shapes; least, mean, most):
+  //   1 / 1  1.31 1.49 1.72 (1024 x 512, K = 512 8.2 / 5.3 us; 4096 x 512, K = 2048 15.5 / 10.2)
+  //   2 / 2  1.18 1.34 1.50 (4096 x 1152, K = 384 with rotation 11.3 / 7.5)
+  //   2 / 1, 3 / 2, 4 / 3  up to K = 1024 0.95 1.10 1.27, beyond 0.88 0.98 1.10; N <= 256, K > 512 0.86 - 0.95
+  //   4 / 2, 5 / 3  up to K = 1024 0.83 0.93 1.10, beyond 0.8 - 0.9
+  // Equal work's operands are twice as many bytes in 128-wide tiles: from K = 512 on a further turn of them takes as
+  // long as one of pairs, and with N <= 256 a pair reads A once.
+  // The norm of q and k needs 256-wide tiles: a warp's 64 columns are then one whole 64-channel head.
   constexpr bool QKV = EPI == EPI_QKV_ROPE || EPI == EPI_QKV_NORM;
+  const int tiles128 = ((p.M + GEMM_BM - 1) / GEMM_BM) * ((p.N + 127) / 128);
   if (p.M >= 1024 && (p.N > 128 || QKV)) {
-    if (!QKV && p.N % 256 == 128 && p.K >= 32 && 128 % p.K == 0)
+    const int pairs = sm_count / 2, tiles_pair = ((p.M + 2 * GEMM_BM - 1) / (2 * GEMM_BM)) * ((p.N + 255) / 256);
+    const int turns = (tiles128 + sm_count - 1) / sm_count, turns_pair = (tiles_pair + pairs - 1) / pairs;
+    const bool few = turns <= turns_pair || (turns == turns_pair + 1 && turns <= 4 && p.K <= (p.N > 256 ? 1024 : 512));
+    if (EPI != EPI_QKV_NORM && (few || (!QKV && p.N % 256 == 128 && p.K >= 32 && 128 % p.K == 0)))
       return launch_gemm_t<128, EPI, false>(A, lda, W, ldw, p, sm_count, stream);
     return launch_gemm_t<256, EPI, true>(A, lda, W, ldw, p, sm_count, stream);
   }
   // Few rows: a launch is one tile's latency long, and a 128-wide tile has half the epilogue of a 256-wide
-  // one, as long as there are SMs for twice as many (256 x 512, K = 128: 5.6 -> 4.1 us; 256 x 384 with rotation: 5.9 -> 4.3). The qk norm needs
-  // 256-wide tiles: a warp's 64 columns are then one whole 64-channel head.
-  const int tiles128 = ((p.M + GEMM_BM - 1) / GEMM_BM) * ((p.N + 127) / 128);
+  // one, as long as there are SMs for twice as many (256 x 512, K = 128: 5.6 -> 4.1 us; 256 x 384 with rotation: 5.9 -> 4.3).
   if (EPI == EPI_QKV_NORM || (tiles128 > sm_count && (QKV || p.N % 256 == 0 || p.N > 512)))
     return launch_gemm_t<256, EPI, false>(A, lda, W, ldw, p, sm_count, stream);
   return launch_gemm_t<128, EPI, false>(A, lda, W, ldw, p, sm_count, stream);

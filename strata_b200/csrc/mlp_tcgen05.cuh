@@ -548,14 +548,19 @@ inline int launch_mlp_t(const __nv_bfloat16* x, long long ldx, const __nv_bfloat
 // Whether the kernel takes these sizes (weights contiguous, everything else as the GEMMs want it).
 inline bool mlp_fused_sizes(int C, int H) { return C % 64 == 0 && C > 0 && C <= MLP_MAX_C && H % MLP_CHUNK == 0 && H > 0; }
 
-// Whether it is the faster way: two GEMMs / this kernel, microseconds with a residual, from a cold L2, at 256, 1024,
-// 8192, 24576, 131072 and 442368 rows, H = 4 C:
-//   C =  64: 13.1 / 11.0, 15.3 / 11.1, 17.3 / 11.2, 21.4 / 14.3, 46 / 31, 132 / 80
-//   C = 128: 13.3 / 14.3, 17.3 / 14.2, 17.4 / 14.3, 25.6 / 20.5, 79 / 51, 232 / 145
-//   C = 192: 15.3 / 20.4, 21.5 / 19.4, 23.6 / 20.5, 35.8 / 34.7, 116 / 100, 345 / 301
-//   C = 256: 17.4 / 24.5, 23.6 / 23.6, 27.6 / 24.5, 44.0 / 43.0, 155 / 129, 480 / 412
-// A few row blocks of a wide model leave most SMs idle through all of its chunks.
-inline bool mlp_fused_pays(int M, int C, int H) { return mlp_fused_sizes(C, H) && (C <= 128 || M >= 1024); }
+// Whether it is the faster way: two GEMMs / this kernel, microseconds with a residual, from a cold L2, H = 4 C:
+//            1024       4096       8192       12288      18944      24576      49152      442368 rows
+//   C = 128: 15 / 14    15 / 14    17 / 14    17 / 16    21 / 16    26 / 22    34 / 29    232 / 145
+//   C = 192: 15 / 20    17 / 20    19 / 20    24 / 22    28 / 22    32 / 35    48 / 49    345 / 301
+//   C = 256: 15 / 25    19 / 25    24 / 25    28 / 27    32 / 29    42 / 45    69 / 63    480 / 412
+// and at C = 64 13.1 / 11.0, 17.3 / 11.2, 46 / 31, 132 / 80 at 256, 8192, 131072, 442368 rows. A few row blocks of a
+// wide model leave SMs idle through all of its chunks, and so does a second turn of the blocks that is less than half full.
+inline bool mlp_fused_pays(int M, int C, int H, int sm_count) {
+  if (!mlp_fused_sizes(C, H)) return false;
+  if (C <= 128) return true;
+  const int blocks = (M + GEMM_BM - 1) / GEMM_BM;
+  return blocks > sm_count / 2 && (blocks <= sm_count || 2 * blocks > 3 * sm_count);
+}
 
 inline int launch_mlp(int C, const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w1, const __nv_bfloat16* w2,
                       __nv_bfloat16* y, long long ldy, const MlpParams& p, int sm_count, cudaStream_t stream) {

@@ -551,8 +551,22 @@ def test_linear_half_last_tile(ops, M, N, K):
     assert torch.equal(y, ops.linear(x, w, b)[:, :N])          # N + 128 is a multiple of 256: pairs
 
 
+@pytest.mark.parametrize("M,N,K", [(1024, 512, 64), (4600, 1000, 200), (2100, 2056, 72), (4096, 1152, 64), (18000, 256, 520),
+                                   (24500, 320, 136), (24500, 320, 1032), (30000, 136, 64), (40000, 320, 200), (9000, 1160, 64)])
+def test_linear_does_not_depend_on_the_tiles(ops, M, N, K):
+    # few turns of the chip go to 128-wide tiles of one CTA, the others to pairs of 256: the same columns as part
+    # of a wide output, which takes pairs
+    g = torch.Generator("cuda").manual_seed(M + N)
+    R = lambda *s: torch.randn(*s, generator=g, device="cuda", dtype=torch.bfloat16)
+    x, w, b = R(M, K), R(10240, K) * K ** -0.5, torch.randn(10240, generator=g, device="cuda")
+    y = ops.linear(x, w[:N], b[:N])
+    assert _status() == 0
+    assert rel_max_err(y.cpu(), (x.float() @ w[:N].float().T + b[:N]).cpu()) < TOL_BF16
+    assert torch.equal(y, ops.linear(x, w, b)[:, :N])
+
+
 @pytest.mark.parametrize("C,grid,tiles,gated", [(64, (1, 5, 6), 1, False), (128, (2, 9, 13), 2, True), (192, (3, 8, 8), 3, False),
-                                                (256, (2, 7, 9), 1, True), (192, (4, 20, 53), 1, True), (256, (8, 24, 50), 2, False),
+                                                (256, (2, 7, 9), 1, True), (192, (10, 20, 53), 1, True), (256, (16, 74, 112), 1, False),
                                                 (128, (8, 40, 63), 2, False), (64, (3, 31, 67), 1, True)])
 def test_narrow_block_is_its_steps(ops, C, grid, tiles, gated):
     # up to 256 channels the projection writes the norm behind it and the MLP is one kernel: the same bits as one
