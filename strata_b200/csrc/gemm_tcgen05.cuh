@@ -94,7 +94,7 @@ struct GemmSmem {
   static constexpr int A_BYTES = GEMM_BM * GEMM_BK * 2;
   static constexpr int B_BYTES = (PAIR ? BN / 2 : BN) * GEMM_BK * 2;   // a pair splits the W tile
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int STAGES = BN == 256 && !PAIR ? (TABLE ? 3 : 4) : (TABLE ? 5 : 6);
+  static constexpr int STAGES = BN == 256 && !PAIR ? (TABLE ? 3 : 4) : (TABLE ? 5 : 6);   // (BN = 64: 8 gain nothing)
   static constexpr int STAGING_BYTES = 32 * 32 * 2;             // one 32-row x 32-col bf16 box
   // TABLE: the rotary table rows of a tile's 128 output rows, 128 bytes each, twice (QKV epilogues), or the
   // LayerNorm's sums of 8 columns of every row, for the mean and the variance
@@ -550,7 +550,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const int e = warp - 2;
     const int quarter = warp & 3;            // TMEM lane quarter this warp may read
     const int cg = e >> 2;                   // which quarter of the BN columns
-    constexpr int WARP_COLS = BN / 4;
+    constexpr int WARP_COLS = BN < 128 ? 32 : BN / 4;   // (tiles of 64: the warps of the upper quarters have none)
     constexpr int NSUB = WARP_COLS / 32;
     const uint32_t stage_s = smem_base + S::STAGING_OFF + e * S::STAGING_BYTES;
     [[maybe_unused]] const uint32_t my_row_s = stage_s + lane * 64;               // (row form: this lane's row, its swizzle)
@@ -732,7 +732,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
 #pragma unroll 1
       for (int c = 0; c < NSUB; ++c) {
         const int n0 = n_warp0 + c * 32;
-        const bool chunk_live = (n0 < p.N) && (m_warp < p.M);   // warp-uniform
+        const bool chunk_live = (n0 < p.N) && (m_warp < p.M) && cg * WARP_COLS < BN;   // warp-uniform
         if constexpr (FRAG) {
           uint64_t bias[4];
           gemm_lane_bias(p, n0, lane, bias);
@@ -1038,6 +1038,15 @@ inline int launch_gemm(const __nv_bfloat16* A, long long lda, const __nv_bfloat1
   // The norm of q and k needs 256-wide tiles: a warp's 64 columns are then one whole 64-channel head.
   constexpr bool QKV = EPI == EPI_QKV_ROPE || EPI == EPI_QKV_NORM;
   const int tiles128 = ((p.M + GEMM_BM - 1) / GEMM_BM) * ((p.N + 127) / 128);
+  // One tile per SM at most, as narrow as 64: a launch is the latency of one tile, and half as wide a one has half
+  // the epilogue and two thirds of the bytes for each k-block. 128-wide tiles / these, microseconds: 256 x 384 with
+  // rotation, K = 128 4.4 / 4.2; 1024 x 512, K = 512 5.3 / 4.6; 1024 x 256, K = 1024 6.5 / 5.5; 256 x 1024,
+  // K = 4096 13.5 / 11.6; 1.03 - 1.2 times as fast at 64 to 4096 rows, 64 to 1024 channels. (With rotation a tile's table
+  // rows are the same for every width: 0.97 - 1.16.)
+  if constexpr (EPI != EPI_QKV_NORM) {
+    if (((p.M + GEMM_BM - 1) / GEMM_BM) * ((p.N + 63) / 64) <= sm_count)
+      return launch_gemm_t<64, EPI, false>(A, lda, W, ldw, p, sm_count, stream);
+  }
   if (p.M >= 1024 && (p.N > 128 || QKV)) {
     const int pairs = sm_count / 2, tiles_pair = ((p.M + 2 * GEMM_BM - 1) / (2 * GEMM_BM)) * ((p.N + 255) / 256);
     const int turns = (tiles128 + sm_count - 1) / sm_count, turns_pair = (tiles_pair + pairs - 1) / pairs;
@@ -1046,8 +1055,7 @@ inline int launch_gemm(const __nv_bfloat16* A, long long lda, const __nv_bfloat1
       return launch_gemm_t<128, EPI, false>(A, lda, W, ldw, p, sm_count, stream);
     return launch_gemm_t<256, EPI, true>(A, lda, W, ldw, p, sm_count, stream);
   }
-  // Few rows: a launch is one tile's latency long, and a 128-wide tile has half the epilogue of a 256-wide
-  // one, as long as there are SMs for twice as many (256 x 512, K = 128: 5.6 -> 4.1 us; 256 x 384 with rotation: 5.9 -> 4.3).
+  // Few rows of many columns: the same against 256-wide tiles, as long as there are SMs for twice as many.
   if (EPI == EPI_QKV_NORM || (tiles128 > sm_count && (QKV || p.N % 256 == 0 || p.N > 512)))
     return launch_gemm_t<256, EPI, false>(A, lda, W, ldw, p, sm_count, stream);
   return launch_gemm_t<128, EPI, false>(A, lda, W, ldw, p, sm_count, stream);

@@ -552,10 +552,9 @@ def test_linear_half_last_tile(ops, M, N, K):
 
 
 @pytest.mark.parametrize("M,N,K", [(1024, 512, 64), (4600, 1000, 200), (2100, 2056, 72), (4096, 1152, 64), (18000, 256, 520),
-                                   (24500, 320, 136), (24500, 320, 1032), (30000, 136, 64), (40000, 320, 200), (9000, 1160, 64)])
+                                   (24500, 320, 136), (24500, 320, 1032), (1, 64, 72), (127, 200, 136), (513, 1032, 64), (1100, 1000, 72), (30000, 136, 64), (40000, 320, 200), (9000, 1160, 64)])
 def test_linear_does_not_depend_on_the_tiles(ops, M, N, K):
-    # few turns of the chip go to 128-wide tiles of one CTA, the others to pairs of 256: the same columns as part
-    # of a wide output, which takes pairs
+    # one turn of the chip of 64-wide tiles, few of 128-wide ones, pairs of 256: the same columns as part of a wide output
     g = torch.Generator("cuda").manual_seed(M + N)
     R = lambda *s: torch.randn(*s, generator=g, device="cuda", dtype=torch.bfloat16)
     x, w, b = R(M, K), R(10240, K) * K ** -0.5, torch.randn(10240, generator=g, device="cuda")
