@@ -550,11 +550,12 @@ inline bool mlp_fused_sizes(int C, int H) { return C % 64 == 0 && C > 0 && C <= 
 
 // Whether it is the faster way: two GEMMs / this kernel, microseconds with a residual, from a cold L2, H = 4 C:
 //            1024       4096       8192       12288      18944      24576      49152      442368 rows
-//   C = 128: 15 / 14    15 / 14    17 / 14    17 / 16    21 / 16    26 / 22    34 / 29    232 / 145
-//   C = 192: 15 / 20    17 / 20    19 / 20    24 / 22    28 / 22    32 / 35    48 / 49    345 / 301
-//   C = 256: 15 / 25    19 / 25    24 / 25    28 / 27    32 / 29    42 / 45    69 / 63    480 / 412
-// and at C = 64 13.1 / 11.0, 17.3 / 11.2, 46 / 31, 132 / 80 at 256, 8192, 131072, 442368 rows. A few row blocks of a
-// wide model leave SMs idle through all of its chunks, and so does a second turn of the blocks that is less than half full.
+//   C = 128: 13 / 14    15 / 15    15 / 15    17 / 16    21 / 16    26 / 22    34 / 29    232 / 145
+//   C = 192: 15 / 20    17 / 21    19 / 21    24 / 22    28 / 22    32 / 35    48 / 49    345 / 301
+//   C = 256: 15 / 24    17 / 25    24 / 26    28 / 27    32 / 29    42 / 45    69 / 63    480 / 412
+// and at C = 64 11 / 11, 13 / 11, 46 / 31, 132 / 80 at 256, 8192, 131072, 442368 rows. A few row blocks of a wide model leave
+// SMs idle through all of its chunks, and so does a second turn of the blocks that is less than half full. At C = 128 the
+// two are level on few rows, where the host, which launches one kernel less, is what a small model waits for.
 inline bool mlp_fused_pays(int M, int C, int H, int sm_count) {
   if (!mlp_fused_sizes(C, H)) return false;
   if (C <= 128) return true;
