@@ -550,7 +550,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     const int e = warp - 2;
     const int quarter = warp & 3;            // TMEM lane quarter this warp may read
     const int cg = e >> 2;                   // which quarter of the BN columns
-    constexpr int WARP_COLS = BN < 128 ? 32 : BN / 4;   // (tiles of 64: the warps of the upper quarters have none)
+    // (the q/k norm takes a head to a warp; in narrow tiles the warps of the upper quarters have no columns)
+    constexpr int WARP_COLS = EPI == EPI_QKV_NORM ? 64 : BN < 128 ? 32 : BN / 4;
     constexpr int NSUB = WARP_COLS / 32;
     const uint32_t stage_s = smem_base + S::STAGING_OFF + e * S::STAGING_BYTES;
     [[maybe_unused]] const uint32_t my_row_s = stage_s + lane * 64;               // (row form: this lane's row, its swizzle)
@@ -1034,29 +1035,30 @@ inline int launch_gemm(const __nv_bfloat16* A, long long lda, const __nv_bfloat1
   //   2 / 1, 3 / 2, 4 / 3  up to K = 1024 0.95 1.10 1.27, beyond 0.88 0.98 1.10; N <= 256, K > 512 0.86 - 0.95
   //   4 / 2, 5 / 3  up to K = 1024 0.83 0.93 1.10, beyond 0.8 - 0.9
   // Equal work's operands are twice as many bytes in 128-wide tiles: from K = 512 on a further turn of them takes as
-  // long as one of pairs, and with N <= 256 a pair reads A once.
-  // The norm of q and k needs 256-wide tiles: a warp's 64 columns are then one whole 64-channel head.
+  // long as one of pairs, and with N <= 256 a pair reads A once. The norm of q and k keeps a head to a warp, so that half
+  // the warps of a 128-wide tile have none: 1 / 1 1.21 - 1.25 (1536 x 1536, K = 512 9.6 / 7.9), 2 / 2 1.21, 2 / 1 and 3 / 2 0.83 - 0.97.
   constexpr bool QKV = EPI == EPI_QKV_ROPE || EPI == EPI_QKV_NORM;
   const int tiles128 = ((p.M + GEMM_BM - 1) / GEMM_BM) * ((p.N + 127) / 128);
   // One tile per SM at most, as narrow as 64: a launch is the latency of one tile, and half as wide a one has half
   // the epilogue and two thirds of the bytes for each k-block. 128-wide tiles / these, microseconds: 256 x 384 with
   // rotation, K = 128 4.4 / 4.2; 1024 x 512, K = 512 5.3 / 4.6; 1024 x 256, K = 1024 6.5 / 5.5; 256 x 1024,
-  // K = 4096 13.5 / 11.6; 1.03 - 1.2 times as fast at 64 to 4096 rows, 64 to 1024 channels. (With rotation a tile's table
-  // rows are the same for every width: 0.97 - 1.16.)
-  if constexpr (EPI != EPI_QKV_NORM) {
-    if (((p.M + GEMM_BM - 1) / GEMM_BM) * ((p.N + 63) / 64) <= sm_count)
-      return launch_gemm_t<64, EPI, false>(A, lda, W, ldw, p, sm_count, stream);
-  }
+  // K = 4096 13.5 / 11.6; 1.03 - 1.2 times as fast at 64 to 4096 rows, 64 to 1024 channels. A QKV launch is
+  // 0.97 - 1.16 times as fast with rotation and 1.16 - 1.35 with the norm, but the attention behind it, whose CTAs come
+  // up while it runs, has no room beside it: from half the SMs on a model is slower with these tiles (five blocks
+  // on 1512 x 192 204 -> 214 us, eight on 864 x 320 with the norm 302 -> 314).
+  if (((p.M + GEMM_BM - 1) / GEMM_BM) * ((p.N + 63) / 64) <= (QKV ? sm_count / 2 : sm_count))
+    return launch_gemm_t<64, EPI, false>(A, lda, W, ldw, p, sm_count, stream);
   if (p.M >= 1024 && (p.N > 128 || QKV)) {
     const int pairs = sm_count / 2, tiles_pair = ((p.M + 2 * GEMM_BM - 1) / (2 * GEMM_BM)) * ((p.N + 255) / 256);
     const int turns = (tiles128 + sm_count - 1) / sm_count, turns_pair = (tiles_pair + pairs - 1) / pairs;
-    const bool few = turns <= turns_pair || (turns == turns_pair + 1 && turns <= 4 && p.K <= (p.N > 256 ? 1024 : 512));
-    if (EPI != EPI_QKV_NORM && (few || (!QKV && p.N % 256 == 128 && p.K >= 32 && 128 % p.K == 0)))
+    const bool few = turns <= turns_pair || (EPI != EPI_QKV_NORM && turns == turns_pair + 1 && turns <= 4 &&
+                                             p.K <= (p.N > 256 ? 1024 : 512));
+    if (few || (!QKV && p.N % 256 == 128 && p.K >= 32 && 128 % p.K == 0))
       return launch_gemm_t<128, EPI, false>(A, lda, W, ldw, p, sm_count, stream);
     return launch_gemm_t<256, EPI, true>(A, lda, W, ldw, p, sm_count, stream);
   }
   // Few rows of many columns: the same against 256-wide tiles, as long as there are SMs for twice as many.
-  if (EPI == EPI_QKV_NORM || (tiles128 > sm_count && (QKV || p.N % 256 == 0 || p.N > 512)))
+  if (tiles128 > sm_count && (QKV || p.N % 256 == 0 || p.N > 512))
     return launch_gemm_t<256, EPI, false>(A, lda, W, ldw, p, sm_count, stream);
   return launch_gemm_t<128, EPI, false>(A, lda, W, ldw, p, sm_count, stream);
 }

@@ -427,7 +427,8 @@ def test_linear_edges(ops, epi, M, N, K, bias):
 
 
 @pytest.mark.parametrize("M,C,hd,norm", [(1, 64, 64, True), (129, 128, 64, True), (129, 64, 32, True), (1100, 192, 64, True),
-                                         (1100, 320, 32, True), (2500, 576, 64, True), (1100, 192, 64, False),
+                                         (1100, 320, 32, True), (2500, 576, 64, True), (1100, 192, 64, False), (300, 256, 64, True), (257, 320, 32, True),
+                                         (1500, 512, 64, True), (1500, 512, 32, True), (4100, 384, 64, True), (3000, 320, 64, True),
                                          (129, 192, 32, False)])
 def test_qkv_rotation_and_norm_edges(ops, M, C, hd, norm):
     # a table row of its own for every token, rows and heads at the edges of tiles and of column tiles that
