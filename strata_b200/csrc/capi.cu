@@ -237,7 +237,8 @@ static int qkv_rope_impl(const void* x, int64_t ldx, const void* w, int64_t ldw,
     // microseconds at 1024, 24576, 262144 and 1572864 rows (the pixel stage of one production tile): C = 64 13.3 / 13.3,
     // 17.4 / 17.4, 54 / 56, 327 / 282; C = 128 11.2 / 13.4, 19.5 / 20.5, 103 / 98, 570 / 520; C = 192 13.3 / 14.3, 25.6 /
     // 26.6, 183 / 171, 1157 / 949 - in favour of two kernels where a launch is short. From C = 256 on fused is
-    // ahead: 212 / 173, 24.6 / 21.9, 9.6 / 9.6; C = 512 at 262144 rows 491 / 377. (Here the norm sees q and k rounded
+    // ahead: 212 / 173, 24.6 / 21.9, 9.6 / 9.6; C = 512 at 262144 rows 491 / 377. (All with 256-wide tiles in the fused
+    // one, which takes narrow ones on few rows today; its sums and so its bits are others than the row kernel's.) (Here the norm sees q and k rounded
     // to bf16, there the fp32 accumulators: error against 64 bits 2.1e-3 and 1.7e-3 of the result.)
     int r = launch_gemm<EPI_BIAS>(A, ldx, W, ldw, p, sms, as_stream(stream));
     if (r != 0) return r;

@@ -9,10 +9,10 @@
 //   warps 2-17  epilogue (16 warps: four per SM sub-partition, because the epilogue of a
 //               128 x 256 tile is bound by the latency of each warp's instruction stream
 //               rather than by issue slots): read the finished accumulator with tcgen05.ld
-//               (each thread owns one output row, 16 columns at a time), apply bias and the
-//               selected epilogue, store bf16. The other accumulator is being filled meanwhile.
+//               (as matrix fragments, or each thread one output row, 16 columns at a time), apply bias
+//               and the selected epilogue, store bf16. The other accumulator is being filled meanwhile.
 //
-// PAIR variant (large problems): two CTAs of a cluster share every MMA (tcgen05 cta_group::2,
+// BN = 256, 128 or 64 by the rule of launch_gemm. PAIR variant (large problems): two CTAs of a cluster share every MMA (tcgen05 cta_group::2,
 // M = 256): each CTA loads its own 128 rows of A and HALF of the W tile, the instruction reads
 // both halves, and each CTA's tensor memory receives its 128 rows x BN accumulator. A CTA then
 // moves 32 KB per k-block through shared memory instead of 48 KB, which matters because the
@@ -25,9 +25,9 @@
 //   EPI_BIAS           y = acc + b                                   (generic Linear)
 //   EPI_GELU           y = gelu_tanh(acc + b)                        (mlp.layers.0 + tanh GELU)
 //   EPI_RESIDUAL       y = acc + b + R[m,n]                          (attn.proj / mlp.layers.2)
+//   EPI_RESIDUAL_LN    the same, and layernorm(y) besides            (attn.proj and the norm behind it)
 //   EPI_QKV_ROPE       y = rope(acc + b) on q,k columns              (attn.qkv + RoPE + pack)
 //   EPI_QKV_NORM       y = rope(rmsnorm(acc + b)) on q,k columns     (the same with the q/k norm)
-//   EPI_RESIDUAL_LN    the same, and layernorm(y) besides            (attn.proj and the norm behind it)
 //   EPI_GATE           y = G[m,n] * sigmoid(acc + b)                 (attn.gate_proj)
 #pragma once
 #include <cuda_fp16.h>
