@@ -191,8 +191,8 @@ halo_gather_fields_kernel(float* __restrict__ out, const __grid_constant__ PeerP
                           const int* __restrict__ src_a, const int* __restrict__ src_b,
                           int n_out_cells, int cells_per_rank, int L) {
   chain_begin();
-  const int oc = (blockIdx.x * 256 + threadIdx.x) * V;
-  if (oc >= n_out_cells) return;
+  const int oc = static_cast<int>((blockIdx.x * 256 + threadIdx.x) * V);
+  if (static_cast<unsigned>(oc) >= static_cast<unsigned>(n_out_cells)) return;   // (the last block may reach past 2^31)
   const bool failed = halo_exchange_failed();
   int a[V], b[V];
   ld_cells<V>(a, src_a + oc);
