@@ -71,6 +71,8 @@ struct MlpSmem {
   static constexpr int BAR_OFF = LN_OFF + (LN ? 2 * 4 * 16 * 32 * 4 : 0);
   static constexpr int TOTAL = BAR_OFF + 512 + 1024;             // + alignment slack
   static constexpr int OUT_COL = 256, OUT_BUFS = AHEAD ? 2 : 1, OUT_STRIDE = 128;
+  // Warps that read a tile's output: those whose box of 32 columns begins below C (16 warps, four boxes side by side).
+  static constexpr int OUT_READERS = C < 128 ? 4 * (C / 32) : GEMM_EPI_WARPS;
   static_assert(GEMM_EPI_WARPS * STAGING_BYTES <= H_BYTES, "the staging boxes fit the hidden chunk's buffer");
   static_assert(TOTAL <= 232448, "shared memory of an SM");
 };
@@ -120,7 +122,7 @@ mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       mbar_init(h_full(b), GEMM_EPI_WARPS / S::SETS);
       mbar_init(h_empty(b), 1);
       mbar_init(out_full(b), 1);
-      mbar_init(out_free(b), GEMM_EPI_WARPS);
+      mbar_init(out_free(b), S::OUT_READERS);
     }
     for (int s = 0; s < S::S1; ++s) { mbar_init(w1_full(s), 1); mbar_init(w1_empty(s), 1); }
     for (int s = 0; s < S::S2; ++s) { mbar_init(w2_full(s), 1); mbar_init(w2_empty(s), 1); }
@@ -431,10 +433,15 @@ mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
           tma_store_commit();
         }
       }
-      // the output columns may be accumulated into again
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(out_free(ob));
+      // The output columns may be accumulated into again. Every arrival follows its warp's own wait for out_full of
+      // this tile, so a phase of out_free is made of one tile's readers. A warp without columns waits for nothing here
+      // and runs ahead by as many tiles as its chunks let it, so it has no say: else two of its tiles would fill a phase
+      // before the readers of the first are done (C = 64, one chunk a tile, from the fourth tile of a CTA on).
+      if (box0 < C) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(out_free(ob));
+      }
       if constexpr (LN) {
         if (box0 < C && m_warp < p.M) {      // (the whole quarter has rows or none)
 #pragma unroll

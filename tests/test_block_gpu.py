@@ -592,3 +592,28 @@ def test_narrow_block_is_its_steps(ops, C, grid, tiles, gated):
     h = ops.linear(ops.layernorm(x1), w["w_fc1"], w["b_fc1"], ops.EPI_GELU)
     want = ops.linear(h, w["w_fc2"], w["b_fc2"], ops.EPI_RESIDUAL, x1)
     assert torch.equal(y.view(M, C), want)
+
+
+# hidden layers of 1, 2 and 8 times the width; 64 and 128 channels on more rows than three 128-row tiles for each SM
+@pytest.mark.parametrize("C,hidden,grid,tiles", [(64, 128, (15, 62, 64), 1), (64, 64, (2, 9, 13), 1),
+                                                 (64, 512, (15, 62, 64), 1), (128, 128, (15, 62, 64), 1),
+                                                 (192, 384, (10, 60, 64), 1), (256, 512, (4, 40, 63), 2),
+                                                 (256, 2048, (4, 40, 63), 2)])
+def test_narrow_block_of_other_hidden_widths(ops, C, hidden, grid, tiles):
+    g = torch.Generator("cuda").manual_seed(C + hidden)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    D, H, W = grid
+    M, heads, kernel = tiles * D * H * W, C // 64, (1, 3, 3)
+    w = {}
+    for n, (o, i) in {"qkv": (3 * C, C), "proj": (C, C), "fc1": (hidden, C), "fc2": (C, hidden)}.items():
+        w[f"w_{n}"], w[f"b_{n}"] = (rnd(o, i) * i ** -0.5).bfloat16(), rnd(o) * 0.1
+    x = (rnd(M, C) * 2 + 0.5).bfloat16()
+    y = ops.block_forward(x.view(tiles, D * H * W, C), w, grid=grid, num_heads=heads, kernel=kernel, rope_cos=None,
+                          rope_sin=None)
+    assert _status() == 0
+    qkv = ops.qkv_rope(ops.layernorm(x), w["w_qkv"], w["b_qkv"], 64, None, None, D * H * W, H * W)
+    q6 = qkv.view(tiles, D, H, W, 3, heads, 64)
+    attn = ops.na3d(*(q6[..., i, :, :] for i in range(3)), kernel).reshape(M, C)
+    x1 = ops.linear(attn, w["w_proj"], w["b_proj"], ops.EPI_RESIDUAL, x)
+    h = ops.linear(ops.layernorm(x1), w["w_fc1"], w["b_fc1"], ops.EPI_GELU)
+    assert torch.equal(y.view(M, C), ops.linear(h, w["w_fc2"], w["b_fc2"], ops.EPI_RESIDUAL, x1))

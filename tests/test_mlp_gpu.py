@@ -69,6 +69,15 @@ def test_mlp_is_the_two_gemms(ops, M, C, H, mode, pad, bias):
     assert float((out.double() - t).norm() / t.norm()) < 4e-3
 
 
+# 64 channels leave half of the epilogue warps without output columns, and with one chunk a tile those take only every
+# other tile's: four tiles a CTA and more (148 x 128 rows are one), where such warps run ahead of the readers
+@pytest.mark.parametrize("M,C,H,mode", [
+    (60007, 64, 128, "residual"), (60007, 64, 256, "gate"), (200003, 64, 128, "gate"), (200003, 64, 128, "bias"),
+    (200003, 64, 256, "residual"), (200003, 64, 384, "residual"), (100003, 128, 128, "residual")])
+def test_mlp_of_many_tiles_a_cta(ops, M, C, H, mode):
+    test_mlp_is_the_two_gemms(ops, M, C, H, mode, 0, True)
+
+
 def test_mlp_in_place_and_through_ops(ops):
     d = _data(5000, 128, 512, 3)
     want = ops.linear(ops.linear(d["x"], d["w1"], d["b1"], ops.EPI_GELU), d["w2"], d["b2"], ops.EPI_RESIDUAL, d["aux"])

@@ -118,6 +118,34 @@ def test_norms_written_by_the_kernels_before_them(dim, layers, size, gated):
         assert torch.equal(m(x, idx), y)
 
 
+@pytest.mark.parametrize("two_stage", [False, True])
+def test_short_hidden_layers_on_many_rows(two_stage):
+    # 64 channels and 128 hidden ones on more rows than three 128-row tiles for each SM: the next norm written by the
+    # MLP (one stage), the gated residual (pixel stage, whose single steps are the GEMMs)
+    from strata_b200.wrappers import StrataBackboneModel, StrataModel
+    D, H, W = (5, 96, 72) if two_stage else (16, 172, 180)
+    kw = dict(depth=D, height=H, width=W, n_layers=1 if two_stage else 3, patch_size_horiz=4, in_chans=5,
+              base_out_chans=4, embed_dim=128 if two_stage else 64, num_heads=2 if two_stage else 1, attn_kernel=(1, 3, 3),
+              do_rope_2d_stereographic=True, index_is_latlon=True)
+    if two_stage:
+        kw.update(embed_dim_pixel=64, n_layers_pixel=2, mlp_ratio_pixel=2.0, attn_kernel_pixel=(1, 3, 3),
+                  use_bilinear_dw_gelu_project_adaln_pixel=True)
+    else:
+        kw.update(mlp_ratio=2.0)
+    m = _randomised((StrataModel if two_stage else StrataBackboneModel)(**kw).cuda())
+    x = torch.randn(2, 5, D, H, W, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    lat, lon = tile_latlon(2, H, W)
+    idx = {"lat": lat.cuda(), "lon": lon.cuda()}
+
+    class StepByStep:
+        def forward(self, *a):
+            return None
+    with torch.no_grad():
+        y = m(x, idx)
+        m.strata._network = StepByStep()
+        assert torch.equal(m(x, idx), y)
+
+
 def _own_block_code(m, seen):
     """Replaces parts of a model's blocks; every replaced part reports itself in `seen`."""
     import types
