@@ -120,8 +120,10 @@ def mlp(x: torch.Tensor, w1: torch.Tensor, b1: torch.Tensor | None, w2: torch.Te
     M, C = x.shape
     H = w1.shape[0]
     rows = (x, residual) if out is None else (x, residual, out)
+    # whatever is not of the kernel's form goes to the two GEMMs, which take it or say what is wrong with it
     if not (x.is_cuda and _lib.load().strata_mlp_fused(M, C, H) and w1.is_contiguous() and w2.is_contiguous() and
-            tuple(w2.shape) == (C, H) and all(t.shape == x.shape and t.stride(1) == 1 for t in rows)):
+            tuple(w1.shape) == (H, C) and tuple(w2.shape) == (C, H) and
+            all(t.shape == x.shape and t.stride(1) == 1 for t in rows)):
         return linear(linear(x, w1, b1, EPI_GELU), w2, b2, EPI_RESIDUAL, residual, out=out)
     for t, n in ((x, "x"), (w1, "w1"), (w2, "w2"), (residual, "residual")):
         _require_cuda_bf16(t, n)

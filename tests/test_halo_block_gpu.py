@@ -122,6 +122,19 @@ def test_tiled_block_matches_oracle(gated, qk_norm, kernel, halo, runner_kw):
     assert rel_max_err(y, ref) < TOL_BF16
 
 
+def test_tiled_block_of_wrong_mlp_weights_raises():
+    run, topo, p, x, okw = _setup(2, (1, 5, 5))
+    w = device_block_weights(p, "cuda")
+    C = x.shape[-1]
+    for cols in (C // 2, 2 * C):
+        bad = torch.zeros(w["w_fc1"].shape[0], cols, device="cuda", dtype=torch.bfloat16)
+        with pytest.raises(ValueError):
+            run.block_forward(x.cuda(), {**w, "w_fc1": bad})
+    with pytest.raises(ValueError):
+        run.block_forward(x.cuda(), {**w, "w_fc2": w["w_fc2"][:, :-64].contiguous()})
+    run.check_status()
+
+
 @pytest.mark.skipif(not (torch.cuda.is_available() and torch.cuda.device_count() >= 2),
                     reason="needs 2 GPUs on one node")
 def test_two_rank_tiled_block_stack():

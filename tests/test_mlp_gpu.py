@@ -96,3 +96,19 @@ def test_mlp_refuses_what_it_has_no_kernel_for(ops):
     assert f(p, 320, p, None, p, None, None, 0, None, 0, p, 320, 128, 128, 320, 0) == -2      # part of a chunk
     assert f(p, 320, p, None, p, None, None, 0, p, 320, p, 320, 128, 128, 128, 0) == -1       # a gate without aux
     assert f(p + 2, 320, p, None, p, None, None, 0, None, 0, p, 320, 128, 128, 128, 0) == -1  # alignment
+
+
+def test_mlp_of_wrong_weights_raises(ops):
+    z = lambda *s: torch.zeros(*s, device="cuda", dtype=torch.bfloat16)
+    x, w1, w2 = z(256, 128), z(512, 128), z(128, 512)
+    b1, b2 = torch.zeros(512, device="cuda"), torch.zeros(128, device="cuda")
+    assert ops.mlp(x, w1, b1, w2, b2, x).shape == x.shape
+    for bad in (z(512, 64), z(512, 192), z(512), z(512, 128, 1)):
+        with pytest.raises(ValueError):
+            ops.mlp(x, bad, b1, w2, b2, x)
+    for bad in (z(128, 384), z(64, 512), z(128, 640)):
+        with pytest.raises(ValueError):
+            ops.mlp(x, w1, b1, bad, b2, x)
+    for bad in (z(256, 64), z(128, 128)):
+        with pytest.raises(ValueError):
+            ops.mlp(x, w1, b1, w2, b2, bad)
