@@ -555,19 +555,42 @@ inline int launch_mlp_t(const __nv_bfloat16* x, long long ldx, const __nv_bfloat
 // Whether the kernel takes these sizes (weights contiguous, everything else as the GEMMs want it).
 inline bool mlp_fused_sizes(int C, int H) { return C % 64 == 0 && C > 0 && C <= MLP_MAX_C && H % MLP_CHUNK == 0 && H > 0; }
 
-// Whether it is the faster way: two GEMMs / this kernel, microseconds with a residual, from a cold L2, H = 4 C:
-//            1024       4096       8192       12288      18944      24576      49152      442368 rows
-//   C = 128: 13 / 14    15 / 15    15 / 15    17 / 16    21 / 16    26 / 22    34 / 29    232 / 145
-//   C = 192: 15 / 20    17 / 21    19 / 21    24 / 22    28 / 22    32 / 35    48 / 49    345 / 301
-//   C = 256: 15 / 24    17 / 25    24 / 26    28 / 27    32 / 29    42 / 45    69 / 63    480 / 412
-// and at C = 64 11 / 11, 13 / 11, 46 / 31, 132 / 80 at 256, 8192, 131072, 442368 rows. A few row blocks of a wide model leave
-// SMs idle through all of its chunks, and so does a second turn of the blocks that is less than half full. At C = 128 the
-// two are level on few rows, where the host, which launches one kernel less, is what a small model waits for.
+// Whether it is the faster way. Two GEMMs/this kernel, microseconds with a residual, passes back to back on inputs and
+// outputs that do not stay in L2, by row blocks of 128 (148 of them are one turn of the chip):
+//              16        75        148       149       222       296       352       445       592       3456
+//   C = 192 H = 2C 8.0/11.2  13.6/12.8 15.9/14.0 17.7/21.2 22.8/22.6 26.9/23.4 31.5/32.0 37.8/39.2 42.7/41.7 218/220
+//           H = 4C 9.6/15.0  18.7/16.5 21.7/17.8 25.6/28.4 29.1/29.9 32.6/30.8 40.9/42.6 51.6/53.5 64.5/56.2 329/311
+//           H = 8C 12.7/22.0 24.5/23.5 31.1/25.1 37.3/41.9 47.9/44.5 60.5/45.3 75.3/63.6 94.1/81.0 116/84.8  612/490
+//   C = 256 H = 2C 9.1/13.9  15.5/15.2 20.0/16.6 22.8/25.6 25.2/27.5 29.4/28.6 34.9/38.9 42.1/48.2 50.9/52.0 272/274
+//           H = 4C 10.7/18.7 22.6/20.5 26.9/22.1 32.2/35.9 36.5/38.3 45.3/39.3 58.1/54.3 73.6/69.0 90.7/76.2 473/435
+//           H = 8C 14.5/29.1 32.0/31.2 42.8/33.1 52.8/56.2 68.0/61.7 85.4/62.2 104/87.5  138/130   163/135   915/705
+//              1         16        48        64        149       296       592       3456
+//   C = 64  H = 2C 6.5/5.2   7.0/5.3   7.1/5.3   7.5/5.6   10.7/7.5  12.6/8.3  18.6/12.6 81.9/57.7
+//           H = 4C 6.8/6.1   7.3/6.1   8.2/6.4   8.4/6.7   12.4/9.2  16.5/10.2 25.0/16.5 122/78.3
+//           H = 8C 7.3/8.3   7.9/8.4   9.8/8.8   10.3/9.0  17.6/13.5 22.4/14.6 38.9/25.0 211/131
+//   C = 128 H = 2C 6.9/6.6   7.4/6.8   8.8/7.3   9.3/7.5   13.7/11.2 18.4/12.2 26.9/19.1 132/87.6
+//           H = 4C 7.3/8.8   8.2/9.0   10.6/9.6  10.9/9.8  18.6/15.3 22.8/16.8 40.8/28.1 219/141
+//           H = 8C 8.8/13.1  9.9/13.4  13.1/13.9 15.3/14.3 25.1/24.0 36.5/25.9 74.7/46.0 390/249
+// The kernel's time goes by turns of the chip, each a fixed part and one for every chunk of hidden channels, however
+// many row blocks the turn has; the GEMMs spread columns over the SMs too, and theirs goes by row blocks and chunks.
+// Up to half a turn the kernel leaves SMs idle through all of its chunks; from there to the turn's end it is ahead. Of
+// two turns the second has to be half full, a quarter where the chunks are many. From three on a 192-wide block of few
+// chunks, whose turn takes as long as the GEMMs' share of one, wants two thirds of the last turn full (H = 2C: at 370
+// blocks 31.9/32.2, at 400 33.7/32.4, at 520 41.0/41.3, at 560 42.2/41.6); elsewhere the two lines compare the times,
+// in units of their own, as fitted to 22 numbers of blocks from 297 to 3456: the slower way by more than 2.4 % nowhere.
+// Narrower blocks have the kernel ahead from few rows on; with more than four chunks its chain is longer than the two
+// GEMMs' until a third of the SMs have work, and with four the two are within 1.5 us there, where the host, which
+// launches one kernel less, is what a small model waits for.
 inline bool mlp_fused_pays(int M, int C, int H, int sm_count) {
   if (!mlp_fused_sizes(C, H)) return false;
-  if (C <= 128) return true;
-  const int blocks = (M + GEMM_BM - 1) / GEMM_BM;
-  return blocks > sm_count / 2 && (blocks <= sm_count || 2 * blocks > 3 * sm_count);
+  const int blocks = (M + GEMM_BM - 1) / GEMM_BM, turns = (blocks + sm_count - 1) / sm_count, chunks = H / MLP_CHUNK;
+  if (C <= 128) return chunks <= 4 || 3 * blocks > sm_count;
+  if (turns <= 1) return 2 * blocks > sm_count;
+  if (turns == 2) return 4 * blocks > (chunks >= 10 ? 5 : 6) * sm_count;
+  if (C <= 192 && chunks <= 4) return 3 * (turns * sm_count - blocks) <= sm_count;
+  const float passes = static_cast<float>(blocks) / static_cast<float>(sm_count);
+  return C <= 192 ? turns * (4.5f + 1.1f * chunks) <= 2.5f + passes * 2.15f * chunks
+                  : turns * (5.75f + 1.1f * chunks) <= 2.f + passes * 2.35f * chunks;
 }
 
 inline int launch_mlp(int C, const __nv_bfloat16* x, long long ldx, const __nv_bfloat16* w1, const __nv_bfloat16* w2,

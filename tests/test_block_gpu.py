@@ -598,7 +598,12 @@ def test_narrow_block_is_its_steps(ops, C, grid, tiles, gated):
 @pytest.mark.parametrize("C,hidden,grid,tiles", [(64, 128, (15, 62, 64), 1), (64, 64, (2, 9, 13), 1),
                                                  (64, 512, (15, 62, 64), 1), (128, 128, (15, 62, 64), 1),
                                                  (192, 384, (10, 60, 64), 1), (256, 512, (4, 40, 63), 2),
-                                                 (256, 2048, (4, 40, 63), 2)])
+                                                 (256, 2048, (4, 40, 63), 2),
+                                                 # either side of the rule: turns of 148 row blocks, chunks
+                                                 (128, 1024, (4, 28, 41), 1), (128, 1024, (5, 32, 41), 1),
+                                                 (192, 768, (10, 60, 64), 1), (192, 1536, (10, 60, 64), 1),
+                                                 (256, 1024, (4, 80, 119), 1), (256, 512, (9, 70, 90), 1),
+                                                 (192, 1536, (5, 61, 80), 1)])
 def test_narrow_block_of_other_hidden_widths(ops, C, hidden, grid, tiles):
     g = torch.Generator("cuda").manual_seed(C + hidden)
     rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")

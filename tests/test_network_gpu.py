@@ -118,20 +118,23 @@ def test_norms_written_by_the_kernels_before_them(dim, layers, size, gated):
         assert torch.equal(m(x, idx), y)
 
 
-@pytest.mark.parametrize("two_stage", [False, True])
-def test_short_hidden_layers_on_many_rows(two_stage):
+@pytest.mark.parametrize("two_stage,dim,ratio,size", [(False, 64, 2.0, (16, 172, 180)), (True, 64, 2.0, (5, 96, 72)),
+                                                      (False, 128, 8.0, (4, 100, 92)), (True, 128, 8.0, (2, 40, 24))])
+def test_short_and_long_hidden_layers(two_stage, dim, ratio, size):
     # 64 channels and 128 hidden ones on more rows than three 128-row tiles for each SM: the next norm written by the
-    # MLP (one stage), the gated residual (pixel stage, whose single steps are the GEMMs)
+    # MLP (one stage), the gated residual (pixel stage, whose single steps are the GEMMs). 128 channels and 1024 hidden
+    # ones on so few rows that the two GEMMs are taken, though the projection writes the norm before them
     from strata_b200.wrappers import StrataBackboneModel, StrataModel
-    D, H, W = (5, 96, 72) if two_stage else (16, 172, 180)
+    D, H, W = size
     kw = dict(depth=D, height=H, width=W, n_layers=1 if two_stage else 3, patch_size_horiz=4, in_chans=5,
-              base_out_chans=4, embed_dim=128 if two_stage else 64, num_heads=2 if two_stage else 1, attn_kernel=(1, 3, 3),
+              base_out_chans=4, embed_dim=128 if two_stage else dim, num_heads=2 if two_stage else dim // 64,
+              attn_kernel=(1, 3, 3),
               do_rope_2d_stereographic=True, index_is_latlon=True)
     if two_stage:
-        kw.update(embed_dim_pixel=64, n_layers_pixel=2, mlp_ratio_pixel=2.0, attn_kernel_pixel=(1, 3, 3),
+        kw.update(embed_dim_pixel=dim, n_layers_pixel=2, mlp_ratio_pixel=ratio, attn_kernel_pixel=(1, 3, 3),
                   use_bilinear_dw_gelu_project_adaln_pixel=True)
     else:
-        kw.update(mlp_ratio=2.0)
+        kw.update(mlp_ratio=ratio)
     m = _randomised((StrataModel if two_stage else StrataBackboneModel)(**kw).cuda())
     x = torch.randn(2, 5, D, H, W, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
     lat, lon = tile_latlon(2, H, W)
