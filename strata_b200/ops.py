@@ -128,14 +128,15 @@ def mlp(x: torch.Tensor, w1: torch.Tensor, b1: torch.Tensor | None, w2: torch.Te
     for t, n in ((x, "x"), (w1, "w1"), (w2, "w2"), (residual, "residual")):
         _require_cuda_bf16(t, n)
     b1, b2 = _f32_or_none(b1, "b1"), _f32_or_none(b2, "b2")
+    (_, _, _, ldx), (_, _, _, ldr) = _as_rows(x, "x"), _as_rows(residual, "residual")
     if out is None:
         out = torch.empty((M, C), dtype=torch.bfloat16, device=x.device)
     else:
         _require_cuda_bf16(out, "out")
     with _lib.on_device(x):
         _lib.check(_lib.load().strata_mlp_bf16(
-            x.data_ptr(), x.stride(0), w1.data_ptr(), None if b1 is None else b1.data_ptr(), w2.data_ptr(),
-            None if b2 is None else b2.data_ptr(), residual.data_ptr(), residual.stride(0), None, 0,
+            x.data_ptr(), ldx, w1.data_ptr(), None if b1 is None else b1.data_ptr(), w2.data_ptr(),
+            None if b2 is None else b2.data_ptr(), residual.data_ptr(), ldr, None, 0,
             out.data_ptr(), out.stride(0), M, C, H, _stream_ptr(x)), "strata_mlp_bf16")
     return out
 

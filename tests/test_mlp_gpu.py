@@ -112,3 +112,13 @@ def test_mlp_of_wrong_weights_raises(ops):
     for bad in (z(256, 64), z(128, 128)):
         with pytest.raises(ValueError):
             ops.mlp(x, w1, b1, w2, b2, bad)
+
+
+def test_mlp_of_one_row_with_any_row_stride(ops):
+    # the row stride of a single row says nothing: linear takes such a view, and so does this
+    d = _data(1, 128, 512, 5)
+    x, aux = (t.contiguous().view(128, 1).t() for t in (d["x"], d["aux"]))
+    assert x.stride() == (1, 1)
+    h = ops.linear(x, d["w1"], d["b1"], ops.EPI_GELU)
+    want = ops.linear(h, d["w2"], d["b2"], ops.EPI_RESIDUAL, aux)
+    assert torch.equal(ops.mlp(x, d["w1"], d["b1"], d["w2"], d["b2"], aux), want)
