@@ -63,7 +63,8 @@ const char* strata_error_string(int code) {
     case STRATA_ERR_TENSORMAP:
     case -21:
     case -22:
-    case -23: return "TMA tensor map could not be encoded for this operand layout";
+    case -23:
+    case -25: return "TMA tensor map could not be encoded for this operand layout";
     default: break;
   }
   if (code <= -1000) return cudaGetErrorString(static_cast<cudaError_t>(-(code + 1000)));

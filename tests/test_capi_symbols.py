@@ -35,6 +35,12 @@ def test_error_strings_and_version():
     assert lib.strata_block_workspace_bytes(128, 64, 256) == 3 * 128 * 64 * 2 + 128 * 192 * 2 + 128 * 256 * 2
 
 
+@pytest.mark.parametrize("code", [-20, -21, -22, -23, -25])   # one for every operand that a launch describes to TMA
+def test_tensor_map_errors_have_a_text(code):
+    from strata_b200 import _lib
+    assert b"tensor map" in _lib.load().strata_error_string(code)
+
+
 def test_ops_refuse_cpu_tensors():
     import torch
     from strata_b200 import ops, _lib
