@@ -62,8 +62,8 @@ int strata_linear_bf16(const void* x, int64_t ldx, const void* w, int64_t ldw, c
                        int64_t ldaux, void* stream);
 
 /* y[M,C] = aux + [gate *] (W2 gelu(W1 x + b1) + b2): the MLP of a narrow block in one kernel, same bits as
- * strata_linear_bf16 with STRATA_EPI_GELU and then with STRATA_EPI_RESIDUAL (aux, no gate), STRATA_EPI_BIAS (neither) or
- * STRATA_EPI_BIAS followed by the gated residual of strata_adaln_rows_bf16 (gate). W1 [hidden,C] and
+ * strata_linear_bf16 with STRATA_EPI_GELU and then with STRATA_EPI_RESIDUAL (aux, no gate), STRATA_EPI_BIAS (neither)
+ * or STRATA_EPI_BIAS followed by the gated residual of strata_adaln_rows_bf16 (gate). W1 [hidden,C] and
  * W2 [C,hidden] are contiguous. C = 64, 128, 192 or 256 and hidden a multiple of 128, otherwise
  * STRATA_ERR_UNSUPPORTED. y may be aux. */
 int strata_mlp_bf16(const void* x, int64_t ldx, const void* w1, const float* b1, const void* w2,

@@ -161,7 +161,8 @@ static int mlp_impl(const void* x, int64_t ldx, const void* w1, const float* b1,
   p.gate = static_cast<const __nv_bfloat16*>(gate); p.ldgate = ldgate;
   p.ln_out = static_cast<__nv_bfloat16*>(ln_out); p.ldln = ldln; p.ln_eps = ln_eps;
   return launch_mlp(C, static_cast<const __nv_bfloat16*>(x), ldx, static_cast<const __nv_bfloat16*>(w1),
-                    static_cast<const __nv_bfloat16*>(w2), static_cast<__nv_bfloat16*>(y), ldy, p, sms, as_stream(stream));
+                    static_cast<const __nv_bfloat16*>(w2), static_cast<__nv_bfloat16*>(y), ldy, p, sms,
+                    as_stream(stream));
 }
 
 int strata_mlp_bf16(const void* x, int64_t ldx, const void* w1, const float* b1, const void* w2, const float* b2,
@@ -233,14 +234,17 @@ static int qkv_rope_impl(const void* x, int64_t ldx, const void* w, int64_t ldw,
   const auto* W = static_cast<const __nv_bfloat16*>(w);
   if (!rope_cs && !qk_norm) return launch_gemm<EPI_BIAS>(A, ldx, W, ldw, p, sms, as_stream(stream));
   if (!rope_cs && C < 256 && head_dim == 64) {
-    // qk norm without rotation at a small width: a plain projection and the in-place row kernel, which
-    // normalises the q and k heads, against the fused epilogue with an identity table. Two kernels / fused,
-    // microseconds at 1024, 24576, 262144 and 1572864 rows (the pixel stage of one production tile): C = 64 13.3 / 13.3,
-    // 17.4 / 17.4, 54 / 56, 327 / 282; C = 128 11.2 / 13.4, 19.5 / 20.5, 103 / 98, 570 / 520; C = 192 13.3 / 14.3, 25.6 /
-    // 26.6, 183 / 171, 1157 / 949 - in favour of two kernels where a launch is short. From C = 256 on fused is
-    // ahead: 212 / 173, 24.6 / 21.9, 9.6 / 9.6; C = 512 at 262144 rows 491 / 377. (All with 256-wide tiles in the fused
-    // one, which takes narrow ones on few rows today; its sums and so its bits are others than the row kernel's.) (Here the norm sees q and k rounded
-    // to bf16, there the fp32 accumulators: error against 64 bits 2.1e-3 and 1.7e-3 of the result.)
+    // qk norm without rotation at a small width: a plain projection and the in-place row kernel, which normalises the q
+    // and k heads. Beside the fused epilogue with an identity table, two kernels / fused in microseconds, passes back
+    // to back on buffers that do not stay in L2:
+    //   rows      256         4096        8192        24576       65536       262144      1572864
+    //   C = 64    5.0 / 5.4   6.0 / 6.3   7.3 / 6.6   10.2 / 10.5 18.2 / 17.3 50.4 / 50.9 323 / 279
+    //   C = 128   5.5 / 5.7   7.4 / 6.6   8.7 / 8.5   14.8 / 14.4 26.7 / 27.2 99.7 / 91.6 589 / 519
+    //   C = 192   5.7 / 6.0   9.2 / 8.6   11.2 / 12.4 20.4 / 20.1 42.8 / 47.1 178 / 165   1107 / 954
+    //   C = 256   5.9 / 6.1   9.2 / 8.7   11.9 / 12.4 23.0 / 19.3 49.9 / 42.8 203 / 152   1258 / 903
+    // Below 256 channels neither is ahead by much until a launch is the pixel stage of a whole production tile; the
+    // norm there sees q and k rounded to bf16, in the epilogue the fp32 accumulators (error against 64 bits 2.1e-3 and
+    // 1.7e-3 of the result), so the choice is one of bits too and is kept. From 256 channels on the epilogue is ahead.
     int r = launch_gemm<EPI_BIAS>(A, ldx, W, ldw, p, sms, as_stream(stream));
     if (r != 0) return r;
     long long rows = M;
@@ -336,13 +340,13 @@ int64_t strata_block_workspace_bytes(int64_t M, int C, int hidden) {
   return r256(M * C * 2) * 3 + r256(M * 3 * C * 2) + r256(M * static_cast<int64_t>(hidden) * 2);
 }
 
-// Where the projection writes the block's second norm, and the MLP (C <= 128) the norm that comes next: up to 256 channels
-// (whole rows in a tile), a power of two, so that the division by their number is exact and the norm has the
+// Where the projection writes the block's second norm, and the MLP (C <= 128) the norm that comes next: up to 256
+// channels (whole rows in a tile), a power of two, so that the division by their number is exact and the norm has the
 // bits of the kernel of its own. 442368 x 256: projection and norm 122 + 109 us, in one 178; a block on 8192 x 128
 // 39.7 -> 38.4 us, three on 18480 x 128 219 -> 206. A short launch's own norm is spread over all SMs and overlaps
 // its neighbours, here it is at the end of every CTA's chain: on 256 and 1024 rows of 128 level (0.99 - 1.01), and with
-// 256 channels, where one tile is all of a row's columns, a block on 8192 rows 52.9 -> 55.0 us, on 65536 213.7 -> 216.8,
-// on 131072 387 -> 386.
+// 256 channels, where one tile is all of a row's columns, a block on 8192 rows 52.9 -> 55.0 us, on 65536 213.7 ->
+// 216.8, on 131072 387 -> 386.
 static bool ln_fused_pays(int M, int C) {
   return C == 256 ? M >= 131072 : M >= 4096 && (C == 64 || C == 128);
 }
@@ -351,8 +355,8 @@ static bool ln_fused_pays(int M, int C) {
 // may be the workspace's beginning; *ln_done says whether it did.
 static int block_impl(const void* x, void* y, int n_tiles, int D, int H, int W, int C, int heads, int hidden, int kd,
                       int kh, int kw, const strata_block_weights* wts, const void* rope_cs, int qk_norm, float ln_eps,
-                      float qk_eps, void* workspace, int64_t workspace_bytes, bool xn_ready, void* ln_out, bool* ln_done,
-                      void* stream) {
+                      float qk_eps, void* workspace, int64_t workspace_bytes, bool xn_ready, void* ln_out,
+                      bool* ln_done, void* stream) {
   if (ln_done) *ln_done = false;
   if (!x || !y || !wts || !workspace || n_tiles < 0 || D <= 0 || H <= 0 || W <= 0)
     return STRATA_ERR_ARG;
@@ -396,8 +400,9 @@ static int block_impl(const void* x, void* y, int n_tiles, int D, int H, int W, 
     p.aux = static_cast<const __nv_bfloat16*>(x); p.ldaux = C;
     p.ln_eps = ln_eps;
     if (!aligned16(x) || !aligned16(wts->w_proj) || (wts->b_proj && !aligned16(wts->b_proj))) return STRATA_ERR_ARG;
-    if ((r = launch_gemm_residual_ln(static_cast<const __nv_bfloat16*>(attn), C, static_cast<const __nv_bfloat16*>(wts->w_proj), C,
-                                     static_cast<__nv_bfloat16*>(xn), C, p, current_sm_count(), as_stream(stream))) != 0)
+    if ((r = launch_gemm_residual_ln(static_cast<const __nv_bfloat16*>(attn), C,
+                                     static_cast<const __nv_bfloat16*>(wts->w_proj), C, static_cast<__nv_bfloat16*>(xn),
+                                     C, p, current_sm_count(), as_stream(stream))) != 0)
       return r;
   } else {
     if ((r = strata_linear_bf16(attn, C, wts->w_proj, C, wts->b_proj, x1, C, M, C, C,
@@ -407,8 +412,8 @@ static int block_impl(const void* x, void* y, int n_tiles, int D, int H, int W, 
   }
   if (mlp_fused_pays(M, C, hidden, current_sm_count())) {
     const bool ln = ln_out && ln_fused_pays(M, C) && C <= 128;
-    r = mlp_impl(xn, C, wts->w_fc1, wts->b_fc1, wts->w_fc2, wts->b_fc2, x1, C, nullptr, 0, y, C, ln ? ln_out : nullptr, C,
-                 ln_eps, M, C, hidden, stream);
+    r = mlp_impl(xn, C, wts->w_fc1, wts->b_fc1, wts->w_fc2, wts->b_fc2, x1, C, nullptr, 0, y, C,
+                 ln ? ln_out : nullptr, C, ln_eps, M, C, hidden, stream);
     if (ln_done) *ln_done = ln && r == 0;
     return r;
   }

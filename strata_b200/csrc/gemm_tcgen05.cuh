@@ -12,7 +12,8 @@
 //               (as matrix fragments, or each thread one output row, 16 columns at a time), apply bias
 //               and the selected epilogue, store bf16. The other accumulator is being filled meanwhile.
 //
-// BN = 256, 128 or 64 by the rule of launch_gemm. PAIR variant (large problems): two CTAs of a cluster share every MMA (tcgen05 cta_group::2,
+// BN = 256, 128 or 64 by the rule of launch_gemm. PAIR variant (large problems): two CTAs of a cluster share every MMA
+// (tcgen05 cta_group::2,
 // M = 256): each CTA loads its own 128 rows of A and HALF of the W tile, the instruction reads
 // both halves, and each CTA's tensor memory receives its 128 rows x BN accumulator. A CTA then
 // moves 32 KB per k-block through shared memory instead of 48 KB, which matters because the
@@ -171,8 +172,9 @@ __device__ __forceinline__ void gemm_epilogue_16(float (&v)[16], bool rotate, fl
   }
 }
 
-// The other epilogues read the accumulator as matrix fragments, 16 rows x 32 columns a load: registers 4 i + {0, 1} hold row lane / 4,
-// columns 8 i + 2 (lane % 4) + {0, 1}, registers 4 i + {2, 3} the same of row lane / 4 + 8. A lane then needs eight
+// The other epilogues read the accumulator as matrix fragments, 16 rows x 32 columns a load: registers 4 i + {0, 1}
+// hold row lane / 4, columns 8 i + 2 (lane % 4) + {0, 1}, registers 4 i + {2, 3} the same of row lane / 4 + 8. A lane
+// then needs eight
 // biases for 32 columns (with a row per lane all 32) and holds the pairs that the rotation turns, a row's
 // squares are summed within a quad, and 8 x 8 pieces go to the staging boxes and come from them with stmatrix and
 // ldmatrix.
@@ -205,7 +207,8 @@ __device__ __forceinline__ void gemm_lane_bias(const GemmParams& p, int n0, int 
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int k = n + 8 * i;
-      bias[i] = p.bias == nullptr ? 0ull : pack2(k < p.N ? __ldg(p.bias + k) : 0.f, k + 1 < p.N ? __ldg(p.bias + k + 1) : 0.f);
+      bias[i] = p.bias == nullptr ? 0ull
+                                  : pack2(k < p.N ? __ldg(p.bias + k) : 0.f, k + 1 < p.N ? __ldg(p.bias + k + 1) : 0.f);
     }
   }
 }
@@ -213,7 +216,8 @@ __device__ __forceinline__ void gemm_lane_bias(const GemmParams& p, int n0, int 
 // Epilogue math on a pair of neighbouring columns of one row (bias added); aux: the residual / gated operand of the
 // pair (bf16); cs: its (cos, sin) half pair; scale: the RMS factor of the row's head.
 template <int EPI>
-__device__ __forceinline__ uint32_t gemm_epilogue_pair(uint64_t x, uint32_t aux, bool rotate, uint32_t cs, float scale) {
+__device__ __forceinline__ uint32_t gemm_epilogue_pair(uint64_t x, uint32_t aux, bool rotate, uint32_t cs,
+                                                       float scale) {
   float a, b;
   if constexpr (EPI == EPI_GELU) {
     unpack2(gelu_pair(x), a, b);
@@ -288,9 +292,10 @@ __device__ __noinline__ float2 gemm_qk_norm_scales(uint32_t taddr, const float* 
 }
 
 // LayerNorm of a row that four warps (a lane quarter) hold in parts, a row per lane, bf16 in and out: what
-// layernorm_rows_kernel computes, with its order of additions - pairs, the four pairs of 8 columns in turn, then the 8-column
-// sums i with i ^ 16, i ^ 8, ... - so that the result is the same bits. Each warp leaves its 8-column sums in shared
-// memory ([groups][32 rows] of its quarter, one buffer for the mean and one for the variance) and reads all of them.
+// layernorm_rows_kernel computes, with its order of additions - pairs, the four pairs of 8 columns in turn, then the
+// 8-column sums i with i ^ 16, i ^ 8, ... - so that the result is the same bits. Each warp leaves its 8-column sums
+// in shared memory ([groups][32 rows] of its quarter, one buffer for the mean and one for the variance) and reads all
+// of them.
 __device__ __forceinline__ float ln_group_sum(const uint32_t* w) {   // 8 columns
   float s = 0.f;
 #pragma unroll
@@ -317,10 +322,12 @@ __device__ __forceinline__ float ln_total(uint32_t buf, int lane) {
   float g[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(g[i]) : "r"(buf + static_cast<uint32_t>(i * 32 + lane) * 4u) : "memory");
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(g[i])
+                 : "r"(buf + static_cast<uint32_t>(i * 32 + lane) * 4u) : "memory");
     if constexpr (GROUPS == 32) {
       float h;
-      asm volatile("ld.shared.f32 %0, [%1];" : "=f"(h) : "r"(buf + static_cast<uint32_t>((i + 16) * 32 + lane) * 4u) : "memory");
+      asm volatile("ld.shared.f32 %0, [%1];" : "=f"(h)
+                   : "r"(buf + static_cast<uint32_t>((i + 16) * 32 + lane) * 4u) : "memory");
       g[i] += h;
     }
   }
@@ -374,10 +381,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   constexpr bool LN = EPI == EPI_RESIDUAL_LN;
   constexpr bool TABLE = EPI == EPI_QKV_ROPE || EPI == EPI_QKV_NORM;
   // The accumulator as matrix fragments (see above) or a row per lane. Fragments / rows, microseconds: residual
-  // 262144 x 512, K = 512 115 / 121, 442368 x 256, K = 256 91 / 101; GELU 442368 x 1024, K = 256 231 / 267, 103000 x 1536,
-  // K = 384 103 / 110, level from K = 512 on; q/k norm and rotation 262144 x 1536, K = 512 377 / 383, 98304 x 2304,
-  // K = 768 243 / 267, 103000 x 1152, K = 384 150 / 167. The other way: rotation alone 346 / 338, 252 / 246, 121 / 120
-  // (without the norm's code in the kernel rows take 324, 245, 121); bias alone 295 / 291, 171 / 166.
+  // 262144 x 512, K = 512 115 / 121, 442368 x 256, K = 256 91 / 101; GELU 442368 x 1024, K = 256 231 / 267, 103000 x
+  // 1536, K = 384 103 / 110, level from K = 512 on; q/k norm and rotation 262144 x 1536, K = 512 377 / 383, 98304
+  // x 2304, K = 768 243 / 267, 103000 x 1152, K = 384 150 / 167. The other way: rotation alone 346 / 338, 252 / 246,
+  // 121 / 120 (without the norm's code in the kernel rows take 324, 245, 121); bias alone 295 / 291, 171 / 166.
   constexpr bool FRAG = EPI != EPI_BIAS && EPI != EPI_QKV_ROPE && !LN;
   using S = GemmSmem<BN, PAIR, TABLE || LN>;
   // PAIR: this CTA is rank 0 or 1 of a cluster of two that computes 256 x BN tiles together
@@ -404,7 +411,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   uint8_t* tail = smem_gen + S::BAR_OFF + 8 * (2 * S::STAGES + 4 + GEMM_EPI_WARPS);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tail);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tail + 8);
-  [[maybe_unused]] const uint32_t ln_bar0 = bar_base + 8u * (2 * S::STAGES + 4 + GEMM_EPI_WARPS) + 16u;   // one per lane quarter
+  // one per lane quarter
+  [[maybe_unused]] const uint32_t ln_bar0 = bar_base + 8u * (2 * S::STAGES + 4 + GEMM_EPI_WARPS) + 16u;
 
   const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
@@ -554,13 +562,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
     constexpr int WARP_COLS = EPI == EPI_QKV_NORM ? 64 : BN < 128 ? 32 : BN / 4;
     constexpr int NSUB = WARP_COLS / 32;
     const uint32_t stage_s = smem_base + S::STAGING_OFF + e * S::STAGING_BYTES;
-    [[maybe_unused]] const uint32_t my_row_s = stage_s + lane * 64;               // (row form: this lane's row, its swizzle)
+    [[maybe_unused]] const uint32_t my_row_s = stage_s + lane * 64;   // (row form: this lane's row, its swizzle)
     [[maybe_unused]] const uint32_t sw = static_cast<uint32_t>((lane >> 1) & 3);
     // this lane's row of the four 8 x 8 pieces (rows 16 hf + {0, 8}, columns 16 q + {0, 8}) of a staging box: 64-byte
     // rows, 64-byte swizzle
     const uint32_t box_row = stage_s + static_cast<uint32_t>(((lane >> 3) & 1) * 8 + (lane & 7)) * 64u;
     auto box_addr = [&](int hf, int q) -> uint32_t {
-      return box_row + hf * 1024u + ((static_cast<uint32_t>(2 * q + (lane >> 4)) ^ static_cast<uint32_t>((lane >> 1) & 3)) << 4);
+      return box_row + hf * 1024u +
+             ((static_cast<uint32_t>(2 * q + (lane >> 4)) ^ static_cast<uint32_t>((lane >> 1) & 3)) << 4);
     };
     const uint32_t acce_remote0 = PAIR ? map_to_cta(acce_bar(0), 0) : 0u;
     const uint32_t acce_remote1 = PAIR ? map_to_cta(acce_bar(1), 0) : 0u;
@@ -628,12 +637,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             for (int q = 0; q < 2; ++q) {
               const uint32_t addr = my_row_s + ((static_cast<uint32_t>(2 * g + q) ^ sw) << 4);
               uint32_t ax[4];
-              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(ax[0]), "=r"(ax[1]), "=r"(ax[2]), "=r"(ax[3])
-                           : "r"(addr) : "memory");
+              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                           : "=r"(ax[0]), "=r"(ax[1]), "=r"(ax[2]), "=r"(ax[3]) : "r"(addr) : "memory");
 #pragma unroll
               for (int h = 0; h < 2; ++h) {       // four columns: N is a multiple of 64
                 float4 b4 = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (p.bias != nullptr) b4 = __ldg(reinterpret_cast<const float4*>(p.bias + n0 + 16 * g + 8 * q + 4 * h));
+                if (p.bias != nullptr)
+                  b4 = __ldg(reinterpret_cast<const float4*>(p.bias + n0 + 16 * g + 8 * q + 4 * h));
                 const int k = 8 * q + 4 * h;
                 w[c][8 * g + 4 * q + 2 * h] = pack_bf16(__uint_as_float(r[k]) + b4.x + bf16_lo(ax[2 * h]),
                                                         __uint_as_float(r[k + 1]) + b4.y + bf16_hi(ax[2 * h]));
@@ -641,7 +651,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                                                             __uint_as_float(r[k + 3]) + b4.w + bf16_hi(ax[2 * h + 1]));
               }
               asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w[c][8 * g + 4 * q]),
-                           "r"(w[c][8 * g + 4 * q + 1]), "r"(w[c][8 * g + 4 * q + 2]), "r"(w[c][8 * g + 4 * q + 3]) : "memory");
+                           "r"(w[c][8 * g + 4 * q + 1]), "r"(w[c][8 * g + 4 * q + 2]), "r"(w[c][8 * g + 4 * q + 3])
+                           : "memory");
             }
           }
         }
@@ -655,7 +666,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         }
         if (m_warp < p.M) {                        // (columns behind N count as zero)
 #pragma unroll
-          for (int k = 0; k < 4; ++k) ln_put(sums, cg * (WARP_COLS / 8) + 4 * c + k, lane, live ? ln_group_sum(&w[c][4 * k]) : 0.f);
+          for (int k = 0; k < 4; ++k)
+            ln_put(sums, cg * (WARP_COLS / 8) + 4 * c + k, lane, live ? ln_group_sum(&w[c][4 * k]) : 0.f);
         }
       }
       if (m_warp >= p.M) return true;              // all four warps of the quarter
@@ -667,7 +679,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       for (int c = 0; c < NSUB; ++c)
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          ln_put(squares, cg * (WARP_COLS / 8) + 4 * c + k, lane, n_warp0 + 32 * c < p.N ? ln_group_squares(&w[c][4 * k], mean) : 0.f);
+          ln_put(squares, cg * (WARP_COLS / 8) + 4 * c + k, lane,
+                 n_warp0 + 32 * c < p.N ? ln_group_squares(&w[c][4 * k], mean) : 0.f);
       __syncwarp();
       if (lane == 0) mbar_arrive(ln_bar);
       if (!gemm_wait(ln_bar, 1u, abort_flag, ST_TIMEOUT_EPILOGUE)) return false;
@@ -717,7 +730,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
             break;
           }
           if (t + n_units < num_tiles && !(one_row && it != 0))
-            gemm_fetch_table(p, tile_rows(t + n_units), cg * 8, tab_quarter + static_cast<uint32_t>(buf ^ 1) * (GEMM_BM * 128u), one_row);
+            gemm_fetch_table(p, tile_rows(t + n_units), cg * 8,
+                             tab_quarter + static_cast<uint32_t>(buf ^ 1) * (GEMM_BM * 128u), one_row);
         }
       }
       if constexpr (LN) {
@@ -861,7 +875,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                 const int pair0 = ((p.head_dim == 64) ? (n0 & 63) >> 1 : 0) + 8 * g;
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {
-                  const uint32_t addr = tab_base + lane * 128u + ((static_cast<uint32_t>((pair0 >> 2) + q) ^ (lane & 7u)) << 4);
+                  const uint32_t addr =
+                      tab_base + lane * 128u + ((static_cast<uint32_t>((pair0 >> 2) + q) ^ (lane & 7u)) << 4);
                   asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
                                : "=r"(cs[4 * q]), "=r"(cs[4 * q + 1]), "=r"(cs[4 * q + 2]), "=r"(cs[4 * q + 3])
                                : "r"(addr) : "memory");
@@ -1035,8 +1050,9 @@ inline int launch_gemm(const __nv_bfloat16* A, long long lda, const __nv_bfloat1
   //   2 / 1, 3 / 2, 4 / 3  up to K = 1024 0.95 1.10 1.27, beyond 0.88 0.98 1.10; N <= 256, K > 512 0.86 - 0.95
   //   4 / 2, 5 / 3  up to K = 1024 0.83 0.93 1.10, beyond 0.8 - 0.9
   // Equal work's operands are twice as many bytes in 128-wide tiles: from K = 512 on a further turn of them takes as
-  // long as one of pairs, and with N <= 256 a pair reads A once. The norm of q and k keeps a head to a warp, so that half
-  // the warps of a 128-wide tile have none: 1 / 1 1.21 - 1.25 (1536 x 1536, K = 512 9.6 / 7.9), 2 / 2 1.21, 2 / 1 and 3 / 2 0.83 - 0.97.
+  // long as one of pairs, and with N <= 256 a pair reads A once. The norm of q and k keeps a head to a warp, so that
+  // half the warps of a 128-wide tile have none: 1 / 1 1.21 - 1.25 (1536 x 1536, K = 512 9.6 / 7.9), 2 / 2 1.21, 2 / 1
+  // and 3 / 2 0.83 - 0.97.
   constexpr bool QKV = EPI == EPI_QKV_ROPE || EPI == EPI_QKV_NORM;
   const int tiles128 = ((p.M + GEMM_BM - 1) / GEMM_BM) * ((p.N + 127) / 128);
   // One tile per SM at most, as narrow as 64: a launch is the latency of one tile, and half as wide a one has half
@@ -1066,7 +1082,8 @@ inline int launch_gemm(const __nv_bfloat16* A, long long lda, const __nv_bfloat1
 // y = A W^T + bias + aux and layernorm(y) into ln_out, for whole rows in a tile: N a multiple of 64, at most 256.
 // For calls of many rows: pairs of CTAs where one 128-wide tile does not hold a row.
 inline int launch_gemm_residual_ln(const __nv_bfloat16* A, long long lda, const __nv_bfloat16* W, long long ldw,
-                                   __nv_bfloat16* ln_out, long long ldln, const GemmParams& p, int sm_count, cudaStream_t stream) {
+                                   __nv_bfloat16* ln_out, long long ldln, const GemmParams& p, int sm_count,
+                                   cudaStream_t stream) {
   if (p.N % 64 != 0 || p.N > 256) return -2;
   if (p.N <= 128) return launch_gemm_t<128, EPI_RESIDUAL_LN, false>(A, lda, W, ldw, p, sm_count, stream, ln_out, ldln);
   return launch_gemm_t<256, EPI_RESIDUAL_LN, true>(A, lda, W, ldw, p, sm_count, stream, ln_out, ldln);

@@ -133,7 +133,8 @@ halo_gather_tokens_kernel(__nv_bfloat16* __restrict__ out, const PeerPtrs src,
 // Measured, microseconds (24 tiles of 64 x 64, halo 8; 512 leading indices are 516 MB read + written):
 //   leading indices                     1     16    64    512    | 96 x 96, halo 16: 256 | 128 x 128, halo 32: 64
 //   copy, 1 cell a thread, UL 8         8     12    22    104    | 133                    | 84
-//   copy, 4 cells, UL 4                 8     11    20     93    | 121                    | 74   (UL 2: 100, UL 8: 98 at 512)
+//   copy, 4 cells, UL 4                 8     11    20     93    | 121                    | 74
+//   ..., UL 2 (UL 8)                                       100 (98)
 //   4 neighbours, UL 4 (UL 8, 16)      10     18    29    196 (233, 199)
 //   overlap-add, UL 8                  12     16    29    128    | 162                    | 120
 //   ..., every entry in its turn, UL 12  14   23    37    145    | 195                    | 154

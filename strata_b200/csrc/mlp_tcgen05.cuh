@@ -3,8 +3,8 @@
 //   y = aux + [gate *] (W2 gelu(W1 x + b1) + b2)        x, aux, gate, y: [M, C] bf16; W1 [H, C], W2 [C, H]
 //
 // As two GEMMs the hidden rows [M, H] are written and read again: at C = 256, H = 1024 that is 4 of every 5
-// bytes the two move, and they are bound by it. Here a CTA keeps 128 rows: the hidden channels are made 128 at a time in
-// tensor memory, leave it as bf16 through the GELU into shared memory and are multiplied on from there.
+// bytes the two move, and they are bound by it. Here a CTA keeps 128 rows: the hidden channels are made 128 at a time
+// in tensor memory, leave it as bf16 through the GELU into shared memory and are multiplied on from there.
 //
 //   warp 0      TMA producer: the x tile, and the weights of every chunk of 128 hidden channels through two
 //               rings (W1: 128 x 64 boxes, W2: C x 64 boxes); the weights come from L2, 16 C^2 bytes per tile.
@@ -81,7 +81,8 @@ template <int C, bool LN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW1,
                    const __grid_constant__ CUtensorMap tmW2, const __grid_constant__ CUtensorMap tmOut,
-                   const __grid_constant__ CUtensorMap tmAux, const __grid_constant__ CUtensorMap tmLn, const MlpParams p) {
+                   const __grid_constant__ CUtensorMap tmAux, const __grid_constant__ CUtensorMap tmLn,
+                   const MlpParams p) {
   using S = MlpSmem<C, LN>;
   constexpr bool AHEAD = S::AHEAD;
   extern __shared__ uint8_t smem_raw[];
@@ -109,7 +110,8 @@ mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   const int lane = threadIdx.x & 31;
   const int tiles = (p.M + 127) / 128;
   const int nj = p.H / MLP_CHUNK;
-  const int n_my = (tiles - static_cast<int>(blockIdx.x) + static_cast<int>(gridDim.x) - 1) / static_cast<int>(gridDim.x);
+  const int ctas = static_cast<int>(gridDim.x);
+  const int n_my = (tiles - static_cast<int>(blockIdx.x) + ctas - 1) / ctas;
   const int chunks = n_my * nj;              // of this CTA, numbered through its tiles
 
   if (threadIdx.x == 0) {
@@ -130,12 +132,13 @@ mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     mbar_init(x_empty, 1);
     mbar_init(staged, GEMM_EPI_WARPS);
     for (int w = 0; w < GEMM_EPI_WARPS; ++w) mbar_init(aux_full(w), 1);
-    for (int q = 0; q < 4; ++q) mbar_init(ln_bar(q), C < 128 ? C / 32 : 4);   // the warps of a quarter that have columns
+    for (int q = 0; q < 4; ++q) mbar_init(ln_bar(q), S::OUT_READERS / 4);   // the warps of a quarter that have columns
     *abort_flag = 0;
     fence_mbar_init();
   }
   if constexpr (LN && C == 64)   // groups that no warp has
-    for (int i = threadIdx.x; i < 2 * 4 * 16 * 32; i += GEMM_THREADS) *reinterpret_cast<float*>(smem_gen + S::LN_OFF + 4 * i) = 0.f;
+    for (int i = threadIdx.x; i < 2 * 4 * 16 * 32; i += GEMM_THREADS)
+      *reinterpret_cast<float*>(smem_gen + S::LN_OFF + 4 * i) = 0.f;
   if (warp == 1) {
     tmem_alloc(smem_u32(tmem_slot), 512);
     tmem_relinquish();
@@ -259,8 +262,9 @@ mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     const uint32_t stage_s = smem_base + S::STAGING_OFF + e * S::STAGING_BYTES;
     const uint32_t my_row_s = stage_s + lane * 64;
     const uint32_t sw = static_cast<uint32_t>((lane >> 1) & 3);   // 64-byte swizzle of a staging box's row
-    const uint32_t h_row0 = smem_base + S::H_OFF + set * S::H_BYTES + quarter * 32 * 128;   // the quarter's rows of the hidden chunk
-    auto tile_row = [&](int t) { return (static_cast<int>(blockIdx.x) + t * static_cast<int>(gridDim.x)) * 128 + quarter * 32; };
+    // the quarter's rows of the hidden chunk
+    const uint32_t h_row0 = smem_base + S::H_OFF + set * S::H_BYTES + quarter * 32 * 128;
+    auto tile_row = [&](int t) { return (static_cast<int>(blockIdx.x) + t * ctas) * 128 + quarter * 32; };
 
     // A chunk's accumulator is read as matrix fragments (lane: rows lane / 4 and + 8, columns 2 (lane % 4) and + 1
     // of every 8): a lane then needs two biases per 8 columns, eight for its 32 channels, which are asked for before
@@ -284,7 +288,8 @@ mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         const int col = (cg * SETS + pc) * 32;
         uint32_t acc[2][16], h[2][8];
 #pragma unroll
-        for (int hf = 0; hf < 2; ++hf) tmem_ld_16x256_x4(lane_taddr + (static_cast<uint32_t>(16 * hf) << 16) + buf * MLP_CHUNK + col, acc[hf]);
+        for (int hf = 0; hf < 2; ++hf)
+          tmem_ld_16x256_x4(lane_taddr + (static_cast<uint32_t>(16 * hf) << 16) + buf * MLP_CHUNK + col, acc[hf]);
         tmem_ld_wait();
         if (pc == SETS - 1) {
           tc_fence_before();
@@ -304,7 +309,7 @@ mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf)
 #pragma unroll
-          for (int q = 0; q < 2; ++q) {      // columns 16 q: k-block col / 64, 16-byte pieces (col % 64) / 8 + 2 q and + 1
+          for (int q = 0; q < 2; ++q) {      // columns 16 q: k-block col / 64, 16-byte pieces (col % 64) / 8 + 2 q, + 1
             const uint32_t piece = static_cast<uint32_t>((col & 32) / 8 + 2 * q + (lane >> 4));
             const uint32_t addr = st_row + hf * 2048 + (col >> 6) * 16384 + ((piece ^ (lane & 7u)) << 4);
             stmatrix_x4(addr, &h[hf][4 * q]);
@@ -342,7 +347,8 @@ mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       const int m_warp = tile_row(t);
       bool ready = false;
       [[maybe_unused]] uint32_t keep[16];          // LN: the row's columns of this warp
-      [[maybe_unused]] const uint32_t sums = smem_base + S::LN_OFF + static_cast<uint32_t>(quarter) * 2048u, squares = sums + 8192u;
+      [[maybe_unused]] const uint32_t sums = smem_base + S::LN_OFF + static_cast<uint32_t>(quarter) * 2048u;
+      [[maybe_unused]] const uint32_t squares = sums + 8192u;
 #pragma unroll 1
       for (int n0 = box0; n0 < C; n0 += 128) {
         uint4 aux[4], gate[4];
@@ -368,8 +374,8 @@ mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               const uint32_t addr = my_row_s + ((static_cast<uint32_t>(q) ^ sw) << 4);
-              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(aux[q].x), "=r"(aux[q].y), "=r"(aux[q].z), "=r"(aux[q].w)
-                           : "r"(addr) : "memory");
+              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                           : "=r"(aux[q].x), "=r"(aux[q].y), "=r"(aux[q].z), "=r"(aux[q].w) : "r"(addr) : "memory");
             }
           } else {
             if (elect_one()) tma_store_wait_read0();
@@ -423,7 +429,8 @@ mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
               w[i] = pack_bf16(v[8 * q + 2 * i], v[8 * q + 2 * i + 1]);
               if constexpr (LN) keep[8 * g + 4 * q + i] = w[i];
             }
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+                         "r"(w[3]) : "memory");
           }
         }
         fence_proxy_async_smem();
@@ -435,8 +442,8 @@ mlp_tcgen05_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
       }
       // The output columns may be accumulated into again. Every arrival follows its warp's own wait for out_full of
       // this tile, so a phase of out_free is made of one tile's readers. A warp without columns waits for nothing here
-      // and runs ahead by as many tiles as its chunks let it, so it has no say: else two of its tiles would fill a phase
-      // before the readers of the first are done (C = 64, one chunk a tile, from the fourth tile of a CTA on).
+      // and runs ahead by as many tiles as its chunks let it, so it has no say: else two of its tiles would fill a
+      // phase before the readers of the first are done (C = 64, one chunk a tile, from the fourth tile of a CTA on).
       if (box0 < C) {
         tc_fence_before();
         __syncwarp();
@@ -553,7 +560,9 @@ inline int launch_mlp_t(const __nv_bfloat16* x, long long ldx, const __nv_bfloat
 }
 
 // Whether the kernel takes these sizes (weights contiguous, everything else as the GEMMs want it).
-inline bool mlp_fused_sizes(int C, int H) { return C % 64 == 0 && C > 0 && C <= MLP_MAX_C && H % MLP_CHUNK == 0 && H > 0; }
+inline bool mlp_fused_sizes(int C, int H) {
+  return C % 64 == 0 && C > 0 && C <= MLP_MAX_C && H % MLP_CHUNK == 0 && H > 0;
+}
 
 // Whether it is the faster way. Two GEMMs/this kernel, microseconds with a residual, passes back to back on inputs and
 // outputs that do not stay in L2, by row blocks of 128 (148 of them are one turn of the chip):

@@ -292,7 +292,7 @@ __device__ __noinline__ void na_store_o_rows(uint32_t o_taddr, float inv, __nv_b
       __nv_bfloat16* pg = reinterpret_cast<__nv_bfloat16*>(g ? p1 : p0);
       uint32_t y[2][4];                    // chunks 2 (lane % 4) and the next of the row
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {        // chunks q, q + 2, q + 4, q + 6: a word of each per lane -> one chunk per lane
+      for (int q = 0; q < 2; ++q) {        // chunks q, q + 2, q + 4, q + 6: a word of each per lane, one chunk per lane
         uint32_t w[4], x[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -329,7 +329,8 @@ __device__ __forceinline__ bool na_wait(uint32_t bar, uint32_t parity, volatile 
 
 // One arrival for a converged warp (lane 0's), without a branch.
 __device__ __forceinline__ void na_arrive(uint32_t bar, int lane) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar), "r"(lane) : "memory");
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.eq.s32 p, %1, 0;\n\t"
+               "@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar), "r"(lane) : "memory");
 }
 
 struct NaItem {

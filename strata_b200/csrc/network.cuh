@@ -147,7 +147,8 @@ inline int pixel_block(const strata_backbone_desc& b, const strata_pixel_desc& p
   STRATA_TRY(strata_adaln_rows_bf16(x, C, n.y, C, part(2), ldm, x, C, part(3), part(4), ldm, n.xn, C, M, C,
                                     1e-6f, stream));
   if (mod && mlp_fused_pays(M, C, px.hidden, current_sm_count()))
-    return strata_mlp_bf16(n.xn, C, a.w_fc1, a.b_fc1, a.w_fc2, a.b_fc2, x, C, part(5), ldm, x, C, M, C, px.hidden, stream);
+    return strata_mlp_bf16(n.xn, C, a.w_fc1, a.b_fc1, a.w_fc2, a.b_fc2, x, C, part(5), ldm, x, C, M, C, px.hidden,
+                           stream);
   STRATA_TRY(strata_linear_bf16(n.xn, C, a.w_fc1, C, a.b_fc1, n.hid, px.hidden, M, px.hidden, C,
                                 STRATA_EPI_GELU, nullptr, 0, stream));
   STRATA_TRY(strata_linear_bf16(n.hid, px.hidden, a.w_fc2, px.hidden, a.b_fc2, n.y, C, M, C, px.hidden,
