@@ -706,7 +706,7 @@ def pixel_stage_bench(torch, dev, iters=3):
     1024, pixel 128, 2 heads, 9x9x9 attention, bilinear_dw conditioning) on one 24 x 256 x 256
     pixel tile (1.57 M pixel tokens, 98 k backbone tokens): every kernel of the block alone, with
     its algorithmic bytes or flops, then the whole block (modulation + forward)."""
-    from strata_b200 import ops
+    from strata_b200 import _lib, ops
     from strata_b200.ops import EPI_GELU
     from strata_b200.pixel import StrataPixel3DBlock
     tf_peak, hbm_peak, _ = measured_peaks()
@@ -733,7 +733,15 @@ def pixel_stage_bench(torch, dev, iters=3):
         attn = ops.na3d(q6[:, :, :, :, 0], q6[:, :, :, :, 1], q6[:, :, :, :, 2], c["kernel"]).view(-1, C)
         h = ops.linear(xn, wts["w_fc1"], wts["b_fc1"], EPI_GELU)
         y = ops.linear(attn, wts["w_proj"], wts["b_proj"])
+        hidden, z = wts["w_fc1"].shape[0], torch.empty_like(x)
         kd, kh, kw = c["kernel"]
+
+        def mlp_kernel():                       # as a model's call launches it
+            g = sl(5)
+            _lib.check(_lib.load().strata_mlp_bf16(
+                xn.data_ptr(), C, wts["w_fc1"].data_ptr(), wts["b_fc1"].data_ptr(), wts["w_fc2"].data_ptr(),
+                wts["b_fc2"].data_ptr(), x.data_ptr(), C, g.data_ptr(), g.stride(0), z.data_ptr(), C, M, C, hidden,
+                _lib.stream_of(x)), "strata_mlp_bf16")
         items = [
             ("adaln_cond (2^18 pixels)", lambda: ops.adaln_cond(s, wts["w_dw"], wts["b_dw"], f, 0, n, out=cond),
              "hbm", n * Cb * 2),
@@ -747,11 +755,14 @@ def pixel_stage_bench(torch, dev, iters=3):
             ("proj GEMM", lambda: ops.linear(attn, wts["w_proj"], wts["b_proj"], out=y), "hbm", M * C * 2 * 2),
             ("gated residual + ln_modulate", lambda: ops.adaln_rows(x, y=y, gate=sl(2), shift=sl(3), scale=sl(4)),
              "hbm", M * C * 2 * 7),
-            ("fc1 GEMM + GELU", lambda: ops.linear(xn, wts["w_fc1"], wts["b_fc1"], EPI_GELU, out=h),
+            ("MLP kernel: fc1, GELU, fc2, gated residual", mlp_kernel, "tensor", 4.0 * M * C * hidden),
+            # a block called as a module (hooks, replaced blocks) takes these three for the MLP kernel
+            ("fc1 GEMM + GELU (module)", lambda: ops.linear(xn, wts["w_fc1"], wts["b_fc1"], EPI_GELU, out=h),
              "hbm", M * C * 2 * 5),
-            ("fc2 GEMM", lambda: ops.linear(h, wts["w_fc2"], wts["b_fc2"], out=y), "hbm", M * C * 2 * 5),
-            ("gated residual", lambda: ops.adaln_rows(x, y=y, gate=sl(5), norm=False), "hbm", M * C * 2 * 4),
-            ("whole block (modulation + forward)", lambda: blk(x, (D, H, W), blk.modulation(s, f), 1),
+            ("fc2 GEMM (module)", lambda: ops.linear(h, wts["w_fc2"], wts["b_fc2"], out=y), "hbm", M * C * 2 * 5),
+            ("gated residual (module)", lambda: ops.adaln_rows(x, y=y, gate=sl(5), norm=False), "hbm",
+             M * C * 2 * 4),
+            ("whole block as a module (modulation + forward)", lambda: blk(x, (D, H, W), blk.modulation(s, f), 1),
              None, 0),
         ]
         out = []
