@@ -122,3 +122,17 @@ def test_mlp_of_one_row_with_any_row_stride(ops):
     h = ops.linear(x, d["w1"], d["b1"], ops.EPI_GELU)
     want = ops.linear(h, d["w2"], d["b2"], ops.EPI_RESIDUAL, aux)
     assert torch.equal(ops.mlp(x, d["w1"], d["b1"], d["w2"], d["b2"], aux), want)
+
+
+# the two ways as measured: turns of 148 row blocks (18944 rows), the last one's share, chunks of 128 hidden channels
+@pytest.mark.parametrize("M,C,H,fused", [
+    (37889, 192, 768, 0), (40000, 192, 768, 0), (45000, 192, 768, 0), (57000, 192, 768, 0), (75776, 192, 768, 1),
+    (37889, 256, 1024, 0), (45000, 256, 1024, 1), (57000, 256, 1024, 1), (37889, 192, 1536, 1), (37889, 256, 2048, 1),
+    (57000, 256, 512, 0), (45000, 192, 384, 0), (151552, 192, 384, 1), (9472, 256, 1024, 0), (9473, 256, 1024, 1),
+    (18945, 192, 768, 0), (37888, 192, 768, 1), (128, 128, 512, 1), (128, 128, 1024, 0), (8192, 128, 1024, 1),
+    (128, 64, 128, 1), (128, 128, 320, 0), (1 << 20, 320, 1280, 0)])
+def test_mlp_rule(ops, M, C, H, fused):
+    from strata_b200 import _lib
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the line lies by turns of 148 SMs")
+    assert _lib.load().strata_mlp_fused(M, C, H) == fused
