@@ -27,9 +27,9 @@
 // Bound: C <= 128 by the epilogue warps (tanh on the special-function unit alone: 128 x 512 per tile take
 // 4096 cycles at C = 128, the products as many; a tile takes 11000), C = 256 by shared memory (operands,
 // weights coming in and the hidden chunk: 1.5 times what it moves in the products' own time) and the same warps.
-// 442368 rows, one call from a cold L2 (back to back: at the rule below), two GEMMs -> this kernel: C = 64 132 -> 80 us,
-// 128 232 -> 145, 192 345 -> 301, 256 480 -> 412; with the gated residual of the pixel blocks, which was a third kernel,
-// C = 128 296 -> 180.
+// 442368 rows, one call from a cold L2 (back to back: at the rule below), two GEMMs -> this kernel: C = 64 132 -> 80
+// us, 128 232 -> 145, 192 345 -> 301, 256 480 -> 412; with the gated residual of the pixel blocks, which was a third
+// kernel, C = 128 296 -> 180.
 #pragma once
 #include "gemm_tcgen05.cuh"
 
